@@ -81,23 +81,32 @@ inline int sm_count() {
 	return v;
 }
 
-struct RowSource { const int8_t* hidden; const Scale* scale; };  // nullptr hidden: embed rows[r].token
-struct RowSink { int8_t* hidden; Scale* scale; };                // nullptr hidden: drop
-
 // ---- per-row sites (sslm_rows.cu)
 cudaError_t rows_configure(const Dims& d);
-void launch_begin(const RowBatch& b, const Dims& d, const int8_t* embed, Scale c_embed,
-                  const RowSource* src, const LayerDev* layer, cudaStream_t st);
-void launch_rmsnorm(const RowBatch& b, const Dims& d, const int8_t* gain, Scale site, cudaStream_t st);
-void launch_qkv_post(const RowBatch& b, const Dims& d, const LayerDev* layer, int layer_index,
-                     KvPoolDev pool, const int32_t* cos, const int32_t* sin, cudaStream_t st);
-void launch_ctx_funnel(const RowBatch& b, const Dims& d, const LayerDev* layer, cudaStream_t st);
-void launch_res1(const RowBatch& b, const Dims& d, const LayerDev* layer, cudaStream_t st);
-void launch_res2(const RowBatch& b, const Dims& d, const LayerDev* layer, const LayerDev* next,
-                 cudaStream_t st);
-void launch_act(const RowBatch& b, const Dims& d, const LayerDev* layer, const int32_t* silu,
-                cudaStream_t st);
-void launch_scatter(const RowBatch& b, const Dims& d, const RowSink* sink, cudaStream_t st);
+// (the host's copy `h` of a layer record carries the site constants into the launch parameters)
+// first rows of a call: embed or resume, then an RMSNorm with `gain` (nullptr: none)
+void launch_begin(const RowBatch& b, const Dims& d, const int8_t* embed, Scale c_embed, const RowSource* src, const int8_t* gain,
+                  Scale c_norm, int site_norm, cudaStream_t st);
+void launch_qkv_post(const RowBatch& b, const Dims& d, const LayerDev* layer, const LayerDev& h, int layer_index, KvPoolDev pool,
+                     const int32_t* cos, const int32_t* sin, cudaStream_t st);
+void launch_ctx_funnel(const RowBatch& b, const Dims& d, const LayerDev& h, cudaStream_t st);
+// A residual site: funnel of the projection row, reconciliation with the stream, and the RMSNorm of
+// whatever comes next.
+struct ResSite {
+	const int8_t* stream;        // [m, hidden] the stream the branch joins, and its scales
+	const Scale* stream_scale;
+	const Scale* in_scale;       // scales of the projection's input rows
+	int8_t* out;                 // [m, hidden] the joined stream, and its scales
+	Scale* out_scale;
+	const int8_t* gain;          // of the norm that follows into b.nrm / b.ns, nullptr: none
+	Scale c_proj, c_res, c_norm;
+	int site_proj, site_res, site_norm, norm_layer;
+	int32_t* done;               // [m] set to done_value once the stream is joined, or nullptr
+	int done_value;
+	const RowSink* sink;         // [m] where the joined stream also goes (the call's last layer), or nullptr
+};
+void launch_res(const RowBatch& b, const Dims& d, const ResSite& a, cudaStream_t st);
+void launch_act(const RowBatch& b, const Dims& d, const LayerDev& h, const int32_t* silu, cudaStream_t st);
 
 // ---- int8 linear layers (sslm_gemv.cu, sslm_gemm_tc.cu)
 // out[m, n] = fold_n( sum_k x[m,k] * w[n,k] ) (+ LoRA delta), plus the per-row max |out|

@@ -77,6 +77,9 @@ struct RowDesc {
 	int32_t token;              // token id to embed when the row starts a token
 };
 
+struct RowSource { const int8_t* hidden; const Scale* scale; };  // nullptr hidden: embed rows[r].token
+struct RowSink { int8_t* hidden; Scale* scale; };                // nullptr hidden: drop
+
 // Where in the reference's program order a row was refused. A row's status word holds the
 // reference status in bits 0..7, the site in bits 8..15 and the layer index + 1 in bits 16..31;
 // any non-zero word means "refused". The host needs the place twice: a decode step that fails in
