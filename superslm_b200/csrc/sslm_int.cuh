@@ -579,10 +579,10 @@ SSLM_HD int32_t silu_sigmoid_q15(const int32_t* table, int32_t code, int64_t m, 
 	pos += hi_dom / 2;
 	if (pos < 0) pos = 0;
 	else if (pos > hi_dom) pos = hi_dom;
-	int64_t i0 = pos >> 12;
+	const int32_t p32 = (int32_t)pos;      // 0 .. 1024 * 4096
+	int32_t i0 = p32 >> 12;
 	if (i0 > 1023) i0 = 1023;
-	int64_t frac = pos - (i0 << 12);
-	int64_t lo = table[i0], hi = table[i0 + 1];
+	const int64_t frac = p32 - (i0 << 12), lo = table[i0], hi = table[i0 + 1];
 	return (int32_t)(lo + rdivpot64(frac * (hi - lo), 12));
 }
 SSLM_HD bool silu_scale_in_domain(Scale g) {
@@ -599,12 +599,7 @@ SSLM_HD bool silu_scale_in_domain(Scale g) {
 struct IExpConsts { int64_t q_ln2, q_b, q_c; };
 // IExpScaleConstants with the production coefficients, all formats 30
 // (src/intmath.cpp:702-778). 0 ok, else out of domain.
-SSLM_HD_OUTLINE int iexp_scale_constants(int64_t m, int64_t e, IExpConsts* out) {
-	int64_t sh_l = sat_add64(92, e);
-	int64_t sh_c = sat_add64(154, sat_add64(e, e));
-	int64_t mn = sh_l < sh_c ? sh_l : sh_c;
-	if (mn < 0) return 2;
-	uint64_t rm = (uint64_t)dyn_recip(m);
+SSLM_HD_OUTLINE int iexp_scale_constants_general(int64_t sh_l, int64_t sh_c, uint64_t rm, IExpConsts* out) {
 	U128 n_ln2 = umul64((uint64_t)SSLM_IEXP_LN2_Q, rm);
 	U128 n_b = umul64((uint64_t)SSLM_IEXP_B_Q, rm);
 	U128 n_c = umul128x64(umul64(rm, rm), (uint64_t)SSLM_IEXP_CA_Q);
@@ -619,16 +614,38 @@ SSLM_HD_OUTLINE int iexp_scale_constants(int64_t m, int64_t e, IExpConsts* out) 
 	out->q_c = (int64_t)f_c.lo;
 	return 0;
 }
+SSLM_HD int iexp_scale_constants(int64_t m, int64_t e, IExpConsts* out) {
+	int64_t sh_l = sat_add64(92, e);
+	int64_t sh_c = sat_add64(154, sat_add64(e, e));
+	int64_t mn = sh_l < sh_c ? sh_l : sh_c;
+	if (mn < 0) return 2;
+	const uint64_t rm = (uint64_t)dyn_recip(m);
+	// A canonical mantissa (2^31 <= rm < 2^32) keeps LN2_Q rm, B_Q rm and rm^2 inside 64 bits and
+	// rm^2 CA_Q inside 96; the shifts of every scale a row carries in earnest are below 64 and 128.
+	if (rm < ((uint64_t)1 << 32) && sh_l < 64 && sh_c < 128) {
+		const uint64_t l = ((uint64_t)SSLM_IEXP_LN2_Q * rm) >> sh_l, b = ((uint64_t)SSLM_IEXP_B_Q * rm) >> sh_l, sq = rm * rm;
+		const uint64_t c_lo = sq * (uint64_t)SSLM_IEXP_CA_Q, c_hi = umulhi64(sq, (uint64_t)SSLM_IEXP_CA_Q);
+		const int k = (int)sh_c;
+		const uint64_t v = k >= 64 ? c_hi >> (k - 64) : (k == 0 ? c_lo : (c_lo >> k) | (c_hi << (64 - k)));
+		const uint64_t over = k >= 64 ? 0 : c_hi >> k;
+		if (over != 0 || (int64_t)v < 0) return 3;      // (the other two stay below 2^63)
+		out->q_ln2 = (int64_t)l;
+		out->q_b = (int64_t)b;
+		out->q_c = (int64_t)v;
+		return 0;
+	}
+	return iexp_scale_constants_general(sh_l, sh_c, rm, out);
+}
 // largest row peak the Q15 normalisation can carry (checked_chain_funnel.h:563)
 #define SSLM_SOFTMAX_MAX_SAFE (((int64_t)1 << 62) >> 15)
 // CheckSoftmaxRowWidthDomain (src/forward/checked_chain_funnel.cpp:520-583)
-SSLM_HD_OUTLINE bool softmax_width_in_domain(int64_t q_b, int64_t q_c, uint64_t width, int64_t* peak) {
+SSLM_HD bool softmax_width_in_domain(int64_t q_b, int64_t q_c, uint64_t width, int64_t* peak) {
 	if (q_c < 0 || width == 0) return false;
 	U128 m = uadd(smul64(q_b, q_b), U128{(uint64_t)q_c, 0});
 	if (m.hi != 0 || m.lo > (uint64_t)SSLM_SOFTMAX_MAX_SAFE) return false;
 	*peak = (int64_t)m.lo;
-	if (m.lo != 0 && width > (uint64_t)(INT64_MAX / (int64_t)m.lo)) return false;
-	return true;
+	// width > floor(INT64_MAX / peak) without the division: width * peak > INT64_MAX
+	return umulhi64(width, m.lo) == 0 && width * m.lo <= (uint64_t)INT64_MAX;
 }
 // One softmax element: IExpConstruct + IExpEvaluate on a shifted score q <= 0 followed
 // by SoftmaxRowQ15's per-element bound (src/intmath.cpp:580-668, :870-888), specialised

@@ -47,51 +47,164 @@ __device__ __forceinline__ uint32_t pack4(int a, int b, int c, int d) {
 }
 __device__ __forceinline__ int byte_of(uint32_t w, int j) { return (int)(int8_t)(w >> (8 * j)); }
 
-// ------------------------------------------------------------------ requant codes
-// code = round_half_away(x * 127 R / 2^E), |x| <= the row's maximum (so |code| <= 127), E = 62 - s.
-// v = x * f with f = 127 R / 2^E in float: the three roundings (x, f, the product) put v within
-// 127 * 2^-22 < 3.1e-5 of the exact quotient, so unless v is within 1e-4 of a half-integer its
-// nearest integer IS the code; one element in 5,000 is not and is recomputed with requant_code.
-// Five instructions per element instead of about twenty.
-struct QuadCoder {
-	float f;
-	int64_t r;
-	int s;
+// ------------------------------------------------------------------ the funnel's scalars
+// funnel_finish for the quads: the carried scale, and for the codes 127 / d as a float instead of the
+// normalised reciprocal (R / 2^E = 1 / d up to 2^-32). The reciprocal itself is derived only where an
+// element needs the integer form. About a fifth of funnel_finish's instructions, which every warp of
+// the block executes on the way from one reduction to the next.
+struct QuadFunnel {
+	float f, f_lo;     // 127 / d to one rounding, and the rest of it (both of d rounded, above 2^24)
+	uint32_t d;        // the row's maximum, at least 1
+	Scale out;
+	int32_t status;
 };
-__device__ __forceinline__ QuadCoder make_quad_coder(int64_t r, int s) {
-	QuadCoder c;
-	c.r = r;
-	c.s = s;
-	const int e = 62 - s;      // 32..63
-	c.f = __ull2float_rn((unsigned long long)r) * 127.0f * __int_as_float((127 - e) << 23);
-	return c;
+__device__ __forceinline__ QuadFunnel quad_funnel(unsigned long long mx, const FunnelFold& fold) {
+	QuadFunnel q;
+	const bool wide = mx > (1ull << 31);
+	const uint32_t d = wide ? 1u : max((uint32_t)mx, 1u);
+	q.d = d;
+	const float df = __uint2float_rn(d), rd = __fdividef(1.0f, df), f0 = 127.0f * rd;
+	q.f = fmaf(fmaf(-f0, df, 127.0f), rd, f0);
+	q.f_lo = fmaf(-q.f, df, 127.0f) * rd;
+	const int s = __clz((int)d) - 1;                                   // 30 - floor(log2 d)
+	const uint32_t dn = s >= 0 ? d << s : d >> 1;                      // 2^30 <= dn < 2^31
+	q.status = fold.fold_status;
+	if (fold.run.e > ((int64_t)1 << 61) || fold.run.e < -((int64_t)1 << 61)) {      // exponents that may saturate
+		q.out = combine(fold.run, Scale{(int64_t)dn, -(int64_t)s});
+		if (!fits_i32(q.out.m)) q.status = kCarriedScaleMantissaOutOfDomain;
+	} else {
+		// CombineCarriedScale; the doubling high multiply cannot saturate because dn < 2^31
+		int32_t m = (int32_t)(((int64_t)(int32_t)fold.run.m * (int64_t)dn + ((int64_t)1 << 30)) >> 31);
+		q.out.e = fold.run.e + (31 - s);
+		if (m < (1 << 30)) {
+			if (m < -(1 << 30)) q.status = kCarriedScaleMantissaOutOfDomain;
+			m <<= 1;
+			q.out.e -= 1;
+		}
+		q.out.m = m;
+	}
+	if (wide) q.status = kChainInputOutOfDomain;
+	if (fold.pre_status != kOk) q.status = fold.pre_status;
+	return q;
 }
+
+// ------------------------------------------------------------------ requant codes
+// code = round_half_away(x * 127 R / 2^E), |x| <= the row's maximum (so |code| <= 127).
+// v = x * f: the roundings of x, d, f and the product put v within 127 * 2^-23 < 1.6e-5 of the exact
+// quotient, so unless v is within 2e-5 of a half-integer its nearest integer IS the code: five
+// instructions per element instead of about twenty. One element in 25,000 is closer -- one in most
+// activation rows, and a row waits for its slowest warp -- so those are settled in place by adding
+// x * f_lo to the distance, and only within 1e-6 of the tie (or in a row above 2^24, where x and d
+// themselves round) out of line, at last by requant_code itself.
 constexpr float kRoundMagic = 12582912.0f;      // 1.5 * 2^23: adding it leaves the nearest integer in the low bits
-constexpr float kNearTie = 0.4999f;
+constexpr int kRoundMagicBits = 0x4B400000;
+constexpr float kNearTie = 0.49998f;
 __device__ __forceinline__ float to_float(int32_t x) { return __int2float_rn(x); }
 __device__ __forceinline__ float to_float(int64_t x) { return __ll2float_rn(x); }
 template <typename T>
-static __device__ __noinline__ uint32_t code_quad_exact(T x0, T x1, T x2, T x3, int64_t r, int s) {
+static __device__ __noinline__ uint32_t code_quad_exact(T x0, T x1, T x2, T x3, uint32_t d) {
+	int64_t dn;
+	int s;
+	normalize_scale((int64_t)d, &dn, &s);
+	const int64_t r = dyn_recip(dn);
 	return pack4(requant_code((int64_t)x0, r, s), requant_code((int64_t)x1, r, s), requant_code((int64_t)x2, r, s),
 	             requant_code((int64_t)x3, r, s));
 }
+__device__ __forceinline__ float low_part(int32_t x, float xf) { return (float)((int64_t)x - (int64_t)xf); }
+__device__ __forceinline__ float low_part(int64_t x, float xf) { return (float)(x - (int64_t)xf); }
+template <typename T>
+static __device__ __noinline__ uint32_t code_quad_near_tie(T x0, T x1, T x2, T x3, uint32_t d) {
+	// f + f_lo = 127 / d to about 2^-46
+	const float df = __uint2float_rn(d), dl = (float)(int)((int64_t)d - (int64_t)df), rd = __fdividef(1.0f, df), f0 = 127.0f * rd;
+	const float f = fmaf(fmaf(-f0, df, 127.0f), rd, f0);
+	const float f_lo = fmaf(-f, dl, fmaf(-f, df, 127.0f)) * rd;
+	const T x[4] = {x0, x1, x2, x3};
+	int c[4];
+	bool tie = false;
+#pragma unroll
+	for (int j = 0; j < 4; ++j) {
+		const float xf = to_float(x[j]);
+		const float q = fmaf(xf, f, kRoundMagic) - kRoundMagic;
+		const float off = fmaf(xf, f, -q) + fmaf(xf, f_lo, low_part(x[j], xf) * f);
+		tie = tie || fabsf(fabsf(off) - 0.5f) < 1e-6f;
+		c[j] = (int)q + (off > 0.5f ? 1 : (off < -0.5f ? -1 : 0));
+	}
+	if (tie) return code_quad_exact<T>(x0, x1, x2, x3, d);
+	return pack4(c[0], c[1], c[2], c[3]);
+}
 // four codes, packed; element j in byte j
 template <typename T>
-__device__ __forceinline__ uint32_t code_quad(const T (&x)[4], const QuadCoder& c) {
+__device__ __forceinline__ uint32_t code_quad(const T (&x)[4], const QuadFunnel& q) {
+	int t[4];
+	float off[4], far = 0.0f;
+#pragma unroll
+	for (int j = 0; j < 4; ++j) {
+		const float xf = to_float(x[j]);
+		const float m = fmaf(xf, q.f, kRoundMagic);
+		t[j] = __float_as_int(m);
+		off[j] = fmaf(xf, q.f, kRoundMagic - m);
+		far = fmaxf(far, fabsf(off[j]));
+	}
+	if (far > kNearTie) {
+		far = 1.0f;
+#pragma unroll
+		for (int j = 0; j < 4; ++j) {
+			const float o = fmaf(to_float(x[j]), q.f_lo, off[j]);
+			t[j] += (o > 0.5f ? 1 : 0) - (o < -0.5f ? 1 : 0);
+			far = fminf(far, fabsf(fabsf(o) - 0.5f));
+		}
+		if (far < 1e-6f || q.d > (1u << 24)) return code_quad_near_tie<T>(x[0], x[1], x[2], x[3], q.d);
+	}
+	return pack4(t[0], t[1], t[2], t[3]);
+}
+// The same for rows of small integers (the residual sums), where a true tie 254 |x| = (2 c + 1) d is
+// common: the half of an even maximum usually occurs in the row. On a tie the reference's answer
+// depends on which way its reciprocal R = round(2^E / d), E = 32 + floor(log2 d), was rounded: away
+// from zero if R d >= 2^E, toward it otherwise (off a tie the distance, at least 1 / (2 d), exceeds
+// what R's rounding moves, 63.5 / 2^31). R was rounded up iff floor(2^(E+1) / d) is odd or d is a
+// power of two; the quotient's last bit comes from two 16-bit division steps. d < 2^16.
+__device__ __forceinline__ uint32_t div_step(uint32_t num, uint32_t d, float rd, uint32_t* rem) {      // num / d <= 2^16
+	int32_t q = __float2int_rz(__uint2float_rn(num) * rd), r = (int32_t)(num - (uint32_t)q * d);
+	if (r < 0) { --q; r += (int32_t)d; }
+	if (r >= (int32_t)d) { ++q; r -= (int32_t)d; }
+	*rem = (uint32_t)r;
+	return (uint32_t)q;
+}
+__device__ __forceinline__ bool reciprocal_rounded_up(uint32_t d) {
+	const float rd = __fdividef(1.0f, __uint2float_rn(d));
+	uint32_t rem;
+	div_step(1u << (16 + 31 - __clz((int)d)), d, rd, &rem);      // 2^(p + 16)
+	div_step(rem << 16, d, rd, &rem);                            // ... 2^(p + 32)
+	return 2u * rem >= d || (d & (d - 1u)) == 0u;                // ... 2^(p + 33)
+}
+__device__ __forceinline__ uint32_t code_small_near_tie(float x0, float x1, float x2, float x3, float f, uint32_t d) {
+	const bool up = reciprocal_rounded_up(d);
+	const float x[4] = {x0, x1, x2, x3};
+	int c[4];
+#pragma unroll
+	for (int j = 0; j < 4; ++j) {
+		const int a = (int)fabsf(x[j]), k = (int)rintf(fabsf(x[j]) * f);
+		const int u = 254 * a - 2 * k * (int)d, dd = (int)d;      // the quotient is k + u / (2 d)
+		const int up_by = (u > dd || (u == dd && up)) ? 1 : ((u < -dd || (u == -dd && !up)) ? -1 : 0);
+		c[j] = x[j] < 0.0f ? -(k + up_by) : k + up_by;
+	}
+	return pack4(c[0], c[1], c[2], c[3]);
+}
+// elements: integers below 2^16 in floats, as is the row's maximum
+__device__ __forceinline__ uint32_t code_small_quad(const float (&x)[4], const QuadFunnel& q) {
 	int t[4];
 	float far = 0.0f;
 #pragma unroll
 	for (int j = 0; j < 4; ++j) {
-		const float xf = to_float(x[j]);
-		const float m = fmaf(xf, c.f, kRoundMagic);
+		const float m = fmaf(x[j], q.f, kRoundMagic);
 		t[j] = __float_as_int(m);
-		far = fmaxf(far, fabsf(fmaf(xf, c.f, kRoundMagic - m)));
+		far = fmaxf(far, fabsf(fmaf(x[j], q.f, kRoundMagic - m)));
 	}
-	if (far > kNearTie) return code_quad_exact<T>(x[0], x[1], x[2], x[3], c.r, c.s);
+	if (far > kNearTie) return code_small_near_tie(x[0], x[1], x[2], x[3], q.f, q.d);
 	return pack4(t[0], t[1], t[2], t[3]);
 }
 
-// ------------------------------------------------------------------- K/V landing, residual
+// --------------------------------------------------------------------------- K/V landing
 // LandingRescale with the row's (m_a, r_t, exponent) product hoisted: round_half_away(|code| P / 2^k)
 // with P = |m_a| r_t < 2^63, by the 64-bit-word identity landing_rescale states. `fast` when the
 // scales are in the range that identity covers.
@@ -120,6 +233,73 @@ __device__ __forceinline__ uint64_t land_magnitude(uint32_t ac, const Lander& l)
 	return ((uint64_t)ac * l.hi + l.half + __umulhi(ac, l.lo)) >> l.sh;
 }
 
+// ---------------------------------------------------------------------- residual
+// A branch code on the stream's scale, LandingRescale(code) = round_half_away(code * rho) with
+// rho = m_a r_t / 2^k: like the requant codes, in float with the near-ties settled separately. rho is
+// rounded once, so the landed value is known unless it is within 127 rho 2^-23 (+ 1e-6) of a
+// half-integer. Sums with the stream stay below 2^16: exact in float.
+struct Recip {
+	float hi, lo;      // the stream scale's reciprocal r_t as a sum of two floats (0: outside (0, 2^32])
+};
+__device__ __forceinline__ Recip make_recip(int64_t r_t) {
+	Recip r{0.0f, 0.0f};
+	if (r_t > 0 && (uint64_t)r_t <= ((uint64_t)1 << 32)) {
+		r.hi = __ll2float_rn(r_t);
+		r.lo = (float)(r_t - (int64_t)r.hi);
+	}
+	return r;
+}
+struct Branch {
+	float rho, rho_lo, near_tie;
+	bool fast;
+};
+// bs: the branch's scale, ss: the stream's, r: the reciprocal of its mantissa
+__device__ __forceinline__ Branch make_branch(Scale bs, Recip r, Scale ss) {
+	Branch b;
+	const int64_t k64 = 62 - (bs.e - ss.e);
+	const bool e_ok = bs.e < ((int64_t)1 << 61) && bs.e > -((int64_t)1 << 61) && ss.e < ((int64_t)1 << 61) && ss.e > -((int64_t)1 << 61);
+	const bool in = e_ok && k64 >= 33 && k64 <= 94 && r.hi > 0.0f;
+	const float scale = __int_as_float((127 - (in ? (int)k64 : 33)) << 23);      // 2^-k
+	const int32_t m = (int32_t)bs.m;      // (a negative mantissa flips the sign of every landed value)
+	const float mh = __int2float_rn(m), ml = (float)((int64_t)m - (int64_t)mh);
+	const float p = mh * r.hi, e = fmaf(mh, r.hi, -p) + fmaf(mh, r.lo, ml * r.hi);
+	const float rho = p + e;
+	b.rho = rho * scale;
+	b.rho_lo = ((p - rho) + e) * scale;
+	const float top = fabsf(b.rho) * 127.0f;
+	b.near_tie = 0.499999f - top * 1.1920928955078125e-07f;      // 2^-23
+	b.fast = in && top < 32000.0f;
+	return b;
+}
+static __device__ __noinline__ float land_code_exact(int code, int64_t bs_m, int64_t bs_e, int64_t ss_m, int64_t ss_e) {
+	return (float)landing_rescale((int64_t)code, bs_m, dyn_recip(ss_m), bs_e, ss_e, nullptr, nullptr);
+}
+static __device__ __noinline__ float land_code_near_tie(int code, float rho, float rho_lo, int64_t bs_m, int64_t bs_e, int64_t ss_m,
+                                                        int64_t ss_e) {
+	const float cf = (float)code, q = fmaf(cf, rho, kRoundMagic) - kRoundMagic;
+	const float off = fmaf(cf, rho, -q) + cf * rho_lo;      // within 2^-24 + 127 rho 2^-44
+	if (fabsf(fabsf(off) - 0.5f) < 1e-6f) return land_code_exact(code, bs_m, bs_e, ss_m, ss_e);
+	return q + (off > 0.5f ? 1.0f : (off < -0.5f ? -1.0f : 0.0f));
+}
+// w[j] = landed(code j) + stream code j, for four codes packed in c and four in st
+__device__ __forceinline__ void join_quad(uint32_t c, uint32_t st, const Branch& b, Scale bs, Scale ss, float (&w)[4]) {
+	float far[4], worst = 0.0f;
+#pragma unroll
+	for (int j = 0; j < 4; ++j) {
+		const float cf = (float)byte_of(c, j);
+		const float q = fmaf(cf, b.rho, kRoundMagic) - kRoundMagic;
+		far[j] = fabsf(fmaf(cf, b.rho, -q));
+		worst = fmaxf(worst, far[j]);
+		w[j] = q + (float)byte_of(st, j);
+	}
+	if (worst > b.near_tie) {
+#pragma unroll
+		for (int j = 0; j < 4; ++j)
+			if (far[j] > b.near_tie)
+				w[j] = land_code_near_tie(byte_of(c, j), b.rho, b.rho_lo, bs.m, bs.e, ss.m, ss.e) + (float)byte_of(st, j);
+	}
+}
+
 // ---------------------------------------------------------------------- RMSNorm
 // floor((h << 32) / root) for |h| <= 127: with 2^32 = Q root + rem it is h Q + floor(h rem / root),
 // and mulhi(h rem, Q) is that floor or one beside it. Needs root >= 2^16 (Q <= 2^16, every product
@@ -129,23 +309,34 @@ struct NormDiv {
 	bool fast;
 };
 // root of RmsNormSite: max(isqrt(floor(ss 2^32 / n)), 1); the inner floor cannot change the outer one.
-// n <= 131071 and |h| <= 127 keep (root + 1)^2 n inside 64 bits.
+// A double estimate within one of the root, settled by one exact residual x - r^2 n (n <= 131071 and
+// |h| <= 127 keep it inside 64 bits); Q the same way from a float reciprocal (2^32 / root <= 2^16, so
+// the estimate is within one).
 __device__ __forceinline__ NormDiv make_norm_div(uint32_t ss, int n, double inv_n) {
-	const uint64_t x = (uint64_t)ss << 32;
-	uint32_t r = ss == 0u ? 0u : (uint32_t)sqrt_estimate((double)ss * 4294967296.0 * inv_n);      // within one of the root
-	if ((uint64_t)r * r * (uint64_t)n > x) --r;
-	if ((uint64_t)(r + 1u) * (r + 1u) * (uint64_t)n <= x) ++r;
+	const double ms = (double)max(ss, 1u) * 4294967296.0 * inv_n;
+	double y;
+	asm("rsqrt.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(ms));
+	const double g = ms * y;
+	uint32_t r = (uint32_t)__double2int_rz(fma(fma(-g, g, ms), 0.5 * y, g));
+	const int64_t left = (int64_t)(((uint64_t)ss << 32) - (uint64_t)r * r * (uint64_t)(uint32_t)n);
+	if (left < 0) --r;
+	if (left >= (int64_t)(uint64_t)(2u * r + 1u) * n) ++r;
 	NormDiv d;
 	d.fast = r >= 65536u;
 	if (r < 65536u) r = 65536u;
-	uint32_t q = 0xFFFFFFFFu / r, rem = 0u - q * r;
-	if (rem == r) {      // root a power of two
+	int32_t q = __float2int_rz(__fdividef(4294967296.0f, __uint2float_rn(r)));
+	int32_t rem = (int32_t)(0u - (uint32_t)q * r);
+	if (rem < 0) {
+		--q;
+		rem += (int32_t)r;
+	}
+	if (rem >= (int32_t)r) {
 		++q;
-		rem = 0u;
+		rem -= (int32_t)r;
 	}
 	d.root = (int32_t)r;
-	d.q = (int32_t)q;
-	d.rem = (int32_t)rem;
+	d.q = q;
+	d.rem = rem;
 	return d;
 }
 __device__ __forceinline__ int32_t norm_quotient(int h, const NormDiv& d) {

@@ -17,6 +17,7 @@
 #include <type_traits>
 
 #include "sslm_kernels.h"
+#include "sslm_cluster.cuh"
 #include "sslm_quad.cuh"
 
 namespace sslm {
@@ -200,13 +201,12 @@ __device__ __forceinline__ int32_t quad_rmsnorm(const uint32_t (&h)[NV], const u
 		}
 	}
 	mx = block_max_u32(mx, bank);
-	const FunnelParams fp = funnel_finish((unsigned long long)mx, fold);
+	const QuadFunnel fp = quad_funnel((unsigned long long)mx, fold);
 	if (fp.status != kOk) return fp.status;
-	const QuadCoder cd = make_quad_coder(fp.r, fp.s);
 #pragma unroll
 	for (int v = 0; v < NV; ++v) {
 		const int q = threadIdx.x + v * blockDim.x;
-		const uint32_t c = code_quad(w[v], cd);
+		const uint32_t c = code_quad(w[v], fp);
 		if (q < nq) ((uint32_t*)out)[q] = c;
 	}
 	if (threadIdx.x == 0) *out_scale = fp.out;
@@ -259,14 +259,13 @@ k_begin(RowBatch b, Dims d, const int8_t* embed, Scale c_embed, const RowSource*
 #pragma unroll
 			for (int j = 0; j < 4; ++j) mx = max(mx, abs_u32(byte_of(h[v], j)));
 		mx = block_max_u32(mx, bank);
-		const FunnelParams fp = funnel_finish((unsigned long long)mx, fold_e);
+		const QuadFunnel fp = quad_funnel((unsigned long long)mx, fold_e);
 		st = fp.status;
 		if (st == kOk) {
-			const QuadCoder cd = make_quad_coder(fp.r, fp.s);
 #pragma unroll
 			for (int v = 0; v < NV; ++v) {
 				const int32_t w[4] = {byte_of(h[v], 0), byte_of(h[v], 1), byte_of(h[v], 2), byte_of(h[v], 3)};
-				h[v] = code_quad(w, cd);
+				h[v] = code_quad(w, fp);
 			}
 			if (threadIdx.x == 0) b.xs[r] = fp.out;
 		}
@@ -294,15 +293,14 @@ k_begin(RowBatch b, Dims d, const int8_t* embed, Scale c_embed, const RowSource*
 	set_status(b, r, st, site, b.layer);
 }
 
-// acc + bias term, *ok = false when the term or the sum leaves int64. A bias code inside 32 bits keeps
-// the product with the row's reciprocal (at most 2^32) inside 64; others take the 128-bit composite.
-__device__ __forceinline__ int64_t biased(int64_t acc, int64_t bias, int64_t r_a, int bexp, bool* ok) {
-	int64_t term, sum;
-	bool t_ok = true;
-	if (bias == (int64_t)(int32_t)bias && r_a > 0 && (uint64_t)r_a <= ((uint64_t)1 << 32)) term = rdivpot64(bias * r_a, bexp);
-	else t_ok = bias_reconcile(bias, r_a, bexp, &term);
-	*ok = bias_accumulate(acc, term, &sum) && t_ok;
-	return sum;
+// The bias term of one element, false when it leaves int64. A bias code inside 32 bits keeps the
+// product with the row's reciprocal (at most 2^32) inside 64; others take the 128-bit composite.
+__device__ __forceinline__ bool bias_term(int64_t bias, int64_t r_a, int bexp, int64_t* term) {
+	if (bias == (int64_t)(int32_t)bias && r_a > 0 && (uint64_t)r_a <= ((uint64_t)1 << 32)) {
+		*term = rdivpot64(bias * r_a, bexp);
+		return true;
+	}
+	return bias_reconcile(bias, r_a, bexp, term);
 }
 
 // After the fused q/k/v projection: q funnel (ProjectAndFunnel's tail,
@@ -357,6 +355,31 @@ k_qkv_post(RowBatch b, Dims d, const LayerDev* layer, Scale c_q, int layer_index
 		if (e < H + KV) rope_words(e, rc1, rs1);
 		if (e >= H) landing(e, rt1, et1);
 	}
+	// q/k/v bias (BIA1): term_i = round(B_i * Recip(S[x].m) / 2^(92 + S[x].e)) joins the folded
+	// accumulator (after the LoRA delta) before the q funnel and before the K/V landing
+	// (ApplyBiasReconcileRow, forward_sites.cpp:1015-1036). The exponent gate and R_a are per
+	// row; a term or a sum that leaves int64 refuses the row. Biased elements are kept in 64 bits.
+	// Only the sum needs the projection.
+	int bexp = 0;
+	int64_t r_a = 0;
+	bool gate = true;
+	if (BIAS) {
+		r_a = dyn_recip(ns.m);
+		gate = bias_exponent_in_domain(ns.e, &bexp);
+	}
+	auto bias_quad = [&](int q, int64_t (&term)[4], uint32_t& bad) {
+		const int e = q * 4;
+		const int64_t* bp = e < H ? bias_q : (e < H + KV ? bias_k : bias_v);
+		const int off = e < H ? e : (e < H + KV ? e - H : e - H - KV);
+#pragma unroll
+		for (int j = 0; j < 4; ++j) {
+			term[j] = 0;
+			if (!scalar_warp && q < nq && bp != nullptr && gate && !bias_term(bp[off + j], r_a, bexp, &term[j])) bad = 1;
+		}
+	};
+	int64_t term1[4] = {0, 0, 0, 0};
+	uint32_t bad1 = 0;
+	if (BIAS && NV == 1) bias_quad((int)threadIdx.x, term1, bad1);
 	pdl_wait();
 	pdl_release();
 	const T* row = (const T*)b.wide + (size_t)r * b.wide_ld;
@@ -373,10 +396,6 @@ k_qkv_post(RowBatch b, Dims d, const LayerDev* layer, Scale c_q, int layer_index
 	if (threadIdx.x == 0) b.rowmax[(size_t)r * 4] = 0ull;
 	if (refused) return;
 
-	// q/k/v bias (BIA1): term_i = round(B_i * Recip(S[x].m) / 2^(92 + S[x].e)) joins the folded
-	// accumulator (after the LoRA delta) before the q funnel and before the K/V landing
-	// (ApplyBiasReconcileRow, forward_sites.cpp:1015-1036). The exponent gate and R_a are per
-	// row; a term or a sum that leaves int64 refuses the row. Biased elements are kept in 64 bits.
 	using Y = typename WideOf<W64 || BIAS>::T;
 	Y y[NV][4];
 	if constexpr (!BIAS) {
@@ -385,9 +404,6 @@ k_qkv_post(RowBatch b, Dims d, const LayerDev* layer, Scale c_q, int layer_index
 #pragma unroll
 			for (int j = 0; j < 4; ++j) y[v][j] = x[v][j];
 	} else {
-		int bexp = 0;
-		const int64_t r_a = dyn_recip(ns.m);
-		const bool gate = bias_exponent_in_domain(ns.e, &bexp);
 		if (!gate && bias_q != nullptr) {
 			set_status(b, r, kRoundingDivideExponentOutOfDomain, kSiteQ, b.layer);
 			return;
@@ -396,48 +412,45 @@ k_qkv_post(RowBatch b, Dims d, const LayerDev* layer, Scale c_q, int layer_index
 #pragma unroll
 		for (int v = 0; v < NV; ++v) {
 			const int q = (int)threadIdx.x + v * qt, e = q * 4;
-			const int64_t* bp = e < H ? bias_q : (e < H + KV ? bias_k : bias_v);
-			const int off = e < H ? e : (e < H + KV ? e - H : e - H - KV);
-			const bool mine = !scalar_warp && q < nq;
+			int64_t term[4];
+			uint32_t bad = 0;
+			if (NV > 1) bias_quad(q, term, bad);
+			else bad = bad1;
 #pragma unroll
 			for (int j = 0; j < 4; ++j) {
-				int64_t sum = (int64_t)x[v][j];
-				if (mine && bp != nullptr && gate) {
-					bool ok;
-					sum = biased(sum, bp[off + j], r_a, bexp, &ok);
-					if (!ok) (e < H ? bad_q : bad_kv) = 1;
-				}
+				int64_t sum;
+				if (!bias_accumulate((int64_t)x[v][j], NV > 1 ? term[j] : term1[j], &sum)) bad = 1;
 				y[v][j] = sum;
-				if (mine && e < H) {
+				if (!scalar_warp && e < H) {
 					const unsigned long long a = abs_u64(sum);
 					lmx = max(lmx, a > 0xFFFFFFFFull ? 0xFFFFFFFFu : (uint32_t)a);      // (anything above 2^31 is refused alike)
 				}
 			}
+			if (e < H) bad_q |= bad;
+			else bad_kv |= bad;
 		}
 		if (bias_q != nullptr) {
-			// the row maximum the projection reduced does not include the bias: take it here
-			if (block_max_u32(bad_q, bank) != 0u) {
+			// the row maximum the projection reduced does not include the bias: take it here (a q term or
+			// sum outside int64 refuses the row first: it votes with a bit no maximum in the domain has)
+			const uint32_t m = block_max_u32(bad_q != 0u ? 0xFFFFFFFFu : min(lmx, 0xFFFFFFFEu), bank);
+			if (m == 0xFFFFFFFFu) {
 				set_status(b, r, kBiasReconcileProductOutOfDomain, kSiteQ, b.layer);
 				return;
 			}
-			mx = (unsigned long long)block_max_u32(lmx, bank);
+			mx = (unsigned long long)m;
 		}
-		// (K / V terms that cannot be formed refuse the row after the q funnel had its say)
-		const FunnelParams fq = funnel_finish(mx, fold_q);
-		if (fq.status == kOk && (bias_k != nullptr || bias_v != nullptr)) {
-			if (!gate) {
-				set_status(b, r, kRoundingDivideExponentOutOfDomain, kSiteKv, b.layer);
-				return;
-			}
-			// (a bias term outside int64 refuses the row before anything lands, so before anything
-			// could count as saturated: LandTokenKVRow, forward_sites.cpp:1281-1418)
-			if (block_max_u32(bad_kv, bank) != 0u) {
-				set_status(b, r, kBiasReconcileProductOutOfDomain, kSiteKv, b.layer);
+		// (K / V terms that cannot be formed refuse the row after the q funnel had its say, and before
+		// anything lands, so before anything could count as saturated: LandTokenKVRow,
+		// forward_sites.cpp:1281-1418)
+		if (bias_k != nullptr || bias_v != nullptr) {
+			const bool bad = __syncthreads_or((int)bad_kv) != 0;
+			if ((bad || !gate) && quad_funnel(mx, fold_q).status == kOk) {
+				set_status(b, r, gate ? kBiasReconcileProductOutOfDomain : kRoundingDivideExponentOutOfDomain, kSiteKv, b.layer);
 				return;
 			}
 		}
 	}
-	const FunnelParams fp = funnel_finish(mx, fold_q);
+	const QuadFunnel fp = quad_funnel(mx, fold_q);
 	if (fp.status != kOk) {
 		set_status(b, r, fp.status, kSiteQ, b.layer);
 		return;
@@ -478,14 +491,13 @@ k_qkv_post(RowBatch b, Dims d, const LayerDev* layer, Scale c_q, int layer_index
 		return;
 	}
 
-	const QuadCoder cd = make_quad_coder(fp.r, fp.s);
 	uint32_t sat = 0;
 #pragma unroll
 	for (int v = 0; v < NV; ++v) {
 		const int q = (int)threadIdx.x + v * qt, e = q * 4;
 		if (q >= nq) break;
 		if (e < H) {      // q: code, rotate
-			const uint32_t c = code_quad(y[v], cd);
+			const uint32_t c = code_quad(y[v], fp);
 			if (NV > 1) rope_words(e, rc1, rs1);
 			((uint32_t*)(b.qrot + (size_t)r * H))[q] = rope_quad(c, rc1, rs1);
 			continue;
@@ -548,16 +560,15 @@ k_ctx_funnel(RowBatch b, Dims d, Scale c_ctx) {
 	__syncthreads();
 	if (threadIdx.x == 0) b.rowmax[(size_t)r * 4 + 3] = 0ull;
 	if (refused) return;
-	const FunnelParams fp = funnel_finish(mx, fold_ctx);
+	const QuadFunnel fp = quad_funnel(mx, fold_ctx);
 	if (fp.status != kOk) {
 		set_status(b, r, fp.status, kSiteCtx, b.layer);
 		return;
 	}
-	const QuadCoder cd = make_quad_coder(fp.r, fp.s);
 #pragma unroll
 	for (int v = 0; v < NV; ++v) {
 		const int q = threadIdx.x + v * blockDim.x;
-		const uint32_t c = code_quad(x[v], cd);
+		const uint32_t c = code_quad(x[v], fp);
 		if (q < nq) ((uint32_t*)(b.ctx + (size_t)r * n))[q] = c;
 	}
 	if (threadIdx.x == 0) b.cs[r] = fp.out;
@@ -566,14 +577,17 @@ k_ctx_funnel(RowBatch b, Dims d, Scale c_ctx) {
 // The residual site's general form, from the projection row on (the row's scales left the register
 // form's range). Everything it needs is still in global memory.
 template <typename T>
-__device__ __noinline__ int32_t res_site_general(const T* row, int n, int64_t code_r, int code_s, int64_t bs_m, int64_t bs_e,
+__device__ __noinline__ int32_t res_site_general(const T* row, int n, uint32_t peak, int64_t bs_m, int64_t bs_e,
                                                  const int8_t* stream, int64_t ss_m, int64_t ss_e, int64_t site_m, int64_t site_e,
                                                  int8_t* out, Scale* out_scale, unsigned char* smem) {
 	Red red{(unsigned long long*)smem, 0};
 	int64_t* lut = (int64_t*)(smem + kRedBytes);
 	int64_t* wide = (int64_t*)(smem + kRedBytes + kLutBytes);
 	int8_t* so = (int8_t*)(wide + n);
-	const Coder cd = make_coder(code_r, code_s);
+	int64_t dn;
+	int s;
+	normalize_scale((int64_t)peak, &dn, &s);
+	const Coder cd = make_coder(dyn_recip(dn), s);
 	const Scale ss{ss_m, ss_e};
 	__syncthreads();
 #pragma unroll 1
@@ -586,8 +600,8 @@ __device__ __noinline__ int32_t res_site_general(const T* row, int n, int64_t co
 // A projection's funnel -> residual site -> (RMSNorm): the o projection and the attention residual
 // (forward_sites.cpp:1906-1937), or the down projection, the MLP residual and the next layer's
 // attention norm (:1968-1987, :1694-1698).
-template <int NV, bool W64>
-__global__ void __launch_bounds__(512, NV == 1 ? 1 : 2)
+template <int NV, int MAXT, bool W64>
+__global__ void __launch_bounds__(MAXT, NV == 1 ? 2 : 1)
 k_res(RowBatch b, Dims d, ResSite a) {
 	using T = typename WideOf<W64>::T;
 	using WideLoad = typename std::conditional<W64, long long, int>::type;
@@ -609,10 +623,11 @@ k_res(RowBatch b, Dims d, ResSite a) {
 	const FunnelFold fold_res = funnel_prefold(&ss, 1, a.c_res);
 	const FunnelFold fold_n = funnel_prefold(nullptr, 0, a.c_norm);
 	const int64_t r_h = dyn_recip(ss.m);
+	const Recip r_f = make_recip(r_h);
 	const double inv_n = rcp_estimate((double)n);
+	const T* row = (const T*)b.wide + (size_t)r * b.wide_ld;
 	pdl_wait();
 	pdl_release();
-	const T* row = (const T*)b.wide + (size_t)r * b.wide_ld;
 	T x[NV][4];
 #pragma unroll
 	for (int v = 0; v < NV; ++v) {
@@ -622,7 +637,7 @@ k_res(RowBatch b, Dims d, ResSite a) {
 	}
 	const unsigned long long pmx = __ldcg(&b.rowmax[(size_t)r * 4]);
 	const bool refused = __ldcg(&b.status[r]) != 0;
-	const FunnelParams fp = funnel_finish(pmx, fold_p);
+	const QuadFunnel fp = quad_funnel(pmx, fold_p);
 	int32_t st = fp.status;
 	int site = a.site_proj, site_layer = b.layer;
 	if (refused || st != kOk) {
@@ -631,38 +646,31 @@ k_res(RowBatch b, Dims d, ResSite a) {
 		if (!refused) set_status(b, r, st, site, site_layer);
 		return;
 	}
-	// wide_i = LandingRescale(code_i, S[branch], Recip(S[stream].m), ...) + stream_i in 32 bits, when the
-	// largest landed magnitude allows it
-	const Lander l = make_lander(fp.out.m, r_h, fp.out.e, ss.e);
-	const bool fast = l.fast && land_magnitude(127u, l) < (1ull << 30) && fits_i32(ss.m);
+	// wide_i = LandingRescale(code_i, S[branch], Recip(S[stream].m), ...) + stream_i, small integers held
+	// in floats when the largest landed magnitude allows it
+	const Branch br = make_branch(fp.out, r_f, ss);
 	site = a.site_res;
 	uint32_t h[NV];
 	Scale os{0, 0};
-	if (fast) {
-		const QuadCoder cd = make_quad_coder(fp.r, fp.s);
-		int32_t w[NV][4];
-		uint32_t mx = 0;
+	if (br.fast && fits_i32(ss.m)) {
+		float w[NV][4], top = 0.0f;
 #pragma unroll
 		for (int v = 0; v < NV; ++v) {
-			const uint32_t c = code_quad(x[v], cd);
+			const uint32_t c = code_quad(x[v], fp);
+			join_quad(c, sx[v], br, fp.out, ss, w[v]);
 #pragma unroll
-			for (int j = 0; j < 4; ++j) {
-				const int cj = byte_of(c, j);
-				const int32_t m = (int32_t)land_magnitude((uint32_t)abs(cj), l);
-				w[v][j] = (((cj < 0) != l.neg) ? -m : m) + byte_of(sx[v], j);
-				mx = max(mx, abs_u32(w[v][j]));
-			}
+			for (int j = 0; j < 4; ++j) top = fmaxf(top, fabsf(w[v][j]));
 		}
+		uint32_t mx = (uint32_t)top;
 		mx = block_max_u32(mx, bank);
 		if (threadIdx.x == 0) b.rowmax[(size_t)r * 4] = 0ull;      // (every thread has read it)
-		const FunnelParams fr = funnel_finish((unsigned long long)mx, fold_res);
+		const QuadFunnel fr = quad_funnel((unsigned long long)mx, fold_res);
 		st = fr.status;
 		if (st == kOk) {
-			const QuadCoder cr = make_quad_coder(fr.r, fr.s);
 #pragma unroll
 			for (int v = 0; v < NV; ++v) {
 				const int q = threadIdx.x + v * blockDim.x;
-				h[v] = code_quad(w[v], cr);
+				h[v] = code_small_quad(w[v], fr);
 				if (q < nq) ((uint32_t*)(a.out + (size_t)r * n))[q] = h[v];
 			}
 			if (threadIdx.x == 0) a.out_scale[r] = fr.out;
@@ -670,7 +678,7 @@ k_res(RowBatch b, Dims d, ResSite a) {
 		}
 	} else {
 		if (!fits_i32(ss.m)) st = kCarriedScaleMantissaOutOfDomain;
-		else st = res_site_general((const WideLoad*)row, n, fp.r, fp.s, fp.out.m, fp.out.e, a.stream + (size_t)r * n, ss.m, ss.e,
+		else st = res_site_general((const WideLoad*)row, n, fp.d, fp.out.m, fp.out.e, a.stream + (size_t)r * n, ss.m, ss.e,
 		                           a.c_res.m, a.c_res.e, a.out + (size_t)r * n, &a.out_scale[r], smem);
 		__syncthreads();
 		if (threadIdx.x == 0) b.rowmax[(size_t)r * 4] = 0ull;
@@ -713,42 +721,38 @@ k_res(RowBatch b, Dims d, ResSite a) {
 	set_status(b, r, st, site, site_layer);
 }
 
-// ---- thread-block cluster helpers (distributed shared memory)
-__device__ __forceinline__ uint32_t cluster_rank() {
-	uint32_t r;
-	asm volatile("mov.u32 %0, %%cluster_ctarank;" : "=r"(r));
-	return r;
-}
-__device__ __forceinline__ void cluster_arrive() { asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory"); }
-__device__ __forceinline__ void cluster_wait() { asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory"); }
-// store v at the place of `local` (an address in this block's shared memory) in the block of rank `rank`
-__device__ __forceinline__ void peer_store_u32(void* local, uint32_t rank, uint32_t v) {
-	uint32_t a = (uint32_t)__cvta_generic_to_shared(local);
-	asm volatile("{\n\t.reg .b32 ra;\n\tmapa.shared::cluster.u32 ra, %0, %1;\n\tst.shared::cluster.u32 [ra], %2;\n\t}" ::"r"(a), "r"(rank), "r"(v) : "memory");
-}
-
 // gate / up funnels -> SwiGLU activation site (MlpActSite, forward_sites.cpp:796-864).
 //
 // The activation row is the longest a row site walks (intermediate width, three codes per element).
 // While rows are few its time is one block's chain, so a row is cut over a cluster of `gridDim.x`
 // blocks, which meet once, for the maximum of the products; on a prefill chunk two blocks share a row.
 template <int NV, bool W64>
-__global__ void __launch_bounds__(NV == 5 ? 352 : 512, NV == 5 ? 2 : 1)
+__global__ void __launch_bounds__(NV == 5 ? 352 : 384, NV == 1 ? 1 : 2)
 k_act(RowBatch b, Dims d, Scale c_gate, Scale c_up, Scale c_act, const int32_t* silu_table) {
 	using T = typename WideOf<W64>::T;
 	__shared__ uint32_t s_bank[64];
+	__shared__ int32_t table[1025];     // the sigmoid table
 	__shared__ int32_t gsil[256];       // g * sigmoid(g) for the 255 gate codes, this row's scale
 	__shared__ uint32_t s_peer[8];      // every block's largest product
+	__shared__ __align__(8) unsigned long long s_arrived;
 	Bank bank{s_bank, 0};
 	const int r = blockIdx.y, n = d.inter, nq = n >> 2;
 	const uint32_t blocks = gridDim.x, rank = blocks > 1 ? cluster_rank() : 0u;
 	const int per = (nq + (int)blocks - 1) / (int)blocks, q0 = (int)rank * per, q1 = min(nq, q0 + per);
 	// ahead of the gate/up projection: the normed row's scale (written by the residual site
-	// before that projection ran); the sigmoid table asked into the L1
+	// before that projection ran) and the sigmoid table
 	const Scale ns = b.ns[r];
-	if (threadIdx.x < 33) asm volatile("prefetch.global.L1 [%0];" ::"l"(silu_table + 32 * threadIdx.x));
+	for (int i = threadIdx.x; i < 1025; i += blockDim.x) table[i] = silu_table[i];
 	const FunnelFold fold_g = funnel_prefold(&ns, 1, c_gate), fold_u = funnel_prefold(&ns, 1, c_up);
-	if (blocks > 1) cluster_arrive();      // (paired below: a peer's shared memory is written only once the peer runs)
+	const uint32_t arrived = cta_addr(&s_arrived);
+	if (blocks > 1) {
+		if (threadIdx.x == 0) {
+			exchange_init(arrived, 4u * blocks);
+			exchange_fence_init();
+		}
+		cluster_arrive();
+		cluster_wait();
+	}
 	pdl_wait();
 	pdl_release();
 	const T* grow = (const T*)b.wide + (size_t)r * b.wide_ld;
@@ -766,8 +770,8 @@ k_act(RowBatch b, Dims d, Scale c_gate, Scale c_up, Scale c_act, const int32_t* 
 	}
 	const unsigned long long mxg = __ldcg(&b.rowmax[(size_t)r * 4 + 1]), mxu = __ldcg(&b.rowmax[(size_t)r * 4 + 2]);
 	const bool refused = __ldcg(&b.status[r]) != 0;
-	const FunnelParams fg = funnel_finish(mxg, fold_g);
-	const FunnelParams fu = funnel_finish(mxu, fold_u);
+	const QuadFunnel fg = quad_funnel(mxg, fold_g);
+	const QuadFunnel fu = quad_funnel(mxu, fold_u);
 	int32_t st = fg.status != kOk ? fg.status : fu.status;
 	int site = fg.status != kOk ? kSiteGate : kSiteUp;
 	if (st == kOk && !silu_scale_in_domain(fg.out)) {
@@ -775,11 +779,12 @@ k_act(RowBatch b, Dims d, Scale c_gate, Scale c_up, Scale c_act, const int32_t* 
 		site = kSiteSilu;
 	}
 	const bool live = !refused && st == kOk;
+	__syncthreads();      // the table is complete
 	if (live) {
 		// the sigmoid depends only on the gate code and the row's gate scale: 255 evaluations per
 		// block instead of one per element
 		const int ge = (int)fg.out.e;
-		for (int t = threadIdx.x; t < 255; t += blockDim.x) gsil[t] = (t - 127) * silu_sigmoid_q15(silu_table, t - 127, fg.out.m, ge);
+		for (int t = threadIdx.x; t < 255; t += blockDim.x) gsil[t] = (t - 127) * silu_sigmoid_q15(table, t - 127, fg.out.m, ge);
 	}
 	__syncthreads();
 	// products g * sigmoid(g) * u, |.| <= 127 * 2^15 * 127 < 2^29
@@ -788,10 +793,9 @@ k_act(RowBatch b, Dims d, Scale c_gate, Scale c_up, Scale c_act, const int32_t* 
 	int32_t w[NV][4];
 	uint32_t mx = 0;
 	if (live) {
-		const QuadCoder cg = make_quad_coder(fg.r, fg.s), cu = make_quad_coder(fu.r, fu.s);
-#pragma unroll
+		#pragma unroll
 		for (int v = 0; v < NV; ++v) {
-			const uint32_t g = code_quad(xg[v], cg), u = code_quad(xu[v], cu);
+			const uint32_t g = code_quad(xg[v], fg), u = code_quad(xu[v], fu);
 #pragma unroll
 			for (int j = 0; j < 4; ++j) {
 				w[v][j] = gsil[byte_of(g, j) + 127] * byte_of(u, j);
@@ -802,11 +806,12 @@ k_act(RowBatch b, Dims d, Scale c_gate, Scale c_up, Scale c_act, const int32_t* 
 	mx = block_max_u32(mx, bank);
 	if (blocks > 1) {
 		// Every block of the cluster comes through here, refused row or not, so none waits for one
-		// that left; and only behind the barrier is the row maximum cleared, so every block saw it.
-		cluster_wait();
-		if (threadIdx.x < blocks) peer_store_u32(&s_peer[rank], threadIdx.x, mx);
-		cluster_arrive();
-		cluster_wait();
+		// that left; and only behind it is the row maximum cleared, so every block saw it.
+		if (threadIdx.x < blocks) exchange_send(&s_peer[rank], arrived, threadIdx.x, mx);
+		if (!exchange_wait(arrived)) {
+			set_status(b, r, kInternalWaitTimeout, kSiteAct, b.layer);
+			return;
+		}
 		for (uint32_t i = 0; i < blocks; ++i) mx = max(mx, s_peer[i]);
 	}
 	if (rank == 0 && threadIdx.x == 0) {
@@ -817,17 +822,16 @@ k_act(RowBatch b, Dims d, Scale c_gate, Scale c_up, Scale c_act, const int32_t* 
 		if (!refused && rank == 0) set_status(b, r, st, site, b.layer);
 		return;
 	}
-	const FunnelParams fp = funnel_finish((unsigned long long)mx, fold_act);
+	const QuadFunnel fp = quad_funnel((unsigned long long)mx, fold_act);
 	if (fp.status != kOk) {
 		if (rank == 0) set_status(b, r, fp.status, kSiteAct, b.layer);
 		return;
 	}
-	const QuadCoder ca = make_quad_coder(fp.r, fp.s);
 	uint32_t* out = (uint32_t*)(b.act + (size_t)r * n);
 #pragma unroll
 	for (int v = 0; v < NV; ++v) {
 		const int q = q0 + (int)threadIdx.x + v * (int)blockDim.x;
-		const uint32_t c = code_quad(w[v], ca);
+		const uint32_t c = code_quad(w[v], fp);
 		if (q < q1) out[q] = c;
 	}
 	if (rank == 0 && threadIdx.x == 0) b.acts[r] = fp.out;
@@ -887,15 +891,17 @@ void launch_res(const RowBatch& b, const Dims& d, const ResSite& a, cudaStream_t
 	const int nq = d.hidden / 4, nv = quads_per_thread(b.m, nq), t = quad_threads(nq, nv);
 	const size_t sm = general_smem_bytes(d.hidden);
 	auto go = [&](auto kernel) { launch_pdl(kernel, dim3(b.m), dim3(t), sm, st, b, d, a); };
-	if (nv == 1) b.wide64 ? go(k_res<1, true>) : go(k_res<1, false>);
-	else if (nv == 4) b.wide64 ? go(k_res<4, true>) : go(k_res<4, false>);
-	else b.wide64 ? go(k_res<8, true>) : go(k_res<8, false>);
+	// (two blocks of up to 384 threads leave 85 registers per thread, two of 512 only 64, which spill)
+	if (nv == 1 && t <= 384) b.wide64 ? go(k_res<1, 384, true>) : go(k_res<1, 384, false>);
+	else if (nv == 1) b.wide64 ? go(k_res<1, 512, true>) : go(k_res<1, 512, false>);
+	else if (nv == 4) b.wide64 ? go(k_res<4, 512, true>) : go(k_res<4, 512, false>);
+	else b.wide64 ? go(k_res<8, 512, true>) : go(k_res<8, 512, false>);
 }
 void launch_act(const RowBatch& b, const Dims& d, const LayerDev& h, const int32_t* silu, cudaStream_t st) {
 	const int nq = d.inter / 4;
-	// blocks per row: as many (up to 8) as leave at most two blocks for each multiprocessor
+	// blocks per row: as many (up to 8) as the multiprocessors hold at once, three each
 	int blocks = 2;
-	while (blocks < 8 && b.m * blocks * 2 <= 2 * sm_count()) blocks *= 2;
+	while (blocks < 8 && b.m * blocks * 2 <= 3 * sm_count()) blocks *= 2;
 	while (blocks < 8 && quad_threads((nq + blocks - 1) / blocks, 5) > 352) blocks *= 2;      // (very wide rows)
 	const int per = (nq + blocks - 1) / blocks;
 	const int nv = per <= 384 ? 1 : (per <= 2 * 384 ? 2 : 5);
@@ -928,9 +934,10 @@ cudaError_t rows_configure(const Dims& d) {
 		if (e == cudaSuccess) e = cudaFuncSetAttribute(f, cudaFuncAttributePreferredSharedMemoryCarveout, cudaSharedmemCarveoutMaxShared);
 		if (e == cudaSuccess && dynamic) e = cudaFuncSetAttribute(f, cudaFuncAttributeMaxDynamicSharedMemorySize, sm);
 	};
-	for (const void* f : {(const void*)k_begin<1>, (const void*)k_begin<4>, (const void*)k_begin<8>, (const void*)k_res<1, false>,
-	                      (const void*)k_res<1, true>, (const void*)k_res<4, false>, (const void*)k_res<4, true>,
-	                      (const void*)k_res<8, false>, (const void*)k_res<8, true>})
+	for (const void* f : {(const void*)k_begin<1>, (const void*)k_begin<4>, (const void*)k_begin<8>, (const void*)k_res<1, 384, false>,
+	                      (const void*)k_res<1, 384, true>, (const void*)k_res<1, 512, false>, (const void*)k_res<1, 512, true>,
+	                      (const void*)k_res<4, 512, false>, (const void*)k_res<4, 512, true>, (const void*)k_res<8, 512, false>,
+	                      (const void*)k_res<8, 512, true>})
 		set(f, true);
 	for (const void* f : {(const void*)k_qkv_post<1, false, false>, (const void*)k_qkv_post<1, false, true>,
 	                      (const void*)k_qkv_post<1, true, false>, (const void*)k_qkv_post<1, true, true>,
