@@ -23,17 +23,17 @@
 
 #include <atomic>
 
+#include "sslm_cluster.cuh"
 #include "sslm_kernels.h"
+#include "sslm_quad.cuh"
 
 namespace sslm {
-
-// threads per block = 2 * head_dim: one warp per pair of 8-channel blocks of P.V
-constexpr int kAttnMaxWarps = 8;
 
 // One softmax element for constants that passed the gates of k_qkv_post (1 <= q_ln2 <= q_b
 // < 2^24, q_c >= 0, peak = q_b^2 + q_c within the width gate): the value iexp_element()
 // computes, on 32-bit words and without a branch. dq = max - score (0 <= dq < 2^32).
-// z = floor(x / q_ln2) comes from a float estimate (within 1) repaired with the exact remainder.
+// z = floor(x / q_ln2) comes from one fused multiply-add that rounds toward zero onto an integer grid, with a
+// reciprocal a little too small, so that it is z or z - 1 and the exact remainder tells which.
 //
 // The reference also refuses an element whose value leaves [0, peak] (SoftmaxRowQ15's per-element
 // bound, src/intmath.cpp:870-888). Under the gates above that cannot happen, so the kernels carry
@@ -43,7 +43,7 @@ struct IExpFast {
 	uint32_t ln2, clip;     // q_ln2, 30 * q_ln2
 	int32_t qb;
 	int64_t qc;
-	float inv_ln2;
+	float inv_ln2;          // (1 - 2^-21) / q_ln2
 };
 __device__ __forceinline__ IExpFast iexp_fast_prepare(const SoftmaxConsts& k) {
 	IExpFast f;
@@ -51,7 +51,7 @@ __device__ __forceinline__ IExpFast iexp_fast_prepare(const SoftmaxConsts& k) {
 	f.clip = 30u * f.ln2;
 	f.qb = (int32_t)k.c.q_b;
 	f.qc = k.c.q_c;
-	f.inv_ln2 = 1.0f / (float)f.ln2;
+	f.inv_ln2 = (1.0f / (float)f.ln2) * 0.9999995f;
 	return f;
 }
 // *parts = (z << 24) | rem with x = z * q_ln2 + rem (rem < q_ln2 < 2^24, z <= 30): the second
@@ -59,23 +59,39 @@ __device__ __forceinline__ IExpFast iexp_fast_prepare(const SoftmaxConsts& k) {
 constexpr uint32_t kPartsOfZero = 63u << 24;      // parts that rebuild to the value 0 (shift by 63)
 __device__ __forceinline__ int64_t iexp_fast(uint32_t dq, const IExpFast& f, uint32_t* parts) {
 	const uint32_t x = min(dq, f.clip);
-	int32_t z = __float2int_rz(__uint2float_rn(x) * f.inv_ln2);
-	int32_t rem = (int32_t)(x - (uint32_t)z * f.ln2);
-	const int32_t adj = rem < 0 ? -1 : (rem >= (int32_t)f.ln2 ? 1 : 0);
-	z += adj;
-	rem -= adj * (int32_t)f.ln2;
-	const int32_t base = f.qb - rem;
-	*parts = ((uint32_t)z << 24) | (uint32_t)rem;
-	return ((int64_t)base * (int64_t)base + f.qc) >> z;
+	uint32_t z = (uint32_t)__float_as_int(__fmaf_rz(__uint2float_rn(x), f.inv_ln2, 8388608.0f)) - 0x4B000000u;
+	uint32_t rem = x - z * f.ln2;
+	if (rem >= f.ln2) {
+		rem -= f.ln2;
+		++z;
+	}
+	const int32_t base = f.qb - (int32_t)rem;
+	*parts = (z << 24) | rem;
+	return (int64_t)((uint64_t)((int64_t)base * (int64_t)base + f.qc) >> z);
 }
 __device__ __forceinline__ int64_t iexp_from_parts(uint32_t parts, const IExpFast& f) {
 	const int32_t base = f.qb - (int32_t)(parts & 0xFFFFFFu);
 	return ((int64_t)base * (int64_t)base + f.qc) >> (parts >> 24);
 }
-// floor((e << 15) / tot) for 0 <= e <= min(tot, 2^47), 1 <= tot < 2^63, rinv = 32768 / tot in
-// float: the float quotient is within 2^-6 of the true one, so its floor is off by at most one
-// either way, and one signed remainder settles it (|e * 2^15 - p * tot| < 2 * tot stays inside
-// 64 bits because e * 2^15 <= 2^62).
+// Q15 probability floor((e << 15) / tot), 0 <= e <= tot, 1 <= tot < 2^63.
+//
+// The row's constants scale e to 31 bits; the float product is then within pf 2^-21 + 2^-15 of the
+// quotient, and its floor (one add that rounds toward zero) is the answer unless the fraction is that
+// close to an integer -- at most one element in some ten thousand, and never below the first integer,
+// where nearly all elements of a long row lie. Those take prob_q15.
+struct ProbRow {
+	unsigned long long tot;
+	float c;      // 2^(15 + sh) / tot
+	int sh;
+};
+__device__ __forceinline__ ProbRow prob_row(unsigned long long total) {
+	ProbRow r;
+	r.tot = total > 1ull ? total : 1ull;
+	r.sh = max(0, 33 - __clzll((long long)r.tot));
+	r.c = (32768.0f / (float)r.tot) * __int_as_float((127 + r.sh) << 23);
+	return r;
+}
+// the exact form: a float quotient off by at most one, settled by one signed remainder
 __device__ __forceinline__ uint32_t prob_q15(int64_t e, unsigned long long tot, float rinv) {
 	const unsigned long long num = (unsigned long long)e << 15;
 	uint32_t p = min(__float2uint_rz(__ll2float_rn(e) * rinv), 32768u);
@@ -83,6 +99,18 @@ __device__ __forceinline__ uint32_t prob_q15(int64_t e, unsigned long long tot, 
 	p -= r < 0 ? 1u : 0u;
 	p += r >= (long long)tot ? 1u : 0u;
 	return p;
+}
+// bits 0..15 of the result: the probability, unless *unsure came out true
+__device__ __forceinline__ uint32_t prob_fast(int64_t e, const ProbRow& r, bool* unsure) {
+	const float pf = __uint2float_rn((uint32_t)((uint64_t)e >> r.sh)) * r.c;
+	const float t = __fadd_rz(pf, 8388608.0f);
+	const float off = fabsf((pf - (t - 8388608.0f)) - 0.5f), eps = fmaf(pf, 4.76837158203125e-07f, 3.2e-05f);
+	*unsure = *unsure || (off > 0.5f - eps && pf > eps);
+	return (uint32_t)__float_as_int(t);
+}
+static __device__ __noinline__ uint2 prob_pair_exact(int64_t e0, int64_t e1, unsigned long long tot) {
+	const float rinv = 32768.0f / (float)tot;
+	return make_uint2(prob_q15(e0, tot, rinv), prob_q15(e1, tot, rinv));
 }
 // bytes 0 (low plane) or 1 (high plane) of four probabilities, packed into one word
 __device__ __forceinline__ uint32_t pack_plane(uint32_t p0, uint32_t p1, uint32_t p2, uint32_t p3, int byte) {
@@ -131,166 +159,90 @@ __device__ __forceinline__ void load_row_words(const int8_t* row, int c, uint32_
 	}
 }
 
-// ---- thread-block cluster helpers (distributed shared memory)
-__device__ __forceinline__ uint32_t cluster_rank() {
-	uint32_t r;
-	asm volatile("mov.u32 %0, %%cluster_ctarank;" : "=r"(r));
-	return r;
-}
-// the address, in the cluster's shared window, of `local` (a shared-memory address of this
-// block) inside the block of rank `rank`
-__device__ __forceinline__ uint32_t peer_addr(const void* local, uint32_t rank) {
-	uint32_t a = (uint32_t)__cvta_generic_to_shared(local), out;
-	asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(out) : "r"(a), "r"(rank));
-	return out;
-}
-__device__ __forceinline__ uint32_t peer_ld32(uint32_t addr) {
-	uint32_t v;
-	asm volatile("ld.shared::cluster.u32 %0, [%1];" : "=r"(v) : "r"(addr) : "memory");
-	return v;
-}
-__device__ __forceinline__ unsigned long long peer_ld64(uint32_t addr) {
-	unsigned long long v;
-	asm volatile("ld.shared::cluster.u64 %0, [%1];" : "=l"(v) : "r"(addr) : "memory");
-	return v;
-}
-// Hardware barrier over all threads of all blocks of the cluster: everything written to shared
-// memory before it is visible to every block after it. Every block of a cluster executes every
-// barrier of the kernel (no early return), so nothing can wait for a block that left.
-__device__ __forceinline__ void cluster_sync_all() {
-	asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");
-	asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
-}
-
 // What one block keeps in shared memory. `cp` = positions a block can hold (a multiple of 64).
 struct AttnSmem {
-	int64_t* pbase;       // [cp/16] byte offset of each of the block's pages inside a plane
-	int32_t* sc;          // [G][cp] scores, later (shift, remainder) of each element
-	uint8_t* pl;          // [G][cp] low byte of the Q15 probability
-	uint8_t* ph;          // [G][cp] high byte
-	unsigned long long* red;   // [8 heads][warps] partials inside the block
-	// what the other blocks of the cluster read (one block = one slice of one kv head's row):
-	int32_t* x_max;       // [8] largest score per head in this slice
-	unsigned long long* x_sum;   // [8] sum of the slice's exponentials per head
-	int32_t* x_ctx;       // [8][HD] this slice's share of P.V per head
-	uint32_t* x_flags;    // [0] the slice met an element the reference refuses, [1] largest folded |ctx| of the
-	                      //     channels this block reduced, [2] this block sits the row out
-	// local copies of what the exchanges fetched (a few threads read the peers, everybody reads these)
-	int32_t* l_max;       // [8] row maximum per head
-	unsigned long long* l_sum;   // [8] row total per head
-	uint32_t* l_misc;     // [0] some block refused the row, [1] largest folded |ctx| of the row
-	int32_t* l_fold;      // [8][3] context fold (identity, multiplier, shift) of this kv head's q heads
+	int64_t* pbase;            // [cp/16] byte offset of each of the row's pages inside a plane
+	int32_t* sc;               // [G][cp] scores, later (shift, remainder) of each element
+	uint8_t* pl;               // [G][cp] low byte of the Q15 probability
+	uint8_t* ph;               // [G][cp] high byte
+	unsigned long long* sum;   // [8] row total per head
+	int32_t* mx;               // [8] row maximum per head
+	int32_t* fold;             // [8][3] context fold (identity, multiplier, shift) of this kv head's q heads
+	uint32_t* refused;
 };
-__host__ __device__ inline size_t attn_smem_bytes(int group, int cp, int hd) {
-	return (size_t)cp / 16 * 8 + (size_t)group * cp * 6 + 8 * kAttnMaxWarps * 8 + 8 * 4 + 8 * 8 + (size_t)8 * hd * 4 + 16 +
-	       8 * 8 + 8 * 4 + 8 + 24 * 4;
+__host__ __device__ inline size_t attn_smem_bytes(int group, int cp) {
+	return (size_t)cp / 16 * 8 + (size_t)group * cp * 6 + 8 * 8 + 8 * 4 + 24 * 4 + 16;
 }
-__device__ __forceinline__ AttnSmem carve(unsigned char* smem, int group, int cp, int hd) {
+__device__ __forceinline__ AttnSmem carve(unsigned char* smem, int group, int cp) {
 	AttnSmem s;
 	s.pbase = (int64_t*)smem;
-	s.sc = (int32_t*)(smem + (size_t)cp / 16 * 8);
+	s.sum = (unsigned long long*)(s.pbase + cp / 16);
+	s.sc = (int32_t*)(s.sum + 8);
 	s.pl = (uint8_t*)(s.sc + (size_t)group * cp);
 	s.ph = s.pl + (size_t)group * cp;
-	s.red = (unsigned long long*)(s.ph + (size_t)group * cp);
-	s.x_sum = s.red + 8 * kAttnMaxWarps;
-	s.x_max = (int32_t*)(s.x_sum + 8);
-	s.x_ctx = s.x_max + 8;
-	s.x_flags = (uint32_t*)(s.x_ctx + 8 * hd);
-	s.l_sum = (unsigned long long*)(s.x_flags + 4);
-	s.l_max = (int32_t*)(s.l_sum + 8);
-	s.l_misc = (uint32_t*)(s.l_max + 8);
-	s.l_fold = (int32_t*)(s.l_misc + 2);
+	s.mx = (int32_t*)(s.ph + (size_t)group * cp);
+	s.fold = s.mx + 8;
+	s.refused = (uint32_t*)(s.fold + 24);
 	return s;
 }
 // ask for the line at p to be brought into L2; nothing waits for it
 __device__ __forceinline__ void prefetch_l2(const void* p) { asm volatile("prefetch.global.L2 [%0];" ::"l"(p)); }
 
-// One attention row = one token of one sequence, all its q heads over the positions 0..pos.
-// The row is cut two ways: by kv head (a block serves the q heads of one GQA group, so K and V
-// bytes are read once per kv head) and along the context width into `splits` slices of
-// `slice_len(width)` positions. The blocks of a row -- kv_heads x splits of them when
-// `whole_row`, else the `splits` of one kv head -- form one thread-block cluster and meet three
-// times through distributed shared memory, which is what the exact integer softmax needs
-// (SoftmaxRowQ15 is not mergeable online: an element's exponential depends on the row maximum
-// through floor divisions):
-//   1  scores of the slice (tensor cores), slice maximum per head      -> exchange: row maximum
-//   2  e_k per element, slice sum per head, refusal flag               -> exchange: row total
-//   3  p_k = (e_k << 15) / total, the slice's share of P.V (tensor cores) -> exchange: the shares
-//      are added per channel (integer adds: any order), then folded per head
-// and, when the cluster holds the whole row, a fourth time for the attention-context funnel
-// (forward_sites.cpp:1898-1903): largest folded magnitude of the row -> codes and carried scale,
-// so that no separate funnel kernel runs. HD = head_dim (32, 64 or 128); threads = 2 * HD.
+// One attention row = one token of one sequence, all its q heads over the positions 0..pos, cut by kv
+// head: a block serves the q heads of one GQA group, so K and V bytes are read once per kv head. Many
+// rows (a decode batch, the rows of a prefill chunk) run this way, a block meeting nobody:
+//   1  scores (tensor cores) and the row maximum per head
+//   2  e_k per element and the row total, then p_k = (e_k << 15) / total
+//   3  P.V (tensor cores), per-head context fold, row maximum for the funnel kernel that follows
+// HD = head_dim (32, 64 or 128); threads = 2 * HD.
 template <int HD>
 __global__ void __launch_bounds__(2 * HD, HD == 128 ? 4 : 8)
-k_attention(RowBatch b, Dims d, const LayerDev* layer, int layer_index, KvPoolDev pool, int cp, int splits, int whole_row,
-            int reverse_rows) {
+k_attention(RowBatch b, Dims d, const LayerDev* layer, int layer_index, KvPoolDev pool, int cp, int reverse_rows) {
 	extern __shared__ __align__(16) unsigned char smem[];
 	// blocks start in index order: with reverse_rows the last (widest) rows of a prefill chunk go first
 	const int r = reverse_rows ? (int)gridDim.y - 1 - (int)blockIdx.y : (int)blockIdx.y;
-	const int kvh = (int)blockIdx.x / splits, split = (int)blockIdx.x % splits;
+	const int kvh = (int)blockIdx.x;
 	constexpr int kAttnThreads = 2 * HD, kAttnWarps = kAttnThreads / 32;
 	const int G = d.heads / d.kv_heads;
 	const int t = threadIdx.x, warp = t >> 5, lane = t & 31;
 	const int g = lane >> 2, c = lane & 3;
-	const AttnSmem s = carve(smem, G, cp, HD);
-	const uint32_t my_rank = cluster_rank();
-	const uint32_t kv_rank0 = my_rank - (uint32_t)split;     // rank of this kv head's first slice
-	const uint32_t cluster_blocks = whole_row ? (uint32_t)(d.kv_heads * splits) : (uint32_t)splits;
+	const AttnSmem s = carve(smem, G, cp);
 	// Ahead of the kernel that lands this step's K / V rows (it may still be running): the row
 	// descriptor and the page table were uploaded before the step's first launch, and every K / V
 	// row but the newest was written by earlier steps. So the page offsets are staged now, and
-	// the slice's old K rows are asked into L2 while that kernel, which moves little data, finishes.
-	const int width = b.rows[r].pos + 1;
-	// slice length: the row's width over the slices, rounded up to whole 64-position groups
-	const int slen = ((width + splits - 1) / splits + 63) & ~63;
-	const int p0 = split * slen;                                   // first position of this slice
-	const int n = max(0, min(slen, width - p0));                   // positions in it
+	// the old K rows are asked into L2 while that kernel, which moves little data, finishes.
+	const int n = b.rows[r].pos + 1;
 	const int n64 = (n + 63) & ~63;
 	const int8_t* kplane = pool.base + kv_plane_offset(d, pool, layer_index, kvh, 0);
 	const int8_t* vplane = pool.base + kv_plane_offset(d, pool, layer_index, kvh, 1);
 	const int npages = (n + kPageTokens - 1) / kPageTokens;
 	{
-		// entries beyond the slice's last page, up to the 64-position group stage 3 reads, repeat
+		// entries beyond the row's last page, up to the 64-position group stage 3 reads, repeat
 		// that page: their probabilities are zero, so any readable V words will do
-		const int32_t* pages = b.rows[r].pages + p0 / kPageTokens;
+		const int32_t* pages = b.rows[r].pages;
 		for (int j = t; j < (n64 >> 4); j += kAttnThreads)
 			s.pbase[j] = (int64_t)pages[min(j, npages - 1)] * (kPageTokens * HD);
 	}
-	const FunnelFold fold_ctx = funnel_prefold(nullptr, 0, layer->c_ctx);
-	if (t < 3 * G) s.l_fold[t] = layer->f_ctx[3 * kvh * G + t];      // (weights: ahead of the wait)
+	if (t < 3 * G) s.fold[t] = layer->f_ctx[3 * kvh * G + t];      // (weights: ahead of the wait)
 	__syncthreads();
 	constexpr int kRowsPerLine = 128 / HD;
-	for (int pos = t * kRowsPerLine; pos < n - (p0 + n == width ? 1 : 0); pos += kAttnThreads * kRowsPerLine)
+	for (int pos = t * kRowsPerLine; pos < n - 1; pos += kAttnThreads * kRowsPerLine)
 		prefetch_l2(kplane + s.pbase[pos >> 4] + (pos & 15) * HD);
 	pdl_wait();
 	pdl_release();
-	// A row that an earlier site refused is sat out: no loads, zero contributions, but every
-	// barrier. One thread reads the word for the block; blocks of a cluster may see different
-	// words (another block can refuse the row while this one runs), which is harmless: a refused
-	// row's outputs are never used.
-	if (t == 0) s.x_flags[2] = __ldcg(&b.status[r]) != 0 ? 1u : 0u;
+	if (t == 0) *s.refused = __ldcg(&b.status[r]) != 0 ? 1u : 0u;
 	if (t < 8) {
-		s.x_max[t] = INT32_MIN;
-		s.x_sum[t] = 0ull;
-		s.l_max[t] = INT32_MIN;
-		s.l_sum[t] = 0ull;
+		s.mx[t] = INT32_MIN;
+		s.sum[t] = 0ull;
 	}
-	if (t == 8) s.x_flags[0] = 0u;
-	if (t == 9) s.x_flags[1] = 0u;
 	const SoftmaxConsts smc = b.smc[(size_t)r * d.kv_heads + kvh];   // wanted after the scores; asked for now
 	__syncthreads();
-	const bool live = s.x_flags[2] == 0u;
-	// A row that is one slice of one kv head has nobody to meet: the block keeps everything local
-	// (and may leave early).
-	const bool solo = splits == 1 && !whole_row;
-	if (solo && !live) return;
+	if (*s.refused != 0u) return;
 
 	// ---- stage 1: scores, 8 positions per MMA group, groups dealt round-robin to the warps, and the
-	// slice's maximum per head on the way. Lanes beyond the slice's end read its last position again
+	// row's maximum per head on the way. Lanes beyond the row's end read its last position again
 	// (no predicated loads); their columns are stored as INT32_MIN, which the maximum ignores.
-	int32_t* const s_max = solo ? s.l_max : s.x_max;
-	unsigned long long* const s_sum = solo ? s.l_sum : s.x_sum;
-	if (live) {
+	{
 		constexpr int NW = HD / 16;
 		uint32_t qw[NW];
 		load_row_words<HD>(b.qrot + (size_t)r * d.hidden + (size_t)(kvh * G + min(g, G - 1)) * HD, c, qw);
@@ -319,26 +271,13 @@ k_attention(RowBatch b, Dims d, const LayerDev* layer, int layer_index, KvPoolDe
 		}
 		rmax = max(rmax, __shfl_xor_sync(0xffffffffu, rmax, 1));
 		rmax = max(rmax, __shfl_xor_sync(0xffffffffu, rmax, 2));
-		if (c == 0 && g < G && rmax != INT32_MIN) atomicMax(&s_max[g], rmax);
+		if (c == 0 && g < G && rmax != INT32_MIN) atomicMax(&s.mx[g], rmax);
 	}
 	__syncthreads();
 
-	// the softmax below moves no data: ask for this slice's V pages (16 lines each) meanwhile
-	if (live)
-		for (int ln = t; ln < npages * (kPageTokens * HD / 128); ln += kAttnThreads)
+	// the softmax below moves no data: ask for the row's V pages (16 lines each) meanwhile
+	for (int ln = t; ln < npages * (kPageTokens * HD / 128); ln += kAttnThreads)
 			prefetch_l2(vplane + s.pbase[ln / (kPageTokens * HD / 128)] + (ln % (kPageTokens * HD / 128)) * 128);
-
-	if (!solo) {
-		cluster_sync_all();      // ---- exchange 1: every slice's maxima are up
-		// (one thread per head fetches the peers' values; reading them from every thread would put
-		// thousands of remote loads on the cluster's shared-memory network)
-		if (t < G) {
-			int m = INT32_MIN;
-			for (int j = 0; j < splits; ++j) m = max(m, (int)peer_ld32(peer_addr(&s.x_max[t], kv_rank0 + (uint32_t)j)));
-			s.l_max[t] = m;
-		}
-		__syncthreads();
-	}
 
 	// ---- stage 2: softmax. The work is dealt to the warps as (head, 128-position chunk) pairs, so
 	// that every warp is busy whatever the width; a lane takes 4 consecutive positions. First the
@@ -346,14 +285,14 @@ k_attention(RowBatch b, Dims d, const LayerDev* layer, int layer_index, KvPoolDe
 	// (shift, remainder), which the probability pass rebuilds it from.
 	const IExpFast fx = iexp_fast_prepare(smc);
 	const int nchunk = (n64 + 127) >> 7;
-	if (live) {
+	{
 #pragma unroll 1
 		for (int pr = warp; pr < G * nchunk; pr += kAttnWarps) {
 			const int h = pr / nchunk, k4 = (pr - h * nchunk) * 128 + lane * 4;
 			unsigned long long tot = 0;
 			if (k4 < n) {
 				int32_t* row = s.sc + (size_t)h * cp;
-				const uint32_t m = (uint32_t)s.l_max[h];
+				const uint32_t m = (uint32_t)s.mx[h];
 				const int4 v = *(const int4*)&row[k4];
 				uint32_t q0, q1, q2, q3;
 				const int64_t e0 = iexp_fast(m - (uint32_t)v.x, fx, &q0);
@@ -373,37 +312,29 @@ k_attention(RowBatch b, Dims d, const LayerDev* layer, int layer_index, KvPoolDe
 			const uint32_t l0 = __reduce_add_sync(0xffffffffu, (uint32_t)tot & 0xFFFFFFu);
 			const uint32_t l1 = __reduce_add_sync(0xffffffffu, (uint32_t)(tot >> 24) & 0xFFFFFFu);
 			const uint32_t l2 = __reduce_add_sync(0xffffffffu, (uint32_t)(tot >> 48));
-			if (lane == 0) atomicAdd(&s_sum[h], (unsigned long long)l0 + ((unsigned long long)l1 << 24) + ((unsigned long long)l2 << 48));
+			if (lane == 0) atomicAdd(&s.sum[h], (unsigned long long)l0 + ((unsigned long long)l1 << 24) + ((unsigned long long)l2 << 48));
 		}
 	}
-	if (solo) {
-		__syncthreads();
-	} else {
-		cluster_sync_all();      // ---- exchange 2: every slice's sums are up
-		if (t < G) {
-			unsigned long long x = 0;
-			for (int j = 0; j < splits; ++j) x += peer_ld64(peer_addr(&s.x_sum[t], kv_rank0 + (uint32_t)j));
-			s.l_sum[t] = x;
-		}
-		__syncthreads();
-	}
-	const bool work = live;
-	// probabilities as two u8 planes, zero beyond the slice up to the next multiple of 64 (stage 3
+	__syncthreads();
+	// probabilities as two u8 planes, zero beyond the row up to the next multiple of 64 (stage 3
 	// reads whole 64-position groups)
-	if (work) {
+	{
 		const int n4 = (n + 3) & ~3;
 #pragma unroll 1
-		for (int pr = warp; pr < G * nchunk; pr += kAttnWarps) {
-			const int h = pr / nchunk, k4 = (pr - h * nchunk) * 128 + lane * 4;
+		for (int task = warp; task < G * nchunk; task += kAttnWarps) {
+			const int h = task / nchunk, k4 = (task - h * nchunk) * 128 + lane * 4;
 			if (k4 < n4) {
-				const unsigned long long x = s.l_sum[h];
-				const unsigned long long tot = x > 1ull ? x : 1ull;
-				const float inv = 32768.0f / (float)tot;
+				const ProbRow pr = prob_row(s.sum[h]);
 				const int4 v = *(const int4*)&s.sc[(size_t)h * cp + k4];
-				const uint32_t p0 = prob_q15(iexp_from_parts((uint32_t)v.x, fx), tot, inv);
-				const uint32_t p1 = prob_q15(iexp_from_parts((uint32_t)v.y, fx), tot, inv);
-				const uint32_t p2 = prob_q15(iexp_from_parts((uint32_t)v.z, fx), tot, inv);
-				const uint32_t p3 = prob_q15(iexp_from_parts((uint32_t)v.w, fx), tot, inv);
+				const int64_t e0 = iexp_from_parts((uint32_t)v.x, fx), e1 = iexp_from_parts((uint32_t)v.y, fx);
+				const int64_t e2 = iexp_from_parts((uint32_t)v.z, fx), e3 = iexp_from_parts((uint32_t)v.w, fx);
+				bool unsure = false;
+				uint32_t p0 = prob_fast(e0, pr, &unsure), p1 = prob_fast(e1, pr, &unsure);
+				uint32_t p2 = prob_fast(e2, pr, &unsure), p3 = prob_fast(e3, pr, &unsure);
+				if (unsure) {
+					const uint2 a = prob_pair_exact(e0, e1, pr.tot), b2 = prob_pair_exact(e2, e3, pr.tot);
+					p0 = a.x; p1 = a.y; p2 = b2.x; p3 = b2.y;
+				}
 				*(uint32_t*)&s.pl[(size_t)h * cp + k4] = pack_plane(p0, p1, p2, p3, 0);
 				*(uint32_t*)&s.ph[(size_t)h * cp + k4] = pack_plane(p0, p1, p2, p3, 1);
 			} else if (k4 < n64) {
@@ -414,7 +345,7 @@ k_attention(RowBatch b, Dims d, const LayerDev* layer, int layer_index, KvPoolDe
 	}
 	__syncthreads();
 
-	// ---- stage 3: the slice's share of ctx = P V. Lane column c owns page 4*grp + c of each
+	// ---- stage 3: ctx = P V. Lane column c owns page 4*grp + c of each
 	// 64-position group; its 16-byte row of the transposed page feeds two MMAs (positions 0..7 and
 	// 8..15). Nothing is predicated: the page table and the planes are padded to whole groups, and
 	// lanes of MMA rows beyond the group's heads read head 0's probabilities (their output rows are
@@ -425,7 +356,7 @@ k_attention(RowBatch b, Dims d, const LayerDev* layer, int layer_index, KvPoolDe
 	for (int i = 0; i < NDB; ++i)
 #pragma unroll
 		for (int j = 0; j < 4; ++j) accl[i][j] = acch[i][j] = 0;
-	if (work) {
+	{
 		const int ngrp = n64 >> 6;
 		const uint8_t* pl = s.pl + (size_t)(g < G ? g : 0) * cp + c * kPageTokens;
 		const uint8_t* ph = s.ph + (size_t)(g < G ? g : 0) * cp + c * kPageTokens;
@@ -464,12 +395,12 @@ k_attention(RowBatch b, Dims d, const LayerDev* layer, int layer_index, KvPoolDe
 			group(grp0, vv);
 		}
 	}
-	if (solo) {
+	{
 		// per-head context fold (forward_sites.cpp:1889-1896), store, row maximum for the funnel
 		uint32_t smax = 0;
 		if (g < G) {
 			const int head = kvh * G + g;
-			const int32_t fi = s.l_fold[3 * g], fm = s.l_fold[3 * g + 1], fs = s.l_fold[3 * g + 2];
+			const int32_t fi = s.fold[3 * g], fm = s.fold[3 * g + 1], fs = s.fold[3 * g + 2];
 #pragma unroll
 			for (int i = 0; i < NDB; ++i) {
 				int2 o;
@@ -485,75 +416,354 @@ k_attention(RowBatch b, Dims d, const LayerDev* layer, int layer_index, KvPoolDe
 #pragma unroll
 		for (int o = 16; o > 0; o >>= 1) smax = max(smax, __shfl_xor_sync(0xffffffffu, smax, o));
 		if (lane == 0 && smax) atomicMax(&b.rowmax[(size_t)r * 4 + 3], (unsigned long long)smax);
-		return;
 	}
-	// the slice's share, [head][channel], for the block that reduces that channel
+}
+
+// ---------------------------------------------------------------- few rows: slices over a cluster
+// While rows are few (a handful of conversations decoding), the time of an attention row is one
+// block's chain of dependent steps, so the row is cut along its width into slices, one block each; the
+// blocks of a row -- all its kv heads when `whole_row`, else those of one kv head -- form a cluster and
+// exchange maxima, sums, shares of P.V and, with the whole row, the funnel's maximum (forward_sites.cpp:
+// 1898-1903; no separate funnel kernel then). The exact integer softmax needs all of these to be exact:
+// an element's exponential depends on the row maximum through floor divisions.
+//
+// The K / V rows of earlier calls are in place, so with STAGED a block copies those of its slice into
+// shared memory (cp.async) ahead of the dependency wait, while the row kernel in front runs; behind the
+// wait it fetches only what this call lands: a decode row's own position, a chunk's positions. One row of 2,011 positions, 1.5B widths:
+// 13.9 us with four slices per kv head read through L2 and cluster barriers around every exchange.
+template <int HD>
+struct FewSmem {
+	static constexpr int kKStride = HD == 128 ? HD + 16 : HD;      // bytes per staged K row (bank conflicts)
+	static constexpr int kVStride = HD * kPageTokens + 32;         // bytes per staged V page
+	int64_t* pbase;            // [cp / 16] byte offset of each of the block's pages inside a plane
+	int32_t* sc;               // [G][cp] scores, later (shift, remainder) of each element
+	uint8_t *pl, *ph;          // [G][cp] low / high byte of the Q15 probability
+	unsigned long long* sum;   // [8] this slice's sums
+	unsigned long long* rx_sum;      // [16][8] every slice's
+	int32_t *rx_max;           // [16][8]
+	int32_t* rx_ctx;           // [splits][G * HD / splits] shares of the channels this block reduces
+	uint32_t* rx_top;          // [16] every block's largest folded magnitude
+	int32_t* mx;               // [8] this slice's maxima
+	int32_t* fold;             // [8][3]
+	uint32_t* misc;            // [0] this block's largest folded magnitude, [1] refused
+	int8_t *ks, *vs;           // staged K rows and V pages
+	__host__ __device__ static size_t fixed_bytes() { return 8 * 8 + 16 * 8 * 8 + 16 * 8 * 4 + (size_t)8 * HD * 4 + 16 * 4 + 8 * 4 + 24 * 4 + 4 * 4; }
+	__host__ __device__ static size_t bytes(int group, int cp, bool staged) {
+		return (size_t)cp / 16 * 8 + (size_t)group * cp * 6 + fixed_bytes() + (staged ? (size_t)cp * kKStride + (size_t)cp / 16 * kVStride + 32 : 0);
+	}
+	__device__ static FewSmem carve(unsigned char* p, int group, int cp) {
+		FewSmem s;
+		s.pbase = (int64_t*)p;
+		s.sum = (unsigned long long*)(s.pbase + cp / 16);
+		s.rx_sum = s.sum + 8;
+		s.sc = (int32_t*)(s.rx_sum + 128);
+		s.pl = (uint8_t*)(s.sc + (size_t)group * cp);
+		s.ph = s.pl + (size_t)group * cp;
+		s.rx_ctx = (int32_t*)(s.ph + (size_t)group * cp);
+		s.rx_max = s.rx_ctx + 8 * HD;
+		s.rx_top = (uint32_t*)(s.rx_max + 128);
+		s.mx = (int32_t*)(s.rx_top + 16);
+		s.fold = s.mx + 8;
+		s.misc = (uint32_t*)(s.fold + 24);
+		s.ks = (int8_t*)(((uintptr_t)(s.misc + 4) + 15) & ~(uintptr_t)15);
+		s.vs = s.ks + (size_t)cp * kKStride;
+		return s;
+	}
+};
+__device__ __forceinline__ void cp_async16(void* dst, const void* src) {
+	asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"((uint32_t)__cvta_generic_to_shared(dst)), "l"(src) : "memory");
+}
+// the words of load_row_words from a staged K row (plain shared-memory loads)
+template <int HD>
+__device__ __forceinline__ void shared_row_words(const int8_t* row, int c, uint32_t (&w)[HD / 16]) {
+	if constexpr (HD == 32) {
+		const int2 x = *(const int2*)(row + c * 8);
+		w[0] = (uint32_t)x.x; w[1] = (uint32_t)x.y;
+	} else {
+#pragma unroll
+		for (int h = 0; h < HD / 64; ++h) {
+			const int4 x = *(const int4*)(row + c * (HD / 4) + 16 * h);
+			w[4 * h] = (uint32_t)x.x; w[4 * h + 1] = (uint32_t)x.y; w[4 * h + 2] = (uint32_t)x.z; w[4 * h + 3] = (uint32_t)x.w;
+		}
+	}
+}
+
+template <int HD, bool STAGED>
+__global__ void __launch_bounds__(2 * HD)
+k_attention_few(RowBatch b, Dims d, const LayerDev* layer, Scale c_ctx, int layer_index, KvPoolDev pool, int cp, int splits,
+                int whole_row, int chunk) {
+	using S = FewSmem<HD>;
+	extern __shared__ __align__(16) unsigned char smem[];
+	__shared__ __align__(8) unsigned long long s_bars[4];
+	constexpr int kThreads = 2 * HD, kWarps = kThreads / 32, NW = HD / 16;
+	const int r = (int)blockIdx.y, kvh = (int)blockIdx.x / splits, split = (int)blockIdx.x % splits;
+	const int G = d.heads / d.kv_heads;
+	const int t = threadIdx.x, warp = t >> 5, lane = t & 31, g = lane >> 2, c = lane & 3;
+	const S s = S::carve(smem, G, cp);
+	const uint32_t my_rank = cluster_rank(), kv_rank0 = my_rank - (uint32_t)split;      // rank of this kv head's first slice
+	const uint32_t cluster_blocks = whole_row ? (uint32_t)(d.kv_heads * splits) : (uint32_t)splits;
+	const int per = HD / splits, ch0 = split * per;                  // channels this block reduces
+	auto bar = [&](int i) { return cta_addr(&s_bars[i]); };
+	if (t == 0) {
+		exchange_init(bar(0), (uint32_t)(splits * G * 4));
+		exchange_init(bar(1), (uint32_t)(splits * G * 8));
+		exchange_init(bar(2), (uint32_t)(G * HD * 4));
+		exchange_init(bar(3), 4u * cluster_blocks);
+		exchange_fence_init();
+	}
+	// ahead of the kernel that lands this step's K / V rows: the page table, the old rows
+	const int width = b.rows[r].pos + 1;
+	const int slen = ((width + splits - 1) / splits + 63) & ~63;
+	const int p0 = split * slen;                                   // first position of this slice
+	const int n = max(0, min(slen, width - p0));                   // positions in it
+	const int n64 = (n + 63) & ~63, npages = (n + kPageTokens - 1) / kPageTokens;
+	// positions of the slice that were there before this call (the rows of a chunk are consecutive positions)
+	const int old = max(0, min(n, (chunk ? b.rows[0].pos : width - 1) - p0)), old_pages = old / kPageTokens;
+	const int8_t* kplane = pool.base + kv_plane_offset(d, pool, layer_index, kvh, 0);
+	const int8_t* vplane = pool.base + kv_plane_offset(d, pool, layer_index, kvh, 1);
+	{
+		// entries beyond the slice's last page repeat it: their probabilities are zero, any V words will do
+		const int32_t* pages = b.rows[r].pages + p0 / kPageTokens;
+		for (int j = t; j < (n64 >> 4); j += kThreads) s.pbase[j] = (int64_t)pages[min(j, npages - 1)] * (kPageTokens * HD);
+	}
+	if (t < 3 * G) s.fold[t] = layer->f_ctx[3 * kvh * G + t];
+	if (t < 8) {
+		s.mx[t] = INT32_MIN;
+		s.sum[t] = 0ull;
+	}
+	if (t == 8) s.misc[0] = 0u;
+	const FunnelFold fold_ctx = funnel_prefold(nullptr, 0, c_ctx);
+	__syncthreads();
+	auto stage_k = [&](int from, int to) {
+		for (int i = from * (HD / 16) + t; i < to * (HD / 16); i += kThreads) {
+			const int pos = i / (HD / 16), piece = i % (HD / 16);
+			cp_async16(s.ks + (size_t)pos * S::kKStride + piece * 16, kplane + s.pbase[pos >> 4] + (pos & 15) * HD + piece * 16);
+		}
+	};
+	auto stage_v = [&](int from, int to) {      // pages
+		for (int i = from * HD + t; i < to * HD; i += kThreads) {
+			const int pg = i / HD, piece = i % HD;
+			cp_async16(s.vs + (size_t)pg * S::kVStride + piece * 16, vplane + s.pbase[pg] + piece * 16);
+		}
+	};
+	if (STAGED) {
+		stage_k(0, old);
+		stage_v(0, old_pages);
+		// (pages between the slice's end and the next group of four are read against zero probabilities)
+		for (int i = npages * HD + t; i < (n64 >> 4) * HD; i += kThreads)
+			*(int4*)(s.vs + (size_t)(i / HD) * S::kVStride + (i % HD) * 16) = make_int4(0, 0, 0, 0);
+	} else {
+		constexpr int kRowsPerLine = 128 / HD;
+		for (int pos = t * kRowsPerLine; pos < old; pos += kThreads * kRowsPerLine)
+			prefetch_l2(kplane + s.pbase[pos >> 4] + (pos & 15) * HD);
+	}
+	cluster_arrive();
+	cluster_wait();
+	pdl_wait();
+	pdl_release();
+	// A row that an earlier site refused is sat out: zero contributions, but every exchange. (Only this
+	// kernel's last step can refuse the row, when every block has long read the word.)
+	const bool live = __ldcg(&b.status[r]) == 0;
+	const IExpFast fx = iexp_fast_prepare(b.smc[(size_t)r * d.kv_heads + kvh]);
+	uint32_t qw[NW];
+	load_row_words<HD>(b.qrot + (size_t)r * d.hidden + (size_t)(kvh * G + min(g, G - 1)) * HD, c, qw);
+	if (STAGED) {
+		stage_k(old, n);
+		stage_v(old_pages, npages);
+		asm volatile("cp.async.wait_all;" ::: "memory");
+		__syncthreads();
+	}
+
+	// ---- stage 1: scores, 8 positions per MMA group, groups dealt round-robin to the warps; lanes beyond
+	// the slice's end read its last position again, their columns are stored as INT32_MIN
+	if (live && n > 0) {
+		const int nblk = (n + 7) >> 3;
+		constexpr int U = 4;
+		int rmax = INT32_MIN;
+#pragma unroll 1
+		for (int blk0 = warp * U; blk0 < nblk; blk0 += kWarps * U) {
+			uint32_t kw[U][NW];
+#pragma unroll
+			for (int u = 0; u < U; ++u) {
+				const int pos = min((blk0 + u) * 8 + g, n - 1);
+				if (STAGED) shared_row_words<HD>(s.ks + (size_t)pos * S::kKStride, c, kw[u]);
+				else load_row_words<HD>(kplane + s.pbase[pos >> 4] + (pos & 15) * HD, c, kw[u]);
+			}
+#pragma unroll
+			for (int u = 0; u < U; ++u) {
+				int acc[4] = {0, 0, 0, 0};
+#pragma unroll
+				for (int j = 0; j < NW / 2; ++j) mma_s8s8(acc, qw[2 * j], qw[2 * j + 1], kw[u][2 * j], kw[u][2 * j + 1]);
+				const int k = (blk0 + u) * 8 + c * 2;
+				if (g < G && blk0 + u < nblk) {
+					const int v0 = k < n ? acc[0] : INT32_MIN, v1 = k + 1 < n ? acc[1] : INT32_MIN;
+					*(int2*)&s.sc[(size_t)g * cp + k] = make_int2(v0, v1);
+					rmax = max(rmax, max(v0, v1));
+				}
+			}
+		}
+		rmax = max(rmax, __shfl_xor_sync(0xffffffffu, rmax, 1));
+		rmax = max(rmax, __shfl_xor_sync(0xffffffffu, rmax, 2));
+		if (c == 0 && g < G && rmax != INT32_MIN) atomicMax(&s.mx[g], rmax);
+	}
+	if (!STAGED && live)      // the softmax below moves no data: ask for this slice's V pages meanwhile
+		for (int ln = t; ln < npages * (kPageTokens * HD / 128); ln += kThreads)
+			prefetch_l2(vplane + s.pbase[ln / (kPageTokens * HD / 128)] + (ln % (kPageTokens * HD / 128)) * 128);
+	__syncthreads();
+	// ---- exchange 1: every slice's maxima
+	for (int i = t; i < splits * G; i += kThreads) exchange_send(&s.rx_max[split * 8 + i % G], bar(0), kv_rank0 + (uint32_t)(i / G), (uint32_t)s.mx[i % G]);
+	bool ok = exchange_wait(bar(0));
+
+	// ---- stage 2: softmax, (head, 128-position chunk) pairs dealt to the warps, a lane takes 4 consecutive
+	// positions: exponentials and their sums, the score's place then holds the element's (shift, remainder)
+	const int nchunk = (n64 + 127) >> 7;
+	if (live) {
+#pragma unroll 1
+		for (int task = warp; task < G * nchunk; task += kWarps) {
+			const int h = task / nchunk, k4 = (task - h * nchunk) * 128 + lane * 4;
+			unsigned long long tot = 0;
+			if (k4 < n) {
+				int m = s.rx_max[h];
+				for (int j = 1; j < splits; ++j) m = max(m, s.rx_max[j * 8 + h]);
+				int32_t* row = s.sc + (size_t)h * cp;
+				const int4 v = *(const int4*)&row[k4];
+				uint32_t q0, q1, q2, q3;
+				const int64_t e0 = iexp_fast((uint32_t)m - (uint32_t)v.x, fx, &q0);
+				int64_t e1 = iexp_fast((uint32_t)m - (uint32_t)v.y, fx, &q1);
+				int64_t e2 = iexp_fast((uint32_t)m - (uint32_t)v.z, fx, &q2);
+				int64_t e3 = iexp_fast((uint32_t)m - (uint32_t)v.w, fx, &q3);
+				if (k4 + 3 >= n) {       // the slice's last group: positions beyond its end count for nothing
+					if (k4 + 1 >= n) { e1 = 0; q1 = kPartsOfZero; }
+					if (k4 + 2 >= n) { e2 = 0; q2 = kPartsOfZero; }
+					e3 = 0; q3 = kPartsOfZero;
+				}
+				tot = (unsigned long long)(e0 + e1) + (unsigned long long)(e2 + e3);
+				*(int4*)&row[k4] = make_int4((int)q0, (int)q1, (int)q2, (int)q3);
+			}
+			// a lane's partial is below 2^50: three 24-bit limbs add up across the warp inside 32 bits
+			const uint32_t l0 = __reduce_add_sync(0xffffffffu, (uint32_t)tot & 0xFFFFFFu);
+			const uint32_t l1 = __reduce_add_sync(0xffffffffu, (uint32_t)(tot >> 24) & 0xFFFFFFu);
+			const uint32_t l2 = __reduce_add_sync(0xffffffffu, (uint32_t)(tot >> 48));
+			if (lane == 0) atomicAdd(&s.sum[h], (unsigned long long)l0 + ((unsigned long long)l1 << 24) + ((unsigned long long)l2 << 48));
+		}
+	}
+	__syncthreads();
+	// ---- exchange 2: every slice's sums
+	for (int i = t; i < splits * G; i += kThreads) exchange_send(&s.rx_sum[split * 8 + i % G], bar(1), kv_rank0 + (uint32_t)(i / G), s.sum[i % G]);
+	ok = exchange_wait(bar(1)) && ok;
+	// probabilities as two u8 planes, zero beyond the slice up to the next multiple of 64
+	if (live) {
+		const int n4 = (n + 3) & ~3;
+#pragma unroll 1
+		for (int task = warp; task < G * nchunk; task += kWarps) {
+			const int h = task / nchunk, k4 = (task - h * nchunk) * 128 + lane * 4;
+			if (k4 < n4) {
+				unsigned long long total = s.rx_sum[h];
+				for (int j = 1; j < splits; ++j) total += s.rx_sum[j * 8 + h];
+				const ProbRow pr = prob_row(total);
+				const int4 v = *(const int4*)&s.sc[(size_t)h * cp + k4];
+				const int64_t e0 = iexp_from_parts((uint32_t)v.x, fx), e1 = iexp_from_parts((uint32_t)v.y, fx);
+				const int64_t e2 = iexp_from_parts((uint32_t)v.z, fx), e3 = iexp_from_parts((uint32_t)v.w, fx);
+				bool unsure = false;
+				uint32_t q0 = prob_fast(e0, pr, &unsure), q1 = prob_fast(e1, pr, &unsure);
+				uint32_t q2 = prob_fast(e2, pr, &unsure), q3 = prob_fast(e3, pr, &unsure);
+				if (unsure) {
+					const uint2 a = prob_pair_exact(e0, e1, pr.tot), a2 = prob_pair_exact(e2, e3, pr.tot);
+					q0 = a.x; q1 = a.y; q2 = a2.x; q3 = a2.y;
+				}
+				*(uint32_t*)&s.pl[(size_t)h * cp + k4] = pack_plane(q0, q1, q2, q3, 0);
+				*(uint32_t*)&s.ph[(size_t)h * cp + k4] = pack_plane(q0, q1, q2, q3, 1);
+			} else if (k4 < n64) {
+				*(uint32_t*)&s.pl[(size_t)h * cp + k4] = 0u;
+				*(uint32_t*)&s.ph[(size_t)h * cp + k4] = 0u;
+			}
+		}
+	}
+	__syncthreads();
+
+	// ---- stage 3: the slice's share of ctx = P V. Lane column c owns page 4 grp + c of each 64-position
+	// group; its 16-byte row of the transposed page feeds two MMAs
+	constexpr int NDB = 2;            // 8-channel blocks per warp
+	int accl[NDB][4], acch[NDB][4];
+#pragma unroll
+	for (int i = 0; i < NDB; ++i)
+#pragma unroll
+		for (int j = 0; j < 4; ++j) accl[i][j] = acch[i][j] = 0;
+	if (live) {
+		const int ngrp = n64 >> 6;
+		const uint8_t* pl = s.pl + (size_t)(g < G ? g : 0) * cp + c * kPageTokens;
+		const uint8_t* ph = s.ph + (size_t)(g < G ? g : 0) * cp + c * kPageTokens;
+		const int chan = (warp * NDB * 8 + g) * kPageTokens;
+#pragma unroll 4
+		for (int grp = 0; grp < ngrp; ++grp) {
+			const int4 al = *(const int4*)(pl + grp * 64), ah = *(const int4*)(ph + grp * 64);
+			const int8_t* vp = STAGED ? s.vs + (size_t)(grp * 4 + c) * S::kVStride + chan : vplane + s.pbase[grp * 4 + c] + chan;
+#pragma unroll
+			for (int i = 0; i < NDB; ++i) {
+				const int4 v = *(const int4*)(vp + i * 8 * kPageTokens);
+				mma_u8s8(accl[i], (uint32_t)al.x, (uint32_t)al.y, (uint32_t)v.x, (uint32_t)v.y);
+				mma_u8s8(accl[i], (uint32_t)al.z, (uint32_t)al.w, (uint32_t)v.z, (uint32_t)v.w);
+				mma_u8s8(acch[i], (uint32_t)ah.x, (uint32_t)ah.y, (uint32_t)v.x, (uint32_t)v.y);
+				mma_u8s8(acch[i], (uint32_t)ah.z, (uint32_t)ah.w, (uint32_t)v.z, (uint32_t)v.w);
+			}
+		}
+	}
+	// ---- exchange 3: each share goes to the slice that reduces its channels
 	if (g < G) {
 #pragma unroll
 		for (int i = 0; i < NDB; ++i) {
 			const int ch = (warp * NDB + i) * 8 + c * 2;
-			*(int2*)&s.x_ctx[g * HD + ch] = make_int2(accl[i][0] + 256 * acch[i][0], accl[i][1] + 256 * acch[i][1]);
+			exchange_send(&s.rx_ctx[(split * G + g) * per + ch % per], bar(2), kv_rank0 + (uint32_t)(ch / per),
+			              make_int2(accl[i][0] + 256 * acch[i][0], accl[i][1] + 256 * acch[i][1]));
 		}
 	}
-	cluster_sync_all();      // ---- exchange 3: every slice's share of P.V is up
-
-	// Slice `split` of a kv head reduces channels [split * HD / splits, ...) of each of its heads:
-	// add the shares, per-head context fold (forward_sites.cpp:1889-1896), row maximum.
-	const int per = (HD + splits - 1) / splits;                    // channels per block
-	const int ch0 = split * per, nch = max(0, min(per, HD - ch0));
-	// element e of this block = (head e / nch, channel ch0 + e % nch); at most G * HD <= 2 * threads * ... per block
-	uint32_t lmax = 0;
-	constexpr int kMaxMine = 4;                                   // G * per <= 8 * HD = 4 * threads
+	ok = exchange_wait(bar(2)) && ok;
+	// add the shares, per-head context fold (forward_sites.cpp:1889-1896), row maximum
+	uint32_t top = 0;
+	constexpr int kMaxMine = 4;                                   // G * per <= 8 HD = 4 threads' worth
 	int32_t mine[kMaxMine];
 #pragma unroll
 	for (int q = 0; q < kMaxMine; ++q) {
 		mine[q] = 0;
-		const int e = q * kAttnThreads + t;
-		if (e < G * nch) {
-			const int h = e / nch, ch = ch0 + e - h * nch;
+		const int e = q * kThreads + t;
+		if (e < G * per) {
+			const int h = e / per, ch = ch0 + e - h * per;
 			int32_t sum = 0;
-			for (int j = 0; j < splits; ++j) sum += (int32_t)peer_ld32(peer_addr(&s.x_ctx[h * HD + ch], kv_rank0 + (uint32_t)j));
-			const int32_t o = fold(sum, s.l_fold[3 * h], s.l_fold[3 * h + 1], s.l_fold[3 * h + 2]);
+			for (int j = 0; j < splits; ++j) sum += s.rx_ctx[j * G * per + e];
+			const int32_t o = fold(sum, s.fold[3 * h], s.fold[3 * h + 1], s.fold[3 * h + 2]);
 			mine[q] = o;
-			lmax = max(lmax, o < 0 ? 0u - (uint32_t)o : (uint32_t)o);
-			if (!whole_row && work) b.ctxw[(size_t)r * d.hidden + (size_t)(kvh * G + h) * HD + ch] = o;
+			top = max(top, o < 0 ? 0u - (uint32_t)o : (uint32_t)o);
+			if (!whole_row && live) b.ctxw[(size_t)r * d.hidden + (size_t)(kvh * G + h) * HD + ch] = o;
 		}
 	}
-#pragma unroll
-	for (int o = 16; o > 0; o >>= 1) lmax = max(lmax, __shfl_xor_sync(0xffffffffu, lmax, o));
+	top = __reduce_max_sync(0xffffffffu, top);
+	if (!ok && t == 0) atomicCAS(&b.status[r], 0, pack_status(kInternalWaitTimeout, kSiteCtx, b.layer));
 	if (!whole_row) {
-		if (lane == 0 && lmax && work) atomicMax(&b.rowmax[(size_t)r * 4 + 3], (unsigned long long)lmax);
-		cluster_sync_all();  // nobody leaves while its shared memory may still be read
+		if (lane == 0 && top && live) atomicMax(&b.rowmax[(size_t)r * 4 + 3], (unsigned long long)top);
 		return;
 	}
-	// ---- the cluster holds the whole row: its funnel runs here
-	if (lane == 0 && lmax) atomicMax(&s.x_flags[1], lmax);
-	cluster_sync_all();      // ---- exchange 4: every block's largest folded magnitude is up
-	if (t == 0) {
-		uint32_t v = 0;
-		for (uint32_t j = 0; j < cluster_blocks; ++j) v = max(v, peer_ld32(peer_addr(&s.x_flags[1], j)));
-		s.l_misc[1] = v;
-	}
+	// ---- exchange 4: the cluster holds the whole row, its funnel runs here
+	if (lane == 0 && top) atomicMax(&s.misc[0], top);
 	__syncthreads();
-	const uint32_t rowmx = s.l_misc[1];
-	const FunnelParams fp = funnel_finish((unsigned long long)rowmx, fold_ctx);
-	if (work) {
-		if (fp.status != kOk) {
-			if (my_rank == 0 && t == 0) atomicCAS(&b.status[r], 0, pack_status(fp.status, kSiteCtx, b.layer));
-		} else {
-			const Coder cd = make_coder(fp.r, fp.s);
+	if (t < (int)cluster_blocks) exchange_send(&s.rx_top[my_rank], bar(3), (uint32_t)t, s.misc[0]);
+	ok = exchange_wait(bar(3)) && ok;
+	if (!live || !ok) return;
+	for (uint32_t j = 0; j < cluster_blocks; ++j) top = max(top, s.rx_top[j]);
+	const QuadFunnel fp = quad_funnel((unsigned long long)top, fold_ctx);
+	if (fp.status != kOk) {
+		if (my_rank == 0 && t == 0) atomicCAS(&b.status[r], 0, pack_status(fp.status, kSiteCtx, b.layer));
+		return;
+	}
+	const uint32_t codes = code_quad(mine, fp);
 #pragma unroll
-			for (int q = 0; q < kMaxMine; ++q) {
-				const int e = q * kAttnThreads + t;
-				if (e < G * nch) {
-					const int h = e / nch, ch = ch0 + e - h * nch;
-					b.ctx[(size_t)r * d.hidden + (size_t)(kvh * G + h) * HD + ch] = code_of(mine[q], cd);
-				}
-			}
-			if (my_rank == 0 && t == 0) b.cs[r] = fp.out;
+	for (int q = 0; q < kMaxMine; ++q) {
+		const int e = q * kThreads + t;
+		if (e < G * per) {
+			const int h = e / per, ch = ch0 + e - h * per;
+			b.ctx[(size_t)r * d.hidden + (size_t)(kvh * G + h) * HD + ch] = (int8_t)byte_of(codes, q);
 		}
 	}
-	cluster_sync_all();      // nobody leaves while its shared memory may still be read
+	if (my_rank == 0 && t == 0) b.cs[r] = fp.out;
 }
 
 // ------------------------------------------------------------ prefill: query-tiled attention
@@ -587,9 +797,6 @@ __device__ __forceinline__ void mma_u8s8_full(int (&c)[4], uint32_t a0, uint32_t
 	    "mma.sync.aligned.m16n8k32.row.col.s32.u8.s8.s32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%0,%1,%2,%3};"
 	    : "+r"(c[0]), "+r"(c[1]), "+r"(c[2]), "+r"(c[3])
 	    : "r"(a0), "r"(a1), "r"(a2), "r"(a3), "r"(b0), "r"(b1));
-}
-__device__ __forceinline__ void cp_async16(void* dst, const void* src) {
-	asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"((uint32_t)__cvta_generic_to_shared(dst)), "l"(src) : "memory");
 }
 
 template <int HD>
@@ -778,8 +985,7 @@ k_attention_tile(RowBatch b, Dims d, const LayerDev* layer, int layer_index, KvP
 	__syncthreads();
 	sum_a = wsum[rho_a] + wsum[kTileRows + rho_a];
 	sum_b = wsum[rho_b] + wsum[kTileRows + rho_b];
-	const unsigned long long tot_a = sum_a > 1ull ? sum_a : 1ull, tot_b = sum_b > 1ull ? sum_b : 1ull;
-	const float inv_a = 32768.0f / (float)tot_a, inv_b = 32768.0f / (float)tot_b;
+	const ProbRow pr_a = prob_row(sum_a), pr_b = prob_row(sum_b);
 	const bool go_a = in_a, go_b = in_b;
 
 	// ---- walk 3: probabilities and P.V
@@ -796,13 +1002,25 @@ k_attention_tile(RowBatch b, Dims d, const LayerDev* layer, int layer_index, KvP
 			const int col = 32 * ph + 8 * j + 2 * c;
 			const int k0 = blk * kTileKeys + col;
 			uint32_t pa[2], pb[2];
+			int64_t ea[2], eb[2];
+			bool unsure = false;
 #pragma unroll
 			for (int q = 0; q < 2; ++q) {
 				uint32_t parts;
-				const uint32_t va = prob_q15(iexp_fast((uint32_t)mx_a - (uint32_t)acc[j][q], fa, &parts), tot_a, inv_a);
-				const uint32_t vb = prob_q15(iexp_fast((uint32_t)mx_b - (uint32_t)acc[j][2 + q], fb, &parts), tot_b, inv_b);
-				pa[q] = k0 + q <= lim_a ? va : 0u;
-				pb[q] = k0 + q <= lim_b ? vb : 0u;
+				ea[q] = iexp_fast((uint32_t)mx_a - (uint32_t)acc[j][q], fa, &parts);
+				eb[q] = iexp_fast((uint32_t)mx_b - (uint32_t)acc[j][2 + q], fb, &parts);
+				// (an element beyond its row's limit may exceed the row's total: it is dropped below, whatever it gives)
+				pa[q] = prob_fast(ea[q], pr_a, &unsure);
+				pb[q] = prob_fast(eb[q], pr_b, &unsure);
+			}
+			if (unsure) {
+				const uint2 xa = prob_pair_exact(ea[0], ea[1], pr_a.tot), xb = prob_pair_exact(eb[0], eb[1], pr_b.tot);
+				pa[0] = xa.x; pa[1] = xa.y; pb[0] = xb.x; pb[1] = xb.y;
+			}
+#pragma unroll
+			for (int q = 0; q < 2; ++q) {
+				pa[q] = k0 + q <= lim_a ? pa[q] & 0xFFFFu : 0u;
+				pb[q] = k0 + q <= lim_b ? pb[q] & 0xFFFFu : 0u;
 			}
 			*(uint16_t*)(Pl + (size_t)rho_a * kTilePStride + col) = (uint16_t)((pa[0] & 0xffu) | ((pa[1] & 0xffu) << 8));
 			*(uint16_t*)(Ph + (size_t)rho_a * kTilePStride + col) = (uint16_t)((pa[0] >> 8) | ((pa[1] >> 8) << 8));
@@ -874,17 +1092,15 @@ static int pad64(int w) { return (w + 63) / 64 * 64; }
 constexpr int kAttnMaxSlice = 2048;      // positions one block holds at most
 
 struct AttnPlan {
-	int splits;       // slices along the width
+	int splits;       // slices along the width (k_attention_few), or 0: whole rows (k_attention)
 	int whole_row;    // the cluster spans every kv head of the row (the funnel is fused)
 	int cp;           // positions per block (shared-memory capacity)
 };
-// How a launch over `m` rows of up to `max_width` positions is cut. A cluster has at most 8
-// blocks (the portable size), 16 only when a row is too wide for 8 slices; a row's funnel is
-// fused when all its kv heads fit into the cluster beside the slices.
+// How a launch over `m` rows of up to `max_width` positions is cut.
 static std::atomic<int> g_forced_splits{-1};     // -1: not set yet (the environment decides), 0: automatic
 void attn_force_splits(int splits) { g_forced_splits.store(splits < 0 ? 0 : splits); }
 
-static AttnPlan attn_plan(const Dims& d, int m, int max_width, bool one_sequence) {
+static AttnPlan attn_plan(const Dims& d, int m, int max_width) {
 	AttnPlan p;
 	int forced = g_forced_splits.load();
 	if (forced < 0) {      // SSLM_B200_ATTN_SPLITS=n fixes the slices per kv head (tuning, tests)
@@ -892,42 +1108,47 @@ static AttnPlan attn_plan(const Dims& d, int m, int max_width, bool one_sequence
 		forced = e ? atoi(e) : 0;
 		g_forced_splits.store(forced < 0 ? 0 : forced);
 	}
-	const int per_kv_max = d.kv_heads <= 8 ? 8 / d.kv_heads : 1;   // slices per kv head with the whole row in one cluster
+	// Clusters of 16 blocks need a GPC to themselves and there are eight: up to six rows get one each.
+	// Otherwise a cluster has at most 8 blocks (the portable size).
+	const int cluster_max = m <= 6 ? 16 : 8;
+	const int per_kv_max = d.kv_heads <= cluster_max ? cluster_max / d.kv_heads : 1;   // slices with the whole row in one cluster
 	int splits = 1;
 	if (forced > 0) {
 		while (splits * 2 <= forced && splits * 2 <= 16) splits *= 2;
 	} else {
-		// A block's time is mostly a fixed chain of dependent steps, and blocks of a cluster wait
-		// for one another at every exchange, so cutting rows into slices pays only when the rows
-		// are so few that most multiprocessors would otherwise idle (a single long sequence): then
-		// the width is cut until the blocks fill a fifth of the machine. Otherwise a row is one
-		// slice per kv head, unclustered, and the funnel kernel follows.
+		// A slice shortens every stage of a block's chain and four exchanges cost under a microsecond, so
+		// rows are cut while all blocks still run at once.
+		static const int lim = [] { const char* e = getenv("SSLM_ATTN_LIM"); return e ? atoi(e) : 100; }();
 		const int blocks = m * d.kv_heads;
-		int want = 1;
-		while (want < 8 && blocks * want * 2 <= sm_count() / 5) want *= 2;
-		while (splits * 2 <= want && splits * 2 <= 8) splits *= 2;
-		if (splits > per_kv_max) splits = per_kv_max;              // prefer the fused funnel ...
+		while (splits < 8 && blocks * splits * 2 * 100 <= sm_count() * lim) splits *= 2;
+		if (splits > per_kv_max) splits = per_kv_max;              // prefer the fused funnel
 	}
 	while (splits > 1 && splits * 64 > pad64(max_width)) splits /= 2;
 	// ... unless the width does not fit the slices: then up to 16 slices of one kv head per cluster
 	while (splits < 16 && pad64((max_width + splits - 1) / splits) > kAttnMaxSlice) splits *= 2;
 	p.whole_row = splits <= per_kv_max ? 1 : 0;
-	// The rows of a prefill chunk are many and of very different widths: blocks that wait for one
-	// another at cluster barriers cost more there than the separate funnel kernel does.
-	if (forced <= 0 && splits == 1) p.whole_row = 0;
 	p.splits = splits;
 	p.cp = pad64((max_width + splits - 1) / splits);
+	if (forced <= 0 && splits == 1 && m * d.kv_heads > sm_count() / 2) {      // many rows: a block meets nobody
+		p.whole_row = 0;
+		p.splits = 0;
+	}
 	return p;
 }
+constexpr size_t kFewSmemMax = 225 * 1024;
 
 template <int HD>
-static cudaError_t launch_attn(const RowBatch& b, const Dims& d, const LayerDev* layer, int layer_index, KvPoolDev pool,
+static cudaError_t launch_attn(const RowBatch& b, const Dims& d, const LayerDev* layer, const LayerDev& h, int layer_index, KvPoolDev pool,
                                const AttnPlan& p, int reverse_rows, cudaStream_t st) {
-	const size_t sm = attn_smem_bytes(d.heads / d.kv_heads, p.cp, HD);
+	const int G = d.heads / d.kv_heads;
+	if (p.splits == 0)
+		return launch_pdl(k_attention<HD>, dim3(d.kv_heads, b.m), dim3(2 * HD), attn_smem_bytes(G, p.cp), st, b, d, layer, layer_index,
+		                  pool, p.cp, reverse_rows);
+	const bool staged = FewSmem<HD>::bytes(G, p.cp, true) <= kFewSmemMax;
 	cudaLaunchConfig_t cfg = {};
 	cfg.gridDim = dim3(d.kv_heads * p.splits, b.m);
 	cfg.blockDim = dim3(2 * HD);
-	cfg.dynamicSmemBytes = sm;
+	cfg.dynamicSmemBytes = FewSmem<HD>::bytes(G, p.cp, staged);
 	cfg.stream = st;
 	cudaLaunchAttribute attr[2];
 	attr[0].id = cudaLaunchAttributeClusterDimension;
@@ -938,7 +1159,25 @@ static cudaError_t launch_attn(const RowBatch& b, const Dims& d, const LayerDev*
 	attr[1].val.programmaticStreamSerializationAllowed = 1;
 	cfg.attrs = attr;
 	cfg.numAttrs = pdl_enabled() ? 2 : 1;
-	return cudaLaunchKernelEx(&cfg, k_attention<HD>, b, d, layer, layer_index, pool, p.cp, p.splits, p.whole_row, reverse_rows);
+	return cudaLaunchKernelEx(&cfg, staged ? k_attention_few<HD, true> : k_attention_few<HD, false>, b, d, layer, h.c_ctx, layer_index, pool,
+	                          p.cp, p.splits, p.whole_row, reverse_rows);
+}
+
+template <int HD>
+static cudaError_t configure_hd(int group) {
+	auto set = [](const void* f, int smem, bool big_cluster) {
+		cudaError_t e = cudaFuncSetAttribute(f, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
+		// clusters of 16 blocks are an opt-in size
+		if (e == cudaSuccess && big_cluster) e = cudaFuncSetAttribute(f, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
+		// same carve-out as the kernels around it (see rows_configure)
+		if (e == cudaSuccess) e = cudaFuncSetAttribute(f, cudaFuncAttributePreferredSharedMemoryCarveout, cudaSharedmemCarveoutMaxShared);
+		return e;
+	};
+	cudaError_t e = set((const void*)k_attention<HD>, (int)attn_smem_bytes(group, kAttnMaxSlice), false);
+	if (e == cudaSuccess) e = set((const void*)k_attention_few<HD, true>, (int)kFewSmemMax, true);
+	if (e == cudaSuccess) e = set((const void*)k_attention_few<HD, false>, (int)FewSmem<HD>::bytes(group, kAttnMaxSlice, false), true);
+	if (e == cudaSuccess) e = set((const void*)k_attention_tile<HD>, (int)TileSmem<HD>::kBytes, false);
+	return e;
 }
 
 cudaError_t attn_configure(const Dims& d) {
@@ -946,33 +1185,14 @@ cudaError_t attn_configure(const Dims& d) {
 	if (group < 1 || group > 8 || d.heads % d.kv_heads != 0) return cudaErrorInvalidConfiguration;
 	// widest row the plan can serve: 16 slices of kAttnMaxSlice positions
 	if (d.context_cap > 16 * kAttnMaxSlice) return cudaErrorInvalidConfiguration;
-	const size_t need = attn_smem_bytes(group, kAttnMaxSlice, d.head_dim);
-	if (need > 227 * 1024) return cudaErrorInvalidConfiguration;
-	const int n = (int)need;
-	const void* f = nullptr;
-	if (d.head_dim == 128) f = (const void*)k_attention<128>;
-	else if (d.head_dim == 64) f = (const void*)k_attention<64>;
-	else if (d.head_dim == 32) f = (const void*)k_attention<32>;
-	else return cudaErrorInvalidConfiguration;
-	cudaError_t e = cudaFuncSetAttribute(f, cudaFuncAttributeMaxDynamicSharedMemorySize, n);
-	if (e != cudaSuccess) return e;
-	// clusters of 16 blocks (rows wider than 8 slices) are an opt-in size
-	e = cudaFuncSetAttribute(f, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
-	if (e != cudaSuccess) return e;
-	// same carve-out as the kernels around it (see rows_configure)
-	e = cudaFuncSetAttribute(f, cudaFuncAttributePreferredSharedMemoryCarveout, cudaSharedmemCarveoutMaxShared);
-	if (e != cudaSuccess) return e;
-	const void* ft = nullptr;
-	size_t tile_bytes = 0;
-	if (d.head_dim == 128) { ft = (const void*)k_attention_tile<128>; tile_bytes = TileSmem<128>::kBytes; }
-	else if (d.head_dim == 64) { ft = (const void*)k_attention_tile<64>; tile_bytes = TileSmem<64>::kBytes; }
-	else { ft = (const void*)k_attention_tile<32>; tile_bytes = TileSmem<32>::kBytes; }
-	e = cudaFuncSetAttribute(ft, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)tile_bytes);
-	if (e != cudaSuccess) return e;
-	return cudaFuncSetAttribute(ft, cudaFuncAttributePreferredSharedMemoryCarveout, cudaSharedmemCarveoutMaxShared);
+	if (attn_smem_bytes(group, kAttnMaxSlice) > 225 * 1024) return cudaErrorInvalidConfiguration;
+	if (d.head_dim == 128) return configure_hd<128>(group);
+	if (d.head_dim == 64) return configure_hd<64>(group);
+	if (d.head_dim == 32) return configure_hd<32>(group);
+	return cudaErrorInvalidConfiguration;
 }
 
-bool launch_attention(const RowBatch& b, const Dims& d, const LayerDev* layer, int layer_index,
+bool launch_attention(const RowBatch& b, const Dims& d, const LayerDev* layer, const LayerDev& h, int layer_index,
                       KvPoolDev pool, int max_width, int reverse_rows, cudaStream_t st, cudaError_t* err) {
 	// the rows of a prefill chunk (consecutive positions of one sequence) take the query-tiled kernel
 	static const bool tile_off = [] {
@@ -994,11 +1214,11 @@ bool launch_attention(const RowBatch& b, const Dims& d, const LayerDev* layer, i
 		if (err) *err = e;
 		return false;
 	}
-	const AttnPlan p = attn_plan(d, b.m, max_width, reverse_rows != 0);
+	const AttnPlan p = attn_plan(d, b.m, max_width);
 	cudaError_t e;
-	if (d.head_dim == 128) e = launch_attn<128>(b, d, layer, layer_index, pool, p, reverse_rows, st);
-	else if (d.head_dim == 64) e = launch_attn<64>(b, d, layer, layer_index, pool, p, reverse_rows, st);
-	else e = launch_attn<32>(b, d, layer, layer_index, pool, p, reverse_rows, st);
+	if (d.head_dim == 128) e = launch_attn<128>(b, d, layer, h, layer_index, pool, p, reverse_rows, st);
+	else if (d.head_dim == 64) e = launch_attn<64>(b, d, layer, h, layer_index, pool, p, reverse_rows, st);
+	else e = launch_attn<32>(b, d, layer, h, layer_index, pool, p, reverse_rows, st);
 	if (err) *err = e;
 	return p.whole_row != 0;
 }
@@ -1051,7 +1271,11 @@ __global__ void k_int_sweep(int which, const int64_t* a, const int64_t* b, const
 		}
 		case 8: {      // Q15 probability: floor((e << 15) / total), 0 <= e <= total
 			const unsigned long long tot = (unsigned long long)b[i];
-			o0 = prob_q15(a[i], tot, 32768.0f / (float)tot);
+			const ProbRow pr = prob_row(tot);
+			bool unsure = false;
+			const uint32_t p = prob_fast(a[i], pr, &unsure) & 0xFFFFu;
+			o0 = unsure ? prob_pair_exact(a[i], a[i], pr.tot).x : p;
+			o1 = prob_q15(a[i], tot, 32768.0f / (float)tot);      // the exact form by itself
 			break;
 		}
 		default: break;

@@ -578,6 +578,16 @@ struct MapKeyHash {
 	}
 };
 
+bool encode_map(const void* ptr, int rows, int k, int box_rows, CUtensorMap* out) {
+	EncodeFn fn = encode_fn();
+	if (!fn) return false;
+	const cuuint64_t dims[2] = {(cuuint64_t)k, (cuuint64_t)rows};
+	const cuuint64_t strides[1] = {(cuuint64_t)k};
+	const cuuint32_t box[2] = {(cuuint32_t)BK, (cuuint32_t)box_rows};
+	const cuuint32_t estr[2] = {1, 1};
+	return fn(out, CU_TENSOR_MAP_DATA_TYPE_UINT8, 2, const_cast<void*>(ptr), dims, strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE,
+	          CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
+}
 // [rows, K] int8 row-major -> 2-D map, box = 128 bytes x box_rows rows, 128-byte swizzle, zero fill
 bool tensor_map(const void* ptr, int rows, int k, int box_rows, CUtensorMap* out) {
 	static std::mutex mu;
@@ -589,17 +599,8 @@ bool tensor_map(const void* ptr, int rows, int k, int box_rows, CUtensorMap* out
 		*out = it->second;
 		return true;
 	}
-	EncodeFn fn = encode_fn();
-	if (!fn) return false;
-	const cuuint64_t dims[2] = {(cuuint64_t)k, (cuuint64_t)rows};
-	const cuuint64_t strides[1] = {(cuuint64_t)k};
-	const cuuint32_t box[2] = {(cuuint32_t)BK, (cuuint32_t)box_rows};
-	const cuuint32_t estr[2] = {1, 1};
 	CUtensorMap m;
-	if (fn(&m, CU_TENSOR_MAP_DATA_TYPE_UINT8, 2, const_cast<void*>(ptr), dims, strides, box, estr,
-	       CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
-	       CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) != CUDA_SUCCESS)
-		return false;
+	if (!encode_map(ptr, rows, k, box_rows, &m)) return false;
 	if (cache.size() > 4096) cache.clear();
 	cache.emplace(key, m);
 	*out = m;
@@ -629,6 +630,14 @@ int pick_splits(const LinearArgs& a, int tiles) {
 
 std::atomic<int> g_debug_withhold{0};
 
+}  // namespace
+bool tc_debug_take() {
+	int left = g_debug_withhold.load();
+	while (left > 0 && !g_debug_withhold.compare_exchange_weak(left, left - 1)) {}
+	return left > 0;
+}
+namespace {
+
 template <int MT, int BN>
 bool launch_cfg(const LinearArgs& a_in, cudaStream_t st) {
 	using Cfg = TcCfg<MT, BN>;
@@ -647,12 +656,7 @@ bool launch_cfg(const LinearArgs& a_in, cudaStream_t st) {
 	}
 	const int tiles = ((a.N + BN - 1) / BN) * ((a.M + MT * BM - 1) / (MT * BM));
 	a.splits = pick_splits<MT, BN>(a, tiles);
-	{
-		int left = g_debug_withhold.load();
-		a.debug_withhold = 0;
-		while (left > 0 && !g_debug_withhold.compare_exchange_weak(left, left - 1)) {}
-		if (left > 0) a.debug_withhold = 1;
-	}
+	a.debug_withhold = tc_debug_take() ? 1 : 0;
 	const int items = tiles * a.splits;
 	const int grid = items < sm_count() ? items : sm_count();
 	if (launch_pdl(k_linear_tc<MT, BN>, dim3(grid), dim3(kTcThreads), Cfg::kSmemBytes, st, ma, mb, a) != cudaSuccess) {
@@ -676,6 +680,14 @@ static bool tc_refuse(int reason) {
 	g_tc_refusals.fetch_add(1);
 	g_tc_last_reason.store(reason);
 	return false;
+}
+
+bool tc_tensor_map(const void* ptr, int rows, int k, int box_rows, bool cache, CUtensorMap* out) {
+	return cache ? tensor_map(ptr, rows, k, box_rows, out) : encode_map(ptr, rows, k, box_rows, out);
+}
+void tc_count(bool launched, int reason) {
+	if (launched) g_tc_launches.fetch_add(1);
+	else tc_refuse(reason);
 }
 
 void tc_debug_withhold(int launches) { g_debug_withhold.store(launches < 0 ? 0 : launches); }

@@ -2,6 +2,7 @@
 // stream and returns immediately; errors surface through cudaGetLastError at the call
 // site. Nothing here allocates.
 #pragma once
+#include <cuda.h>
 #include <cuda_runtime.h>
 
 #include <atomic>
@@ -150,6 +151,13 @@ cudaError_t launch_linear_gemv(const LinearArgs& a, cudaStream_t st);
 // tensor-core path for M > 8 rows (tcgen05 kind::i8, TMA-fed). Returns false when the
 // shape is not supported by that kernel (caller then uses the GEMV path).
 bool launch_linear_tc(const LinearArgs& a, cudaStream_t st);
+// tensor-core path for up to 256 rows, weights on the M side of the MMA (sslm_skinny.cu). cache_maps:
+// keep the tensor maps of these pointers (a map costs the host about a microsecond and the cache memory).
+bool launch_linear_skinny(const LinearArgs& a, bool cache_maps, cudaStream_t st);
+// shared by the two tensor-core kernels: [rows, k] int8 map, box 128 bytes x box_rows, 128-byte swizzle
+bool tc_tensor_map(const void* ptr, int rows, int k, int box_rows, bool cache, CUtensorMap* out);
+void tc_count(bool launched, int reason);
+bool tc_debug_take();      // one launch of those tc_debug_withhold asked for
 // Tests of the bounded waits: the next `launches` tensor-core launches arm their first weight-tile
 // barrier in block 0 without requesting the tile, so that the wait on it runs out (no fault, no
 // endless loop: the rows of that tile end with the internal wait-timeout status).
@@ -170,7 +178,7 @@ cudaError_t attn_configure(const Dims& d);
 void attn_force_splits(int splits);
 // Returns true when the launch also ran the attention-context funnel (codes in b.ctx, scale in
 // b.cs); otherwise b.ctxw / rowmax slot 3 are filled and launch_ctx_funnel must follow.
-bool launch_attention(const RowBatch& b, const Dims& d, const LayerDev* layer, int layer_index,
+bool launch_attention(const RowBatch& b, const Dims& d, const LayerDev* layer, const LayerDev& h, int layer_index,
                       KvPoolDev pool, int max_width, int reverse_rows, cudaStream_t st, cudaError_t* err);
 // gather a sequence's pages into the reference's canonical block layout
 // [layer][K|V][kv_head][position][head_dim]; positions beyond `valid(layer)` are zero
