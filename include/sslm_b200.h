@@ -221,7 +221,8 @@ SSLM_API sslm_status sslm_b200_set_device(int ordinal);
  * src/forward/forward_sites.cpp:1114-1146, :1182-1203.) Outputs that are NULL are skipped.
  * in_scales: M pairs (m, e); out_scales: M pairs; row_status: M reference
  * SslmForwardStatus ordinals (0 = Ok). use_tensor_cores: 0 forces the streaming GEMV
- * kernel, 1 lets M > 8 take the tcgen05 kernel. */
+ * kernel, 1 lets M > 8 take the activation-major tcgen05 kernel, 2 lets up to 256 rows take the
+ * weights-first one where it is the better of the two. */
 SSLM_API sslm_status sslm_b200_linear(const int8_t* x, const int8_t* w, const int32_t* fold, int32_t M,
                              int32_t N, int32_t K, const int64_t* in_scales, int64_t site_m,
                              int64_t site_e, int32_t use_tensor_cores, int32_t* out_folded,
@@ -322,7 +323,7 @@ SSLM_API size_t sslm_b200_model_device_bytes(sslm_model model);
  *  - All calls on a device share the array. It reads zero at load time and every call leaves
  *    it zero again; calls whose kernels may overlap in time (other streams or threads) race
  *    on it and must be ordered by the caller.
- * Always the streaming dp4a kernel (the tensor-core path keeps host-side caches). */
+ * From two rows on it runs on the tensor cores, its tensor maps encoded on the stack of the call. */
 #define SSLM_B200_RESIDENT_MAX_ROWS 256
 SSLM_API sslm_status sslm_b200_linear_resident(const int8_t* d_x, const int8_t* d_w, const int32_t* d_fold,
                                                int32_t M, int32_t N, int32_t K, const int64_t* d_in_scales,

@@ -340,6 +340,14 @@ k_linear_tc(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ C
 		// straight-line path: int32 rows, fold present, no adapters, not the head
 		const bool fast_ok = vec_ok && a.fold != nullptr && a.rows == nullptr && a.best == nullptr;
 		const bool wide_ok = (a.out_ld & 7) == 0 && (((uintptr_t)a.out) & 31) == 0;   // 32-byte stores line up
+		auto refuse = [&](int m0) {
+			for (int mt = 0; mt < MT; ++mt) {
+				const int row = m0 + mt * BM + q * 32 + lane;
+				if (row >= a.M) break;
+				if (a.status != nullptr) atomicCAS(&a.status[row], 0, (int32_t)kInternalWaitTimeout);
+				else if (a.rowmax != nullptr) atomicMax(&a.rowmax[(size_t)row * 4], kRowmaxTimeout);
+			}
+		};
 		uint32_t tc = 0;
 		for (int w = blockIdx.x; w < items; w += gridDim.x, ++tc) {
 			const uint32_t as = tc & 1u;
@@ -372,12 +380,7 @@ k_linear_tc(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ C
 			    : "r"(odd_column)
 			    : "memory");
 			if (s_stop[as] != 0) {
-				if (a.status != nullptr) {
-					for (int mt = 0; mt < MT; ++mt) {
-						const int row = m0 + mt * BM + q * 32 + lane;
-						if (row < a.M) atomicCAS(&a.status[row], 0, (int32_t)kInternalWaitTimeout);
-					}
-				}
+				refuse(m0);
 				break;
 			}
 			// (the MMA thread commits a tile it gave up on as well, so that nobody waits out a second
@@ -386,12 +389,7 @@ k_linear_tc(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ C
 			asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
 			if (!acc_ok) {
 				s_timeout = 1;
-				if (a.status != nullptr) {
-					for (int mt = 0; mt < MT; ++mt) {
-						const int row = m0 + mt * BM + q * 32 + lane;
-						if (row < a.M) atomicCAS(&a.status[row], 0, (int32_t)kInternalWaitTimeout);
-					}
-				}
+				refuse(m0);
 			}
 			bool finish = true;                        // this block runs the tile's epilogue
 			if (splits > 1) {
@@ -650,7 +648,7 @@ bool launch_cfg(const LinearArgs& a_in, cudaStream_t st) {
 		return false;
 	}
 	CUtensorMap ma, mb;
-	if (!tensor_map(a.x, a.M, a.K, BM, &ma) || !tensor_map(a.w, a.N, a.K, BN, &mb)) {
+	if (!tc_tensor_map(a.x, a.M, a.K, BM, a.caller_memory == 0, &ma) || !tc_tensor_map(a.w, a.N, a.K, BN, a.caller_memory == 0, &mb)) {
 		g_tc_last_reason.store(encode_fn() ? 4 : 3);
 		return false;
 	}
@@ -659,7 +657,7 @@ bool launch_cfg(const LinearArgs& a_in, cudaStream_t st) {
 	a.debug_withhold = tc_debug_take() ? 1 : 0;
 	const int items = tiles * a.splits;
 	const int grid = items < sm_count() ? items : sm_count();
-	if (launch_pdl(k_linear_tc<MT, BN>, dim3(grid), dim3(kTcThreads), Cfg::kSmemBytes, st, ma, mb, a) != cudaSuccess) {
+	if (launch_ordered(a.caller_memory == 0, k_linear_tc<MT, BN>, dim3(grid), dim3(kTcThreads), Cfg::kSmemBytes, st, ma, mb, a) != cudaSuccess) {
 		g_tc_last_reason.store(5);
 		return false;
 	}

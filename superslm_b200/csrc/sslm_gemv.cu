@@ -232,7 +232,10 @@ k_gemv(LinearArgs a, GemvPlan p) {
 	__syncthreads();
 
 	if (*(volatile int*)&s_timeout) {
-		if (a.status != nullptr && t < mcount) atomicCAS(&a.status[m0 + t], 0, (int32_t)kInternalWaitTimeout);
+		if (t < mcount) {
+			if (a.status != nullptr) atomicCAS(&a.status[m0 + t], 0, (int32_t)kInternalWaitTimeout);
+			else if (a.rowmax != nullptr) atomicMax(&a.rowmax[(size_t)(m0 + t) * 4], kRowmaxTimeout);
+		}
 		return;
 	}
 	// ---- epilogue: thread i takes output (m, n) = (i / nrows, i % nrows)
@@ -363,7 +366,7 @@ static cudaError_t launch_mt(const LinearArgs& a, int grid_y, cudaStream_t st) {
 	const size_t smem = gemv_smem_bytes(MT, a.K, rpb, slots, slot_bytes);
 	if (smem > 220 * 1024) return cudaErrorInvalidConfiguration;
 	const int gx = (a.N + rpb - 1) / rpb;
-	return launch_pdl(k_gemv<MT>, dim3(gx, grid_y), dim3(kGemvThreads), smem, st, a, p);
+	return launch_ordered(a.caller_memory == 0, k_gemv<MT>, dim3(gx, grid_y), dim3(kGemvThreads), smem, st, a, p);
 }
 
 cudaError_t launch_linear_gemv(const LinearArgs& a, cudaStream_t st) {

@@ -35,7 +35,7 @@ inline bool pdl_enabled() {
 	return on;
 }
 template <typename... KArgs, typename... Args>
-cudaError_t launch_pdl(void (*kernel)(KArgs...), dim3 grid, dim3 block, size_t smem, cudaStream_t st, Args&&... args) {
+cudaError_t launch_ordered(bool programmatic, void (*kernel)(KArgs...), dim3 grid, dim3 block, size_t smem, cudaStream_t st, Args&&... args) {
 	cudaLaunchConfig_t cfg = {};
 	cfg.gridDim = grid;
 	cfg.blockDim = block;
@@ -45,8 +45,12 @@ cudaError_t launch_pdl(void (*kernel)(KArgs...), dim3 grid, dim3 block, size_t s
 	attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
 	attr[0].val.programmaticStreamSerializationAllowed = 1;
 	cfg.attrs = attr;
-	cfg.numAttrs = pdl_enabled() ? 1 : 0;
+	cfg.numAttrs = programmatic && pdl_enabled() ? 1 : 0;
 	return cudaLaunchKernelEx(&cfg, kernel, std::forward<Args>(args)...);
+}
+template <typename... KArgs, typename... Args>
+cudaError_t launch_pdl(void (*kernel)(KArgs...), dim3 grid, dim3 block, size_t smem, cudaStream_t st, Args&&... args) {
+	return launch_ordered(true, kernel, grid, block, smem, st, std::forward<Args>(args)...);
 }
 
 // ---- per-device one-time set-up
@@ -112,6 +116,7 @@ void launch_act(const RowBatch& b, const Dims& d, const LayerDev& h, const int32
 // ---- int8 linear layers (sslm_gemv.cu, sslm_gemm_tc.cu)
 // out[m, n] = fold_n( sum_k x[m,k] * w[n,k] ) (+ LoRA delta), plus the per-row max |out|
 // of each column segment, reduced into rowmax[m][slot].
+constexpr unsigned long long kRowmaxTimeout = ~0ull;
 struct LinearArgs {
 	const int8_t* x;      // [M, K] row-major activations
 	const int8_t* w;      // [N, K] row-major weights
@@ -136,7 +141,8 @@ struct LinearArgs {
 	// src/forward/forward_sites.cpp:2443-2449), or nullptr for an unconstrained row; the array
 	// itself may be nullptr
 	const uint8_t* const* row_mask;
-	int32_t* status;      // [M] row statuses (a bounded device wait that ran out is reported here), or nullptr
+	int32_t* status;      // [M] row statuses: a bounded device wait that ran out is reported here, or, where this is
+	                      // nullptr, as the row maximum kRowmaxTimeout
 	// split-K scratch of the tensor-core path (optional): partial accumulators and one
 	// arrival counter per output tile. Counters are zero between launches.
 	int32_t* partial;
@@ -144,6 +150,8 @@ struct LinearArgs {
 	unsigned int* tile_counters;
 	int n_tile_counters;
 	int splits;           // filled in by launch_linear_tc
+	int caller_memory;    // 1: operands are a caller's own, on a caller's stream: the weights may have been written by
+	                      //    the kernel in front (plain stream order), and no tensor map is kept
 	int debug_withhold;   // tests only (tc_debug_withhold): block 0 never requests its first weight tile
 };
 // HBM-bound small-M path: bulk-copy weight streaming through a shared-memory ring, dp4a.
@@ -151,9 +159,9 @@ cudaError_t launch_linear_gemv(const LinearArgs& a, cudaStream_t st);
 // tensor-core path for M > 8 rows (tcgen05 kind::i8, TMA-fed). Returns false when the
 // shape is not supported by that kernel (caller then uses the GEMV path).
 bool launch_linear_tc(const LinearArgs& a, cudaStream_t st);
-// tensor-core path for up to 256 rows, weights on the M side of the MMA (sslm_skinny.cu). cache_maps:
-// keep the tensor maps of these pointers (a map costs the host about a microsecond and the cache memory).
-bool launch_linear_skinny(const LinearArgs& a, bool cache_maps, cudaStream_t st);
+// tensor-core path for up to 256 rows, weights on the M side of the MMA (sslm_skinny.cu). Returns false
+// where another kernel is the better one as well.
+bool launch_linear_skinny(const LinearArgs& a, cudaStream_t st);
 // shared by the two tensor-core kernels: [rows, k] int8 map, box 128 bytes x box_rows, 128-byte swizzle
 bool tc_tensor_map(const void* ptr, int rows, int k, int box_rows, bool cache, CUtensorMap* out);
 void tc_count(bool launched, int reason);

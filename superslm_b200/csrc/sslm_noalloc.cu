@@ -29,6 +29,7 @@
 
 #include "../../include/sslm_b200.h"
 #include "sslm_kernels.h"
+#include "sslm_quad.cuh"
 
 // The scratch: 4 slots of 8 bytes per row (the projection kernels index row * 4 + slot; this
 // layer uses slot 0), 256 rows = 8 KiB of device image. All zero at module load and after
@@ -43,25 +44,37 @@ constexpr int kResidentMaxK = 16384;        // the streaming kernel stages 8 act
 
 // Funnel of the projected rows (FunnelProjectedRow's tail, src/forward/forward_sites.cpp:
 // 1114-1146): the same arithmetic as the funnel behind sslm_b200_linear, reading the row
-// peak from the fixed array and leaving the slot zero for the next call.
-__global__ void __launch_bounds__(256)
+// peak from the fixed array and leaving the slot zero for the next call. One block per row, four
+// elements per thread and pass: 45 rows of 8,960 took 30 us with one element each and the integer coder.
+__global__ void __launch_bounds__(1024)
 k_resident_funnel(const int32_t* wide, int n, unsigned long long* row_peak, const Scale* in_scales, Scale site,
                   int8_t* codes, Scale* out_scales, int32_t* status) {
-	__shared__ unsigned long long s_peak;
 	const int r = blockIdx.x;
-	if (threadIdx.x == 0) {
-		s_peak = row_peak[(size_t)r * 4];
-		row_peak[(size_t)r * 4] = 0ull;
-	}
+	pdl_wait();
+	const FunnelFold fold = funnel_prefold(&in_scales[r], 1, site);
+	const unsigned long long peak = __ldcg(&row_peak[(size_t)r * 4]);
 	__syncthreads();
-	const FunnelParams fp = funnel_params(s_peak, &in_scales[r], 1, site);
+	if (threadIdx.x == 0) row_peak[(size_t)r * 4] = 0ull;
+	const QuadFunnel fp = quad_funnel(peak, fold);
 	if (threadIdx.x == 0) {
-		if (status != nullptr && status[r] == 0) status[r] = fp.status;
-		if (out_scales != nullptr) out_scales[r] = fp.out;
+		if (status != nullptr) status[r] = peak == kRowmaxTimeout ? (int32_t)kInternalWaitTimeout : fp.status;
+		if (out_scales != nullptr) out_scales[r] = fp.status == kOk ? fp.out : funnel_finish(peak, fold).out;
 	}
 	if (fp.status != kOk || codes == nullptr) return;
-	for (int i = threadIdx.x; i < n; i += blockDim.x)
-		codes[(size_t)r * n + i] = requant_code((int64_t)wide[(size_t)r * n + i], fp.r, fp.s);
+	const int32_t* row = wide + (size_t)r * n;
+	int8_t* out = codes + (size_t)r * n;
+	if ((n & 3) == 0 && ((uintptr_t)codes & 3) == 0) {
+		for (int q = threadIdx.x; q < (n >> 2); q += blockDim.x) {
+			int32_t x[4];
+			load_quad(row + 4 * q, x);
+			((uint32_t*)out)[q] = code_quad(x, fp);
+		}
+	} else {
+		for (int i = threadIdx.x; i < n; i += blockDim.x) {
+			const int32_t x[4] = {__ldcg(row + i), 0, 0, 0};
+			out[i] = (int8_t)code_quad(x, fp);
+		}
+	}
 }
 
 // device address of g_row_peak, per device ordinal; resolved by the first call on a device
@@ -97,8 +110,6 @@ extern "C" sslm_status sslm_b200_linear_resident(const int8_t* d_x, const int8_t
 		g_peak_addr[dev].store(peak, std::memory_order_release);
 	}
 	cudaStream_t st = (cudaStream_t)stream;
-	if (d_row_status != nullptr && cudaMemsetAsync(d_row_status, 0, (size_t)M * 4, st) != cudaSuccess)
-		return SSLM_ALLOCATION_FAILED;
 
 	LinearArgs a{};
 	a.x = d_x; a.w = d_w; a.fold = d_fold;
@@ -109,11 +120,14 @@ extern "C" sslm_status sslm_b200_linear_resident(const int8_t* d_x, const int8_t
 	a.seg_end[0] = a.seg_end[1] = a.seg_end[2] = N;
 	a.seg_slot[0] = 0; a.seg_slot[1] = a.seg_slot[2] = -1;
 	a.seg_lora[0] = a.seg_lora[1] = a.seg_lora[2] = -1;
-	a.status = d_row_status;
-	// nothing ran yet if the projection's launch is refused: the array still reads zero
-	if (launch_linear_gemv(a, st) != cudaSuccess) return SSLM_ALLOCATION_FAILED;
-	k_resident_funnel<<<M, 256, 0, st>>>(d_out_folded, N, peak, (const Scale*)d_in_scales, Scale{site_m, site_e},
-	                                     d_out_codes, (Scale*)d_out_scales, d_row_status);
+	a.caller_memory = 1;
+	// nothing ran yet if the projection's launch is refused: the array still reads zero. From two rows on
+	// the tensor cores (45 rows of 1536 x 8960: 85 us as six passes of the streaming kernel).
+	const bool tc = M >= 2 && (launch_linear_skinny(a, st) || (M > 8 && launch_linear_tc(a, st)));
+	if (!tc && launch_linear_gemv(a, st) != cudaSuccess) return SSLM_ALLOCATION_FAILED;
+	const int threads = N >= 4096 ? 1024 : (N >= 1024 ? 256 : 128);
+	launch_pdl(k_resident_funnel, dim3(M), dim3(threads), 0, st, (const int32_t*)d_out_folded, (int)N, peak, (const Scale*)d_in_scales,
+	           Scale{site_m, site_e}, d_out_codes, (Scale*)d_out_scales, d_row_status);
 	if (cudaGetLastError() != cudaSuccess) {
 		// The projection is enqueued and will leave its row peaks in the array, but the kernel that
 		// consumes and clears them is not: clear the rows this call used, in stream order, so the

@@ -351,8 +351,10 @@ k_skinny(const __grid_constant__ CUtensorMap map_w, const __grid_constant__ CUte
 		constexpr int kCols = NB / (Cfg::kEpiWarps / 4);          // columns (rows of x) this warp takes
 		const int col0 = part * kCols;
 		auto refuse = [&]() {
-			if (a.status != nullptr)
-				for (int m = et; m < a.M; m += kEpi) atomicCAS(&a.status[m], 0, (int32_t)kInternalWaitTimeout);
+			for (int m = et; m < a.M; m += kEpi) {
+				if (a.status != nullptr) atomicCAS(&a.status[m], 0, (int32_t)kInternalWaitTimeout);
+				else if (a.rowmax != nullptr) atomicMax(&a.rowmax[(size_t)m * 4], kRowmaxTimeout);
+			}
 		};
 		Channel c = channel_of(a, tile0 * kWRows + q * 32 + lane);      // (fold constants: ahead of the wait)
 		pdl_wait();
@@ -509,7 +511,7 @@ k_skinny(const __grid_constant__ CUtensorMap map_w, const __grid_constant__ CUte
 // stream and its MMAs, and the exchange costs under a microsecond. Ring stages: all of the block's
 // k-blocks when they fit, so that its whole weight stream is requested ahead of the wait.
 template <int NB, int MODE>
-bool launch_mode(const LinearArgs& a_in, bool cache_maps, cudaStream_t st, int* reason) {
+bool launch_mode(const LinearArgs& a_in, cudaStream_t st, int* reason) {
 	using Cfg = SkCfg<NB>;
 	LinearArgs a = a_in;
 	static PerDeviceOnce configured;
@@ -524,7 +526,7 @@ bool launch_mode(const LinearArgs& a_in, bool cache_maps, cudaStream_t st, int* 
 		return false;
 	}
 	CUtensorMap mw, mx;
-	if (!tc_tensor_map(a.w, a.N, a.K, kWRows, cache_maps, &mw) || !tc_tensor_map(a.x, a.M, a.K, NB, cache_maps, &mx)) {
+	if (!tc_tensor_map(a.w, a.N, a.K, kWRows, a.caller_memory == 0, &mw) || !tc_tensor_map(a.x, a.M, a.K, NB, a.caller_memory == 0, &mx)) {
 		*reason = 4;
 		return false;
 	}
@@ -559,7 +561,7 @@ bool launch_mode(const LinearArgs& a_in, bool cache_maps, cudaStream_t st, int* 
 	cfg.stream = st;
 	cudaLaunchAttribute attr[2];
 	int n = 0;
-	if (pdl_enabled()) {
+	if (pdl_enabled() && a.caller_memory == 0) {
 		attr[n].id = cudaLaunchAttributeProgrammaticStreamSerialization;
 		attr[n++].val.programmaticStreamSerializationAllowed = 1;
 	}
@@ -580,11 +582,11 @@ bool launch_mode(const LinearArgs& a_in, bool cache_maps, cudaStream_t st, int* 
 
 }  // namespace
 
-bool launch_linear_skinny(const LinearArgs& a, bool cache_maps, cudaStream_t st) {
+bool launch_linear_skinny(const LinearArgs& a, cudaStream_t st) {
 	auto launch = [&](auto nb, int* reason) {
 		constexpr int NB = decltype(nb)::value;
-		if (a.best != nullptr) return launch_mode<NB, kHead>(a, cache_maps, st, reason);
-		return a.out64 ? launch_mode<NB, kRows64>(a, cache_maps, st, reason) : launch_mode<NB, kRows32>(a, cache_maps, st, reason);
+		if (a.best != nullptr) return launch_mode<NB, kHead>(a, st, reason);
+		return a.out64 ? launch_mode<NB, kRows64>(a, st, reason) : launch_mode<NB, kRows32>(a, st, reason);
 	};
 	if (a.best != nullptr && a.fold != nullptr) return false;      // (no caller folds logits)
 	if (a.M < 1 || a.M > 256) return false;
