@@ -135,6 +135,7 @@ struct sslm_adapter_s {
 	DeviceArena arena;
 	sslm::LoraLayerDev* d_layers = nullptr;  // [layers]
 	uint32_t rank = 0;
+	uint32_t slots = 0;                      // bit LoraSlot: some layer adapts that projection
 	std::atomic<uint32_t> live_refs{0};
 };
 
