@@ -1292,12 +1292,12 @@ void launch_int_sweep(int which, const int64_t* a, const int64_t* b, const int64
 
 // ------------------------------------------------------------ canonical KV export
 // Writes the sequence's K and V in the reference's save layout, [layer][K|V][kv head]
-// [context_cap][head_dim] with zeros past the valid positions, undoing the paging and the
+// [span][head_dim] with zeros past the valid positions, undoing the paging and the
 // V-page transposition.
 __global__ void k_kv_export(Dims d, KvPoolDev pool, const int32_t* pages, int context_length,
-                            int layer_index, int8_t* out) {
+                            int layer_index, int span, int8_t* out) {
 	const int hd = d.head_dim, vec = hd / 16;
-	const int64_t per_plane = (int64_t)d.context_cap * vec;
+	const int64_t per_plane = (int64_t)span * vec;
 	const int64_t total = (int64_t)d.layers * 2 * d.kv_heads * per_plane;
 	for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < total;
 	     i += (int64_t)gridDim.x * blockDim.x) {
@@ -1327,16 +1327,16 @@ __global__ void k_kv_export(Dims d, KvPoolDev pool, const int32_t* pages, int co
 }
 
 void launch_kv_export(const Dims& d, KvPoolDev pool, const int32_t* pages, int context_length,
-                      int layer_index, int8_t* out, cudaStream_t st) {
-	k_kv_export<<<148 * 4, 256, 0, st>>>(d, pool, pages, context_length, layer_index, out);
+                      int layer_index, int span, int8_t* out, cudaStream_t st) {
+	k_kv_export<<<148 * 4, 256, 0, st>>>(d, pool, pages, context_length, layer_index, span, out);
 }
 
 // The inverse: scatter a canonical block (a save blob's K/V) into the sequence's pages.
 // Only the valid positions are written; everything else in the pages is never read.
 __global__ void k_kv_import(Dims d, KvPoolDev pool, const int32_t* pages, int context_length,
-                            int layer_index, const int8_t* in) {
+                            int layer_index, int span, const int8_t* in) {
 	const int hd = d.head_dim, vec = hd / 16;
-	const int64_t per_plane = (int64_t)d.context_cap * vec;
+	const int64_t per_plane = (int64_t)span * vec;
 	const int64_t total = (int64_t)d.layers * 2 * d.kv_heads * per_plane;
 	for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < total;
 	     i += (int64_t)gridDim.x * blockDim.x) {
@@ -1361,23 +1361,28 @@ __global__ void k_kv_import(Dims d, KvPoolDev pool, const int32_t* pages, int co
 	}
 }
 
-// Copy one page id to another in every (layer, kv head, K|V) plane: the private copy a
-// sequence takes of an adopted prefix's last, partly filled page.
-__global__ void k_page_copy(Dims d, KvPoolDev pool, int src_page, int dst_page) {
+// Block 0 takes over the page ids and the state; the others, one per (layer, kv head, K|V) plane, copy
+// the last, partly filled page.
+__global__ void k_adopt(Dims d, KvPoolDev pool, AdoptArgs a) {
+	if (blockIdx.x == 0) {
+		for (int i = threadIdx.x; i < a.full_pages; i += blockDim.x) a.dst_pages[i] = a.src_pages[i];
+		if (threadIdx.x == 0 && a.copy_to >= 0) a.dst_pages[a.full_pages] = a.copy_to;
+		for (int i = threadIdx.x; i < a.state_bytes / 16; i += blockDim.x) ((int4*)a.dst_state)[i] = ((const int4*)a.src_state)[i];
+		return;
+	}
 	const int64_t page_bytes = (int64_t)kPageTokens * d.head_dim;
-	const int64_t plane_stride = pool.num_pages * page_bytes;
-	int8_t* plane = pool.base + (int64_t)blockIdx.x * plane_stride;
-	const int4* src = (const int4*)(plane + (int64_t)src_page * page_bytes);
-	int4* dst = (int4*)(plane + (int64_t)dst_page * page_bytes);
+	int8_t* plane = pool.base + (int64_t)(blockIdx.x - 1) * (pool.num_pages * page_bytes);
+	const int4* src = (const int4*)(plane + (int64_t)a.copy_from * page_bytes);
+	int4* dst = (int4*)(plane + (int64_t)a.copy_to * page_bytes);
 	for (int i = threadIdx.x; i < (int)(page_bytes / 16); i += blockDim.x) dst[i] = src[i];
 }
-void launch_page_copy(const Dims& d, KvPoolDev pool, int src_page, int dst_page, cudaStream_t st) {
-	k_page_copy<<<d.layers * d.kv_heads * 2, 128, 0, st>>>(d, pool, src_page, dst_page);
+void launch_adopt(const Dims& d, KvPoolDev pool, const AdoptArgs& a, cudaStream_t st) {
+	k_adopt<<<a.copy_from >= 0 ? 1 + d.layers * d.kv_heads * 2 : 1, 128, 0, st>>>(d, pool, a);
 }
 
 void launch_kv_import(const Dims& d, KvPoolDev pool, const int32_t* pages, int context_length,
-                      int layer_index, const int8_t* in, cudaStream_t st) {
-	k_kv_import<<<148 * 4, 256, 0, st>>>(d, pool, pages, context_length, layer_index, in);
+                      int layer_index, int span, const int8_t* in, cudaStream_t st) {
+	k_kv_import<<<148 * 4, 256, 0, st>>>(d, pool, pages, context_length, layer_index, span, in);
 }
 
 }  // namespace sslm

@@ -9,6 +9,8 @@
 #include <cstdlib>
 #include <cstring>
 #include <new>
+#include <thread>
+#include <type_traits>
 #include <unordered_set>
 
 using namespace sslm;
@@ -31,6 +33,10 @@ bool cuda_ok(cudaError_t e) { return e == cudaSuccess; }
 bool is_aligned64(const void* p) { return ((uintptr_t)p % SSLM_ABI_ALIGNMENT_BYTES) == 0; }
 
 size_t align_up(size_t v, size_t a) { return (v + a - 1) / a * a; }
+
+// one hidden-state slot of a sequence: codes, then the carried scale
+size_t seq_scale_offset(const Dims& d) { return align_up(d.hidden, 16); }
+size_t seq_state_stride(const Dims& d) { return align_up(seq_scale_offset(d) + sizeof(Scale), 256); }
 
 sslm_status map_forward_status(int32_t st) {
 	// MapForwardStatus, src/sslm_abi.cpp:1352-1370
@@ -133,6 +139,7 @@ extern "C" sslm_status sslm_model_map(const void* data, size_t size, sslm_model*
 	auto fail = [&](sslm_status st) {
 		cudaFree(m->arena.base);
 		cudaFree(m->d_schema_pages);
+		if (m->aux) cudaStreamDestroy(m->aux);
 		delete m;
 		return st;
 	};
@@ -281,6 +288,9 @@ extern "C" sslm_status sslm_model_map(const void* data, size_t size, sslm_model*
 	}
 	m->weight_bytes = m->arena.used;
 	if (!cuda_ok(rows_configure(d)) || !cuda_ok(attn_configure(d))) return fail(SSLM_ARTIFACT_REJECTED);
+	if (!cuda_ok(cudaStreamCreateWithFlags(&m->aux, cudaStreamNonBlocking)) ||
+	    !cuda_ok(cudaEventCreateWithFlags(&m->aux_done, cudaEventDisableTiming)))
+		return fail(SSLM_ALLOCATION_FAILED);
 	cudaDeviceSynchronize();
 	*out = m;
 	return SSLM_OK;
@@ -293,6 +303,11 @@ extern "C" sslm_status sslm_model_unmap(sslm_model model) {
 	if (model->live_refs.load(std::memory_order_acquire) != 0) return SSLM_MODEL_HAS_LIVE_SEQUENCES;
 	cudaSetDevice(model->device);
 	if (model->default_ws) destroy_workspace(model->default_ws);
+	cudaStreamSynchronize(model->aux);
+	cudaStreamDestroy(model->aux);
+	cudaEventDestroy(model->aux_done);
+	cudaFreeHost(model->h_stage);
+	cudaFree(model->d_stage);
 	cudaFree(model->arena.base);
 	cudaFree(model->d_schema_pages);
 	delete model;
@@ -333,11 +348,16 @@ extern "C" sslm_status sslm_kv_pool_create(sslm_model model, void* buf, size_t b
 	p->pages_per_block = (d.context_cap + kPageTokens - 1) / kPageTokens;
 	p->dev.num_pages = (int64_t)p->pages_per_block * block_count;
 	const size_t bytes = (size_t)d.layers * d.kv_heads * 2 * p->dev.num_pages * kPageTokens * d.head_dim;
-	if (!cuda_ok(cudaMalloc((void**)&p->dev.base, bytes))) {
+	p->seq_stride = 2 * seq_state_stride(d) + align_up((size_t)p->pages_per_block * 4, 256);
+	const size_t kv_bytes = align_up(bytes, 256);
+	if (!cuda_ok(cudaMalloc((void**)&p->dev.base, kv_bytes + p->seq_stride * block_count))) {
 		delete p;
 		return SSLM_ALLOCATION_FAILED;
 	}
+	p->d_seq = (uint8_t*)p->dev.base + kv_bytes;
 	try {
+		p->free_slots.reserve(block_count);
+		for (int32_t i = (int32_t)block_count - 1; i >= 0; --i) p->free_slots.push_back(i);
 		p->free_pages.reserve(p->dev.num_pages);
 		for (int64_t i = p->dev.num_pages - 1; i >= 0; --i) p->free_pages.push_back((int32_t)i);
 		p->page_refs.assign((size_t)p->dev.num_pages, 0u);
@@ -369,6 +389,31 @@ bool config_ok(const sslm_model_s* model, const sslm_config* c) {
 	return c->reserved == 0;
 }
 
+constexpr size_t kUpBytesPerRow = sizeof(RowDesc) + sizeof(RowSource) + sizeof(RowSink) + sizeof(void*);
+constexpr size_t kDownBytesPerRow = 8 + 8 + 4 + 4;      // arg-max key, saturations, status, finished layers
+
+// Lay the upload and read-back blocks out for a call of n rows.
+void bind_rows(sslm_workspace_s* w, int n) {
+	size_t off = 0;
+	auto up = [&](auto*& h, auto*& d, size_t bytes) {
+		h = (std::remove_reference_t<decltype(h)>)(w->h_up + off);
+		d = (std::remove_reference_t<decltype(d)>)(w->d_up + off);
+		off += bytes;
+	};
+	up(w->h_rows, w->d_rows, n * sizeof(RowDesc));
+	up(w->h_src, w->d_src, n * sizeof(RowSource));
+	up(w->h_sink, w->d_sink, n * sizeof(RowSink));
+	up(w->h_row_mask, w->d_row_mask, n * sizeof(void*));
+	w->h_best = (unsigned long long*)w->h_down;
+	w->h_sat = w->h_best + n;
+	w->h_status = (int32_t*)(w->h_sat + n);
+	w->h_done = w->h_status + n;
+	w->base.best = (unsigned long long*)w->d_down;
+	w->base.sat = w->base.best + n;
+	w->base.status = (int32_t*)(w->base.sat + n);
+	w->base.done = w->base.status + n;
+}
+
 // Carve the per-row buffers for `rows` rows out of one device allocation.
 size_t carve(const Dims& d, int rows, uint8_t* basep, RowBatch* b, size_t* wide_ld_out, int32_t** d_logits) {
 	size_t off = 0;
@@ -390,13 +435,9 @@ size_t carve(const Dims& d, int rows, uint8_t* basep, RowBatch* b, size_t* wide_
 	b->act = (int8_t*)take(R * I);    b->acts = (Scale*)take(R * sizeof(Scale));
 	b->rowmax = (unsigned long long*)take(R * 4 * 8);
 	b->smc = (SoftmaxConsts*)take(R * d.kv_heads * sizeof(SoftmaxConsts));
-	b->status = (int32_t*)take(R * 4);
-	b->done = (int32_t*)take(R * 4);
-	b->sat = (unsigned long long*)take(R * 8);
 	b->sat_layer = (uint32_t*)take(R * d.layers * 4);
 	b->sat_ld = (int)d.layers;
 	b->lora_u = (int8_t*)take(R * 3 * kMaxLoraRank);
-	b->best = (unsigned long long*)take(R * 8);
 	*d_logits = (int32_t*)take((size_t)d.vocab * 4 * std::min<size_t>(R, 64));
 	*wide_ld_out = wide_ld;
 	return align_up(off, 256);
@@ -417,18 +458,10 @@ sslm_workspace_s* create_workspace(sslm_model_s* model, const sslm_config& cfg, 
 	bool ok = cuda_ok(cudaMalloc((void**)&w->d_scratch, w->scratch_bytes));
 	ok = ok && cuda_ok(cudaMemset(w->d_scratch, 0, w->scratch_bytes));
 	ok = ok && cuda_ok(cudaStreamCreateWithFlags(&w->stream, cudaStreamNonBlocking));
-	ok = ok && cuda_ok(cudaMallocHost((void**)&w->h_rows, rows * sizeof(RowDesc)));
-	ok = ok && cuda_ok(cudaMallocHost((void**)&w->h_src, rows * sizeof(RowSource)));
-	ok = ok && cuda_ok(cudaMallocHost((void**)&w->h_sink, rows * sizeof(RowSink)));
-	ok = ok && cuda_ok(cudaMallocHost((void**)&w->h_status, rows * 4));
-	ok = ok && cuda_ok(cudaMallocHost((void**)&w->h_done, rows * 4));
-	ok = ok && cuda_ok(cudaMallocHost((void**)&w->h_sat, rows * 8));
-	ok = ok && cuda_ok(cudaMallocHost((void**)&w->h_best, rows * 8));
-	ok = ok && cuda_ok(cudaMalloc((void**)&w->d_rows, rows * sizeof(RowDesc)));
-	ok = ok && cuda_ok(cudaMalloc((void**)&w->d_src, rows * sizeof(RowSource)));
-	ok = ok && cuda_ok(cudaMalloc((void**)&w->d_sink, rows * sizeof(RowSink)));
-	ok = ok && cuda_ok(cudaMallocHost((void**)&w->h_row_mask, rows * sizeof(void*)));
-	ok = ok && cuda_ok(cudaMalloc((void**)&w->d_row_mask, rows * sizeof(void*)));
+	ok = ok && cuda_ok(cudaMallocHost((void**)&w->h_up, rows * kUpBytesPerRow));
+	ok = ok && cuda_ok(cudaMalloc((void**)&w->d_up, rows * kUpBytesPerRow));
+	ok = ok && cuda_ok(cudaMallocHost((void**)&w->h_down, rows * kDownBytesPerRow));
+	ok = ok && cuda_ok(cudaMalloc((void**)&w->d_down, rows * kDownBytesPerRow));
 	ok = ok && cuda_ok(cudaEventCreate(&w->ev0)) && cuda_ok(cudaEventCreate(&w->ev1));
 	if (ok && rows > 8) {
 		// K slices times tiles never exceeds the SM count, and a tile is at most 256 x 64
@@ -456,18 +489,10 @@ static void destroy_workspace(sslm_workspace_s* w) {
 	cudaFree(w->d_scratch);
 	cudaFree(w->d_tc_partial);
 	cudaFree(w->d_tc_counters);
-	cudaFree(w->d_rows);
-	cudaFree(w->d_src);
-	cudaFree(w->d_sink);
-	cudaFree(w->d_row_mask);
-	cudaFreeHost(w->h_row_mask);
-	cudaFreeHost(w->h_rows);
-	cudaFreeHost(w->h_src);
-	cudaFreeHost(w->h_sink);
-	cudaFreeHost(w->h_status);
-	cudaFreeHost(w->h_done);
-	cudaFreeHost(w->h_sat);
-	cudaFreeHost(w->h_best);
+	cudaFree(w->d_up);
+	cudaFree(w->d_down);
+	cudaFreeHost(w->h_up);
+	cudaFreeHost(w->h_down);
 	if (w->ev0) cudaEventDestroy(w->ev0);
 	if (w->ev1) cudaEventDestroy(w->ev1);
 	for (cudaEvent_t e : w->prof_events) cudaEventDestroy(e);

@@ -35,21 +35,16 @@ struct sslm_workspace_s {
 	cudaStream_t stream = nullptr;
 	uint8_t* d_scratch = nullptr;
 	size_t scratch_bytes = 0;
-	// pinned host staging, row_cap entries each
-	sslm::RowDesc* h_rows = nullptr;
-	sslm::RowSource* h_src = nullptr;
-	sslm::RowSink* h_sink = nullptr;
-	int32_t* h_status = nullptr;
-	int32_t* h_done = nullptr;
-	unsigned long long* h_sat = nullptr;
-	unsigned long long* h_best = nullptr;
-	// device mirrors
-	sslm::RowDesc* d_rows = nullptr;
-	sslm::RowSource* d_src = nullptr;
-	sslm::RowSink* d_sink = nullptr;
+	// What a call uploads and reads back, one copy each way: pinned blocks and their device twins, laid
+	// out for the rows of the call (bind_rows); the pointers below are those of the current call.
+	uint8_t *h_up = nullptr, *d_up = nullptr, *h_down = nullptr, *d_down = nullptr;
+	sslm::RowDesc *h_rows = nullptr, *d_rows = nullptr;
+	sslm::RowSource *h_src = nullptr, *d_src = nullptr;
+	sslm::RowSink *h_sink = nullptr, *d_sink = nullptr;
 	// head rows of constrained sequences: the mask page of the row's DFA state (else nullptr)
-	const uint8_t** h_row_mask = nullptr;   // pinned
-	const uint8_t** d_row_mask = nullptr;
+	const uint8_t **h_row_mask = nullptr, **d_row_mask = nullptr;
+	unsigned long long *h_best = nullptr, *h_sat = nullptr;
+	int32_t *h_status = nullptr, *h_done = nullptr;
 	// carved row buffers (base pointers for row 0)
 	sslm::RowBatch base{};
 	size_t wide_ld = 0;
@@ -113,6 +108,17 @@ struct sslm_model_s {
 	sslm::SchemaTable schemas;
 	std::vector<sslm_schema_s> schema_handles;
 	uint8_t* d_schema_pages = nullptr;
+	// Work of the verbs that move sequence state (adoption, save, restore) runs on a stream of its own;
+	// aux_done is recorded after every piece of it, and the streams of prefill and decode wait for it
+	// when one of their sequences has such work outstanding (sslm_seq_s::pending).
+	cudaStream_t aux = nullptr;
+	cudaEvent_t aux_done = nullptr;
+	std::mutex aux_mutex;
+	// staging of save and restore: a pinned block and its device twin, at most one sequence's K/V, kept
+	// from call to call (under stage_mutex) and freed with the model
+	std::mutex stage_mutex;
+	uint8_t *h_stage = nullptr, *d_stage = nullptr;
+	size_t stage_bytes = 0;
 };
 
 struct sslm_kv_pool_s {
@@ -126,6 +132,11 @@ struct sslm_kv_pool_s {
 	// holders per page: a frozen prefix's full pages are shared, read-only, by every sequence
 	// that adopted it; a page returns to the free list when its last holder lets go
 	std::vector<uint32_t> page_refs;
+	// state slots and page tables of the block_count sequences that can exist, behind the pages in the
+	// same allocation: creating or releasing a sequence calls no allocator of the device
+	uint8_t* d_seq = nullptr;
+	size_t seq_stride = 0;
+	std::vector<int32_t> free_slots;
 	std::atomic<uint32_t> live_refs{0};
 };
 
@@ -142,11 +153,16 @@ struct sslm_adapter_s {
 struct sslm_seq_s {
 	sslm_model_s* model = nullptr;
 	sslm_kv_pool_s* pool = nullptr;
+	int32_t pool_slot = -1;
 	uint8_t* d_state = nullptr;     // two (hidden codes + carried scale) slots
+	bool state_zero = true;         // the committed slot counts as zero bytes, whatever it holds
+	bool pending = false;           // an adoption is on its way on the model's aux stream
 	size_t state_stride = 0, scale_off = 0;
 	int cur = 0;                    // slot holding the committed stream
 	std::vector<int32_t> pages;     // page ids in position order
 	int32_t* d_pages = nullptr;     // device page table, pages_per_block entries
+	size_t pages_on_device = 0;     // entries of it that are in place
+	uint64_t batch_mark = 0;        // the decode batch the sequence was last put into
 	int64_t context_length = 0;
 	uint32_t layer_index = 0;
 	int32_t current_token = -1;

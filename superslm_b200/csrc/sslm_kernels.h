@@ -189,16 +189,27 @@ void attn_force_splits(int splits);
 bool launch_attention(const RowBatch& b, const Dims& d, const LayerDev* layer, const LayerDev& h, int layer_index,
                       KvPoolDev pool, int max_width, int reverse_rows, cudaStream_t st, cudaError_t* err);
 // gather a sequence's pages into the reference's canonical block layout
-// [layer][K|V][kv_head][position][head_dim]; positions beyond `valid(layer)` are zero
+// [layer][K|V][kv_head][position][head_dim] with `span` positions per plane; positions beyond
+// `valid(layer)` are zero
 void launch_kv_export(const Dims& d, KvPoolDev pool, const int32_t* pages, int context_length,
-                      int layer_index, int8_t* out, cudaStream_t st);
+                      int layer_index, int span, int8_t* out, cudaStream_t st);
 // tests: the device integer primitives over arrays of operands (device pointers)
 void launch_int_sweep(int which, const int64_t* a, const int64_t* b, const int64_t* c, const int64_t* e, long long n, int64_t* out0,
                       int64_t* out1, int64_t* out2, cudaStream_t st);
-// copy page src_page to dst_page in every (layer, kv head, K|V) plane
-void launch_page_copy(const Dims& d, KvPoolDev pool, int src_page, int dst_page, cudaStream_t st);
+// What a sequence takes over from a frozen prefix of its pool: the page ids of the full pages, a private
+// copy of the last, partly filled one (copy_from < 0: none), the stream state.
+struct AdoptArgs {
+	const int32_t* src_pages;
+	int32_t* dst_pages;
+	int full_pages;
+	int32_t copy_from, copy_to;
+	const int8_t* src_state;
+	int8_t* dst_state;
+	int state_bytes;      // a multiple of 16
+};
+void launch_adopt(const Dims& d, KvPoolDev pool, const AdoptArgs& a, cudaStream_t st);
 // the inverse: scatter a canonical block into the sequence's pages (valid positions only)
 void launch_kv_import(const Dims& d, KvPoolDev pool, const int32_t* pages, int context_length,
-                      int layer_index, const int8_t* in, cudaStream_t st);
+                      int layer_index, int span, const int8_t* in, cudaStream_t st);
 
 }  // namespace sslm

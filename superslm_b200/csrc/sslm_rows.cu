@@ -239,6 +239,8 @@ k_begin(RowBatch b, Dims d, const int8_t* embed, Scale c_embed, const RowSource*
 		b.sat[r] = 0ull;
 		b.done[r] = 0;
 		b.best[r] = 0ull;      // the head accumulates its arg-max key here
+		const RowDesc& rd = b.rows[r];
+		if (rd.new_page >= 0) ((int32_t*)rd.pages)[rd.pos / kPageTokens] = rd.new_page;
 	}
 	for (int i = threadIdx.x; i < b.sat_ld; i += blockDim.x) b.sat_layer[(size_t)r * b.sat_ld + i] = 0u;
 	const RowSource s = src[r];

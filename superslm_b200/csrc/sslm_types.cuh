@@ -75,6 +75,8 @@ struct RowDesc {
 	const LoraLayerDev* lora;   // the sequence's adapter, per-layer array, or nullptr
 	int32_t pos;                // position this token occupies
 	int32_t token;              // token id to embed when the row starts a token
+	int32_t new_page;           // page id of position pos that the table does not hold yet (k_begin writes it), or -1
+	int32_t pad;
 };
 
 struct RowSource { const int8_t* hidden; const Scale* scale; };  // nullptr hidden: embed rows[r].token
