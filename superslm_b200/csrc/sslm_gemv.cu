@@ -16,7 +16,11 @@
 // little data) finishes, this kernel's weight stream is already running.
 //
 // The epilogue applies the per-channel weight-scale fold, adds the LoRA delta, stores the wide
-// row and reduces the per-row max |x| the funnel needs (or the argmax key for the head).
+// row and reduces the per-row max |x| the funnel needs (or the argmax key for the head). It runs once
+// per launch, so it is short and there is a kernel for each of its uses (int32 rows, int64 rows with
+// adapters, the head): with all uses in one body it took 1.3 us of a 3.6 us launch, mostly instruction
+// fetches. The fold rows are asked for before the first weights: behind the weight stream they came
+// 2 us after the dependency wait would have returned (gate/up of one row, 27.5 MB).
 // (GemmInt8AccumulateRow + ApplyWeightScaleFold + AddAmplifyingLoraDelta,
 //  src/matmul.cpp:455-464, src/forward/forward_sites.cpp:461-470, :1051-1103.)
 // int32 accumulation is exact: K * 127 * 128 < 2^31 for every K the loader accepts, and integer
@@ -96,7 +100,8 @@ struct GemvPlan {
 };
 
 // MT rows of x per pass (grid.y walks the row groups).
-template <int MT>
+enum GemvMode { kGemvRows32 = 0, kGemvRows64, kGemvHead };
+template <int MT, int MODE>
 __global__ void __launch_bounds__(kGemvThreads)
 k_gemv(LinearArgs a, GemvPlan p) {
 	extern __shared__ __align__(128) unsigned char smem[];
@@ -106,13 +111,13 @@ k_gemv(LinearArgs a, GemvPlan p) {
 	const int m0 = blockIdx.y * MT;
 	const int mcount = min(MT, a.M - m0);
 	const int slot_bytes = p.rows_per_item * p.seg16 * 16;
-	// carve: rings | x rows | accumulators | fold rows | maxima | barriers
+	// carve: rings | x rows | accumulators | fold rows | arg-max keys | barriers
 	unsigned char* rings = smem;
 	int8_t* sx = (int8_t*)(rings + (size_t)kGemvWarps * p.slots * slot_bytes);
 	int* sacc = (int*)(sx + (size_t)MT * K);                                   // [MT][rows_per_block]
 	int32_t* sfold = sacc + (size_t)MT * p.rows_per_block;                     // [rows_per_block][3]
-	unsigned long long* smax = (unsigned long long*)(((uintptr_t)(sfold + 3 * (size_t)p.rows_per_block) + 7) & ~(uintptr_t)7);   // [4][MT]
-	const uint32_t bars = smem_addr(smax + 4 * MT);                            // [warps][kMaxSlots]
+	unsigned long long* sbest = (unsigned long long*)(((uintptr_t)(sfold + 3 * (size_t)p.rows_per_block) + 7) & ~(uintptr_t)7);   // [MT]
+	const uint32_t bars = smem_addr(sbest + MT);                               // [warps][kMaxSlots]
 	__shared__ int s_timeout;
 
 	const int t = threadIdx.x, warp = t >> 5, lane = t & 31;
@@ -148,17 +153,18 @@ k_gemv(LinearArgs a, GemvPlan p) {
 	}
 	if (t == 0) s_timeout = 0;
 	__syncwarp();
-	// ahead of the dependency wait: the first copies of every ring, the block's fold rows, cleared
+	// ahead of the dependency wait: the block's fold rows, the first copies of every ring, cleared
 	// accumulators and maxima
+	if (MODE != kGemvHead && a.fold != nullptr) {
+		const int32_t* f = a.fold + (size_t)n0 * 3;
+		for (int i = t; i < nrows * 3; i += kGemvThreads)
+			asm volatile("cp.async.ca.shared.global [%0], [%1], 4;" ::"r"(smem_addr(sfold + i)), "l"(f + i) : "memory");
+	}
 	int issued = items < p.slots ? items : p.slots;      // items whose copies have been requested
 	if (lane == 0)
 		for (int i = 0; i < issued; ++i) issue();
-	if (a.fold != nullptr) {
-		const int32_t* f = a.fold + (size_t)n0 * 3;
-		for (int i = t; i < nrows * 3; i += kGemvThreads) sfold[i] = __ldg(f + i);
-	}
 	for (int i = t; i < MT * p.rows_per_block; i += kGemvThreads) sacc[i] = 0;
-	if (t < 4 * MT) smax[t] = 0ull;
+	if (t < MT) sbest[t] = 0ull;
 	pdl_wait();
 	pdl_release();
 	// the activation rows (written by the kernel in front: read past the L1)
@@ -185,24 +191,38 @@ k_gemv(LinearArgs a, GemvPlan p) {
 		const int nr = min(p.rows_per_item, nrows - row0);
 		const int first = c_s * p.seg16, count = min(p.seg16, k16 - first);
 		const int4* wv = (const int4*)(ring + (size_t)sl * slot_bytes);
-		for (int rr = 0; rr < nr; ++rr) {
-			int acc[MT];
+		// RU weight rows side by side; one reduction per (row of x, weight row segment). Segments of one
+		// weight row may belong to different warps, so the sums meet in shared memory.
+		constexpr int RU = MT == 1 ? 3 : 1;
+#pragma unroll 1
+		for (int rr = 0; rr < nr; rr += RU) {
+			int acc[RU][MT];
 #pragma unroll
-			for (int m = 0; m < MT; ++m) acc[m] = 0;
+			for (int u = 0; u < RU; ++u)
+#pragma unroll
+				for (int m = 0; m < MT; ++m) acc[u][m] = 0;
 #pragma unroll 2
 			for (int c = lane; c < count; c += 32) {
-				const int4 w4 = wv[rr * count + c];
+				int4 xv[MT];
 #pragma unroll
-				for (int m = 0; m < MT; ++m) acc[m] = dot16(w4, ((const int4*)(sx + (size_t)m * K))[first + c], acc[m]);
+				for (int m = 0; m < MT; ++m) xv[m] = ((const int4*)(sx + (size_t)m * K))[first + c];
+#pragma unroll
+				for (int u = 0; u < RU; ++u) {
+					const int4 w4 = wv[min(rr + u, nr - 1) * count + c];
+#pragma unroll
+					for (int m = 0; m < MT; ++m) acc[u][m] = dot16(w4, xv[m], acc[u][m]);
+				}
 			}
-			// one reduction per (row of x, weight row segment); segments of one weight row may
-			// belong to different warps, so the sums meet in shared memory
 #pragma unroll
-			for (int m = 0; m < MT; ++m) {
-				const int v = __reduce_add_sync(0xffffffffu, acc[m]);
-				if (lane == 0) {
-					if (p.nseg == 1) sacc[m * p.rows_per_block + row0 + rr] = v;
-					else atomicAdd(&sacc[m * p.rows_per_block + row0 + rr], v);
+			for (int u = 0; u < RU; ++u) {
+#pragma unroll
+				for (int m = 0; m < MT; ++m) {
+					const int v = __reduce_add_sync(0xffffffffu, acc[u][m]);
+					if (lane == 0 && (RU == 1 || rr + u < nr)) {
+						int* to = &sacc[m * p.rows_per_block + row0 + rr + u];
+						if (p.nseg == 1) *to = v;
+						else atomicAdd(to, v);
+					}
 				}
 			}
 		}
@@ -229,6 +249,7 @@ k_gemv(LinearArgs a, GemvPlan p) {
 			bar_wait(full_bar(s), (uint32_t)(last / p.slots) & 1u);
 		}
 	}
+	asm volatile("cp.async.wait_all;" ::: "memory");
 	__syncthreads();
 
 	if (*(volatile int*)&s_timeout) {
@@ -238,94 +259,95 @@ k_gemv(LinearArgs a, GemvPlan p) {
 		}
 		return;
 	}
-	// ---- epilogue: thread i takes output (m, n) = (i / nrows, i % nrows)
-	unsigned long long lmax[3] = {0ull, 0ull, 0ull};
-	unsigned long long lbest = 0ull;
-	int my_m = -1;
-	auto flush = [&]() {
-		if (my_m < 0) return;
-		if (a.best != nullptr) {
-			if (lbest) atomicMax(&smax[3 * MT + my_m], lbest);
-		} else {
-#pragma unroll
-			for (int sg = 0; sg < 3; ++sg)
-				if (lmax[sg]) atomicMax(&smax[sg * MT + my_m], lmax[sg]);
-		}
-		lmax[0] = lmax[1] = lmax[2] = 0ull;
-		lbest = 0ull;
-	};
-	for (int i = t; i < mcount * nrows; i += kGemvThreads) {
-		const int m = i / nrows, nl0 = i - m * nrows;
-		if (m != my_m) {      // (a thread's outputs belong to one row of x except when the block has few channels)
-			flush();
-			my_m = m;
-		}
+	// ---- epilogue: thread i takes output (m, n) = (i / nrows, i % nrows); a warp's outputs mostly belong to
+	// one row and segment and then share one atomic
+	const int outputs = mcount * nrows;
+#pragma unroll 1
+	for (int i0 = 0; i0 < outputs; i0 += kGemvThreads) {
+		const int i = i0 + t;
+		if (i0 + (t & ~31) >= outputs) break;
+		const bool in = i < outputs;
+		const int m = MT == 1 ? 0 : min(i, outputs - 1) / nrows, nl0 = in ? i - m * nrows : 0;
 		const int n = n0 + nl0, rowg = m0 + m;
-		const int mine = sacc[m * p.rows_per_block + nl0];
-		int seg = 0;
-		while (seg + 1 < a.nseg && n >= a.seg_end[seg]) ++seg;
-		int32_t v32 = mine;
-		if (a.fold) v32 = fold(mine, sfold[3 * nl0], sfold[3 * nl0 + 1], sfold[3 * nl0 + 2]);
-		int64_t v = v32;
-		if (a.rows != nullptr && a.seg_lora[seg] >= 0) {
-			const LoraLayerDev* ll = a.rows[rowg].lora;
-			if (ll != nullptr) {
-				const LoraLayerDev& L = ll[a.layer];
-				const LoraProjDev& pj = L.p[a.seg_lora[seg]];
-				if (pj.a != nullptr) {
-					const int nl = n - (seg ? a.seg_end[seg - 1] : 0);
-					const int8_t* brow = pj.b + (size_t)nl * L.rank;
-					const int8_t* u = a.lora_u + ((size_t)rowg * 3 + seg) * kMaxLoraRank;
-					int dsum = 0;
-					for (uint32_t r = 0; r < L.rank; ++r) dsum += (int)brow[r] * (int)u[r];
-					v += (int64_t)amp_fold(dsum, pj.df[3 * nl], pj.df[3 * nl + 1], pj.df[3 * nl + 2]);
-				}
-			}
-		}
-		if (a.best != nullptr) {
-			if (a.row_mask != nullptr) {
+		const int32_t mine = sacc[m * p.rows_per_block + nl0];
+		// (the exchanges stand by themselves: every lane of the warp takes part in them)
+		const int m_first = __shfl_sync(0xffffffffu, m, 0);
+		const bool same_m = __all_sync(0xffffffffu, !in || m == m_first) != 0;
+		if (MODE == kGemvHead) {
+			int32_t v32 = mine;
+			if (in && a.row_mask != nullptr) {
 				const uint8_t* page = a.row_mask[rowg];
 				if (page != nullptr && !((page[n >> 3] >> (n & 7)) & 1u)) v32 = INT32_MIN;
 			}
-			const unsigned long long key =
-			    ((unsigned long long)((uint32_t)v32 ^ 0x80000000u) << 32) | (0xFFFFFFFFu - (uint32_t)n);
-			lbest = key > lbest ? key : lbest;
-			if (a.logits) a.logits[(size_t)rowg * a.N + n] = v32;
-		} else {
-			if (a.out64) ((int64_t*)a.out)[(size_t)rowg * a.out_ld + n] = v;
-			else ((int32_t*)a.out)[(size_t)rowg * a.out_ld + n] = (int32_t)v;
-			if (a.seg_slot[seg] >= 0) {
-				const unsigned long long ab = v < 0 ? (~(unsigned long long)v + 1ull) : (unsigned long long)v;
-				lmax[seg] = ab > lmax[seg] ? ab : lmax[seg];
+			if (in && a.logits != nullptr) a.logits[(size_t)rowg * a.N + n] = v32;
+			const uint32_t u = in ? (uint32_t)v32 ^ 0x80000000u : 0u;
+			if (same_m) {      // lanes ascend in n: the first lane that holds the maximum is the lowest index
+				const uint32_t top = __reduce_max_sync(0xffffffffu, u);
+				const uint32_t who = __ballot_sync(0xffffffffu, in && u == top);
+				if (lane == __ffs(who) - 1) atomicMax(&sbest[m], ((unsigned long long)top << 32) | (0xFFFFFFFFu - (uint32_t)n));
+			} else if (in) {
+				atomicMax(&sbest[m], ((unsigned long long)u << 32) | (0xFFFFFFFFu - (uint32_t)n));
 			}
+			continue;
+		}
+		const int seg = (n >= a.seg_end[0] && a.nseg > 1 ? 1 : 0) + (n >= a.seg_end[1] && a.nseg > 2 ? 1 : 0);
+		int32_t v32 = mine;
+		if (a.fold != nullptr) v32 = fold(mine, sfold[3 * nl0], sfold[3 * nl0 + 1], sfold[3 * nl0 + 2]);
+		uint32_t mag = v32 < 0 ? 0u - (uint32_t)v32 : (uint32_t)v32;
+		if (MODE == kGemvRows32) {
+			if (in) ((int32_t*)a.out)[(size_t)rowg * a.out_ld + n] = v32;
+		} else {
+			int64_t v = v32;
+			if (in && a.rows != nullptr && a.seg_lora[seg] >= 0) {
+				const LoraLayerDev* ll = a.rows[rowg].lora;
+				if (ll != nullptr) {
+					const LoraLayerDev& L = ll[a.layer];
+					const LoraProjDev& pj = L.p[a.seg_lora[seg]];
+					if (pj.a != nullptr) {
+						const int nl = n - (seg ? a.seg_end[seg - 1] : 0);
+						const int8_t* brow = pj.b + (size_t)nl * L.rank;
+						const int8_t* u = a.lora_u + ((size_t)rowg * 3 + seg) * kMaxLoraRank;
+						int dsum = 0;
+						for (uint32_t r = 0; r < L.rank; ++r) dsum += (int)brow[r] * (int)u[r];
+						v += (int64_t)amp_fold(dsum, pj.df[3 * nl], pj.df[3 * nl + 1], pj.df[3 * nl + 2]);
+					}
+				}
+			}
+			if (in) ((int64_t*)a.out)[(size_t)rowg * a.out_ld + n] = v;
+			// (magnitudes above 32 bits count as 2^32 - 1: the funnel refuses everything above 2^31)
+			const unsigned long long ab = v < 0 ? (~(unsigned long long)v + 1ull) : (unsigned long long)v;
+			mag = ab > 0xFFFFFFFFull ? 0xFFFFFFFFu : (uint32_t)ab;
+		}
+		if (!in) mag = 0u;
+		if (a.rowmax != nullptr) {
+			const int seg_first = __shfl_sync(0xffffffffu, seg, 0);
+			const bool same = __all_sync(0xffffffffu, !in || (m == m_first && seg == seg_first)) != 0;
+			if (same) {
+				mag = __reduce_max_sync(0xffffffffu, mag);
+				if (lane != 0) mag = 0u;
+			}
+			if (mag != 0u && a.seg_slot[seg] >= 0) atomicMax(&a.rowmax[(size_t)rowg * 4 + a.seg_slot[seg]], (unsigned long long)mag);
 		}
 	}
-	flush();
-	__syncthreads();
-	if (t < 4 * MT) {
-		const int sg = t / MT, m = t % MT;
-		const unsigned long long v = smax[t];
-		if (v != 0ull && m < mcount) {
-			if (sg == 3) atomicMax(&a.best[m0 + m], v);
-			else if (a.rowmax != nullptr && sg < a.nseg && a.seg_slot[sg] >= 0)
-				atomicMax(&a.rowmax[(size_t)(m0 + m) * 4 + a.seg_slot[sg]], v);
-		}
+	if (MODE == kGemvHead) {
+		__syncthreads();
+		if (t < mcount && sbest[t] != 0ull) atomicMax(&a.best[m0 + t], sbest[t]);
 	}
 }
 
-// shared memory of one block: rings, activation rows, accumulators, fold rows, maxima, barriers
+// shared memory of one block: rings, activation rows, accumulators, fold rows, arg-max keys, barriers
 static size_t gemv_smem_bytes(int mt, int K, int rows_per_block, int slots, int slot_bytes) {
 	return (size_t)kGemvWarps * slots * slot_bytes + (size_t)mt * K + (size_t)mt * rows_per_block * 4 +
-	       (size_t)rows_per_block * 12 + 8 + (size_t)4 * mt * 8 + (size_t)kGemvWarps * kMaxSlots * 8 + 16;
+	       (size_t)rows_per_block * 12 + 8 + (size_t)mt * 8 + (size_t)kGemvWarps * kMaxSlots * 8 + 16;
 }
 
-template <int MT>
-static cudaError_t launch_mt(const LinearArgs& a, int grid_y, cudaStream_t st) {
+template <int MT, int MODE>
+static cudaError_t launch_mode(const LinearArgs& a, int grid_y, cudaStream_t st) {
 	static PerDeviceOnce configured;
 	cudaError_t e = once_per_device(configured, [] {
-		cudaError_t c = cudaFuncSetAttribute(k_gemv<MT>, cudaFuncAttributeMaxDynamicSharedMemorySize, 220 * 1024);
+		cudaError_t c = cudaFuncSetAttribute(k_gemv<MT, MODE>, cudaFuncAttributeMaxDynamicSharedMemorySize, 220 * 1024);
 		if (c != cudaSuccess) return c;
-		return cudaFuncSetAttribute(k_gemv<MT>, cudaFuncAttributePreferredSharedMemoryCarveout, cudaSharedmemCarveoutMaxShared);
+		return cudaFuncSetAttribute(k_gemv<MT, MODE>, cudaFuncAttributePreferredSharedMemoryCarveout, cudaSharedmemCarveoutMaxShared);
 	});
 	if (e != cudaSuccess) return e;
 	GemvPlan p;
@@ -366,7 +388,13 @@ static cudaError_t launch_mt(const LinearArgs& a, int grid_y, cudaStream_t st) {
 	const size_t smem = gemv_smem_bytes(MT, a.K, rpb, slots, slot_bytes);
 	if (smem > 220 * 1024) return cudaErrorInvalidConfiguration;
 	const int gx = (a.N + rpb - 1) / rpb;
-	return launch_ordered(a.caller_memory == 0, k_gemv<MT>, dim3(gx, grid_y), dim3(kGemvThreads), smem, st, a, p);
+	return launch_ordered(a.caller_memory == 0, k_gemv<MT, MODE>, dim3(gx, grid_y), dim3(kGemvThreads), smem, st, a, p);
+}
+
+template <int MT>
+static cudaError_t launch_mt(const LinearArgs& a, int grid_y, cudaStream_t st) {
+	if (a.best != nullptr) return launch_mode<MT, kGemvHead>(a, grid_y, st);
+	return a.out64 ? launch_mode<MT, kGemvRows64>(a, grid_y, st) : launch_mode<MT, kGemvRows32>(a, grid_y, st);
 }
 
 cudaError_t launch_linear_gemv(const LinearArgs& a, cudaStream_t st) {

@@ -447,17 +447,28 @@ k_skinny(const __grid_constant__ CUtensorMap map_w, const __grid_constant__ CUte
 						tmem_ld16(tmem + ((uint32_t)(q * 32) << 16) + as * NB + col0 + c0, r);
 						const int mine = col0 + c0 + (lane >> 1);      // the row whose maximum this lane ends up with
 						if (MODE == kHead) {
-							if (a.row_mask != nullptr || a.logits != nullptr) {
+							if (a.row_mask != nullptr) {
+								// lane j fetches the mask word of row j for this warp's 32 channels
+								uint32_t allowed = 0xFFFFFFFFu;
+								const int m = col0 + c0 + lane, w0 = (n0 + q * 32) >> 3;
+								if (lane < 16 && m < a.M) {
+									const uint8_t* page = a.row_mask[m];
+									if (page != nullptr) {
+										const int last = (a.N + 7) >> 3;
+										allowed = 0u;
 #pragma unroll
-								for (int j = 0; j < 16; ++j) {
-									const int m = col0 + c0 + j;
-									if (m >= a.M || !c.in) continue;
-									if (a.row_mask != nullptr) {
-										const uint8_t* page = a.row_mask[m];
-										if (page != nullptr && !((page[c.n >> 3] >> (c.n & 7)) & 1u)) r[j] = 0x80000000u;      // INT32_MIN
+										for (int b = 0; b < 4; ++b)
+											if (w0 + b < last) allowed |= (uint32_t)__ldg(page + w0 + b) << (8 * b);
 									}
-									if (a.logits != nullptr) a.logits[(size_t)m * a.N + c.n] = (int32_t)r[j];
 								}
+#pragma unroll
+								for (int j = 0; j < 16; ++j)
+									if (!((__shfl_sync(0xffffffffu, allowed, j) >> lane) & 1u)) r[j] = 0x80000000u;      // INT32_MIN
+							}
+							if (a.logits != nullptr) {
+#pragma unroll
+								for (int j = 0; j < 16; ++j)
+									if (col0 + c0 + j < a.M && c.in) a.logits[(size_t)(col0 + c0 + j) * a.N + c.n] = (int32_t)r[j];
 							}
 							// greedy argmax key, lowest index wins ties
 #pragma unroll
