@@ -21,6 +21,7 @@
 // GemmProbQ15Accumulate (src/matmul.cpp:522-538).
 #include <cuda_runtime.h>
 
+#include <algorithm>
 #include <atomic>
 
 #include "sslm_cluster.cuh"
@@ -1088,6 +1089,521 @@ static cudaError_t launch_attn_tile(const RowBatch& b, const Dims& d, const Laye
 	                  d, layer, layer_index, pool, tq);
 }
 
+// ------------------------------------------------------------ prefill chunks
+// The rows of a prefill chunk are consecutive positions of ONE sequence, so neighbouring tokens read
+// almost the same K / V prefix. A block takes 32 query rows -- tq consecutive tokens times the q heads of
+// one kv head, two 16-row MMA blocks -- and up to 512 positions of their prefix in steps of 128. The exact
+// integer softmax needs the row maximum before any exponential and the row total before any probability;
+// a block keeps its scores in shared memory, every thread its own elements, so K is multiplied once, V
+// once, and the softmax passes touch no other thread's data:
+//   1  scores of a step on the tensor cores, masked by each row's causal limit; row maxima
+//   2  exponentials and row totals; a score's place then holds the element's (shift, base)
+//   3  probabilities, packed in place as the A fragments of P.V (two u8 planes)
+//   4  P.V on the tensor cores, a warp per quarter of the channels, context fold
+// The K rows of a 16-position group are read in an order (0 1 4 5 8 9 12 13 | 2 3 6 7 10 11 14 15) that
+// leaves a lane of the score MMAs with four neighbouring positions, which is what a lane of the P.V MMAs
+// holds: probabilities go from one to the other as whole words.
+// A tile whose prefix is longer is split over the blocks of a cluster (step s goes to block s mod `sub`),
+// which exchange maxima, totals and shares of P.V. Clusters have one size per launch: one takes a single
+// wide tile, or two of half the width, or four ... (ChunkPlan). The widest tiles start first.
+//
+// Bound by the integer instructions of the softmax. One layer, before: the prefix walked three times with
+// recomputed scores, 64 rows per block, 186 us for 2,047 positions at the 1.5B widths; one block per row,
+// 21 us for 512 positions at the 0.5B widths.
+constexpr int kChunkRows = 32, kChunkStep = 128, kChunkThreads = 256, kChunkSteps = 4;
+struct ChunkPlan {
+	int tq;            // tokens per tile
+	int steps;         // steps of 128 positions a block holds at most
+	int cluster;       // blocks per cluster
+	int count[4];      // tiles split `cluster`, cluster / 2, cluster / 4, cluster / 8 ways, widest first
+};
+
+template <int HD>
+struct ChunkSmem {
+	static constexpr int kKStride = HD + 16;
+	static constexpr size_t kStage = (size_t)2 * kChunkStep * kKStride;              // two K steps, or two V steps, or received shares
+	static constexpr size_t kScores = (size_t)kChunkRows * kChunkStep * 4;           // per step
+	static constexpr size_t kMisc = kChunkRows * sizeof(IExpFast) + kChunkRows * (8 + 4 + 4) + 8 * 3 * 4 + kChunkSteps * 8 * 8 +
+	                                8 * kChunkRows * (4 + 8);
+	__host__ __device__ static constexpr size_t bytes(int steps) { return kStage + kScores * steps + kMisc; }
+};
+
+__device__ __forceinline__ void ldmatrix4(uint32_t addr, uint32_t& r0, uint32_t& r1, uint32_t& r2, uint32_t& r3) {
+	asm volatile("ldmatrix.sync.aligned.m8n8.x4.shared.b16 {%0, %1, %2, %3}, [%4];" : "=r"(r0), "=r"(r1), "=r"(r2), "=r"(r3) : "r"(addr) : "memory");
+}
+
+// A row's constants of the probability pass. pf = (base^2 + q_c) 2^-z 32768 / total in float is within
+// pf 2^-21 (five roundings) + 32768 / total (the element's own floor) of the quotient, so its floor is the
+// probability unless the nearest integer from 1 up is that close; those take prob_q15. Below 1 it is 0.
+struct ChunkProb {
+	float c, qc, eps;
+};
+__device__ __forceinline__ ChunkProb chunk_prob(unsigned long long total, const IExpFast& f) {
+	ChunkProb p;
+	p.c = 32768.0f / (float)(total > 1ull ? total : 1ull);
+	p.qc = (float)f.qc;
+	p.eps = p.c * 1.01f;
+	return p;
+}
+constexpr uint32_t kBaseOfZero = 63u << 24;      // (shift, base) of an element that counts for nothing
+__device__ __forceinline__ int64_t chunk_exp(uint32_t dq, const IExpFast& f, uint32_t* parts) {
+	const uint32_t x = min(dq, f.clip);
+	uint32_t z = (uint32_t)__float_as_int(__fmaf_rz(__uint2float_rn(x), f.inv_ln2, 8388608.0f)) - 0x4B000000u;
+	uint32_t rem = x - z * f.ln2;
+	if (rem >= f.ln2) {
+		rem -= f.ln2;
+		++z;
+	}
+	const uint32_t base = (uint32_t)f.qb - rem;      // 1 .. q_b < 2^24
+	*parts = (z << 24) + base;
+	return (int64_t)(((uint64_t)base * base + (uint64_t)f.qc) >> z);
+}
+__device__ __forceinline__ uint32_t chunk_prob_of(uint32_t parts, const ChunkProb& p, float* near) {
+	const float bf = __uint2float_rn(parts & 0xFFFFFFu);
+	const float pf = fmaf(bf, bf, p.qc) * __int_as_float(__float_as_int(p.c) - (int)((parts >> 24) << 23));
+	const float whole = fmaxf((pf + 8388608.0f) - 8388608.0f, 1.0f);
+	*near = fminf(*near, fmaf(pf, -4.76837158203125e-07f, fabsf(pf - whole)));
+	return (uint32_t)__float_as_int(__fadd_rz(pf, 8388608.0f));      // (low 16 bits)
+}
+static __device__ __noinline__ uint4 chunk_prob_exact(uint32_t p0, uint32_t p1, uint32_t p2, uint32_t p3, int64_t qc, unsigned long long total) {
+	const unsigned long long tot = total > 1ull ? total : 1ull;
+	const float rinv = 32768.0f / (float)tot;
+	auto one = [&](uint32_t p) {
+		const uint64_t base = p & 0xFFFFFFu;
+		return (p >> 24) == 63u ? 0u : prob_q15((int64_t)((base * base + (uint64_t)qc) >> (p >> 24)), tot, rinv);
+	};
+	return make_uint4(one(p0), one(p1), one(p2), one(p3));
+}
+
+template <int HD>
+__global__ void __launch_bounds__(kChunkThreads, 2)
+k_attention_chunk(RowBatch b, Dims d, const LayerDev* layer, int layer_index, KvPoolDev pool, ChunkPlan pl) {
+	using L = ChunkSmem<HD>;
+	constexpr int KS = HD / 32;          // MMA steps along the head dimension
+	constexpr int NT = HD / 32;          // 8-channel tiles a warp owns in P.V (a quarter of the channels)
+	extern __shared__ __align__(16) unsigned char smem[];
+	__shared__ __align__(8) unsigned long long s_bars[3];
+	int8_t* stage = (int8_t*)smem;
+	int4* sc = (int4*)(smem + L::kStage);                                     // [step][4][threads]
+	IExpFast* fxs = (IExpFast*)(smem + L::kStage + L::kScores * pl.steps);
+	unsigned long long* rsum = (unsigned long long*)(fxs + kChunkRows);       // [32]
+	unsigned long long* rx_sum = rsum + kChunkRows;                           // [sub][32]
+	int64_t* pbase = (int64_t*)(rx_sum + 8 * kChunkRows);                     // [steps * 8] page offsets inside a plane
+	int32_t* rmax = (int32_t*)(pbase + kChunkSteps * 8);                      // [32]
+	int32_t* rx_max = rmax + kChunkRows;                                      // [sub][32]
+	int32_t* tok_ok = rx_max + 8 * kChunkRows;                                // [32] 1: the token takes part
+	int32_t* l_fold = tok_ok + kChunkRows;                                    // [8][3]
+	int32_t* rx_ctx = (int32_t*)stage;                                        // [sub][32 / sub][HD]
+
+	// which tile, split how many ways
+	const int kvh = blockIdx.z, G = d.heads / d.kv_heads;
+	const int C = pl.cluster, crank = (int)blockIdx.x, total = (b.m + pl.tq - 1) / pl.tq;
+	int sub = C, item = (int)blockIdx.y, before = 0;
+#pragma unroll
+	for (int i = 0; i < 4; ++i) {
+		const int per = C / sub, clusters = (pl.count[i] + per - 1) / per;
+		if (item < clusters || sub == 1 || i == 3) {
+			item = item * per + crank / sub;
+			if (item >= pl.count[i]) item = -1;
+			break;
+		}
+		item -= clusters;
+		before += pl.count[i];
+		sub >>= 1;
+	}
+	const int rank = crank % sub, rank0 = crank - rank;      // in the group of blocks that share the tile
+	const int t = threadIdx.x, warp = t >> 5, lane = t & 31, g = lane >> 2, c = lane & 3;
+	if (sub > 1) {
+		if (t == 0) {
+			exchange_init(cta_addr(&s_bars[0]), (uint32_t)(sub * kChunkRows * 4));
+			exchange_init(cta_addr(&s_bars[1]), (uint32_t)(sub * kChunkRows * 8));
+			exchange_init(cta_addr(&s_bars[2]), (uint32_t)(kChunkRows * HD * 4));
+			exchange_fence_init();
+		}
+		cluster_arrive();
+		cluster_wait();
+	}
+	if (item < 0) {      // no tile for this block: it only meets the others of its cluster
+		if (sub > 1) {
+			cluster_arrive();
+			cluster_wait();
+		}
+		return;
+	}
+	const int tile = total - 1 - before - item;
+	const int r0 = tile * pl.tq, nt = min(pl.tq, b.m - r0);
+	const int rb = warp >> 2, kq = warp & 3;
+	const int rho_a = rb * 16 + g, rho_b = rho_a + 8;
+	const int tok_a = rho_a / G, tok_b = rho_b / G;
+	const int head_a = rho_a - tok_a * G, head_b = rho_b - tok_b * G;
+	// uploaded before the call's first launch: the tile's first position and the sequence's page table
+	const int pos0 = b.rows[r0].pos, old = b.rows[0].pos;
+	const int32_t* pages = b.rows[r0].pages;
+	const int width = pos0 + nt;
+	const int nsteps = ((width + kChunkStep - 1) / kChunkStep - rank + sub - 1) / sub;      // this block's: rank, rank + sub, ...
+	const int8_t* kplane = pool.base + kv_plane_offset(d, pool, layer_index, kvh, 0);
+	const int8_t* vplane = pool.base + kv_plane_offset(d, pool, layer_index, kvh, 1);
+	for (int i = t; i < nsteps * 8; i += kChunkThreads) {
+		const int page = (rank + (i >> 3) * sub) * 8 + (i & 7);
+		pbase[i] = page * kPageTokens < width ? (int64_t)pages[page] * (kPageTokens * HD) : 0;
+	}
+	if (t < 3 * G) l_fold[t] = layer->f_ctx[3 * kvh * G + t];
+	if (t < kChunkRows) {
+		rmax[t] = INT32_MIN;
+		rsum[t] = 0ull;
+	}
+	__syncthreads();
+	// step i of this block into half i & 1 of the stage; positions beyond the tile's width are left as they are
+	// (their scores are masked, their probabilities zero)
+	auto load_k = [&](int i) {
+		int8_t* kd = stage + (size_t)(i & 1) * kChunkStep * L::kKStride;
+		const int base = (rank + i * sub) * kChunkStep;
+		for (int idx = t; idx < kChunkStep * (HD / 16); idx += kChunkThreads) {
+			const int row = idx / (HD / 16), piece = idx % (HD / 16);
+			if (base + row < width)
+				cp_async16(kd + (size_t)row * L::kKStride + piece * 16, kplane + pbase[i * 8 + (row >> 4)] + (row & 15) * HD + piece * 16);
+		}
+		asm volatile("cp.async.commit_group;" ::: "memory");
+	};
+	auto load_v = [&](int i) {
+		int8_t* vd = stage + (size_t)(i & 1) * kChunkStep * HD;
+		const int base = (rank + i * sub) * kChunkStep;
+		for (int idx = t; idx < 8 * HD; idx += kChunkThreads) {
+			const int pg = idx / HD, piece = idx % HD;
+			if (base + pg * kPageTokens < width)
+				cp_async16(vd + (size_t)pg * HD * kPageTokens + piece * 16, vplane + pbase[i * 8 + pg] + piece * 16);
+		}
+		asm volatile("cp.async.commit_group;" ::: "memory");
+	};
+	// positions of earlier calls are in place: the first step need not wait for the kernel in front
+	const bool early = nsteps > 0 && (rank + 1) * kChunkStep <= old;
+	if (early) load_k(0);
+	pdl_wait();
+	pdl_release();
+	if (t < kChunkRows) {
+		int okv = 0;
+		if (t < nt) {
+			okv = __ldcg(&b.status[r0 + t]) == 0 ? 1 : 0;
+			fxs[t] = iexp_fast_prepare(b.smc[(size_t)(r0 + t) * d.kv_heads + kvh]);
+		}
+		tok_ok[t] = okv;
+	}
+	if (nsteps > 0 && !early) load_k(0);
+	__syncthreads();
+	const bool in_a = tok_a < nt && tok_ok[tok_a] != 0, in_b = tok_b < nt && tok_ok[tok_b] != 0;
+	const int lim_a = in_a ? pos0 + tok_a : -1, lim_b = in_b ? pos0 + tok_b : -1;    // last position each row sees
+	bool ok = true;
+
+	// ---- pass 1: scores, kept per thread; row maxima. acc[j]: MMA j = 2 * group + half of a 16-position group
+	{
+		uint32_t qa[KS][4];      // q fragments (A operand) of this warp's rows
+		const int8_t* qpa = b.qrot + (size_t)(r0 + (in_a ? tok_a : 0)) * d.hidden + (size_t)(kvh * G + head_a) * HD;
+		const int8_t* qpb = b.qrot + (size_t)(r0 + (in_b ? tok_b : 0)) * d.hidden + (size_t)(kvh * G + head_b) * HD;
+#pragma unroll
+		for (int ks = 0; ks < KS; ++ks) {
+			qa[ks][0] = in_a ? *(const uint32_t*)(qpa + 32 * ks + 4 * c) : 0u;
+			qa[ks][1] = in_b ? *(const uint32_t*)(qpb + 32 * ks + 4 * c) : 0u;
+			qa[ks][2] = in_a ? *(const uint32_t*)(qpa + 32 * ks + 16 + 4 * c) : 0u;
+			qa[ks][3] = in_b ? *(const uint32_t*)(qpb + 32 * ks + 16 + 4 * c) : 0u;
+		}
+		// the K row that matrix row lane & 7 of half h stands for: 4 * (i / 2) + 2 h + (i & 1)
+		const int krow = 4 * ((lane & 7) >> 1) + (lane & 1);
+		int mx_a = INT32_MIN, mx_b = INT32_MIN;
+#pragma unroll 1
+		for (int i = 0; i < nsteps; ++i) {
+			if (i + 1 < nsteps) {
+				load_k(i + 1);
+				asm volatile("cp.async.wait_group 1;" ::: "memory");
+			} else {
+				asm volatile("cp.async.wait_group 0;" ::: "memory");
+			}
+			__syncthreads();
+			const int base = (rank + i * sub) * kChunkStep;
+			const bool full = base + kChunkStep - 1 <= pos0;      // every row of the tile sees the whole step
+			const uint32_t kd = cta_addr(stage + (size_t)((i & 1) * kChunkStep + kq * 32) * L::kKStride);
+			int acc[4][4];
+#pragma unroll
+			for (int j = 0; j < 4; ++j)
+#pragma unroll
+				for (int q = 0; q < 4; ++q) acc[j][q] = 0;
+			if constexpr (HD == 32) {
+#pragma unroll
+				for (int j = 0; j < 4; j += 2) {      // both halves of a group in one load
+					uint32_t b0, b1, b2, b3;
+					ldmatrix4(kd + (8 * j + krow + 2 * (lane >> 4)) * L::kKStride + ((lane >> 3) & 1) * 16, b0, b1, b2, b3);
+					mma_s8s8_full(acc[j], qa[0][0], qa[0][1], qa[0][2], qa[0][3], b0, b1);
+					mma_s8s8_full(acc[j + 1], qa[0][0], qa[0][1], qa[0][2], qa[0][3], b2, b3);
+				}
+			} else {
+#pragma unroll
+				for (int ks = 0; ks < KS; ks += 2) {
+#pragma unroll
+					for (int j = 0; j < 4; ++j) {
+						uint32_t b0, b1, b2, b3;
+						ldmatrix4(kd + (16 * (j >> 1) + 2 * (j & 1) + krow) * L::kKStride + 32 * ks + (lane >> 3) * 16, b0, b1, b2, b3);
+						mma_s8s8_full(acc[j], qa[ks][0], qa[ks][1], qa[ks][2], qa[ks][3], b0, b1);
+						mma_s8s8_full(acc[j], qa[ks + 1][0], qa[ks + 1][1], qa[ks + 1][2], qa[ks + 1][3], b2, b3);
+					}
+				}
+			}
+			// row a, group p (positions 16 p + 4 c ..): acc[2p][0], acc[2p][1], acc[2p + 1][0], acc[2p + 1][1]; row b: [2], [3]
+			if (!full) {
+#pragma unroll
+				for (int j = 0; j < 4; ++j) {
+					const int k0 = base + kq * 32 + 16 * (j >> 1) + 4 * c + 2 * (j & 1);
+					acc[j][0] = k0 <= lim_a ? acc[j][0] : INT32_MIN;
+					acc[j][1] = k0 + 1 <= lim_a ? acc[j][1] : INT32_MIN;
+					acc[j][2] = k0 <= lim_b ? acc[j][2] : INT32_MIN;
+					acc[j][3] = k0 + 1 <= lim_b ? acc[j][3] : INT32_MIN;
+				}
+			}
+#pragma unroll
+			for (int j = 0; j < 4; ++j) {
+				mx_a = max(mx_a, max(acc[j][0], acc[j][1]));
+				mx_b = max(mx_b, max(acc[j][2], acc[j][3]));
+			}
+#pragma unroll
+			for (int p = 0; p < 2; ++p) {
+				sc[(i * 4 + 2 * p) * kChunkThreads + t] = make_int4(acc[2 * p][0], acc[2 * p][1], acc[2 * p + 1][0], acc[2 * p + 1][1]);
+				sc[(i * 4 + 2 * p + 1) * kChunkThreads + t] = make_int4(acc[2 * p][2], acc[2 * p][3], acc[2 * p + 1][2], acc[2 * p + 1][3]);
+			}
+			__syncthreads();      // the step may be overwritten
+		}
+		mx_a = max(mx_a, __shfl_xor_sync(0xffffffffu, mx_a, 1));
+		mx_a = max(mx_a, __shfl_xor_sync(0xffffffffu, mx_a, 2));
+		mx_b = max(mx_b, __shfl_xor_sync(0xffffffffu, mx_b, 1));
+		mx_b = max(mx_b, __shfl_xor_sync(0xffffffffu, mx_b, 2));
+		if (c == 0) {
+			atomicMax(&rmax[rho_a], mx_a);
+			atomicMax(&rmax[rho_b], mx_b);
+		}
+	}
+	// (the stage is free: V arrives during the softmax)
+	if (nsteps > 0) load_v(0);
+	if (nsteps > 1) load_v(1);
+	__syncthreads();
+	int mx_a = rmax[rho_a], mx_b = rmax[rho_b];
+	if (sub > 1) {
+		if (t < sub * kChunkRows) exchange_send(&rx_max[rank * kChunkRows + (t & 31)], cta_addr(&s_bars[0]), (uint32_t)(rank0 + (t >> 5)), (uint32_t)rmax[t & 31]);
+		ok = exchange_wait(cta_addr(&s_bars[0]));
+		for (int i = 0; i < sub; ++i) {
+			mx_a = max(mx_a, rx_max[i * kChunkRows + rho_a]);
+			mx_b = max(mx_b, rx_max[i * kChunkRows + rho_b]);
+		}
+	}
+
+	// ---- pass 2: exponentials and row totals
+	const IExpFast fa = fxs[in_a ? tok_a : 0], fb = fxs[in_b ? tok_b : 0];
+	{
+		unsigned long long sum[2] = {0ull, 0ull};
+#pragma unroll 1
+		for (int i = 0; i < nsteps; ++i) {
+			const bool full = (rank + i * sub) * kChunkStep + kChunkStep - 1 <= pos0;
+#pragma unroll
+			for (int j = 0; j < 4; ++j) {      // (row j & 1, group j / 2)
+				int4* at = &sc[(i * 4 + j) * kChunkThreads + t];
+				const int4 v = *at;
+				const IExpFast& f = (j & 1) ? fb : fa;
+				const uint32_t m = (uint32_t)((j & 1) ? mx_b : mx_a);
+				uint32_t p0, p1, p2, p3;
+				int64_t e0 = chunk_exp(m - (uint32_t)v.x, f, &p0), e1 = chunk_exp(m - (uint32_t)v.y, f, &p1);
+				int64_t e2 = chunk_exp(m - (uint32_t)v.z, f, &p2), e3 = chunk_exp(m - (uint32_t)v.w, f, &p3);
+				if (!full) {      // positions beyond a row's limit count for nothing
+					if (v.x == INT32_MIN) { e0 = 0; p0 = kBaseOfZero; }
+					if (v.y == INT32_MIN) { e1 = 0; p1 = kBaseOfZero; }
+					if (v.z == INT32_MIN) { e2 = 0; p2 = kBaseOfZero; }
+					if (v.w == INT32_MIN) { e3 = 0; p3 = kBaseOfZero; }
+				}
+				sum[j & 1] += (unsigned long long)(e0 + e1) + (unsigned long long)(e2 + e3);
+				*at = make_int4((int)p0, (int)p1, (int)p2, (int)p3);
+			}
+		}
+#pragma unroll
+		for (int h = 0; h < 2; ++h) {
+			sum[h] += __shfl_xor_sync(0xffffffffu, sum[h], 1);
+			sum[h] += __shfl_xor_sync(0xffffffffu, sum[h], 2);
+			if (c == 0) atomicAdd(&rsum[h ? rho_b : rho_a], sum[h]);
+		}
+	}
+	__syncthreads();
+	unsigned long long tot[2] = {rsum[rho_a], rsum[rho_b]};
+	if (sub > 1) {
+		if (t < sub * kChunkRows) exchange_send(&rx_sum[rank * kChunkRows + (t & 31)], cta_addr(&s_bars[1]), (uint32_t)(rank0 + (t >> 5)), rsum[t & 31]);
+		ok = exchange_wait(cta_addr(&s_bars[1])) && ok;
+		tot[0] = tot[1] = 0;
+		for (int i = 0; i < sub; ++i) {
+			tot[0] += rx_sum[i * kChunkRows + rho_a];
+			tot[1] += rx_sum[i * kChunkRows + rho_b];
+		}
+	}
+
+	// ---- pass 3: probabilities. Slots 0 and 1 of a step then hold this warp's A fragments of P.V, low and high
+	// plane: (row a group 0, row b group 0, row a group 1, row b group 1), four positions per word
+	{
+		const ChunkProb pa = chunk_prob(tot[0], fa), pb = chunk_prob(tot[1], fb);
+#pragma unroll 1
+		for (int i = 0; i < nsteps; ++i) {
+			uint32_t lo[4], hi[4];
+#pragma unroll
+			for (int j = 0; j < 4; ++j) {
+				const int4 v = sc[(i * 4 + j) * kChunkThreads + t];
+				const ChunkProb& p = (j & 1) ? pb : pa;
+				float near = 1.0f;
+				uint32_t p0 = chunk_prob_of((uint32_t)v.x, p, &near), p1 = chunk_prob_of((uint32_t)v.y, p, &near);
+				uint32_t p2 = chunk_prob_of((uint32_t)v.z, p, &near), p3 = chunk_prob_of((uint32_t)v.w, p, &near);
+				if (near < p.eps) {
+					const uint4 x = chunk_prob_exact((uint32_t)v.x, (uint32_t)v.y, (uint32_t)v.z, (uint32_t)v.w, (j & 1) ? fb.qc : fa.qc, tot[j & 1]);
+					p0 = x.x; p1 = x.y; p2 = x.z; p3 = x.w;
+				}
+				lo[j] = pack_plane(p0, p1, p2, p3, 0);
+				hi[j] = pack_plane(p0, p1, p2, p3, 1);
+			}
+			sc[(i * 4) * kChunkThreads + t] = make_int4((int)lo[0], (int)lo[1], (int)lo[2], (int)lo[3]);
+			sc[(i * 4 + 1) * kChunkThreads + t] = make_int4((int)hi[0], (int)hi[1], (int)hi[2], (int)hi[3]);
+		}
+	}
+
+	// ---- pass 4: P.V of this warp's rows and quarter of the channels, over the positions of all four warps
+	int accl[NT][4], acch[NT][4];
+#pragma unroll
+	for (int i = 0; i < NT; ++i)
+#pragma unroll
+		for (int q = 0; q < 4; ++q) accl[i][q] = acch[i][q] = 0;
+#pragma unroll 1
+	for (int i = 0; i < nsteps; ++i) {
+		if (i + 1 < nsteps) asm volatile("cp.async.wait_group 1;" ::: "memory");
+		else asm volatile("cp.async.wait_group 0;" ::: "memory");
+		__syncthreads();      // V of the step (and, the first time, everybody's probabilities) are there
+		const uint32_t vd = cta_addr(stage + (size_t)(i & 1) * kChunkStep * HD);
+#pragma unroll
+		for (int ks = 0; ks < kChunkStep / 32; ++ks) {
+			const int4 l = sc[(i * 4) * kChunkThreads + (rb * 4 + ks) * 32 + lane], h = sc[(i * 4 + 1) * kChunkThreads + (rb * 4 + ks) * 32 + lane];
+			if constexpr (NT == 1) {
+				const uint32_t at = vd + (uint32_t)((2 * ks + ((lane >> 3) & 1)) * HD + 8 * kq + (lane & 7)) * kPageTokens;
+				uint32_t b0, b1, b2, b3;      // (the upper half of the lanes repeats the lower half's rows)
+				ldmatrix4(at, b0, b1, b2, b3);
+				mma_u8s8_full(accl[0], l.x, l.y, l.z, l.w, b0, b1);
+				mma_u8s8_full(acch[0], h.x, h.y, h.z, h.w, b0, b1);
+			} else {
+#pragma unroll
+				for (int n = 0; n < NT; n += 2) {      // two 8-channel tiles, two pages each
+					const uint32_t at = vd + (uint32_t)((2 * ks + ((lane >> 3) & 1)) * HD + 8 * (kq * NT + n + (lane >> 4)) + (lane & 7)) * kPageTokens;
+					uint32_t b0, b1, b2, b3;
+					ldmatrix4(at, b0, b1, b2, b3);
+					mma_u8s8_full(accl[n], l.x, l.y, l.z, l.w, b0, b1);
+					mma_u8s8_full(acch[n], h.x, h.y, h.z, h.w, b0, b1);
+					mma_u8s8_full(accl[n + 1], l.x, l.y, l.z, l.w, b2, b3);
+					mma_u8s8_full(acch[n + 1], h.x, h.y, h.z, h.w, b2, b3);
+				}
+			}
+		}
+		__syncthreads();      // the step may be overwritten
+		if (i + 2 < nsteps) load_v(i + 2);
+	}
+
+	// ---- per-head context fold (forward_sites.cpp:1889-1896), store, row maximum for the funnel
+	if (sub == 1) {
+		uint32_t top_a = 0, top_b = 0;
+#pragma unroll
+		for (int n = 0; n < NT; ++n) {
+			const int ch = 8 * (kq * NT + n) + 2 * c;
+			auto put = [&](int tok, int head, int v0, int v1, uint32_t& top) {
+				int2 o;
+				o.x = fold(v0, l_fold[3 * head], l_fold[3 * head + 1], l_fold[3 * head + 2]);
+				o.y = fold(v1, l_fold[3 * head], l_fold[3 * head + 1], l_fold[3 * head + 2]);
+				*(int2*)(b.ctxw + (size_t)(r0 + tok) * d.hidden + (size_t)(kvh * G + head) * HD + ch) = o;
+				top = max(top, max(abs_u32(o.x), abs_u32(o.y)));
+			};
+			if (in_a) put(tok_a, head_a, accl[n][0] + 256 * acch[n][0], accl[n][1] + 256 * acch[n][1], top_a);
+			if (in_b) put(tok_b, head_b, accl[n][2] + 256 * acch[n][2], accl[n][3] + 256 * acch[n][3], top_b);
+		}
+		top_a = max(top_a, __shfl_xor_sync(0xffffffffu, top_a, 1));
+		top_a = max(top_a, __shfl_xor_sync(0xffffffffu, top_a, 2));
+		top_b = max(top_b, __shfl_xor_sync(0xffffffffu, top_b, 1));
+		top_b = max(top_b, __shfl_xor_sync(0xffffffffu, top_b, 2));
+		if (c == 0 && top_a) atomicMax(&b.rowmax[(size_t)(r0 + tok_a) * 4 + 3], (unsigned long long)top_a);
+		if (c == 0 && top_b) atomicMax(&b.rowmax[(size_t)(r0 + tok_b) * 4 + 3], (unsigned long long)top_b);
+		return;
+	}
+	// the shares go to the blocks that reduce their rows; a peer's stage is free once the peer has got here
+	cluster_arrive();
+	cluster_wait();
+	const int rows = kChunkRows / sub;
+	auto send = [&](int rho, int ch, int v0, int v1) {
+		exchange_send(&rx_ctx[(rank * rows + rho % rows) * HD + ch], cta_addr(&s_bars[2]), (uint32_t)(rank0 + rho / rows), make_int2(v0, v1));
+	};
+#pragma unroll
+	for (int n = 0; n < NT; ++n) {
+		const int ch = 8 * (kq * NT + n) + 2 * c;
+		send(rho_a, ch, accl[n][0] + 256 * acch[n][0], accl[n][1] + 256 * acch[n][1]);
+		send(rho_b, ch, accl[n][2] + 256 * acch[n][2], accl[n][3] + 256 * acch[n][3]);
+	}
+	ok = exchange_wait(cta_addr(&s_bars[2])) && ok;
+	for (int e = t; e < rows * HD; e += kChunkThreads) {
+		const int rho = rank * rows + e / HD, ch = e % HD, tok = rho / G, head = rho - tok * G;      // (a warp's elements lie in one row)
+		int32_t sum = 0;
+		for (int i = 0; i < sub; ++i) sum += rx_ctx[i * rows * HD + e];
+		const int32_t o = fold(sum, l_fold[3 * head], l_fold[3 * head + 1], l_fold[3 * head + 2]);
+		const bool in = tok < nt && tok_ok[tok] != 0;
+		if (in) b.ctxw[(size_t)(r0 + tok) * d.hidden + (size_t)(kvh * G + head) * HD + ch] = o;
+		const uint32_t top = __reduce_max_sync(0xffffffffu, in ? abs_u32(o) : 0u);
+		if (lane == 0 && top) atomicMax(&b.rowmax[(size_t)(r0 + tok) * 4 + 3], (unsigned long long)top);
+	}
+	if (!ok && t < nt) atomicCAS(&b.status[r0 + t], 0, pack_status(kInternalWaitTimeout, kSiteCtx, b.layer));
+}
+
+// How a chunk of m rows whose last row is `width` wide is cut: tiles of 32 query rows; a block holds up to
+// 512 positions, fewer while twice the blocks still run at once. False when the widest tile needs more
+// than the eight blocks of a cluster.
+static bool chunk_plan(const Dims& d, int m, int width, ChunkPlan* out) {
+	const int tq = kChunkRows / (d.heads / d.kv_heads), tiles = (m + tq - 1) / tq, first = width - m;
+	bool found = false;
+	for (int steps = kChunkSteps; steps >= 1; steps /= 2) {
+		ChunkPlan p{tq, steps, 1, {0, 0, 0, 0}};
+		auto ways = [&](int tile) {
+			const int w = first + std::min((tile + 1) * tq, m);
+			int s = 1;
+			while (s * steps * kChunkStep < w) s *= 2;
+			return s;
+		};
+		p.cluster = ways(tiles - 1);
+		if (p.cluster > 8) break;
+		int blocks = 0;
+		for (int i = 0; i < tiles; ++i) {
+			const int s = ways(i);
+			int at = 0;
+			while (p.cluster >> at > s) ++at;
+			++p.count[at];
+			blocks += s * d.kv_heads;
+		}
+		*out = p;
+		found = true;
+		if (blocks > sm_count()) break;
+	}
+	return found;
+}
+template <int HD>
+static cudaError_t launch_attn_chunk(const RowBatch& b, const Dims& d, const LayerDev* layer, int layer_index, KvPoolDev pool,
+                                     const ChunkPlan& p, cudaStream_t st) {
+	int clusters = 0;
+	for (int i = 0, s = p.cluster; i < 4 && s >= 1; ++i, s /= 2) clusters += (p.count[i] + p.cluster / s - 1) / (p.cluster / s);
+	cudaLaunchConfig_t cfg = {};
+	cfg.gridDim = dim3(p.cluster, clusters, d.kv_heads);
+	cfg.blockDim = dim3(kChunkThreads);
+	cfg.dynamicSmemBytes = ChunkSmem<HD>::bytes(p.steps);
+	cfg.stream = st;
+	cudaLaunchAttribute attr[2];
+	attr[0].id = cudaLaunchAttributeClusterDimension;
+	attr[0].val.clusterDim.x = (unsigned)p.cluster;
+	attr[0].val.clusterDim.y = 1;
+	attr[0].val.clusterDim.z = 1;
+	attr[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+	attr[1].val.programmaticStreamSerializationAllowed = 1;
+	cfg.attrs = attr;
+	cfg.numAttrs = pdl_enabled() ? 2 : 1;
+	return cudaLaunchKernelEx(&cfg, k_attention_chunk<HD>, b, d, layer, layer_index, pool, p);
+}
+
 static int pad64(int w) { return (w + 63) / 64 * 64; }
 constexpr int kAttnMaxSlice = 2048;      // positions one block holds at most
 
@@ -1177,6 +1693,7 @@ static cudaError_t configure_hd(int group) {
 	if (e == cudaSuccess) e = set((const void*)k_attention_few<HD, true>, (int)kFewSmemMax, true);
 	if (e == cudaSuccess) e = set((const void*)k_attention_few<HD, false>, (int)FewSmem<HD>::bytes(group, kAttnMaxSlice, false), true);
 	if (e == cudaSuccess) e = set((const void*)k_attention_tile<HD>, (int)TileSmem<HD>::kBytes, false);
+	if (e == cudaSuccess) e = set((const void*)k_attention_chunk<HD>, (int)ChunkSmem<HD>::bytes(kChunkSteps), false);
 	return e;
 }
 
@@ -1194,14 +1711,26 @@ cudaError_t attn_configure(const Dims& d) {
 
 bool launch_attention(const RowBatch& b, const Dims& d, const LayerDev* layer, const LayerDev& h, int layer_index,
                       KvPoolDev pool, int max_width, int reverse_rows, cudaStream_t st, cudaError_t* err) {
-	// the rows of a prefill chunk (consecutive positions of one sequence) take the query-tiled kernel
+	// the rows of a prefill chunk (consecutive positions of one sequence): tiles of queries
+	static const int chunk_min = [] {
+		const char* e = getenv("SSLM_B200_ATTN_CHUNK_MIN");      // tuning: rows of a chunk from which tiles are used
+		return e ? atoi(e) : 64;
+	}();
+	ChunkPlan cp;
+	if (reverse_rows && b.m >= chunk_min && chunk_plan(d, b.m, max_width, &cp)) {
+		cudaError_t e;
+		if (d.head_dim == 128) e = launch_attn_chunk<128>(b, d, layer, layer_index, pool, cp, st);
+		else if (d.head_dim == 64) e = launch_attn_chunk<64>(b, d, layer, layer_index, pool, cp, st);
+		else e = launch_attn_chunk<32>(b, d, layer, layer_index, pool, cp, st);
+		if (err) *err = e;
+		return false;
+	}
+	// ... and where a row is wider than a cluster of blocks can hold (beyond 4,096 positions), the kernel that
+	// walks the prefix three times and keeps nothing
 	static const bool tile_off = [] {
 		const char* e = getenv("SSLM_B200_ATTN_TILE");
 		return e && e[0] == '0';
 	}();
-	// ... once their prefix is long: up to about a thousand positions the per-row kernel, with
-	// thousands of independent blocks, is as fast or faster; beyond that re-reading the prefix per
-	// token costs more than the tiled kernel's lower parallelism (measured on the 0.5B / 1.5B / 3B widths).
 	static const int tile_min = [] {
 		const char* e = getenv("SSLM_B200_ATTN_TILE_MIN");      // tuning: the width from which the tiled kernel runs
 		return e ? atoi(e) : 1536;
