@@ -1114,8 +1114,11 @@ constexpr int kChunkRows = 32, kChunkStep = 128, kChunkThreads = 256, kChunkStep
 struct ChunkPlan {
 	int tq;            // tokens per tile
 	int steps;         // steps of 128 positions a block holds at most
-	int cluster;       // blocks per cluster
+	int cluster;       // blocks per cluster, a power of two
 	int count[4];      // tiles split `cluster`, cluster / 2, cluster / 4, cluster / 8 ways, widest first
+	int cshift;        // log2 cluster
+	int ginv;          // ceil(65536 / q heads per kv head): row / heads = row * ginv >> 16 for the rows of a tile
+	int tiles;
 };
 
 template <int HD>
@@ -1197,21 +1200,21 @@ k_attention_chunk(RowBatch b, Dims d, const LayerDev* layer, int layer_index, Kv
 
 	// which tile, split how many ways
 	const int kvh = blockIdx.z, G = d.heads / d.kv_heads;
-	const int C = pl.cluster, crank = (int)blockIdx.x, total = (b.m + pl.tq - 1) / pl.tq;
-	int sub = C, item = (int)blockIdx.y, before = 0;
+	const int crank = (int)blockIdx.x;
+	int shift = pl.cshift, item = (int)blockIdx.y, before = 0;      // shift = log2 of the ways the tile is split
 #pragma unroll
 	for (int i = 0; i < 4; ++i) {
-		const int per = C / sub, clusters = (pl.count[i] + per - 1) / per;
-		if (item < clusters || sub == 1 || i == 3) {
-			item = item * per + crank / sub;
+		const int per = pl.cshift - shift, clusters = (pl.count[i] + (1 << per) - 1) >> per;
+		if (item < clusters || shift == 0 || i == 3) {
+			item = (item << per) + (crank >> shift);
 			if (item >= pl.count[i]) item = -1;
 			break;
 		}
 		item -= clusters;
 		before += pl.count[i];
-		sub >>= 1;
+		--shift;
 	}
-	const int rank = crank % sub, rank0 = crank - rank;      // in the group of blocks that share the tile
+	const int sub = 1 << shift, rank = crank & (sub - 1), rank0 = crank - rank;      // the group of blocks that share the tile
 	const int t = threadIdx.x, warp = t >> 5, lane = t & 31, g = lane >> 2, c = lane & 3;
 	if (sub > 1) {
 		if (t == 0) {
@@ -1230,17 +1233,17 @@ k_attention_chunk(RowBatch b, Dims d, const LayerDev* layer, int layer_index, Kv
 		}
 		return;
 	}
-	const int tile = total - 1 - before - item;
+	const int tile = pl.tiles - 1 - before - item;
 	const int r0 = tile * pl.tq, nt = min(pl.tq, b.m - r0);
 	const int rb = warp >> 2, kq = warp & 3;
 	const int rho_a = rb * 16 + g, rho_b = rho_a + 8;
-	const int tok_a = rho_a / G, tok_b = rho_b / G;
+	const int tok_a = rho_a * pl.ginv >> 16, tok_b = rho_b * pl.ginv >> 16;
 	const int head_a = rho_a - tok_a * G, head_b = rho_b - tok_b * G;
 	// uploaded before the call's first launch: the tile's first position and the sequence's page table
 	const int pos0 = b.rows[r0].pos, old = b.rows[0].pos;
 	const int32_t* pages = b.rows[r0].pages;
 	const int width = pos0 + nt;
-	const int nsteps = ((width + kChunkStep - 1) / kChunkStep - rank + sub - 1) / sub;      // this block's: rank, rank + sub, ...
+	const int nsteps = ((width + kChunkStep - 1) / kChunkStep - rank + sub - 1) >> shift;      // this block's: rank, rank + sub, ...
 	const int8_t* kplane = pool.base + kv_plane_offset(d, pool, layer_index, kvh, 0);
 	const int8_t* vplane = pool.base + kv_plane_offset(d, pool, layer_index, kvh, 1);
 	for (int i = t; i < nsteps * 8; i += kChunkThreads) {
@@ -1528,9 +1531,9 @@ k_attention_chunk(RowBatch b, Dims d, const LayerDev* layer, int layer_index, Kv
 	// the shares go to the blocks that reduce their rows; a peer's stage is free once the peer has got here
 	cluster_arrive();
 	cluster_wait();
-	const int rows = kChunkRows / sub;
+	const int rows = kChunkRows >> shift, rshift = 5 - shift;
 	auto send = [&](int rho, int ch, int v0, int v1) {
-		exchange_send(&rx_ctx[(rank * rows + rho % rows) * HD + ch], cta_addr(&s_bars[2]), (uint32_t)(rank0 + rho / rows), make_int2(v0, v1));
+		exchange_send(&rx_ctx[(rank * rows + (rho & (rows - 1))) * HD + ch], cta_addr(&s_bars[2]), (uint32_t)(rank0 + (rho >> rshift)), make_int2(v0, v1));
 	};
 #pragma unroll
 	for (int n = 0; n < NT; ++n) {
@@ -1540,7 +1543,7 @@ k_attention_chunk(RowBatch b, Dims d, const LayerDev* layer, int layer_index, Kv
 	}
 	ok = exchange_wait(cta_addr(&s_bars[2])) && ok;
 	for (int e = t; e < rows * HD; e += kChunkThreads) {
-		const int rho = rank * rows + e / HD, ch = e % HD, tok = rho / G, head = rho - tok * G;      // (a warp's elements lie in one row)
+		const int rho = rank * rows + e / HD, ch = e % HD, tok = rho * pl.ginv >> 16, head = rho - tok * G;      // (a warp's elements lie in one row)
 		int32_t sum = 0;
 		for (int i = 0; i < sub; ++i) sum += rx_ctx[i * rows * HD + e];
 		const int32_t o = fold(sum, l_fold[3 * head], l_fold[3 * head + 1], l_fold[3 * head + 2]);
@@ -1556,10 +1559,10 @@ k_attention_chunk(RowBatch b, Dims d, const LayerDev* layer, int layer_index, Kv
 // 512 positions, fewer while twice the blocks still run at once. False when the widest tile needs more
 // than the eight blocks of a cluster.
 static bool chunk_plan(const Dims& d, int m, int width, ChunkPlan* out) {
-	const int tq = kChunkRows / (d.heads / d.kv_heads), tiles = (m + tq - 1) / tq, first = width - m;
+	const int G = d.heads / d.kv_heads, tq = kChunkRows / G, tiles = (m + tq - 1) / tq, first = width - m;
 	bool found = false;
 	for (int steps = kChunkSteps; steps >= 1; steps /= 2) {
-		ChunkPlan p{tq, steps, 1, {0, 0, 0, 0}};
+		ChunkPlan p{tq, steps, 1, {0, 0, 0, 0}, 0, (65536 + G - 1) / G, tiles};
 		auto ways = [&](int tile) {
 			const int w = first + std::min((tile + 1) * tq, m);
 			int s = 1;
@@ -1568,6 +1571,7 @@ static bool chunk_plan(const Dims& d, int m, int width, ChunkPlan* out) {
 		};
 		p.cluster = ways(tiles - 1);
 		if (p.cluster > 8) break;
+		while (1 << p.cshift < p.cluster) ++p.cshift;
 		int blocks = 0;
 		for (int i = 0; i < tiles; ++i) {
 			const int s = ways(i);
@@ -1634,9 +1638,8 @@ static AttnPlan attn_plan(const Dims& d, int m, int max_width) {
 	} else {
 		// A slice shortens every stage of a block's chain and four exchanges cost under a microsecond, so
 		// rows are cut while all blocks still run at once.
-		static const int lim = [] { const char* e = getenv("SSLM_ATTN_LIM"); return e ? atoi(e) : 100; }();
 		const int blocks = m * d.kv_heads;
-		while (splits < 8 && blocks * splits * 2 * 100 <= sm_count() * lim) splits *= 2;
+		while (splits < 8 && blocks * splits * 2 <= sm_count()) splits *= 2;
 		if (splits > per_kv_max) splits = per_kv_max;              // prefer the fused funnel
 	}
 	while (splits > 1 && splits * 64 > pad64(max_width)) splits /= 2;
@@ -1711,22 +1714,14 @@ cudaError_t attn_configure(const Dims& d) {
 
 bool launch_attention(const RowBatch& b, const Dims& d, const LayerDev* layer, const LayerDev& h, int layer_index,
                       KvPoolDev pool, int max_width, int reverse_rows, cudaStream_t st, cudaError_t* err) {
-	// the rows of a prefill chunk (consecutive positions of one sequence): tiles of queries
-	static const int chunk_min = [] {
-		const char* e = getenv("SSLM_B200_ATTN_CHUNK_MIN");      // tuning: rows of a chunk from which tiles are used
-		return e ? atoi(e) : 64;
-	}();
-	ChunkPlan cp;
-	if (reverse_rows && b.m >= chunk_min && chunk_plan(d, b.m, max_width, &cp)) {
-		cudaError_t e;
-		if (d.head_dim == 128) e = launch_attn_chunk<128>(b, d, layer, layer_index, pool, cp, st);
-		else if (d.head_dim == 64) e = launch_attn_chunk<64>(b, d, layer, layer_index, pool, cp, st);
-		else e = launch_attn_chunk<32>(b, d, layer, layer_index, pool, cp, st);
-		if (err) *err = e;
-		return false;
-	}
-	// ... and where a row is wider than a cluster of blocks can hold (beyond 4,096 positions), the kernel that
-	// walks the prefix three times and keeps nothing
+	// Prefill chunks (rows at consecutive positions of one sequence), by what a whole prompt took with each
+	// kernel. Tiles with the scores kept (k_attention_chunk) from 64 rows and 512 positions on: below, a row's
+	// own blocks are as fast and a tile's fixed part is not paid back (300 rows of the 28-layer model: 3.3 ms
+	// against 3.5; 512: 4.0 for either; 2,000 positions in chunks of 128: 55 against 39). The tiles that walk
+	// the prefix three times and keep nothing (k_attention_tile) where a row is wider than a cluster of blocks
+	// can hold (beyond 4,096 positions), and for head dimensions up to 64 in chunks of 1,600 rows or more: a
+	// walk costs half as much there and its 16 times as many blocks fill the device (24-layer model, 1,400 rows:
+	// 6.3 ms against 6.4; 2,047: 9.1 against 8.5).
 	static const bool tile_off = [] {
 		const char* e = getenv("SSLM_B200_ATTN_TILE");
 		return e && e[0] == '0';
@@ -1735,7 +1730,18 @@ bool launch_attention(const RowBatch& b, const Dims& d, const LayerDev* layer, c
 		const char* e = getenv("SSLM_B200_ATTN_TILE_MIN");      // tuning: the width from which the tiled kernel runs
 		return e ? atoi(e) : 1536;
 	}();
-	if (reverse_rows && b.m >= 4 && max_width >= tile_min && !tile_off) {
+	const bool tile_ok = reverse_rows && b.m >= 4 && max_width >= tile_min && !tile_off;
+	const bool prefer_tile = tile_ok && d.head_dim <= 64 && b.m >= 1600;
+	ChunkPlan cp;
+	if (reverse_rows && b.m >= 64 && max_width >= 512 && !prefer_tile && chunk_plan(d, b.m, max_width, &cp)) {
+		cudaError_t e;
+		if (d.head_dim == 128) e = launch_attn_chunk<128>(b, d, layer, layer_index, pool, cp, st);
+		else if (d.head_dim == 64) e = launch_attn_chunk<64>(b, d, layer, layer_index, pool, cp, st);
+		else e = launch_attn_chunk<32>(b, d, layer, layer_index, pool, cp, st);
+		if (err) *err = e;
+		return false;
+	}
+	if (tile_ok) {
 		cudaError_t e;
 		if (d.head_dim == 128) e = launch_attn_tile<128>(b, d, layer, layer_index, pool, st);
 		else if (d.head_dim == 64) e = launch_attn_tile<64>(b, d, layer, layer_index, pool, st);

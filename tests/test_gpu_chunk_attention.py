@@ -1,7 +1,7 @@
 """Attention of prefill chunks in tiles of 32 query rows, against the CPU oracle: chunks around the tile and
-step sizes, one block per tile and tiles split over clusters, prefixes of earlier chunks, head dimensions
-32 and 64 with the real models' group sizes. (Head dimension 128 and widths up to 32,768 are held to records
-of the reference by test_gpu_configs.py.)"""
+step sizes and the sizes where it takes over, one block per tile and tiles split over clusters, prefixes of
+earlier chunks, head dimensions 32 and 64 with the real models' group sizes. (Head dimension 128 and widths
+up to 32,768 are held to records of the reference by test_gpu_configs.py.)"""
 import pytest
 
 from superslm_b200 import abi, artifact as A
@@ -9,8 +9,9 @@ from tests.test_gpu_parity import run_port
 
 pytestmark = pytest.mark.gpu
 
-CASES = [("tiny", [64]), ("tiny", [65, 127, 129]), ("tiny", [513]), ("tiny", [700, 64, 300]), ("tiny", [1300]),
-         ("tiny", [1, 640]), ("tiny", [2100]), ("small", [64, 66]), ("small", [257]), ("small", [520, 200]), ("mini0.5b", [130])]
+CASES = [("tiny", [512]), ("tiny", [448, 64, 65]), ("tiny", [500, 127, 129]), ("tiny", [513]), ("tiny", [700, 64, 300]),
+         ("tiny", [1300]), ("tiny", [1, 640]), ("tiny", [1599, 65]), ("tiny", [1600, 130]), ("small", [520, 200]),
+         ("mini0.5b", [530])]
 
 
 @pytest.mark.parametrize("shape,chunks", CASES)
