@@ -59,4 +59,22 @@ __device__ __forceinline__ bool exchange_wait(uint32_t bar) {
 	return false;
 }
 
+// ---- slots that some threads fill and others empty, turn by turn
+__device__ __forceinline__ void ring_init(uint32_t bar, uint32_t count) { asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(bar), "r"(count)); }
+__device__ __forceinline__ void ring_arrive(uint32_t bar) { asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(bar) : "memory"); }
+__device__ __forceinline__ void copy16(uint32_t dst, const void* src) {      // past the L1
+	asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(dst), "l"(src) : "memory");
+}
+// false when the poll limit (about a second) ran out
+__device__ __forceinline__ bool ring_wait(uint32_t bar, uint32_t parity) {
+	for (uint32_t i = 0; i < (1u << 23); ++i) {
+		uint32_t ok;
+		asm volatile("{\n\t.reg .pred p;\n\tmbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n\tselp.u32 %0, 1, 0, p;\n\t}"
+		             : "=r"(ok) : "r"(bar), "r"(parity) : "memory");
+		if (ok) return true;
+		if (i > 2048) __nanosleep(64);
+	}
+	return false;
+}
+
 }  // namespace sslm

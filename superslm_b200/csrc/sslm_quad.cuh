@@ -132,29 +132,41 @@ static __device__ __noinline__ uint32_t code_quad_near_tie(T x0, T x1, T x2, T x
 	if (tie) return code_quad_exact<T>(x0, x1, x2, x3, d);
 	return pack4(c[0], c[1], c[2], c[3]);
 }
-// four codes, packed; element j in byte j
+// four codes, each kRoundMagicBits + the code, right unless the value returned (the distance of the farthest
+// from its integer) is above kNearTie: then code_quad_settle
 template <typename T>
-__device__ __forceinline__ uint32_t code_quad(const T (&x)[4], const QuadFunnel& q) {
-	int t[4];
-	float off[4], far = 0.0f;
+__device__ __forceinline__ float code_quad_try(const T (&x)[4], const QuadFunnel& q, int (&t)[4]) {
+	float far = 0.0f;
 #pragma unroll
 	for (int j = 0; j < 4; ++j) {
 		const float xf = to_float(x[j]);
 		const float m = fmaf(xf, q.f, kRoundMagic);
 		t[j] = __float_as_int(m);
-		off[j] = fmaf(xf, q.f, kRoundMagic - m);
-		far = fmaxf(far, fabsf(off[j]));
+		far = fmaxf(far, fabsf(fmaf(xf, q.f, kRoundMagic - m)));
 	}
-	if (far > kNearTie) {
-		far = 1.0f;
+	return far;
+}
+template <typename T>
+__device__ __forceinline__ void code_quad_settle(const T (&x)[4], const QuadFunnel& q, int (&t)[4]) {
+	float far = 1.0f;
 #pragma unroll
-		for (int j = 0; j < 4; ++j) {
-			const float o = fmaf(to_float(x[j]), q.f_lo, off[j]);
-			t[j] += (o > 0.5f ? 1 : 0) - (o < -0.5f ? 1 : 0);
-			far = fminf(far, fabsf(fabsf(o) - 0.5f));
-		}
-		if (far < 1e-6f || q.d > (1u << 24)) return code_quad_near_tie<T>(x[0], x[1], x[2], x[3], q.d);
+	for (int j = 0; j < 4; ++j) {
+		const float xf = to_float(x[j]);
+		const float o = fmaf(xf, q.f_lo, fmaf(xf, q.f, kRoundMagic - __int_as_float(t[j])));
+		t[j] += (o > 0.5f ? 1 : 0) - (o < -0.5f ? 1 : 0);
+		far = fminf(far, fabsf(fabsf(o) - 0.5f));
 	}
+	if (far < 1e-6f || q.d > (1u << 24)) {
+		const uint32_t c = code_quad_near_tie<T>(x[0], x[1], x[2], x[3], q.d);
+#pragma unroll
+		for (int j = 0; j < 4; ++j) t[j] = kRoundMagicBits + byte_of(c, j);
+	}
+}
+// four codes, packed; element j in byte j
+template <typename T>
+__device__ __forceinline__ uint32_t code_quad(const T (&x)[4], const QuadFunnel& q) {
+	int t[4];
+	if (code_quad_try(x, q, t) > kNearTie) code_quad_settle(x, q, t);
 	return pack4(t[0], t[1], t[2], t[3]);
 }
 // The same for rows of small integers (the residual sums), where a true tie 254 |x| = (2 c + 1) d is

@@ -839,6 +839,165 @@ k_act(RowBatch b, Dims d, Scale c_gate, Scale c_up, Scale c_act, const int32_t* 
 	if (rank == 0 && threadIdx.x == 0) b.acts[r] = fp.out;
 }
 
+// The activation site of many rows: persistent blocks, one row after another each.
+//
+// With hundreds of rows the form above is held by what every warp repeats for its row (three scale folds
+// and two funnels, the table, 255 sigmoids a block: 840 of its 1,490 instructions) and by a chain of four
+// barriers with nothing in flight. Here two warps derive the scalars and the 255 sigmoid products of the
+// rows to come; the eight workers stream their elements through shared memory (asynchronous copies,
+// each thread its own, kActStages steps ahead and on into the next row, so neither needs a barrier), leave
+// the products there and meet once, for their maximum. The loops stay rolled: kept in registers, the
+// products took so much code that a fifth of the time went into fetching it. Bound by instruction issue
+// (210 a quad and warp, 60 % of the slots): 2,047 rows of 8,960 take 47 us in place of 73, of which the
+// 165 MB that move need 26.
+constexpr int kActWorkers = 256, kActThreads = kActWorkers + 64, kActStages = 4;
+struct ActRow {
+	float fg, fg_lo, fu, fu_lo;
+	uint32_t dg, du;
+	int live;
+	FunnelFold fold;
+};
+__global__ void __launch_bounds__(kActThreads, 3)
+k_act_many(RowBatch b, Dims d, Scale c_gate, Scale c_up, Scale c_act, const int32_t* silu_table) {
+	extern __shared__ __align__(128) int4 stage[];      // [kActStages][gate, up][worker], then the products [quads of a row]
+	__shared__ uint32_t s_top[2][kActWorkers / 32];
+	__shared__ int32_t gsil[2][256];
+	__shared__ ActRow s_row[2];
+	__shared__ __align__(8) unsigned long long s_full[2], s_empty[2];
+	const int n = d.inter, nq = n >> 2, t = threadIdx.x, lane = t & 31;
+	if (t == 0) {
+		for (int i = 0; i < 2; ++i) {
+			ring_init(cta_addr(&s_full[i]), 1);
+			ring_init(cta_addr(&s_empty[i]), kActWorkers / 32);
+		}
+		exchange_fence_init();
+	}
+	__syncthreads();
+	pdl_wait();
+	pdl_release();
+	if (t >= kActWorkers) {
+		const uint32_t slot = (uint32_t)(t - kActWorkers) >> 5;      // the two warps take the rows in turn
+		uint32_t turn = 0;
+		for (int r = blockIdx.x + (int)(slot * gridDim.x); r < b.m; r += 2 * gridDim.x, ++turn) {
+			const unsigned long long mxg = __ldcg(&b.rowmax[(size_t)r * 4 + 1]), mxu = __ldcg(&b.rowmax[(size_t)r * 4 + 2]);
+			const bool refused = __ldcg(&b.status[r]) != 0;
+			const Scale ns = b.ns[r];
+			const QuadFunnel fg = quad_funnel(mxg, funnel_prefold(&ns, 1, c_gate));
+			const QuadFunnel fu = quad_funnel(mxu, funnel_prefold(&ns, 1, c_up));
+			int32_t st = fg.status != kOk ? fg.status : fu.status;
+			int site = fg.status != kOk ? kSiteGate : kSiteUp;
+			if (st == kOk && !silu_scale_in_domain(fg.out)) {
+				st = kSiluScaleOutOfDomain;
+				site = kSiteSilu;
+			}
+			const bool live = !refused && st == kOk;
+			const int freed = turn == 0 || ring_wait(cta_addr(&s_empty[slot]), (turn - 1) & 1);
+			if (!__all_sync(0xffffffffu, freed)) return;      // (the workers' wait for the row runs out in turn)
+			if (live) {
+				const int ge = (int)fg.out.e;
+#pragma unroll 4
+				for (int c = lane; c < 255; c += 32) gsil[slot][c] = (c - 127) * silu_sigmoid_q15(silu_table, c - 127, fg.out.m, ge);
+			}
+			const Scale inc[2] = {fg.out, fu.out};
+			if (lane == 0) {
+				s_row[slot] = ActRow{fg.f, fg.f_lo, fu.f, fu.f_lo, fg.d, fu.d, live, funnel_prefold(inc, 2, c_act)};
+				b.rowmax[(size_t)r * 4 + 1] = 0ull;
+				b.rowmax[(size_t)r * 4 + 2] = 0ull;
+				if (!refused && !live) atomicCAS(&b.status[r], 0, pack_status(st, site, b.layer));
+			}
+			__syncwarp();
+			if (lane == 0) ring_arrive(cta_addr(&s_full[slot]));
+		}
+		return;
+	}
+	// A worker's copies run kActStages quads ahead of its arithmetic, on into the block's next row.
+	const uint32_t stage0 = cta_addr(stage) + 16u * t;
+	constexpr uint32_t kStageBytes = 32u * kActWorkers, kStageMask = kActStages * kStageBytes - 1;
+	int ahead_r = t < nq ? (int)blockIdx.x : b.m, ahead_q = t;
+	uint32_t ahead_slot = 0, slot_at = 0;
+	auto ask = [&]() {
+		if (ahead_r < b.m) {
+			const int4* src = (const int4*)((const int32_t*)b.wide + (size_t)ahead_r * b.wide_ld) + ahead_q;
+			copy16(stage0 + ahead_slot, src);
+			copy16(stage0 + ahead_slot + kStageBytes / 2, src + nq);
+			ahead_slot = (ahead_slot + kStageBytes) & kStageMask;
+			ahead_q += kActWorkers;
+			if (ahead_q >= nq) {
+				ahead_q = t;
+				ahead_r += gridDim.x;
+			}
+		}
+		asm volatile("cp.async.commit_group;" ::: "memory");
+	};
+#pragma unroll 1
+	for (int i = 0; i < kActStages; ++i) ask();
+	int4* const kept = stage + kActStages * 2 * kActWorkers;
+	uint32_t turn = 0;
+	for (int r = blockIdx.x; r < b.m; r += gridDim.x, ++turn) {
+		const uint32_t slot = turn & 1;
+		const bool ok = ring_wait(cta_addr(&s_full[slot]), turn / 2 & 1);
+		const ActRow& a = s_row[slot];
+		const bool live = ok && a.live;
+		// (of a row that is refused: zeros, whatever its words are)
+		QuadFunnel fg{}, fu{};
+		fg.f = live ? a.fg : 0.0f; fg.f_lo = a.fg_lo; fg.d = a.dg;
+		fu.f = live ? a.fu : 0.0f; fu.f_lo = a.fu_lo; fu.d = a.du;
+		const uint32_t products = cta_addr(gsil[slot]) + 4u * 127u - 4u * (uint32_t)kRoundMagicBits;      // + 4 * (biased code)
+		uint32_t mx = 0;
+#pragma unroll 1
+		for (int q = t; q < nq; q += kActWorkers) {
+			asm volatile("cp.async.wait_group %0;" ::"n"(kActStages - 1) : "memory");
+			const int4 g = *(const int4*)((const char*)(stage + t) + slot_at), u = *(const int4*)((const char*)(stage + t) + slot_at + kStageBytes / 2);
+			slot_at = (slot_at + kStageBytes) & kStageMask;
+			const int32_t xg[4] = {g.x, g.y, g.z, g.w}, xu[4] = {u.x, u.y, u.z, u.w};
+			int cg[4], cu[4], w[4];
+			const float far_g = code_quad_try(xg, fg, cg), far_u = code_quad_try(xu, fu, cu);
+			if (fmaxf(far_g, far_u) > kNearTie) {
+				code_quad_settle(xg, fg, cg);
+				code_quad_settle(xu, fu, cu);
+			}
+			ask();
+#pragma unroll
+			for (int j = 0; j < 4; ++j) {
+				int32_t s;
+				asm volatile("ld.shared.s32 %0, [%1];" : "=r"(s) : "r"(products + 4u * (uint32_t)cg[j]));
+				w[j] = s * (cu[j] - kRoundMagicBits);
+				mx = max(mx, abs_u32(w[j]));
+			}
+			kept[q] = make_int4(w[0], w[1], w[2], w[3]);
+		}
+		// products are below 2^29: all ones says that a wait ran out somewhere in the block
+		mx = __reduce_max_sync(0xffffffffu, ok ? mx : 0xffffffffu);
+		uint32_t* top = s_top[slot];
+		if (lane == 0) top[t >> 5] = mx;
+		asm volatile("bar.sync 1, %0;" ::"n"(kActWorkers) : "memory");
+		mx = __reduce_max_sync(0xffffffffu, lane < kActWorkers / 32 ? top[lane] : 0u);
+		if (mx == 0xffffffffu) {
+			if (t == 0)
+				for (; r < b.m; r += gridDim.x) set_status(b, r, kInternalWaitTimeout, kSiteAct, b.layer);
+			break;
+		}
+		if (live) {
+			const QuadFunnel fp = quad_funnel((unsigned long long)mx, a.fold);
+			if (fp.status != kOk) {
+				set_status(b, r, fp.status, kSiteAct, b.layer);
+			} else {
+				uint32_t* out = (uint32_t*)(b.act + (size_t)r * n);
+#pragma unroll 2
+				for (int q = t; q < nq; q += kActWorkers) {
+					const int4 k = kept[q];
+					const int32_t w[4] = {k.x, k.y, k.z, k.w};
+					out[q] = code_quad(w, fp);
+				}
+				if (t == 0) b.acts[r] = fp.out;
+			}
+		}
+		__syncwarp();
+		if (lane == 0) ring_arrive(cta_addr(&s_empty[slot]));
+	}
+	asm volatile("cp.async.wait_all;" ::: "memory");
+}
+
 // ------------------------------------------------------------------ launchers
 // Quads per thread. One quad while the rows are few: the kernel's time is then the chain of a block,
 // and the shortest chain has one quad per thread. A prefill chunk has hundreds of rows and is bound by
@@ -899,8 +1058,18 @@ void launch_res(const RowBatch& b, const Dims& d, const ResSite& a, cudaStream_t
 	else if (nv == 4) b.wide64 ? go(k_res<4, 512, true>) : go(k_res<4, 512, false>);
 	else b.wide64 ? go(k_res<8, 512, true>) : go(k_res<8, 512, false>);
 }
+static int act_many_smem(int nq) { return 16 * (2 * kActStages * kActWorkers + nq); }
+constexpr int kActManySmemMax = 200 * 1024;
 void launch_act(const RowBatch& b, const Dims& d, const LayerDev& h, const int32_t* silu, cudaStream_t st) {
 	const int nq = d.inter / 4;
+	// Many rows: from 512 on (28-layer model, whole prompt: 400 rows 3.77 ms against 3.71, 512 4.00 either way,
+	// 1,024 6.05 against 6.30, 2,047 12.34 against 13.07). Five blocks per multiprocessor where three fit: what
+	// the rows do not divide into evenly is then handed out as blocks leave (3: 6.26 at 1,024 rows; 14: 6.12).
+	if (!b.wide64 && b.m >= 512 && act_many_smem(nq) <= kActManySmemMax) {
+		const int smem = act_many_smem(nq), per_sm = 5;
+		launch_pdl(k_act_many, dim3(std::min(b.m, per_sm * sm_count())), dim3(kActThreads), smem, st, b, d, h.c_gate, h.c_up, h.c_act, silu);
+		return;
+	}
 	// blocks per row: as many (up to 8) as the multiprocessors hold at once, three each
 	int blocks = 2;
 	while (blocks < 8 && b.m * blocks * 2 <= 3 * sm_count()) blocks *= 2;
@@ -951,6 +1120,8 @@ cudaError_t rows_configure(const Dims& d) {
 	                      (const void*)k_act<1, false>, (const void*)k_act<1, true>, (const void*)k_act<2, false>,
 	                      (const void*)k_act<2, true>, (const void*)k_act<5, false>, (const void*)k_act<5, true>})
 		set(f, false);
+	set((const void*)k_act_many, false);
+	if (e == cudaSuccess) e = cudaFuncSetAttribute(k_act_many, cudaFuncAttributeMaxDynamicSharedMemorySize, kActManySmemMax);
 	return e;
 }
 
