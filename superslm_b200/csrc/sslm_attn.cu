@@ -1682,8 +1682,11 @@ static cudaError_t launch_attn(const RowBatch& b, const Dims& d, const LayerDev*
 	                          p.cp, p.splits, p.whole_row, reverse_rows);
 }
 
+// (The attributes are the kernel's, not the model's: limits for the largest group, so that mapping one model
+// takes nothing from another.)
 template <int HD>
-static cudaError_t configure_hd(int group) {
+static cudaError_t configure_hd() {
+	const int group = 8;
 	auto set = [](const void* f, int smem, bool big_cluster) {
 		cudaError_t e = cudaFuncSetAttribute(f, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
 		// clusters of 16 blocks are an opt-in size
@@ -1706,9 +1709,9 @@ cudaError_t attn_configure(const Dims& d) {
 	// widest row the plan can serve: 16 slices of kAttnMaxSlice positions
 	if (d.context_cap > 16 * kAttnMaxSlice) return cudaErrorInvalidConfiguration;
 	if (attn_smem_bytes(group, kAttnMaxSlice) > 225 * 1024) return cudaErrorInvalidConfiguration;
-	if (d.head_dim == 128) return configure_hd<128>(group);
-	if (d.head_dim == 64) return configure_hd<64>(group);
-	if (d.head_dim == 32) return configure_hd<32>(group);
+	if (d.head_dim == 128) return configure_hd<128>();
+	if (d.head_dim == 64) return configure_hd<64>();
+	if (d.head_dim == 32) return configure_hd<32>();
 	return cudaErrorInvalidConfiguration;
 }
 

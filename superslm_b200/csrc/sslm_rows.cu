@@ -1098,8 +1098,10 @@ cudaError_t rows_configure(const Dims& d) {
 	// Every kernel of a step asks for the same (largest) shared-memory carve-out as the
 	// tensor-core GEMM between them, so consecutive launches never make the SMs re-split
 	// their L1 / shared memory.
-	const int sm = (int)general_smem_bytes(d.hidden);
-	if (sm > 227 * 1024) return cudaErrorInvalidConfiguration;
+	// (The limit on dynamic shared memory is the kernel's, not the model's: the most there is, so that mapping
+	// a narrow model does not take it from a wider one.)
+	const int sm = 226 * 1024;
+	if (general_smem_bytes(d.hidden) > (size_t)sm) return cudaErrorInvalidConfiguration;
 	cudaError_t e = cudaSuccess;
 	auto set = [&](const void* f, bool dynamic) {
 		if (e == cudaSuccess) e = cudaFuncSetAttribute(f, cudaFuncAttributePreferredSharedMemoryCarveout, cudaSharedmemCarveoutMaxShared);
