@@ -728,8 +728,9 @@ k_res(RowBatch b, Dims d, ResSite a) {
 // The activation row is the longest a row site walks (intermediate width, three codes per element).
 // While rows are few its time is one block's chain, so a row is cut over a cluster of `gridDim.x`
 // blocks, which meet once, for the maximum of the products; on a prefill chunk two blocks share a row.
-template <int NV, bool W64>
-__global__ void __launch_bounds__(NV == 5 ? 352 : 384, NV == 1 ? 1 : 2)
+// FOUR: in 72 registers, so that four blocks of 224 threads fit a multiprocessor
+template <int NV, bool W64, bool FOUR = false>
+__global__ void __launch_bounds__(FOUR ? 288 : (NV == 5 ? 352 : 384), NV == 1 ? 1 : (FOUR ? 3 : 2))
 k_act(RowBatch b, Dims d, Scale c_gate, Scale c_up, Scale c_act, const int32_t* silu_table) {
 	using T = typename WideOf<W64>::T;
 	__shared__ uint32_t s_bank[64];
@@ -1092,7 +1093,11 @@ void launch_act(const RowBatch& b, const Dims& d, const LayerDev& h, const int32
 	auto go = [&](auto kernel) { cudaLaunchKernelEx(&cfg, kernel, b, d, h.c_gate, h.c_up, h.c_act, silu); };
 	if (nv == 1) b.wide64 ? go(k_act<1, true>) : go(k_act<1, false>);
 	else if (nv == 2) b.wide64 ? go(k_act<2, true>) : go(k_act<2, false>);
-	else b.wide64 ? go(k_act<5, true>) : go(k_act<5, false>);
+	else if (b.wide64) go(k_act<5, true>);
+	// (three blocks fit in 80 registers; where that leaves a second, short wave -- 256 rows of 8,960 -- four in
+	// 72 are 1.5 us faster, and 0.7 us slower where it does not)
+	else if (b.m * blocks > 3 * sm_count() && quad_threads(per, nv) <= 288) go(k_act<5, false, true>);
+	else go(k_act<5, false>);
 }
 cudaError_t rows_configure(const Dims& d) {
 	// Every kernel of a step asks for the same (largest) shared-memory carve-out as the
@@ -1120,7 +1125,8 @@ cudaError_t rows_configure(const Dims& d) {
 	                      (const void*)k_qkv_post<8, true, false>, (const void*)k_qkv_post<8, true, true>,
 	                      (const void*)k_ctx_funnel<1>, (const void*)k_ctx_funnel<4>, (const void*)k_ctx_funnel<8>,
 	                      (const void*)k_act<1, false>, (const void*)k_act<1, true>, (const void*)k_act<2, false>,
-	                      (const void*)k_act<2, true>, (const void*)k_act<5, false>, (const void*)k_act<5, true>})
+	                      (const void*)k_act<2, true>, (const void*)k_act<5, false>, (const void*)k_act<5, true>,
+	                      (const void*)k_act<5, false, true>})
 		set(f, false);
 	set((const void*)k_act_many, false);
 	if (e == cudaSuccess) e = cudaFuncSetAttribute(k_act_many, cudaFuncAttributeMaxDynamicSharedMemorySize, kActManySmemMax);
