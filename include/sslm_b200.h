@@ -265,10 +265,16 @@ SSLM_API sslm_status sslm_b200_trace(sslm_workspace ws, void* buf, size_t capaci
 /* Tests only: every wait of the kernels on an mbarrier is bounded, and this makes one run out on
  * purpose. The next `launches` (0..16) launches of the tensor-core linear kernel arm the barrier of
  * their first weight tile in block 0 without requesting the tile; the wait on it gives up after its
- * poll limit (about a second), the rows of that tile end with an internal status, and the verb
+ * limit (a second or less), the rows of that tile end with an internal status, and the verb
  * that launched the kernel returns SSLM_ALLOCATION_FAILED like any other refusal (a prefill chunk
  * consumes nothing). Nothing faults and nothing spins without a limit; the next call works normally. */
 SSLM_API sslm_status sslm_b200_debug_withhold_tc_load(int32_t launches);
+/* The same for the words that the blocks of a cluster send each other: block 0 of the next launch of
+ * `kernel` waits for more than will come in one of its exchanges. kernel 0: the weights-first linear kernel
+ * where K is cut over a cluster (exchange 0); 1: attention of few rows (0 maxima, 1 sums, 2 contexts, 3 the
+ * funnel's maximum); 2: attention of prefill chunks in tiles cut over a cluster (0 to 2); 3: the activation
+ * site (0). kernel -1 takes the request back. */
+SSLM_API sslm_status sslm_b200_debug_withhold_exchange(int32_t kernel, int32_t exchange);
 
 /* Tests only: the device integer library's primitives evaluated ON THE DEVICE over n operand
  * tuples (host arrays a, b, c, e; three host result arrays), so that their device-only halves

@@ -489,8 +489,10 @@ __device__ __forceinline__ void shared_row_words(const int8_t* row, int c, uint3
 	}
 }
 
+// (Registers: left to itself the compiler takes 56 to 80, and at 64 some forms spill: 24 rows of 500 to
+// 1,500 positions at the 1.5B widths, two slices each, took 1,970 us a token then, 1,810 in 80, 1,730 in 100.)
 template <int HD, bool STAGED>
-__global__ void __launch_bounds__(2 * HD)
+__global__ void __launch_bounds__(2 * HD, 1)
 k_attention_few(RowBatch b, Dims d, const LayerDev* layer, Scale c_ctx, int layer_index, KvPoolDev pool, int cp, int splits,
                 int whole_row, int chunk) {
 	using S = FewSmem<HD>;
@@ -506,10 +508,12 @@ k_attention_few(RowBatch b, Dims d, const LayerDev* layer, Scale c_ctx, int laye
 	const int per = HD / splits, ch0 = split * per;                  // channels this block reduces
 	auto bar = [&](int i) { return cta_addr(&s_bars[i]); };
 	if (t == 0) {
-		exchange_init(bar(0), (uint32_t)(splits * G * 4));
-		exchange_init(bar(1), (uint32_t)(splits * G * 8));
-		exchange_init(bar(2), (uint32_t)(G * HD * 4));
-		exchange_init(bar(3), 4u * cluster_blocks);
+		const int held = (blockIdx.x | blockIdx.y) == 0 ? b.debug_withhold : 0;
+		auto more = [&](int i) { return held == i + 1 ? 4u : 0u; };
+		exchange_init(bar(0), (uint32_t)(splits * G * 4) + more(0));
+		exchange_init(bar(1), (uint32_t)(splits * G * 8) + more(1));
+		exchange_init(bar(2), (uint32_t)(G * HD * 4) + more(2));
+		exchange_init(bar(3), 4u * cluster_blocks + more(3));
 		exchange_fence_init();
 	}
 	// ahead of the kernel that lands this step's K / V rows: the page table, the old rows
@@ -741,6 +745,7 @@ k_attention_few(RowBatch b, Dims d, const LayerDev* layer, Scale c_ctx, int laye
 	if (!ok && t == 0) atomicCAS(&b.status[r], 0, pack_status(kInternalWaitTimeout, kSiteCtx, b.layer));
 	if (!whole_row) {
 		if (lane == 0 && top && live) atomicMax(&b.rowmax[(size_t)r * 4 + 3], (unsigned long long)top);
+		if (__builtin_expect(!__all_sync(0xffffffffu, ok), 0)) exchange_leave(bar(0), 3);
 		return;
 	}
 	// ---- exchange 4: the cluster holds the whole row, its funnel runs here
@@ -748,7 +753,11 @@ k_attention_few(RowBatch b, Dims d, const LayerDev* layer, Scale c_ctx, int laye
 	__syncthreads();
 	if (t < (int)cluster_blocks) exchange_send(&s.rx_top[my_rank], bar(3), (uint32_t)t, s.misc[0]);
 	ok = exchange_wait(bar(3)) && ok;
-	if (!live || !ok) return;
+	if (__builtin_expect(!__all_sync(0xffffffffu, ok), 0)) {
+		exchange_leave(bar(0), 4);
+		return;
+	}
+	if (!live) return;
 	for (uint32_t j = 0; j < cluster_blocks; ++j) top = max(top, s.rx_top[j]);
 	const QuadFunnel fp = quad_funnel((unsigned long long)top, fold_ctx);
 	if (fp.status != kOk) {
@@ -1218,9 +1227,11 @@ k_attention_chunk(RowBatch b, Dims d, const LayerDev* layer, int layer_index, Kv
 	const int t = threadIdx.x, warp = t >> 5, lane = t & 31, g = lane >> 2, c = lane & 3;
 	if (sub > 1) {
 		if (t == 0) {
-			exchange_init(cta_addr(&s_bars[0]), (uint32_t)(sub * kChunkRows * 4));
-			exchange_init(cta_addr(&s_bars[1]), (uint32_t)(sub * kChunkRows * 8));
-			exchange_init(cta_addr(&s_bars[2]), (uint32_t)(kChunkRows * HD * 4));
+			const int held = (blockIdx.x | blockIdx.y | blockIdx.z) == 0 ? b.debug_withhold : 0;
+			auto more = [&](int i) { return held == i + 1 ? 4u : 0u; };
+			exchange_init(cta_addr(&s_bars[0]), (uint32_t)(sub * kChunkRows * 4) + more(0));
+			exchange_init(cta_addr(&s_bars[1]), (uint32_t)(sub * kChunkRows * 8) + more(1));
+			exchange_init(cta_addr(&s_bars[2]), (uint32_t)(kChunkRows * HD * 4) + more(2));
 			exchange_fence_init();
 		}
 		cluster_arrive();
@@ -1553,6 +1564,7 @@ k_attention_chunk(RowBatch b, Dims d, const LayerDev* layer, int layer_index, Kv
 		if (lane == 0 && top) atomicMax(&b.rowmax[(size_t)(r0 + tok) * 4 + 3], (unsigned long long)top);
 	}
 	if (!ok && t < nt) atomicCAS(&b.status[r0 + t], 0, pack_status(kInternalWaitTimeout, kSiteCtx, b.layer));
+	if (__builtin_expect(!__all_sync(0xffffffffu, ok), 0)) exchange_leave(cta_addr(&s_bars[0]), 3);
 }
 
 // How a chunk of m rows whose last row is `width` wide is cut: tiles of 32 query rows; a block holds up to
@@ -1589,6 +1601,8 @@ static bool chunk_plan(const Dims& d, int m, int width, ChunkPlan* out) {
 template <int HD>
 static cudaError_t launch_attn_chunk(const RowBatch& b, const Dims& d, const LayerDev* layer, int layer_index, KvPoolDev pool,
                                      const ChunkPlan& p, cudaStream_t st) {
+	RowBatch rb = b;
+	rb.debug_withhold = p.cluster > 1 ? exchange_debug_take(kExchangeAttnChunk) : 0;
 	int clusters = 0;
 	for (int i = 0, s = p.cluster; i < 4 && s >= 1; ++i, s /= 2) clusters += (p.count[i] + p.cluster / s - 1) / (p.cluster / s);
 	cudaLaunchConfig_t cfg = {};
@@ -1605,7 +1619,7 @@ static cudaError_t launch_attn_chunk(const RowBatch& b, const Dims& d, const Lay
 	attr[1].val.programmaticStreamSerializationAllowed = 1;
 	cfg.attrs = attr;
 	cfg.numAttrs = pdl_enabled() ? 2 : 1;
-	return cudaLaunchKernelEx(&cfg, k_attention_chunk<HD>, b, d, layer, layer_index, pool, p);
+	return cudaLaunchKernelEx(&cfg, k_attention_chunk<HD>, rb, d, layer, layer_index, pool, p);
 }
 
 static int pad64(int w) { return (w + 63) / 64 * 64; }
@@ -1664,6 +1678,8 @@ static cudaError_t launch_attn(const RowBatch& b, const Dims& d, const LayerDev*
 		return launch_pdl(k_attention<HD>, dim3(d.kv_heads, b.m), dim3(2 * HD), attn_smem_bytes(G, p.cp), st, b, d, layer, layer_index,
 		                  pool, p.cp, reverse_rows);
 	const bool staged = FewSmem<HD>::bytes(G, p.cp, true) <= kFewSmemMax;
+	RowBatch rb = b;
+	rb.debug_withhold = exchange_debug_take(kExchangeAttnFew);
 	cudaLaunchConfig_t cfg = {};
 	cfg.gridDim = dim3(d.kv_heads * p.splits, b.m);
 	cfg.blockDim = dim3(2 * HD);
@@ -1678,7 +1694,7 @@ static cudaError_t launch_attn(const RowBatch& b, const Dims& d, const LayerDev*
 	attr[1].val.programmaticStreamSerializationAllowed = 1;
 	cfg.attrs = attr;
 	cfg.numAttrs = pdl_enabled() ? 2 : 1;
-	return cudaLaunchKernelEx(&cfg, staged ? k_attention_few<HD, true> : k_attention_few<HD, false>, b, d, layer, h.c_ctx, layer_index, pool,
+	return cudaLaunchKernelEx(&cfg, staged ? k_attention_few<HD, true> : k_attention_few<HD, false>, rb, d, layer, h.c_ctx, layer_index, pool,
 	                          p.cp, p.splits, p.whole_row, reverse_rows);
 }
 

@@ -5,10 +5,13 @@
 // max / sum exchange of eight blocks takes 420 cycles this way; remote stores (or loads) around
 // barrier.cluster, whose release also waits out the block's global stores, take 1,100 (B200).
 //
-// Rules: a peer's shared memory may be written once the peer runs, i.e. behind one cluster_arrive /
-// cluster_wait pair at the start of the kernel (free: its wait is over before the dependency wait is).
-// A block leaves only after it has received every word its peers send it, whatever became of its row,
-// so no store finds its target gone. Waits are bounded.
+// Rules. A peer's shared memory may be written once the peer runs, i.e. behind one cluster_arrive /
+// cluster_wait pair at the start of the kernel (free: its wait is over before the dependency wait is), and
+// until it leaves. A block that has received every word its peers send it may leave: nothing is on its way
+// to it any more. Waits are bounded in time (kWaitNs), so a block may also have given up on words that a
+// late peer still sends: its warps end in exchange_leave, which outlasts whatever a peer can be late by.
+// (Not a second cluster barrier: passed by every block it cost 1 to 2 % of a decode step, and it would have
+// to be passed by every block, since a barrier that only the warps that gave up arrived at did not return.)
 #pragma once
 #include <cuda_runtime.h>
 #include <stdint.h>
@@ -46,17 +49,53 @@ __device__ __forceinline__ void exchange_send(const void* local, uint32_t bar, u
 	    "{\n\t.reg .b32 ra, rb;\n\tmapa.shared::cluster.u32 ra, %0, %2;\n\tmapa.shared::cluster.u32 rb, %1, %2;\n\t"
 	    "st.async.shared::cluster.mbarrier::complete_tx::bytes.v2.s32 [ra], {%3, %4}, [rb];\n\t}" ::"r"(cta_addr(local)), "r"(bar), "r"(rank), "r"(v.x), "r"(v.y) : "memory");
 }
-// true once every byte is in; false when the poll limit (well under a second) ran out
-__device__ __forceinline__ bool exchange_wait(uint32_t bar) {
-	for (uint32_t i = 0; i < (1u << 22); ++i) {
-		uint32_t ok;
+// A wait on an mbarrier: quick polls, then polls with pauses, kWaitNs (%globaltimer) at most. A limit in polls
+// is none: 2^22 of them took 1 s for one thread and 17 s for a block. The loop stays rolled: a launch passes
+// most of its waits once, so their code is fetched, not run (unrolled, a decode step took 2 to 6 % longer).
+constexpr unsigned long long kWaitNs = 250000000ull;
+constexpr uint32_t kQuickPolls = 2048;
+__device__ __forceinline__ unsigned long long now_ns() {
+	unsigned long long t;
+	asm volatile("mov.u64 %0, %%globaltimer;" : "=l"(t));
+	return t;
+}
+// PEERS: what peers sent is waited for (the scope of the acquire costs 1 to 3 % of a decode step where only
+// this block's own copies and multiplications are)
+template <bool PEERS>
+__device__ __forceinline__ bool bar_try(uint32_t bar, uint32_t parity) {
+	uint32_t ok;
+	if (PEERS)
 		asm volatile(
-		    "{\n\t.reg .pred p;\n\tmbarrier.try_wait.parity.acquire.cluster.shared::cta.b64 p, [%1], 0;\n\tselp.u32 %0, 1, 0, p;\n\t}"
-		    : "=r"(ok) : "r"(bar) : "memory");
-		if (ok) return true;
-		if (i > 2048) __nanosleep(64);
+		    "{\n\t.reg .pred p;\n\tmbarrier.try_wait.parity.acquire.cluster.shared::cta.b64 p, [%1], %2;\n\tselp.u32 %0, 1, 0, p;\n\t}"
+		    : "=r"(ok) : "r"(bar), "r"(parity) : "memory");
+	else
+		asm volatile(
+		    "{\n\t.reg .pred p;\n\tmbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n\tselp.u32 %0, 1, 0, p;\n\t}"
+		    : "=r"(ok) : "r"(bar), "r"(parity) : "memory");
+	return ok != 0;
+}
+// false when the limit ran out
+template <bool PEERS>
+__device__ __forceinline__ bool bounded_wait(uint32_t bar, uint32_t parity) {
+	unsigned long long since = 0;
+#pragma unroll 1
+	for (uint32_t i = 0;; ++i) {
+		if (bar_try<PEERS>(bar, parity)) return true;
+		if (i < kQuickPolls) continue;
+		__nanosleep(64);
+		if (i == kQuickPolls) since = now_ns();
+		else if (now_ns() - since > kWaitNs) return false;
 	}
-	return false;
+}
+// true once every byte is in
+__device__ __forceinline__ bool exchange_wait(uint32_t bar) { return bounded_wait<true>(bar, 0); }
+// The end of a warp in which a wait ran out (bar: the first of the block's n exchanges, side by side). The blocks
+// of a cluster start together and a peer sends its last words after n waits at most (one more in a kernel that
+// waits for its operands), so by this deadline everything that will come has come.
+static __device__ __noinline__ void exchange_leave(uint32_t bar, int n) {
+	const unsigned long long deadline = now_ns() + (unsigned long long)(n + 2) * kWaitNs;
+	for (int i = 0; i < n; ++i)
+		while (!bar_try<true>(bar + 8u * (uint32_t)i, 0) && now_ns() < deadline) __nanosleep(64);
 }
 
 // ---- slots that some threads fill and others empty, turn by turn
@@ -65,16 +104,6 @@ __device__ __forceinline__ void ring_arrive(uint32_t bar) { asm volatile("mbarri
 __device__ __forceinline__ void copy16(uint32_t dst, const void* src) {      // past the L1
 	asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(dst), "l"(src) : "memory");
 }
-// false when the poll limit (about a second) ran out
-__device__ __forceinline__ bool ring_wait(uint32_t bar, uint32_t parity) {
-	for (uint32_t i = 0; i < (1u << 23); ++i) {
-		uint32_t ok;
-		asm volatile("{\n\t.reg .pred p;\n\tmbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n\tselp.u32 %0, 1, 0, p;\n\t}"
-		             : "=r"(ok) : "r"(bar), "r"(parity) : "memory");
-		if (ok) return true;
-		if (i > 2048) __nanosleep(64);
-	}
-	return false;
-}
+__device__ __forceinline__ bool ring_wait(uint32_t bar, uint32_t parity) { return bounded_wait<false>(bar, parity); }
 
 }  // namespace sslm

@@ -288,7 +288,7 @@ k_linear_tc(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ C
 #pragma unroll
 					for (int mt = 0; mt < MT; ++mt) tma_load_2d(sa + mt * BM * BK, &map_a, full_bar(s), kb * BK, m0 + mt * BM);
 					// (tests of the bounded waits leave this one request out, once)
-					if (!(a.debug_withhold != 0 && blockIdx.x == 0 && it == 0))
+					if (!(a.debug_withhold == 1 && blockIdx.x == 0 && it == 0))
 						tma_load_2d(sa + MT * BM * BK, &map_b, full_bar(s), kb * BK, n0);
 				}
 			}

@@ -86,6 +86,18 @@ inline int sm_count() {
 	return v;
 }
 
+// ---- tests of the bounded waits
+// The next launch of one kernel that exchanges words over a cluster arms one of its exchanges, in block 0,
+// with four bytes more than will come: that block's wait runs out. One word: 0 for none, else
+// kernel << 8 | exchange + 1.
+enum ExchangeKernel { kExchangeLinear = 0, kExchangeAttnFew, kExchangeAttnChunk, kExchangeAct, kExchangeKernels };
+inline std::atomic<uint32_t> g_withheld_exchange{0};
+inline int exchange_debug_take(ExchangeKernel kernel) {
+	uint32_t w = g_withheld_exchange.load(std::memory_order_relaxed);
+	if (w == 0 || w >> 8 != (uint32_t)kernel || !g_withheld_exchange.compare_exchange_strong(w, 0)) return 0;
+	return (int)(w & 0xFF);
+}
+
 // ---- per-row sites (sslm_rows.cu)
 cudaError_t rows_configure(const Dims& d);
 // (the host's copy `h` of a layer record carries the site constants into the launch parameters)
@@ -152,7 +164,8 @@ struct LinearArgs {
 	int splits;           // filled in by launch_linear_tc
 	int caller_memory;    // 1: operands are a caller's own, on a caller's stream: the weights may have been written by
 	                      //    the kernel in front (plain stream order), and no tensor map is kept
-	int debug_withhold;   // tests only (tc_debug_withhold): block 0 never requests its first weight tile
+	int debug_withhold;   // tests only: 1 block 0 never requests its first weight tile (tc_debug_withhold), 2 it waits for
+	                      //    four bytes too many in its exchange (exchange_debug_take)
 };
 // HBM-bound small-M path: bulk-copy weight streaming through a shared-memory ring, dp4a.
 cudaError_t launch_linear_gemv(const LinearArgs& a, cudaStream_t st);

@@ -750,7 +750,7 @@ k_act(RowBatch b, Dims d, Scale c_gate, Scale c_up, Scale c_act, const int32_t* 
 	const uint32_t arrived = cta_addr(&s_arrived);
 	if (blocks > 1) {
 		if (threadIdx.x == 0) {
-			exchange_init(arrived, 4u * blocks);
+			exchange_init(arrived, 4u * blocks + ((blockIdx.x | blockIdx.y) == 0 && b.debug_withhold != 0 ? 4u : 0u));
 			exchange_fence_init();
 		}
 		cluster_arrive();
@@ -811,8 +811,10 @@ k_act(RowBatch b, Dims d, Scale c_gate, Scale c_up, Scale c_act, const int32_t* 
 		// Every block of the cluster comes through here, refused row or not, so none waits for one
 		// that left; and only behind it is the row maximum cleared, so every block saw it.
 		if (threadIdx.x < blocks) exchange_send(&s_peer[rank], arrived, threadIdx.x, mx);
-		if (!exchange_wait(arrived)) {
+		const bool ok = exchange_wait(arrived);
+		if (__builtin_expect(!__all_sync(0xffffffffu, ok), 0)) {
 			set_status(b, r, kInternalWaitTimeout, kSiteAct, b.layer);
+			exchange_leave(arrived, 1);
 			return;
 		}
 		for (uint32_t i = 0; i < blocks; ++i) mx = max(mx, s_peer[i]);
@@ -1090,7 +1092,9 @@ void launch_act(const RowBatch& b, const Dims& d, const LayerDev& h, const int32
 	attr[1].val.programmaticStreamSerializationAllowed = 1;
 	cfg.attrs = attr;
 	cfg.numAttrs = pdl_enabled() ? 2 : 1;
-	auto go = [&](auto kernel) { cudaLaunchKernelEx(&cfg, kernel, b, d, h.c_gate, h.c_up, h.c_act, silu); };
+	RowBatch rb = b;
+	rb.debug_withhold = exchange_debug_take(kExchangeAct);
+	auto go = [&](auto kernel) { cudaLaunchKernelEx(&cfg, kernel, rb, d, h.c_gate, h.c_up, h.c_act, silu); };
 	if (nv == 1) b.wide64 ? go(k_act<1, true>) : go(k_act<1, false>);
 	else if (nv == 2) b.wide64 ? go(k_act<2, true>) : go(k_act<2, false>);
 	else if (b.wide64) go(k_act<5, true>);

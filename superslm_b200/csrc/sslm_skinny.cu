@@ -39,7 +39,6 @@ namespace {
 
 constexpr int kWRows = 128, kKBlock = 128, kMmaK = 32;
 constexpr int kMaxStages = 12;
-constexpr uint32_t kPolls = 1u << 22;
 
 template <int NB>
 struct SkCfg {
@@ -61,17 +60,7 @@ __device__ __forceinline__ void bar_expect(uint32_t bar, uint32_t bytes) {
 __device__ __forceinline__ void bar_arrive(uint32_t bar) {
 	asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(bar) : "memory");
 }
-__device__ __forceinline__ bool bar_wait(uint32_t bar, uint32_t parity) {
-	for (uint32_t i = 0; i < kPolls; ++i) {
-		uint32_t ok;
-		asm volatile(
-		    "{\n\t.reg .pred p;\n\tmbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n\tselp.u32 %0, 1, 0, p;\n\t}"
-		    : "=r"(ok) : "r"(bar), "r"(parity) : "memory");
-		if (ok) return true;
-		if (i > 2048) __nanosleep(64);
-	}
-	return false;
-}
+__device__ __forceinline__ bool bar_wait(uint32_t bar, uint32_t parity) { return bounded_wait<false>(bar, parity); }
 __device__ __forceinline__ void tma_2d(uint32_t dst, const CUtensorMap* map, uint32_t bar, int c0, int c1) {
 	asm volatile(
 	    "cp.async.bulk.tensor.2d.shared::cta.global.mbarrier::complete_tx::bytes [%0], [%1, {%3, %4}], [%2];"
@@ -274,7 +263,7 @@ k_skinny(const __grid_constant__ CUtensorMap map_w, const __grid_constant__ CUte
 			bar_init(acce_bar(s), Cfg::kEpiWarps);
 		}
 		s_timeout = 0;
-		if (splits > 1) exchange_init(xch_bar, Cfg::kExchangeBytes);
+		if (splits > 1) exchange_init(xch_bar, Cfg::kExchangeBytes + (a.debug_withhold == 2 && blockIdx.x == 0 ? 4 : 0));
 		exchange_fence_init();
 		// the first weight tiles: no kernel writes weights, so they need not wait for anybody
 		const int early = total < stages ? total : stages;
@@ -282,7 +271,7 @@ k_skinny(const __grid_constant__ CUtensorMap map_w, const __grid_constant__ CUte
 		for (int i = 0; i < early; ++i) {
 			bar_expect(full_bar(i), Cfg::kStageBytes);
 			// (tests of the bounded waits leave the first request out, once)
-			if (!(a.debug_withhold != 0 && blockIdx.x == 0 && i == 0))
+			if (!(a.debug_withhold == 1 && blockIdx.x == 0 && i == 0))
 				tma_2d(base + i * Cfg::kStageBytes, &map_w, full_bar(i), kb * kKBlock, t * kWRows);
 			if (++kb == kb1) { kb = kb0; t += tile_step; }
 		}
@@ -303,6 +292,7 @@ k_skinny(const __grid_constant__ CUtensorMap map_w, const __grid_constant__ CUte
 		cluster_wait();
 	}
 	const uint32_t tmem = s_tmem;
+	bool all_in = true;      // (false: a peer may still be sending)
 
 	if (warp == 0) {
 		if (lane == 0) {
@@ -376,6 +366,7 @@ k_skinny(const __grid_constant__ CUtensorMap map_w, const __grid_constant__ CUte
 				}
 			}
 			const bool ok = exchange_wait(xch_bar);
+			all_in = ok;
 			if (!acc_ok || !ok) refuse();      // (what was sent for a tile given up on is garbage: the rows say so)
 			const int my = et % rows;          // (rows divides 128 and the epilogue's thread count: one channel per thread)
 			c = channel_of(a, tile0 * kWRows + rank * rows + my);
@@ -515,6 +506,7 @@ k_skinny(const __grid_constant__ CUtensorMap map_w, const __grid_constant__ CUte
 		asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
 		asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(Cfg::kTmemCols));
 	}
+	if (__builtin_expect(!__all_sync(0xffffffffu, all_in), 0)) exchange_leave(xch_bar, 1);
 }
 
 // How a launch is cut. K slices (the blocks of a cluster): as many, up to 8, as still fit on the
@@ -564,7 +556,7 @@ bool launch_mode(const LinearArgs& a_in, cudaStream_t st, int* reason) {
 		*reason = 2;
 		return false;
 	}
-	a.debug_withhold = tc_debug_take() ? 1 : 0;
+	a.debug_withhold = tc_debug_take() ? 1 : (splits > 1 && exchange_debug_take(kExchangeLinear) ? 2 : 0);
 	cudaLaunchConfig_t cfg = {};
 	cfg.gridDim = dim3(splits > 1 ? tiles * splits : (tiles < sms ? tiles : sms));
 	cfg.blockDim = dim3(Cfg::kThreads);

@@ -128,6 +128,7 @@ struct RowBatch {
 	int8_t* lora_u;              // [m][3][kMaxLoraRank] clamped u = fold(A x) per projection slot of the current GEMM
 	unsigned long long* best;    // [m] packed (logit, index) argmax key
 	int32_t* logits;             // optional [m, vocab] dump, or nullptr
+	int debug_withhold;          // tests only (exchange_debug_take): 1 + the exchange whose wait runs out in block 0
 };
 
 }  // namespace sslm

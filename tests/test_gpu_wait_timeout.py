@@ -1,14 +1,16 @@
 """A bounded device wait that runs out, made to happen on purpose.
 
-Every mbarrier wait of the kernels has a poll limit. The tensor-core linear kernel's producer is told
+Every mbarrier wait of the kernels has a limit. The tensor-core linear kernel's producer is told
 (test-only hook sslm_b200_debug_withhold_tc_load) to arm the barrier of its first weight tile without
-requesting the tile; the wait on it gives up after the limit (about a second), the tile's rows end
+requesting the tile; the wait on it gives up after the limit (a second or less), the tile's rows end
 with the internal status 100, and the verb that launched the kernel returns SSLM_ALLOCATION_FAILED.
 Nothing faults, nothing spins without a limit, the context stays usable, and the same call then
-succeeds and gives the oracle's results. (The failure is injected on the host side of the launch:
+succeeds and gives the oracle's results. The exchanges between the blocks of a cluster likewise: one
+block waits for four bytes more than its peers send (sslm_b200_debug_withhold_exchange). (The failure is injected on the host side of the launch:
 a request that is never made. No kernel is made to trap or to loop.)
 """
 import ctypes as C
+import time
 
 import numpy as np
 import pytest
@@ -75,4 +77,47 @@ def test_prefill_fails_cleanly_and_the_next_call_succeeds(gpu_lib):
         assert blob["kv"] == ps.kv.tobytes()
     finally:
         arm(0)
+        eng.close()
+
+
+# kernel and exchange, shape, prompt, and the call whose wait runs out: the prefill or the decode step behind it
+EXCHANGES = [(0, 0, "mini1.5b", 40, "prefill"), (1, 0, "mini1.5b", 300, "decode"), (1, 1, "mini1.5b", 300, "decode"),
+             (1, 2, "mini1.5b", 300, "decode"), (2, 0, "tiny", 700, "prefill"), (2, 1, "tiny", 700, "prefill"),
+             (2, 2, "tiny", 700, "prefill")]
+
+
+@pytest.mark.parametrize("kernel,exchange,shape,n,call", EXCHANGES)
+def test_exchange_that_runs_out(gpu_lib, kernel, exchange, shape, n, call):
+    sh = A.SHAPES[shape]
+    art = A.build_synthetic_model(shape, 0x7200 + n, n + 16)
+    prompt = A.stream_uniform(0x7200 + n, "prompt", n, 0, sh.vocab - 1)
+    want_toks, ps = run_port(art, prompt, 3)
+    eng = abi.Engine(gpu_lib, art, blocks=1, max_chunk=n)
+    arm = gpu_lib.dll.sslm_b200_debug_withhold_exchange
+    arm.argtypes = [C.c_int32, C.c_int32]
+    assert arm(kernel, 4) == arm(4, 0) == abi.ST["SSLM_INVALID_ARGUMENT"]
+    failed = abi.ST["SSLM_ALLOCATION_FAILED"]
+    try:
+        s = eng.new_seq()
+        toks = np.ascontiguousarray(prompt, dtype=np.int32)
+        consumed = C.c_int32(-1)
+        t = time.perf_counter()
+        if call == "prefill":
+            assert arm(kernel, exchange) == 0
+            assert gpu_lib.sslm_prefill(eng.model, s.handle, toks.ctypes.data_as(C.POINTER(C.c_int32)), n, n, 0, eng.ws,
+                                        C.byref(consumed)) == failed
+            assert consumed.value == 0
+            took = time.perf_counter() - t
+        assert s.prefill(prompt, n) == n
+        assert s.decode(1, sh.layers) == want_toks[:1]
+        if call == "decode":
+            assert arm(kernel, exchange) == 0
+            t = time.perf_counter()
+            assert eng.decode_step([s], sh.layers)[0] == failed
+            took = time.perf_counter() - t
+        assert 0.2 < took < 5.0      # waits of a quarter of a second: four exchanges and six times that on the way out
+        assert s.decode(2, sh.layers) == want_toks[1:]
+        assert abi.parse_save_blob(s.save(), sh.hidden)["kv"] == ps.kv.tobytes()
+    finally:
+        arm(-1, 0)
         eng.close()
