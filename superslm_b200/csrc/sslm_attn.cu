@@ -742,10 +742,15 @@ k_attention_few(RowBatch b, Dims d, const LayerDev* layer, Scale c_ctx, int laye
 		}
 	}
 	top = __reduce_max_sync(0xffffffffu, top);
-	if (!ok && t == 0) atomicCAS(&b.status[r], 0, pack_status(kInternalWaitTimeout, kSiteCtx, b.layer));
+	// (every thread has its own limit, so every thread whose wait ran out speaks for the row)
+	auto give_up = [&](int exchanges) {
+		if (!ok) atomicCAS(&b.status[r], 0, pack_status(kInternalWaitTimeout, kSiteCtx, b.layer));
+		__syncwarp();
+		exchange_leave(bar(0), exchanges);
+	};
 	if (!whole_row) {
 		if (lane == 0 && top && live) atomicMax(&b.rowmax[(size_t)r * 4 + 3], (unsigned long long)top);
-		if (__builtin_expect(!__all_sync(0xffffffffu, ok), 0)) exchange_leave(bar(0), 3);
+		if (__builtin_expect(!__all_sync(0xffffffffu, ok), 0)) give_up(3);
 		return;
 	}
 	// ---- exchange 4: the cluster holds the whole row, its funnel runs here
@@ -754,7 +759,7 @@ k_attention_few(RowBatch b, Dims d, const LayerDev* layer, Scale c_ctx, int laye
 	if (t < (int)cluster_blocks) exchange_send(&s.rx_top[my_rank], bar(3), (uint32_t)t, s.misc[0]);
 	ok = exchange_wait(bar(3)) && ok;
 	if (__builtin_expect(!__all_sync(0xffffffffu, ok), 0)) {
-		exchange_leave(bar(0), 4);
+		give_up(4);
 		return;
 	}
 	if (!live) return;
@@ -1563,8 +1568,11 @@ k_attention_chunk(RowBatch b, Dims d, const LayerDev* layer, int layer_index, Kv
 		const uint32_t top = __reduce_max_sync(0xffffffffu, in ? abs_u32(o) : 0u);
 		if (lane == 0 && top) atomicMax(&b.rowmax[(size_t)(r0 + tok) * 4 + 3], (unsigned long long)top);
 	}
-	if (!ok && t < nt) atomicCAS(&b.status[r0 + t], 0, pack_status(kInternalWaitTimeout, kSiteCtx, b.layer));
-	if (__builtin_expect(!__all_sync(0xffffffffu, ok), 0)) exchange_leave(cta_addr(&s_bars[0]), 3);
+	if (__builtin_expect(!__all_sync(0xffffffffu, ok), 0)) {      // (the warp's lanes speak for the tile's rows)
+		if (lane < nt) atomicCAS(&b.status[r0 + lane], 0, pack_status(kInternalWaitTimeout, kSiteCtx, b.layer));
+		__syncwarp();
+		exchange_leave(cta_addr(&s_bars[0]), 3);
+	}
 }
 
 // How a chunk of m rows whose last row is `width` wide is cut: tiles of 32 query rows; a block holds up to

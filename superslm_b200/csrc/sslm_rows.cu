@@ -813,7 +813,8 @@ k_act(RowBatch b, Dims d, Scale c_gate, Scale c_up, Scale c_act, const int32_t* 
 		if (threadIdx.x < blocks) exchange_send(&s_peer[rank], arrived, threadIdx.x, mx);
 		const bool ok = exchange_wait(arrived);
 		if (__builtin_expect(!__all_sync(0xffffffffu, ok), 0)) {
-			set_status(b, r, kInternalWaitTimeout, kSiteAct, b.layer);
+			if ((threadIdx.x & 31) == 0) atomicCAS(&b.status[r], 0, pack_status(kInternalWaitTimeout, kSiteAct, b.layer));
+			__syncwarp();
 			exchange_leave(arrived, 1);
 			return;
 		}

@@ -340,8 +340,8 @@ k_skinny(const __grid_constant__ CUtensorMap map_w, const __grid_constant__ CUte
 		const int q = warp & 3, part = (warp - 2) >> 2, et = (int)threadIdx.x - 64;
 		constexpr int kCols = NB / (Cfg::kEpiWarps / 4);          // columns (rows of x) this warp takes
 		const int col0 = part * kCols;
-		auto refuse = [&]() {
-			for (int m = et; m < a.M; m += kEpi) {
+		auto refuse = [&]() {      // (by a whole warp, for all rows)
+			for (int m = lane; m < a.M; m += 32) {
 				if (a.status != nullptr) atomicCAS(&a.status[m], 0, (int32_t)kInternalWaitTimeout);
 				else if (a.rowmax != nullptr) atomicMax(&a.rowmax[(size_t)m * 4], kRowmaxTimeout);
 			}
@@ -367,7 +367,7 @@ k_skinny(const __grid_constant__ CUtensorMap map_w, const __grid_constant__ CUte
 			}
 			const bool ok = exchange_wait(xch_bar);
 			all_in = ok;
-			if (!acc_ok || !ok) refuse();      // (what was sent for a tile given up on is garbage: the rows say so)
+			if (!__all_sync(0xffffffffu, acc_ok && ok)) refuse();      // (what was sent for a tile given up on is garbage: the rows say so)
 			const int my = et % rows;          // (rows divides 128 and the epilogue's thread count: one channel per thread)
 			c = channel_of(a, tile0 * kWRows + rank * rows + my);
 			const int first = tile0 * kWRows + rank * rows;

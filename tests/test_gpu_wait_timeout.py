@@ -82,8 +82,8 @@ def test_prefill_fails_cleanly_and_the_next_call_succeeds(gpu_lib):
 
 # kernel and exchange, shape, prompt, and the call whose wait runs out: the prefill or the decode step behind it
 EXCHANGES = [(0, 0, "mini1.5b", 40, "prefill"), (1, 0, "mini1.5b", 300, "decode"), (1, 1, "mini1.5b", 300, "decode"),
-             (1, 2, "mini1.5b", 300, "decode"), (2, 0, "tiny", 700, "prefill"), (2, 1, "tiny", 700, "prefill"),
-             (2, 2, "tiny", 700, "prefill")]
+             (1, 2, "mini1.5b", 300, "decode"), (1, 3, "mini1.5b", 300, "decode"),
+             (2, 0, "tiny", 700, "prefill"), (2, 1, "tiny", 700, "prefill"), (2, 2, "tiny", 700, "prefill")]
 
 
 @pytest.mark.parametrize("kernel,exchange,shape,n,call", EXCHANGES)
