@@ -83,7 +83,7 @@ def test_prefill_fails_cleanly_and_the_next_call_succeeds(gpu_lib):
 # kernel and exchange, shape, prompt, and the call whose wait runs out: the prefill or the decode step behind it
 EXCHANGES = [(0, 0, "mini1.5b", 40, "prefill"), (1, 0, "mini1.5b", 300, "decode"), (1, 1, "mini1.5b", 300, "decode"),
              (1, 2, "mini1.5b", 300, "decode"), (1, 3, "mini1.5b", 300, "decode"),
-             (2, 0, "tiny", 700, "prefill"), (2, 1, "tiny", 700, "prefill"), (2, 2, "tiny", 700, "prefill")]
+             (2, 0, "tiny", 700, "prefill"), (2, 1, "tiny", 700, "prefill"), (2, 2, "tiny", 700, "prefill"), (3, 0, "mini1.5b", 40, "decode")]
 
 
 @pytest.mark.parametrize("kernel,exchange,shape,n,call", EXCHANGES)
@@ -118,6 +118,33 @@ def test_exchange_that_runs_out(gpu_lib, kernel, exchange, shape, n, call):
         assert 0.2 < took < 5.0      # waits of a quarter of a second: four exchanges and six times that on the way out
         assert s.decode(2, sh.layers) == want_toks[1:]
         assert abi.parse_save_blob(s.save(), sh.hidden)["kv"] == ps.kv.tobytes()
+    finally:
+        arm(-1, 0)
+        eng.close()
+
+
+def test_the_next_sequence_finds_the_workspace_clean(gpu_lib):
+    """The activation site of a sequence's last layer gives up with the row's gate and up maxima still in place;
+    another sequence's row then takes the same place in the workspace, with maxima that may be smaller."""
+    sh = A.SHAPES["tiny"]
+    art = A.build_synthetic_model("tiny", 0x7300, 64)
+    eng = abi.Engine(gpu_lib, art, blocks=2, max_chunk=16)
+    arm = gpu_lib.dll.sslm_b200_debug_withhold_exchange
+    arm.argtypes = [C.c_int32, C.c_int32]
+    try:
+        for i in range(6):
+            a, b = eng.new_seq(), eng.new_seq()
+            for s, salt in ((a, 2 * i), (b, 2 * i + 1)):
+                assert s.prefill(A.stream_uniform(0x7300 + salt, "prompt", 9, 0, sh.vocab - 1), 9) == 9
+                s.decode(1, sh.layers)
+            want, ps = run_port(art, A.stream_uniform(0x7300 + 2 * i + 1, "prompt", 9, 0, sh.vocab - 1), 3)
+            assert sh.layers == 2 and eng.decode_step([a], 1) == (0, [-1])
+            assert arm(3, 0) == 0
+            assert eng.decode_step([a], 1)[0] == abi.ST["SSLM_ALLOCATION_FAILED"]
+            assert b.decode(2, sh.layers) == want[1:]
+            assert abi.parse_save_blob(b.save(), sh.hidden)["kv"] == ps.kv.tobytes(), i
+            a.release()
+            b.release()
     finally:
         arm(-1, 0)
         eng.close()
