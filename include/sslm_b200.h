@@ -275,6 +275,9 @@ SSLM_API sslm_status sslm_b200_debug_withhold_tc_load(int32_t launches);
  * funnel's maximum); 2: attention of prefill chunks in tiles cut over a cluster (0 to 2); 3: the activation
  * site (0). kernel -1 takes the request back. */
 SSLM_API sslm_status sslm_b200_debug_withhold_exchange(int32_t kernel, int32_t exchange);
+/* Tests only: the first kernel of each of the next `launches` (0..16) row groups counts as refused by the CUDA
+ * runtime, as for want of resources. The verb returns SSLM_ALLOCATION_FAILED and launches nothing behind it. */
+SSLM_API sslm_status sslm_b200_debug_refuse_launch(int32_t launches);
 
 /* Tests only: the device integer library's primitives evaluated ON THE DEVICE over n operand
  * tuples (host arrays a, b, c, e; three host result arrays), so that their device-only halves

@@ -579,6 +579,11 @@ extern "C" sslm_status sslm_b200_debug_withhold_tc_load(int32_t launches) {
 	return SSLM_OK;
 }
 
+extern "C" sslm_status sslm_b200_debug_refuse_launch(int32_t launches) {
+	if (launches < 0 || launches > 16) return SSLM_INVALID_ARGUMENT;
+	g_refuse_begin.store(launches);
+	return SSLM_OK;
+}
 extern "C" sslm_status sslm_b200_debug_withhold_exchange(int32_t kernel, int32_t exchange) {
 	static const int kExchanges[kExchangeKernels] = {1, 4, 3, 1};
 	if (kernel >= kExchangeKernels || (kernel >= 0 && (exchange < 0 || exchange >= kExchanges[kernel]))) return SSLM_INVALID_ARGUMENT;

@@ -102,8 +102,10 @@ inline int exchange_debug_take(ExchangeKernel kernel) {
 cudaError_t rows_configure(const Dims& d);
 // (the host's copy `h` of a layer record carries the site constants into the launch parameters)
 // first rows of a call: embed or resume, then an RMSNorm with `gain` (nullptr: none)
-void launch_begin(const RowBatch& b, const Dims& d, const int8_t* embed, Scale c_embed, const RowSource* src, const int8_t* gain,
-                  Scale c_norm, int site_norm, cudaStream_t st);
+// (It enters the call's new pages into the page tables: when it is refused, nothing behind it may be launched.)
+cudaError_t launch_begin(const RowBatch& b, const Dims& d, const int8_t* embed, Scale c_embed, const RowSource* src, const int8_t* gain,
+                         Scale c_norm, int site_norm, cudaStream_t st);
+inline std::atomic<int> g_refuse_begin{0};      // tests: the next launches of it that count as refused by the runtime
 void launch_qkv_post(const RowBatch& b, const Dims& d, const LayerDev* layer, const LayerDev& h, int layer_index, KvPoolDev pool,
                      const int32_t* cos, const int32_t* sin, cudaStream_t st);
 void launch_ctx_funnel(const RowBatch& b, const Dims& d, const LayerDev& h, cudaStream_t st);

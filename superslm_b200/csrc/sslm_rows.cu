@@ -1018,14 +1018,15 @@ static int quads_per_thread(int rows, int nq) {
 }
 static int quad_threads(int nq, int nv) { return ((nq + nv - 1) / nv + 31) / 32 * 32; }
 
-void launch_begin(const RowBatch& b, const Dims& d, const int8_t* embed, Scale c_embed, const RowSource* src, const int8_t* gain,
-                  Scale c_norm, int site_norm, cudaStream_t st) {
+cudaError_t launch_begin(const RowBatch& b, const Dims& d, const int8_t* embed, Scale c_embed, const RowSource* src, const int8_t* gain,
+                         Scale c_norm, int site_norm, cudaStream_t st) {
+	int refuse = g_refuse_begin.load(std::memory_order_relaxed);
+	if (refuse > 0 && g_refuse_begin.compare_exchange_strong(refuse, refuse - 1)) return cudaErrorLaunchOutOfResources;
 	const int nq = d.hidden / 4, nv = quads_per_thread(b.m, nq), t = quad_threads(nq, nv);
 	const size_t sm = general_smem_bytes(d.hidden);
-	auto go = [&](auto kernel) { launch_pdl(kernel, dim3(b.m), dim3(t), sm, st, b, d, embed, c_embed, src, gain, c_norm, site_norm); };
-	if (nv == 1) go(k_begin<1>);
-	else if (nv == 4) go(k_begin<4>);
-	else go(k_begin<8>);
+	auto go = [&](auto kernel) { return launch_pdl(kernel, dim3(b.m), dim3(t), sm, st, b, d, embed, c_embed, src, gain, c_norm, site_norm); };
+	if (nv == 1) return go(k_begin<1>);
+	return nv == 4 ? go(k_begin<4>) : go(k_begin<8>);
 }
 void launch_qkv_post(const RowBatch& b, const Dims& d, const LayerDev* layer, const LayerDev& h, int layer_index, KvPoolDev pool,
                      const int32_t* cos, const int32_t* sin, cudaStream_t st) {
