@@ -1063,6 +1063,8 @@ void launch_res(const RowBatch& b, const Dims& d, const ResSite& a, cudaStream_t
 	else if (nv == 4) b.wide64 ? go(k_res<4, 512, true>) : go(k_res<4, 512, false>);
 	else b.wide64 ? go(k_res<8, 512, true>) : go(k_res<8, 512, false>);
 }
+// the widest activation row: eight blocks of 352 threads with five quads each
+constexpr int kActBlocks = 8, kActQuads = 5, kActBlockThreads = 352;
 static int act_many_smem(int nq) { return 16 * (2 * kActStages * kActWorkers + nq); }
 constexpr int kActManySmemMax = 200 * 1024;
 void launch_act(const RowBatch& b, const Dims& d, const LayerDev& h, const int32_t* silu, cudaStream_t st) {
@@ -1077,8 +1079,8 @@ void launch_act(const RowBatch& b, const Dims& d, const LayerDev& h, const int32
 	}
 	// blocks per row: as many (up to 8) as the multiprocessors hold at once, three each
 	int blocks = 2;
-	while (blocks < 8 && b.m * blocks * 2 <= 3 * sm_count()) blocks *= 2;
-	while (blocks < 8 && quad_threads((nq + blocks - 1) / blocks, 5) > 352) blocks *= 2;      // (very wide rows)
+	while (blocks < kActBlocks && b.m * blocks * 2 <= 3 * sm_count()) blocks *= 2;
+	while (blocks < kActBlocks && quad_threads((nq + blocks - 1) / blocks, kActQuads) > kActBlockThreads) blocks *= 2;      // (very wide rows)
 	const int per = (nq + blocks - 1) / blocks;
 	const int nv = per <= 384 ? 1 : (per <= 2 * 384 ? 2 : 5);
 	cudaLaunchConfig_t cfg = {};
@@ -1113,6 +1115,9 @@ cudaError_t rows_configure(const Dims& d) {
 	// a narrow model does not take it from a wider one.)
 	const int sm = 226 * 1024;
 	if (general_smem_bytes(d.hidden) > (size_t)sm) return cudaErrorInvalidConfiguration;
+	// (The hidden width needs no limit of its own here: 128 heads of 128 are 16,384, which eight quads on each of
+	// 512 threads hold, and q, k and v together 20,480, which 640 hold.)
+	if (quad_threads((d.inter / 4 + kActBlocks - 1) / kActBlocks, kActQuads) > kActBlockThreads) return cudaErrorInvalidConfiguration;
 	cudaError_t e = cudaSuccess;
 	auto set = [&](const void* f, bool dynamic) {
 		if (e == cudaSuccess) e = cudaFuncSetAttribute(f, cudaFuncAttributePreferredSharedMemoryCarveout, cudaSharedmemCarveoutMaxShared);
