@@ -1853,17 +1853,17 @@ void launch_int_sweep(int which, const int64_t* a, const int64_t* b, const int64
 }
 
 // ------------------------------------------------------------ canonical KV export
-// Writes the sequence's K and V in the reference's save layout, [layer][K|V][kv head]
-// [span][head_dim] with zeros past the valid positions, undoing the paging and the
+// Writes `planes` planes of the sequence's K and V, from plane0 on, in the reference's save layout,
+// [layer][K|V][kv head][span][head_dim] with zeros past the valid positions, undoing the paging and the
 // V-page transposition.
 __global__ void k_kv_export(Dims d, KvPoolDev pool, const int32_t* pages, int context_length,
-                            int layer_index, int span, int8_t* out) {
+                            int layer_index, int span, int plane0, int planes, int8_t* out) {
 	const int hd = d.head_dim, vec = hd / 16;
 	const int64_t per_plane = (int64_t)span * vec;
-	const int64_t total = (int64_t)d.layers * 2 * d.kv_heads * per_plane;
+	const int64_t total = planes * per_plane;
 	for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < total;
 	     i += (int64_t)gridDim.x * blockDim.x) {
-		const int64_t plane = i / per_plane, within = i - plane * per_plane;
+		const int64_t nth = i / per_plane, within = i - nth * per_plane, plane = plane0 + nth;
 		const int pos = (int)(within / vec), v = (int)(within % vec);
 		const int kvh = (int)(plane % d.kv_heads);
 		const int is_v = (int)((plane / d.kv_heads) % 2);
@@ -1889,20 +1889,20 @@ __global__ void k_kv_export(Dims d, KvPoolDev pool, const int32_t* pages, int co
 }
 
 void launch_kv_export(const Dims& d, KvPoolDev pool, const int32_t* pages, int context_length,
-                      int layer_index, int span, int8_t* out, cudaStream_t st) {
-	k_kv_export<<<148 * 4, 256, 0, st>>>(d, pool, pages, context_length, layer_index, span, out);
+                      int layer_index, int span, int plane0, int planes, int8_t* out, cudaStream_t st) {
+	k_kv_export<<<148 * 4, 256, 0, st>>>(d, pool, pages, context_length, layer_index, span, plane0, planes, out);
 }
 
-// The inverse: scatter a canonical block (a save blob's K/V) into the sequence's pages.
+// The inverse: scatter planes of a canonical block (a save blob's K/V) into the sequence's pages.
 // Only the valid positions are written; everything else in the pages is never read.
 __global__ void k_kv_import(Dims d, KvPoolDev pool, const int32_t* pages, int context_length,
-                            int layer_index, int span, const int8_t* in) {
+                            int layer_index, int span, int plane0, int planes, const int8_t* in) {
 	const int hd = d.head_dim, vec = hd / 16;
 	const int64_t per_plane = (int64_t)span * vec;
-	const int64_t total = (int64_t)d.layers * 2 * d.kv_heads * per_plane;
+	const int64_t total = planes * per_plane;
 	for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < total;
 	     i += (int64_t)gridDim.x * blockDim.x) {
-		const int64_t plane = i / per_plane, within = i - plane * per_plane;
+		const int64_t nth = i / per_plane, within = i - nth * per_plane, plane = plane0 + nth;
 		const int pos = (int)(within / vec), v = (int)(within % vec);
 		const int kvh = (int)(plane % d.kv_heads);
 		const int is_v = (int)((plane / d.kv_heads) % 2);
@@ -1943,8 +1943,8 @@ void launch_adopt(const Dims& d, KvPoolDev pool, const AdoptArgs& a, cudaStream_
 }
 
 void launch_kv_import(const Dims& d, KvPoolDev pool, const int32_t* pages, int context_length,
-                      int layer_index, int span, const int8_t* in, cudaStream_t st) {
-	k_kv_import<<<148 * 4, 256, 0, st>>>(d, pool, pages, context_length, layer_index, span, in);
+                      int layer_index, int span, int plane0, int planes, const int8_t* in, cudaStream_t st) {
+	k_kv_import<<<148 * 4, 256, 0, st>>>(d, pool, pages, context_length, layer_index, span, plane0, planes, in);
 }
 
 }  // namespace sslm

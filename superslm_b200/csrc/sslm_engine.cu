@@ -140,6 +140,8 @@ extern "C" sslm_status sslm_model_map(const void* data, size_t size, sslm_model*
 		cudaFree(m->arena.base);
 		cudaFree(m->d_schema_pages);
 		if (m->aux) cudaStreamDestroy(m->aux);
+		for (cudaEvent_t e : {m->aux_done, m->stage_done[0], m->stage_done[1]})
+			if (e) cudaEventDestroy(e);
 		delete m;
 		return st;
 	};
@@ -289,7 +291,9 @@ extern "C" sslm_status sslm_model_map(const void* data, size_t size, sslm_model*
 	m->weight_bytes = m->arena.used;
 	if (!cuda_ok(rows_configure(d)) || !cuda_ok(attn_configure(d))) return fail(SSLM_ARTIFACT_REJECTED);
 	if (!cuda_ok(cudaStreamCreateWithFlags(&m->aux, cudaStreamNonBlocking)) ||
-	    !cuda_ok(cudaEventCreateWithFlags(&m->aux_done, cudaEventDisableTiming)))
+	    !cuda_ok(cudaEventCreateWithFlags(&m->aux_done, cudaEventDisableTiming)) ||
+	    !cuda_ok(cudaEventCreateWithFlags(&m->stage_done[0], cudaEventDisableTiming)) ||
+	    !cuda_ok(cudaEventCreateWithFlags(&m->stage_done[1], cudaEventDisableTiming)))
 		return fail(SSLM_ALLOCATION_FAILED);
 	cudaDeviceSynchronize();
 	*out = m;
@@ -306,6 +310,7 @@ extern "C" sslm_status sslm_model_unmap(sslm_model model) {
 	cudaStreamSynchronize(model->aux);
 	cudaStreamDestroy(model->aux);
 	cudaEventDestroy(model->aux_done);
+	for (cudaEvent_t e : model->stage_done) cudaEventDestroy(e);
 	cudaFreeHost(model->h_stage);
 	cudaFree(model->d_stage);
 	cudaFree(model->arena.base);

@@ -26,6 +26,10 @@ struct DeviceArena {
 };
 
 constexpr int kTcTileCounters = 1024;
+// Save and restore move a sequence's K/V in pieces of whole planes. The widest plane (32,768 positions of a
+// 128-wide head) is 4 MiB; a piece of four keeps its eight host threads busy for longer than they take to start,
+// and most sequences are one piece.
+constexpr size_t kStagePiece = (size_t)16 << 20;
 
 struct sslm_workspace_s {
 	sslm_model_s* model = nullptr;
@@ -108,17 +112,19 @@ struct sslm_model_s {
 	sslm::SchemaTable schemas;
 	std::vector<sslm_schema_s> schema_handles;
 	uint8_t* d_schema_pages = nullptr;
-	// Work of the verbs that move sequence state (adoption, save, restore) runs on a stream of its own;
-	// aux_done is recorded after every piece of it, and the streams of prefill and decode wait for it
-	// when one of their sequences has such work outstanding (sslm_seq_s::pending).
+	// Work of the verbs that move sequence state (adoption, save, restore) runs on a stream of its own.
+	// Save and restore wait for theirs; an adoption records aux_done, and the streams of prefill and decode
+	// wait for that when one of their sequences has an adoption outstanding (sslm_seq_s::pending).
 	cudaStream_t aux = nullptr;
 	cudaEvent_t aux_done = nullptr;
 	std::mutex aux_mutex;
-	// staging of save and restore: a pinned block and its device twin, at most one sequence's K/V, kept
-	// from call to call (under stage_mutex) and freed with the model
+	// staging of save and restore: a pinned block and its device twin, two pieces of kStagePiece bytes and one
+	// sequence state at most, kept from call to call (under stage_mutex) and freed with the model; stage_done:
+	// what was last enqueued for either piece
 	std::mutex stage_mutex;
 	uint8_t *h_stage = nullptr, *d_stage = nullptr;
 	size_t stage_bytes = 0;
+	cudaEvent_t stage_done[2] = {nullptr, nullptr};
 };
 
 struct sslm_kv_pool_s {

@@ -203,11 +203,11 @@ void attn_force_splits(int splits);
 // b.cs); otherwise b.ctxw / rowmax slot 3 are filled and launch_ctx_funnel must follow.
 bool launch_attention(const RowBatch& b, const Dims& d, const LayerDev* layer, const LayerDev& h, int layer_index,
                       KvPoolDev pool, int max_width, int reverse_rows, cudaStream_t st, cudaError_t* err);
-// gather a sequence's pages into the reference's canonical block layout
+// gather `planes` planes of a sequence's pages, from plane0 on, into the reference's canonical block layout
 // [layer][K|V][kv_head][position][head_dim] with `span` positions per plane; positions beyond
 // `valid(layer)` are zero
 void launch_kv_export(const Dims& d, KvPoolDev pool, const int32_t* pages, int context_length,
-                      int layer_index, int span, int8_t* out, cudaStream_t st);
+                      int layer_index, int span, int plane0, int planes, int8_t* out, cudaStream_t st);
 // tests: the device integer primitives over arrays of operands (device pointers)
 void launch_int_sweep(int which, const int64_t* a, const int64_t* b, const int64_t* c, const int64_t* e, long long n, int64_t* out0,
                       int64_t* out1, int64_t* out2, cudaStream_t st);
@@ -223,8 +223,8 @@ struct AdoptArgs {
 	int state_bytes;      // a multiple of 16
 };
 void launch_adopt(const Dims& d, KvPoolDev pool, const AdoptArgs& a, cudaStream_t st);
-// the inverse: scatter a canonical block into the sequence's pages (valid positions only)
+// the inverse: scatter planes of a canonical block into the sequence's pages (valid positions only)
 void launch_kv_import(const Dims& d, KvPoolDev pool, const int32_t* pages, int context_length,
-                      int layer_index, int span, const int8_t* in, cudaStream_t st);
+                      int layer_index, int span, int plane0, int planes, const int8_t* in, cudaStream_t st);
 
 }  // namespace sslm
