@@ -520,43 +520,67 @@ k_linear_tc(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ C
 							else if (seg == 1) lmax[1] = mx > lmax[1] ? mx : lmax[1];
 							else lmax[2] = mx > lmax[2] ? mx : lmax[2];
 						} else if (a.out64 != 0 && a.fold != nullptr && a.best == nullptr && any_odd == 0u && full && nb + 32 <= a.seg_end[seg] &&
-						           (a.out_ld & 1) == 0 && (((uintptr_t)a.out) & 15) == 0 && (lora == nullptr || lora->rank == 16)) {
-							// rows with a rank-16 adapter: the same, plus the delta B u. The row's u stays in registers,
-							// a column's B row and delta fold are the same words for every row of the warp.
-							int4 u = make_int4(0, 0, 0, 0);
+						           (a.out_ld & 1) == 0 && (((uintptr_t)a.out) & 15) == 0 && (lora == nullptr || (lora->rank & 3u) == 0u)) {
+							// rows with adapters: the same, plus the delta B u, word by word of the row's u (four or sixteen
+							// bytes, as the rank's multiple allows: rows of B are `rank` bytes apart). A column's B row and delta
+							// fold are the same words for every row of the warp.
 							const LoraProjDev* pj = lora != nullptr && a.seg_lora[seg] >= 0 ? &lora->p[a.seg_lora[seg]] : nullptr;
 							if (pj != nullptr && pj->a == nullptr) pj = nullptr;
 							const int nl = nb - (seg ? a.seg_end[seg - 1] : 0);
-							const int4* brow = nullptr;
+							const int8_t *u = nullptr, *brow = nullptr;
 							const int32_t* df = nullptr;
 							if (pj != nullptr) {
-								u = *(const int4*)(a.lora_u + ((size_t)row * 3 + seg) * kMaxLoraRank);
-								brow = (const int4*)pj->b + nl;
+								u = a.lora_u + ((size_t)row * 3 + seg) * kMaxLoraRank;
+								brow = pj->b + (size_t)nl * lora->rank;
 								df = pj->df + 3 * (size_t)nl;
 							}
+							// (the first sixteen bytes of u stay in registers: a rank of 16 takes no loop)
+							const bool wide_words = pj != nullptr && (lora->rank & 15u) == 0u;
+							const int words = pj != nullptr ? (int)lora->rank >> (wide_words ? 4 : 2) : 0;
+							int4 u0 = make_int4(0, 0, 0, 0);
+							if (wide_words) u0 = *(const int4*)u;
 							int64_t* dst = (int64_t*)a.out + (size_t)row * a.out_ld + nb;
 							unsigned long long mx = 0;
+							constexpr int kAtOnce = 16;      // columns whose deltas are formed side by side (16 and 32 spill registers that the other rows need)
 #pragma unroll
-							for (int j2 = 0; j2 < 32; j2 += 2) {
-								int64_t v[2];
+							for (int j0 = 0; j0 < 32; j0 += kAtOnce) {
+								int delta[kAtOnce];
 #pragma unroll
-								for (int jj = 0; jj < 2; ++jj) {
-									const int j = j2 + jj;
-									const int4 f = sf[c0 + j];
-									uint32_t mag;
-									v[jj] = fold_plain((int32_t)r[j], f.x, f.y, (uint32_t)f.z, &mag);
-									if (pj != nullptr) {
-										const int4 bw = __ldg(brow + j);
-										int d = __dp4a(bw.x, u.x, 0);
-										d = __dp4a(bw.y, u.y, d);
-										d = __dp4a(bw.z, u.z, d);
-										d = __dp4a(bw.w, u.w, d);
-										v[jj] += (int64_t)amp_fold(d, __ldg(df + 3 * j), __ldg(df + 3 * j + 1), __ldg(df + 3 * j + 2));
+								for (int j = 0; j < kAtOnce; ++j) delta[j] = 0;
+								if (wide_words) {
+									auto word = [&](const int4& uw, int k) {
+#pragma unroll
+										for (int j = 0; j < kAtOnce; ++j) {
+											const int4 bw = __ldg((const int4*)brow + (j0 + j) * words + k);
+											delta[j] = __dp4a(bw.x, uw.x, __dp4a(bw.y, uw.y, __dp4a(bw.z, uw.z, __dp4a(bw.w, uw.w, delta[j]))));
+										}
+									};
+									word(u0, 0);
+#pragma unroll 1
+									for (int k = 1; k < words; ++k) word(((const int4*)u)[k], k);
+								} else {
+#pragma unroll 1
+									for (int k = 0; k < words; ++k) {
+										const int uw = ((const int*)u)[k];
+#pragma unroll
+										for (int j = 0; j < kAtOnce; ++j) delta[j] = __dp4a(__ldg((const int*)brow + (j0 + j) * words + k), uw, delta[j]);
 									}
-									const unsigned long long ab = v[jj] < 0 ? (~(unsigned long long)v[jj] + 1ull) : (unsigned long long)v[jj];
-									mx = ab > mx ? ab : mx;
 								}
-								*(longlong2*)(dst + j2) = make_longlong2(v[0], v[1]);
+#pragma unroll
+								for (int j2 = 0; j2 < kAtOnce; j2 += 2) {
+									int64_t v[2];
+#pragma unroll
+									for (int jj = 0; jj < 2; ++jj) {
+										const int j = j0 + j2 + jj;
+										const int4 f = sf[c0 + j];
+										uint32_t mag;
+										v[jj] = fold_plain((int32_t)r[j], f.x, f.y, (uint32_t)f.z, &mag);
+										if (pj != nullptr) v[jj] += (int64_t)amp_fold(delta[j2 + jj], __ldg(df + 3 * j), __ldg(df + 3 * j + 1), __ldg(df + 3 * j + 2));
+										const unsigned long long ab = v[jj] < 0 ? (~(unsigned long long)v[jj] + 1ull) : (unsigned long long)v[jj];
+										mx = ab > mx ? ab : mx;
+									}
+									*(longlong2*)(dst + j0 + j2) = make_longlong2(v[0], v[1]);
+								}
 							}
 							if (seg == 0) lmax[0] = mx > lmax[0] ? mx : lmax[0];
 							else if (seg == 1) lmax[1] = mx > lmax[1] ? mx : lmax[1];
