@@ -551,6 +551,13 @@ bool launch_mode(const LinearArgs& a_in, cudaStream_t st, int* reason) {
 	const size_t fixed = 1024 + (splits > 1 ? Cfg::kExchangeBytes : 0);
 	int stages = (int)((kSmemMax - fixed) / Cfg::kStageBytes);
 	stages = stages > kMaxStages ? kMaxStages : stages;
+	// In clusters, no more than lets two blocks share a multiprocessor: sixteen clusters of eight blocks that take one
+	// each do not fit side by side, nor thirty-six of four (the last ones ran alone: K = 11,008 and 2,048 channels,
+	// 2 rows 22.6 us in place of 14.4, 64 rows 24.7 / 16.5; 4,608 channels 28.9 / 18.5), and where the clusters fit
+	// anyway the shallower ring is as fast (7 to 15 tiles: 0.88 to 1.00 of the time).
+	constexpr int kShare = 113 * 1024 - 1024 - (int)((2 * kMaxStages + 5) * 8 + NB * 4 + 8 + 256);
+	const int shared = (kShare - (int)fixed) / (int)Cfg::kStageBytes;
+	if (splits > 1 && shared >= 2 && stages > shared) stages = shared;
 	if (stages > per_block) stages = per_block;
 	if (stages < 1) {
 		*reason = 2;
