@@ -289,7 +289,15 @@ SSLM_API sslm_status sslm_b200_debug_refuse_launch(int32_t launches);
  *     incoming scale (b, c), site constant (e >> 32, low half of e): out0/out1 the output scale, out2 status
  *   7 one i-exp softmax element: shifted score a, constants (q_ln2 b, q_b c, q_c e >> 32), peak = low
  *     half of e << 16: out0 value, out1 refused, out2 the value rebuilt from its (shift, remainder)
- *   8 Q15 probability floor((a << 15) / b). */
+ *   8 Q15 probability floor((a << 15) / b)
+ * and the short forms of the row and prefill kernels (out1 = 0 where a form does not cover the operands):
+ *   9 code of a in a row of maximum b: out0 32-bit, out1 64-bit elements, out2 0 if the signs agree
+ *  10 the same for small integers in floats: out0 of a, out1 of -a
+ *  11 residual landing of code a: branch scale (b, e >> 32), stream scale (c, low half of e): out0, out1 covered
+ *  12 RMSNorm of code a, sum of squares b over c elements: out0 quotient, out1 covered, out2 root
+ *  13 i-exp element: shifted score a, constants q_ln2 b, q_b c, q_c e: out0 value, out1 (shift, base)
+ *  14 Q15 probability of a (shift, base) word a, row total b, q_c = c: out0, out1 settled exactly
+ *  15 K/V landing as in 4: out0 value, out1 covered. */
 SSLM_API sslm_status sslm_b200_int_sweep(int32_t which, const int64_t* a, const int64_t* b, const int64_t* c,
                                 const int64_t* e, int64_t n, int64_t* out0, int64_t* out1, int64_t* out2);
 

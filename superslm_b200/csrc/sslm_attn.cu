@@ -1840,6 +1840,70 @@ __global__ void k_int_sweep(int which, const int64_t* a, const int64_t* b, const
 			o1 = prob_q15(a[i], tot, 32768.0f / (float)tot);      // the exact form by itself
 			break;
 		}
+		case 9: {      // the row kernels' code of x = a in a row of maximum b
+			const QuadFunnel q = quad_funnel((unsigned long long)b[i], FunnelFold{Scale{1 << 30, 0}, kOk, kOk});
+			const int32_t x32[4] = {(int32_t)a[i], (int32_t)-a[i], 0, (int32_t)a[i]};
+			const int64_t x64[4] = {0, a[i], -a[i], 0};
+			const uint32_t c32 = code_quad(x32, q), c64 = code_quad(x64, q);
+			o0 = byte_of(c32, 0);
+			o1 = byte_of(c64, 1);
+			o2 = (byte_of(c32, 1) == -o0 && byte_of(c32, 3) == o0 && byte_of(c64, 2) == -o1) ? 0 : 1;
+			break;
+		}
+		case 10: {      // the same for small integers held in floats
+			const QuadFunnel q = quad_funnel((unsigned long long)b[i], FunnelFold{Scale{1 << 30, 0}, kOk, kOk});
+			const float x[4] = {(float)a[i], (float)-a[i], 0.0f, (float)a[i]};
+			const uint32_t c4 = code_small_quad(x, q);
+			o0 = byte_of(c4, 0);
+			o1 = byte_of(c4, 1);
+			break;
+		}
+		case 11: {      // the residual site's landing of code a: branch scale (b, e >> 32), stream scale (c, low half of e)
+			const Scale bs{b[i], e[i] >> 32}, ss{c[i], (int64_t)(int32_t)(uint32_t)e[i]};
+			const Branch br = make_branch(bs, make_recip(dyn_recip(ss.m)), ss);
+			float w[4] = {0.0f, 0.0f, 0.0f, 0.0f};
+			if (br.fast) join_quad((uint32_t)(uint8_t)a[i], 0u, br, bs, ss, w);
+			o0 = (int64_t)w[0];
+			o1 = br.fast ? 1 : 0;
+			break;
+		}
+		case 12: {      // RMSNorm: floor((a << 32) / root), the root of a row of c elements whose squares add up to b
+			const NormDiv nd = make_norm_div((uint32_t)b[i], (int)c[i], rcp_estimate((double)c[i]));
+			o0 = norm_quotient((int)a[i], nd);
+			o1 = nd.fast ? 1 : 0;
+			o2 = nd.root;
+			break;
+		}
+		case 13: {      // the prefill kernels' softmax element; o1 its (shift, base) word
+			SoftmaxConsts k;
+			k.c = IExpConsts{b[i], c[i], e[i]};
+			k.peak = 0;
+			const IExpFast f = iexp_fast_prepare(k);
+			uint32_t parts = 0;
+			o0 = chunk_exp((uint32_t)a[i], f, &parts);
+			o1 = parts;
+			break;
+		}
+		case 14: {      // their Q15 probability of the element with the word a: constant q_c = c, row total b
+			IExpFast f{};
+			f.qc = c[i];
+			const ChunkProb p = chunk_prob((unsigned long long)b[i], f);
+			float near = 1.0f;
+			o0 = chunk_prob_of((uint32_t)a[i], p, &near) & 0xFFFFu;
+			o1 = near < p.eps ? 1 : 0;
+			if (o1) o0 = chunk_prob_exact((uint32_t)a[i], kBaseOfZero, kBaseOfZero, kBaseOfZero, f.qc, (unsigned long long)b[i]).x;
+			break;
+		}
+		case 15: {      // K/V landing (operands of case 4), magnitude without the clamp
+			const Lander l = make_lander(b[i], c[i], e[i] >> 32, (int64_t)(int32_t)(uint32_t)e[i]);
+			const uint64_t ac = a[i] < 0 ? (~(uint64_t)a[i] + 1u) : (uint64_t)a[i];
+			o1 = l.fast && ac <= (1ull << 31) ? 1 : 0;
+			if (o1) {
+				const uint64_t m = land_magnitude((uint32_t)ac, l);
+				o0 = ((a[i] < 0) != l.neg) ? -(int64_t)m : (int64_t)m;
+			}
+			break;
+		}
 		default: break;
 		}
 		out0[i] = o0;

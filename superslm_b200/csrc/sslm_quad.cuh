@@ -89,13 +89,16 @@ __device__ __forceinline__ QuadFunnel quad_funnel(unsigned long long mx, const F
 }
 
 // ------------------------------------------------------------------ requant codes
-// code = round_half_away(x * 127 R / 2^E), |x| <= the row's maximum (so |code| <= 127).
-// v = x * f: the roundings of x, d, f and the product put v within 127 * 2^-23 < 1.6e-5 of the exact
-// quotient, so unless v is within 2e-5 of a half-integer its nearest integer IS the code: five
-// instructions per element instead of about twenty. One element in 25,000 is closer -- one in most
-// activation rows, and a row waits for its slowest warp -- so those are settled in place by adding
-// x * f_lo to the distance, and only within 1e-6 of the tie (or in a row above 2^24, where x and d
-// themselves round) out of line, at last by requant_code itself.
+// code = round_half_away(x * 127 R / 2^E), |x| <= the row's maximum d (so |code| <= 127).
+// v = x * f with f = 127 / d rounded once. Up to d = 2^24 nothing else rounds and v is within 127 * 2^-24 of the
+// exact quotient. Above, x and d round as well. Rounding moves a number of mantissa mu by 2^-24 / mu of itself,
+// x moves v by no more than d does, and the mantissa of f is 127/64 / mu (twice that for mu above 127/64): all
+// three together move v by 127 * 2^-24 (1/mu + 1/mu + mu / (127/64)) <= 127 * 2^-24 * 2.504 < 1.896e-5, at mu = 1;
+// products of roundings, R's own (2^-32) and the rounding of the distance add less than 4e-8. So unless v is
+// within 2e-5 of a half-integer its nearest integer IS the code: five instructions per element instead of about
+// twenty. One element in 25,000 is closer -- one in most activation rows, and a row waits for its slowest warp --
+// so those are settled in place by adding x * f_lo to the distance, and only within 1e-6 of the tie (or in a row
+// above 2^24) out of line, at last by requant_code itself.
 constexpr float kRoundMagic = 12582912.0f;      // 1.5 * 2^23: adding it leaves the nearest integer in the low bits
 constexpr int kRoundMagicBits = 0x4B400000;
 constexpr float kNearTie = 0.49998f;

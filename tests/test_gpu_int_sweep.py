@@ -141,3 +141,119 @@ def test_softmax_element_and_probability_on_the_device(gpu_lib):
     got = device_sweep(gpu_lib, 8, ev, tot, zeros(), zeros())
     want = ((ev.astype(np.uint64) << np.uint64(15)) // tot.astype(np.uint64)).astype(I64)
     assert (got[0] == want).all()
+
+
+def funnel_scalars(d):
+    """(R, s) of a row of maximum d, as NormalizeScale and DynamicScaleReciprocal give them."""
+    s = 30 - np.floor(np.log2(d.astype(np.float64))).astype(I64)
+    dn = np.where(s >= 0, d << np.maximum(s, 0), d >> 1)
+    assert ((dn >= 1 << 30) & (dn < 1 << 31)).all()
+    return oracle_sweep(0, dn, np.zeros_like(dn), np.zeros_like(dn), np.zeros_like(dn))[0], s
+
+
+def near_ties(rng, d, low, spread):
+    """elements of rows of maximum d: near (2 c + 1) d / 254, the ties, for |c| from `low` up, and anywhere."""
+    n = d.size
+    c = rng.integers(low, 127, n, dtype=I64)
+    x = ((2 * c + 1) * d) // 254 + rng.integers(-spread, spread + 1, n, dtype=I64)
+    x[::3] = rng.integers(0, 1 << 62, x[::3].size, dtype=I64) % (d[::3] + 1)
+    return np.minimum(np.abs(x), d) * rng.choice(np.array([1, -1], dtype=I64), n)
+
+
+def test_row_codes_on_the_device(gpu_lib):
+    rng = np.random.default_rng(6)
+    for lo, hi, low, spread in [(24, 31, 118, 40), (24, 31, 0, 3), (30, 31, 120, 400), (16, 24, 0, 2), (1, 16, 0, 1)]:
+        d = np.exp2(rng.uniform(lo, hi, N)).astype(I64)
+        d[::11] = (1 << rng.integers(lo, hi + 1, d[::11].size, dtype=I64)) + rng.integers(-3, 4, d[::11].size, dtype=I64)
+        d[::13] = 1 << hi
+        d = np.clip(d, 1, (1 << 31) - 1)
+        if hi == 31:
+            d[5] = 1 << 31      # (the maximum of a row may be 2^31; an element that is no int32 may not be given here)
+        x = np.clip(near_ties(rng, d, low, spread), -(1 << 31) + 1, (1 << 31) - 1)
+        r, s = funnel_scalars(d)
+        want = oracle_sweep(3, x, r, s, zeros())[0]
+        got = device_sweep(gpu_lib, 9, x, d, zeros(), zeros())
+        assert (got[0] == want).all() and (got[1] == want).all() and not got[2].any(), (lo, hi)
+    d = rng.integers(1, 1 << 16, N, dtype=I64)
+    d[::2] = rng.integers(1, 600, d[::2].size, dtype=I64)
+    x = near_ties(rng, d, 0, 1)
+    r, s = funnel_scalars(d)
+    want = oracle_sweep(3, x, r, s, zeros())[0], oracle_sweep(3, -x, r, s, zeros())[0]
+    got = device_sweep(gpu_lib, 10, x, d, zeros(), zeros())
+    assert (got[0] == want[0]).all() and (got[1] == want[1]).all()
+
+
+def test_landings_of_the_row_kernels_on_the_device(gpu_lib):
+    rng = np.random.default_rng(7)
+    code = rng.integers(-127, 128, N, dtype=I64)
+    bs_m, ss_m = canonical(rng, N), canonical(rng, N)
+    bs_m[::4] = np.clip(ss_m[::4] + rng.integers(-300, 301, bs_m[::4].size, dtype=I64), 1 << 30, (1 << 31) - 1)   # ratios near powers of two: true ties
+    bs_m[::17] *= -1
+    bs_e, ss_e = rng.integers(-60, -20, N, dtype=I64), rng.integers(-60, -20, N, dtype=I64)
+    ss_e[::2] = bs_e[::2] + rng.integers(-9, 8, ss_e[::2].size, dtype=I64)
+    e = pack(bs_e, ss_e)
+    want = oracle_sweep(4, code, bs_m, oracle_sweep(0, ss_m, zeros(), zeros(), zeros())[0], e)
+    got = device_sweep(gpu_lib, 11, code, bs_m, ss_m, e)
+    covered = got[1] != 0
+    assert covered.sum() > N // 3 and (np.abs(want[0][covered]) < 1 << 15).all()
+    assert (got[0][covered] == want[0][covered]).all()
+    acc = rng.integers(-(1 << 31), (1 << 31) + 1, N, dtype=I64)
+    acc[::3] = rng.integers(-127, 128, acc[::3].size, dtype=I64)
+    r_t = rng.integers((1 << 31) + 1, (1 << 32) + 1, N, dtype=I64)
+    e = pack(rng.integers(-90, 40, N, dtype=I64), rng.integers(-70, 20, N, dtype=I64))
+    want = oracle_sweep(4, acc, bs_m, r_t, e)
+    got = device_sweep(gpu_lib, 15, acc, bs_m, r_t, e)
+    covered = got[1] != 0
+    assert covered.sum() > N // 4
+    assert (got[0][covered] == want[0][covered]).all()
+
+
+def test_norm_quotients_of_the_row_kernels_on_the_device(gpu_lib):
+    rng = np.random.default_rng(8)
+    n = rng.choice(np.array([128, 256, 896, 1536, 2048, 3584, 8192, 16384], dtype=I64), N)
+    rms = np.exp2(rng.uniform(-1, 6.98, N))
+    ss = np.clip((n * rms * rms).astype(I64), 1, n * 127 * 127)
+    ss[::5] = n[::5] * rng.integers(1, 128, ss[::5].size, dtype=I64) ** 2          # the root a whole code, and its neighbours
+    ss[::5] += rng.integers(-1, 2, ss[::5].size, dtype=I64)
+    h = rng.integers(-127, 128, N, dtype=I64)
+    root = np.maximum(oracle_sweep(1, (ss << 32) // n, zeros(), zeros(), zeros())[0], 1)
+    got = device_sweep(gpu_lib, 12, h, ss, n, zeros())
+    covered = got[1] != 0
+    assert (covered == (root >= 1 << 16)).all() and covered.sum() > N // 2
+    assert (got[2][covered] == root[covered]).all()
+    assert (got[0][covered] == ((h << 32) // root)[covered]).all()
+
+
+def test_prefill_softmax_on_the_device(gpu_lib):
+    rng = np.random.default_rng(9)
+    port = H.port()
+    sets = []
+    for i in range(64):
+        m, e = int(rng.integers(1 << 30, 1 << 31)), int(rng.integers(-51, -33))
+        ln2, qb, qc = C.c_int64(0), C.c_int64(0), C.c_int64(0)
+        if port.osc_iexp_scale_constants(m, e, C.byref(ln2), C.byref(qb), C.byref(qc)) == 0 and ln2.value >= 1 and \
+           qb.value * qb.value + qc.value <= (1 << 47):
+            sets.append((ln2.value, qb.value, qc.value))
+    assert len(sets) >= 16
+    pick = rng.integers(0, len(sets), N)
+    ln2, qb, qc = (np.array([sets[i][k] for i in pick], dtype=I64) for k in range(3))
+    dq = (rng.integers(0, 34, N) * ln2 + rng.integers(-3, 4, N)).clip(0, (1 << 32) - 1).astype(I64)
+    dq[::17] = rng.integers(0, 1 << 32, dq[::17].size, dtype=I64)
+    x = np.minimum(dq, 30 * ln2)
+    value = ((qb - x % ln2) ** 2 + qc) >> (x // ln2)
+    got = device_sweep(gpu_lib, 13, dq, ln2, qb, qc)
+    assert (got[0] == value).all()
+    words = got[1]
+    z, base = words >> 24, words & 0xFFFFFF
+    assert ((base * base + qc) >> z == value).all()
+    # totals from the element alone to rows of 32,768 of the largest; some for quotients beside a whole number
+    tot = np.maximum(value, 1) + (rng.integers(0, 1 << 62, N, dtype=I64) >> rng.integers(0, 61, N)) % ((qb * qb + qc) * 32767)
+    k = rng.integers(1, 1 << 15, N, dtype=I64)
+    near = (value << 15) // k + rng.integers(-2, 3, N, dtype=I64)
+    use = (rng.integers(0, 2, N) == 0) & (near >= value) & (near > 0)
+    tot[use] = near[use]
+    words[::41] = 63 << 24                                                          # elements that count for nothing
+    value[::41] = 0
+    got = device_sweep(gpu_lib, 14, words, tot, qc, zeros())
+    want = ((value.astype(np.uint64) << np.uint64(15)) // tot.astype(np.uint64)).astype(I64)
+    assert (got[0] == want).all()
