@@ -242,8 +242,9 @@ SSLM_API sslm_status sslm_b200_last_call_ms(sslm_workspace ws, float* ms, uint64
 /* Process-wide counters of the tensor-core linear kernel: launches, times it declined a shape
  * (the streaming kernel ran instead) and the reason code of the last refusal. */
 SSLM_API sslm_status sslm_b200_tc_stats(uint64_t* launches, uint64_t* refusals, int32_t* last_reason);
-/* Launches of the tensor-core linear kernel per tile shape (rows x weight columns), first n of:
- * 128 x 64, 128 x 128, 256 x 64, 256 x 128. Lets a test assert which variant served a shape. */
+/* Launches of the tensor-core linear kernels, first n of: the activation-major one per tile shape (rows x weight
+ * columns) 128 x 64, 128 x 128, 256 x 64, 256 x 128; the weights-first one. Lets a test assert which of them
+ * served a shape. */
 SSLM_API sslm_status sslm_b200_tc_variant_counts(uint64_t* counts, int32_t n);
 
 /* Attention cuts a row along its context width into slices that run as the blocks of one

@@ -39,7 +39,7 @@ namespace sslm {
 // 5 the launch itself was refused)
 static std::atomic<unsigned long long> g_tc_launches{0}, g_tc_refusals{0};
 static std::atomic<int> g_tc_last_reason{0};
-// launches per kernel variant: 0 = 128 x 64 tiles, 1 = 128 x 128, 2 = 256 x 64, 3 = 256 x 128
+// launches per kernel variant: 0 = 128 x 64 tiles, 1 = 128 x 128, 2 = 256 x 64, 3 = 256 x 128, 4 = weights first (sslm_skinny.cu)
 static std::atomic<unsigned long long> g_tc_variant[8];
 
 namespace {
@@ -750,8 +750,12 @@ bool tc_tensor_map(const void* ptr, int rows, int k, int box_rows, bool cache, C
 	return cache ? tensor_map(ptr, rows, k, box_rows, out) : encode_map(ptr, rows, k, box_rows, out);
 }
 void tc_count(bool launched, int reason) {
-	if (launched) g_tc_launches.fetch_add(1);
-	else tc_refuse(reason);
+	if (!launched) {
+		tc_refuse(reason);
+		return;
+	}
+	g_tc_launches.fetch_add(1);
+	g_tc_variant[4].fetch_add(1);
 }
 
 void tc_debug_withhold(int launches) { g_debug_withhold.store(launches < 0 ? 0 : launches); }

@@ -72,7 +72,7 @@ def test_resident_linear_matches_the_allocating_entry_twice_in_a_row(gpu_lib):
         got = resident_entry(gpu_lib, torch, x, w, fold, in_scales)
         for a, b, what in zip(got, want, ("folded", "codes", "scales", "status")):
             assert (a == b).all(), (what, seed)
-        # both entry points run the same projection kernel, so the CPU oracle is asked as well
+        # (the other entry point runs the streaming kernel here; both are held to the CPU oracle)
         from tests.test_gpu_parity import oracle_linear
         cpu = oracle_linear(x, w, fold, in_scales, SITE)
         for a, b, what in zip(got, cpu, ("folded", "codes", "scales", "status")):
@@ -90,3 +90,39 @@ def test_resident_linear_refuses_more_rows_than_its_scratch_holds(gpu_lib):
     assert f(p, p, p, 257, 16, 16, p, SITE[0], SITE[1], p, None, None, None, None) == 1     # SSLM_INVALID_ARGUMENT
     assert f(p, p, p, 4, 16, 16400, p, SITE[0], SITE[1], p, None, None, None, None) == 1
     torch.cuda.synchronize()
+
+
+def check_resident(lib, torch, seed, M, N, K):
+    from tests.test_gpu_parity import oracle_linear
+    x, w, fold, in_scales = make_case(seed, M, N, K, 127)
+    got, want = resident_entry(lib, torch, x, w, fold, in_scales), oracle_linear(x, w, fold, in_scales, SITE)
+    for a, b, what in zip(got, want, ("folded", "codes", "scales", "status")):
+        assert (np.asarray(a, dtype=np.int64) == np.asarray(b, dtype=np.int64)).all(), what
+
+
+@pytest.mark.parametrize("M,N,K", [(1, 300, 512), (2, 2048, 1536), (8, 1152, 896), (16, 77, 48), (17, 1536, 4864), (33, 900, 896),
+                                   (64, 1536, 1536), (65, 1536, 1536), (128, 1536, 1536), (100, 4000, 1536), (129, 2048, 1536),
+                                   (130, 17920, 256), (256, 2048, 896), (256, 9728, 896)])
+def test_resident_linear_on_every_kernel(gpu_lib, M, N, K):
+    """one row (streaming), each row padding of the weights-first kernel, clustered and not, and the activation-major one"""
+    torch = pytest.importorskip("torch")
+    torch.cuda.set_device(0)
+    check_resident(gpu_lib, torch, M, M, N, K)
+
+
+@pytest.mark.parametrize("M,N,K,given_up", [(40, 1536, 1536, 40), (40, 20000, 256, 40), (200, 2048, 1536, 128)])
+def test_resident_linear_reports_a_wait_that_ran_out(gpu_lib, M, N, K, given_up):
+    """the weights-first kernel, clustered and not, and the activation-major one (rows of the abandoned tile); there is
+    no status array for the projection to write, so it travels as the row maximum"""
+    torch = pytest.importorskip("torch")
+    torch.cuda.set_device(0)
+    arm = gpu_lib.dll.sslm_b200_debug_withhold_tc_load
+    arm.argtypes = [C.c_int32]
+    x, w, fold, in_scales = make_case(5, M, N, K, 127)
+    assert arm(1) == 0
+    try:
+        status = resident_entry(gpu_lib, torch, x, w, fold, in_scales)[3]
+    finally:
+        arm(0)
+    assert (status[:given_up] == 100).all() and (status[given_up:] == 0).all()
+    check_resident(gpu_lib, torch, 6, M, N, K)      # nothing of it is left in the fixed array
