@@ -728,9 +728,9 @@ k_res(RowBatch b, Dims d, ResSite a) {
 // The activation row is the longest a row site walks (intermediate width, three codes per element).
 // While rows are few its time is one block's chain, so a row is cut over a cluster of `gridDim.x`
 // blocks, which meet once, for the maximum of the products; on a prefill chunk two blocks share a row.
-// FOUR: in 72 registers, so that four blocks of 224 threads fit a multiprocessor
-template <int NV, bool W64, bool FOUR = false>
-__global__ void __launch_bounds__(FOUR ? 288 : (NV == 5 ? 352 : 384), NV == 1 ? 1 : (FOUR ? 3 : 2))
+// DENSE: in 72 registers instead of 80, for one more block per multiprocessor at some widths (launch_act)
+template <int NV, bool W64, bool DENSE = false>
+__global__ void __launch_bounds__(DENSE ? 288 : (NV == 5 ? 352 : 384), NV == 1 ? 1 : (DENSE ? 3 : 2))
 k_act(RowBatch b, Dims d, Scale c_gate, Scale c_up, Scale c_act, const int32_t* silu_table) {
 	using T = typename WideOf<W64>::T;
 	__shared__ uint32_t s_bank[64];
@@ -1099,12 +1099,17 @@ void launch_act(const RowBatch& b, const Dims& d, const LayerDev& h, const int32
 	RowBatch rb = b;
 	rb.debug_withhold = exchange_debug_take(kExchangeAct);
 	auto go = [&](auto kernel) { cudaLaunchKernelEx(&cfg, kernel, rb, d, h.c_gate, h.c_up, h.c_act, silu); };
+	// Registers decide how many blocks a multiprocessor holds: 3 of 224 threads (8,960 elements in two blocks) or 2 of
+	// 288 (11,008) with 80 each, one more with 72, which costs a few instructions. The dense form is the faster one
+	// where the other leaves blocks for a second wave, whole prompts in ms, dense / other: 8,960 x 28 layers, 256 rows
+	// 2.62 / 2.66, 300 3.29 / 3.33, 500 4.00 / 4.04; 11,008 x 4 layers, 215 rows 0.527 / 0.541, 350 0.688 / 0.699.
+	// Where all blocks run at once anyway it is not: 215 rows of 8,960 2.558 / 2.528, 140 of 11,008 0.512 / 0.507.
+	const int threads = quad_threads(per, nv), plain_per_sm = 65536 / (80 * threads), dense_per_sm = 65536 / (72 * threads);
+	const bool dense = threads <= 288 && dense_per_sm > plain_per_sm && b.m * blocks > plain_per_sm * sm_count();
 	if (nv == 1) b.wide64 ? go(k_act<1, true>) : go(k_act<1, false>);
 	else if (nv == 2) b.wide64 ? go(k_act<2, true>) : go(k_act<2, false>);
 	else if (b.wide64) go(k_act<5, true>);
-	// (three blocks fit in 80 registers; where that leaves a second, short wave -- 256 rows of 8,960 -- four in
-	// 72 are 1.5 us faster, and 0.7 us slower where it does not)
-	else if (b.m * blocks > 3 * sm_count() && quad_threads(per, nv) <= 288) go(k_act<5, false, true>);
+	else if (dense) go(k_act<5, false, true>);
 	else go(k_act<5, false>);
 }
 cudaError_t rows_configure(const Dims& d) {

@@ -1,6 +1,7 @@
-"""The activation site of prefill chunks with many rows (persistent blocks), against the CPU oracle: around the
-row count where it takes over, rows shorter and longer than a block is wide with and without a remainder, and
-one, two and more rows per block."""
+"""The activation site of prefill chunks with many rows, against the CPU oracle. Persistent blocks: around the
+row count where they take over, rows shorter and longer than a block is wide with and without a remainder, and
+one, two and more rows per block. Below: either side of the line to the form with one more block per multiprocessor,
+at the two widths that have one."""
 import pytest
 
 from superslm_b200 import abi, artifact as A
@@ -8,7 +9,8 @@ from tests.test_gpu_parity import run_port
 
 pytestmark = pytest.mark.gpu
 
-CASES = [("tiny", 511), ("tiny", 512), ("tiny", 741), ("tiny", 3100), ("small", 800), ("mini0.5b", 515)]
+CASES = [("tiny", 511), ("tiny", 512), ("tiny", 741), ("tiny", 3100), ("small", 800), ("mini0.5b", 515),
+         ("mini1.5b", 222), ("mini1.5b", 223), ("mini3b", 148), ("mini3b", 149)]
 
 
 @pytest.mark.parametrize("shape,n", CASES)
