@@ -1,10 +1,12 @@
-// Integer i-exp softmax attention over the paged int8 KV pool, staged through shared
-// memory, with both contractions on the tensor cores (mma.sync m16n8k32, exact int32
-// accumulation). A row (one token's q heads over positions 0..pos) is cut by kv head and along
-// the context width; a block of head_dim/16 warps owns one slice of one kv head and serves every
-// q head of the GQA group from one pass over its K and V pages, so each K / V byte of the
-// sequence leaves HBM once per kv head. The blocks of a row form a thread-block cluster and
-// exchange maxima, sums and partial contexts through distributed shared memory (k_attention).
+// Integer i-exp softmax attention over the paged int8 KV pool, staged through shared memory, with both
+// contractions on the tensor cores (mma.sync m16n8k32, exact int32 accumulation). A row is one token's q heads
+// over positions 0..pos, cut by kv head, so that each K / V byte of a sequence leaves HBM once per kv head:
+//
+//   k_attention        many decode rows: a block of head_dim/16 warps owns one kv head of a row and meets nobody
+//   k_attention_few    few rows: the row is cut along its width as well; its blocks form a thread-block cluster
+//                      and exchange maxima, sums and partial contexts through distributed shared memory
+//   k_attention_chunk  prefill chunks: tiles of 32 query rows, wide ones cut over a cluster, scores kept
+//   k_attention_tile   prefill chunks: tiles of 64 query rows, the prefix walked three times, nothing kept
 //
 //   stage 1  scores[g][k] = q_rot[g] . K[k]      A = the group's q rows (heads in the M
 //            dimension), B = 8 K rows per MMA straight from the page (16-byte loads; the
@@ -153,10 +155,6 @@ __device__ __forceinline__ void load_row_words(const int8_t* row, int c, uint32_
 	} else {
 		const int4 x = *(const int4*)(row + c * 16);
 		w[0] = (uint32_t)x.x; w[1] = (uint32_t)x.y; w[2] = (uint32_t)x.z; w[3] = (uint32_t)x.w;
-		if constexpr (HD == 128) {
-			const int4 y = *(const int4*)(row + 64 + c * 16);
-			w[4] = (uint32_t)y.x; w[5] = (uint32_t)y.y; w[6] = (uint32_t)y.z; w[7] = (uint32_t)y.w;
-		}
 	}
 }
 

@@ -32,9 +32,7 @@ constexpr int kLutBytes = 256 * 8 + 256;
 // every thread folds the (at most 32) posted values itself. A bank is rewritten only two
 // reductions later, i.e. after a barrier that every reader of its old contents has passed.
 constexpr int kRedBank = 32;                   // one slot per warp
-constexpr int kRedMisc = 2 * kRedBank;         // four more words for single values handed to the block
-constexpr int kRedWords = kRedMisc + 4;
-constexpr int kRedBytes = kRedWords * 8;
+constexpr int kRedBytes = 2 * kRedBank * 8;
 struct Red {
 	unsigned long long* w;
 	int phase;
@@ -65,13 +63,11 @@ __device__ __forceinline__ unsigned long long block_max_u64(unsigned long long v
 	}
 	return m;
 }
-// small: every thread's addend and the warp totals fit 32 bits (a cheaper warp step)
-__device__ __forceinline__ long long block_sum_i64(long long v, Red& red, bool small = false) {
+__device__ __forceinline__ long long block_sum_i64(long long v, Red& red) {
 	const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nw = (blockDim.x + 31) >> 5;
 	unsigned long long* bank = red.w + red.phase * kRedBank;
 	red.phase ^= 1;
-	if (small) v = (long long)__reduce_add_sync(0xffffffffu, (uint32_t)v);
-	else v = warp_sum_i64(v);
+	v = warp_sum_i64(v);
 	if (lane == 0) bank[warp] = (unsigned long long)v;
 	__syncthreads();
 	long long s = (long long)bank[0];
