@@ -848,7 +848,7 @@ k_act(RowBatch b, Dims d, Scale c_gate, Scale c_up, Scale c_act, const int32_t* 
 // each thread its own, kActStages steps ahead and on into the next row, so neither needs a barrier), leave
 // the products there and meet once, for their maximum. The loops stay rolled: kept in registers, the
 // products took so much code that a fifth of the time went into fetching it. Bound by instruction issue
-// (210 a quad and warp, 60 % of the slots): 2,047 rows of 8,960 take 47 us in place of 73, of which the
+// (210 a quad and warp, half of the slots): 2,047 rows of 8,960 take 47 us in place of 73, of which the
 // 165 MB that move need 26.
 constexpr int kActWorkers = 256, kActThreads = kActWorkers + 64, kActStages = 4;
 struct ActRow {
