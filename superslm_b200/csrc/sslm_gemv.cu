@@ -101,7 +101,10 @@ struct GemvPlan {
 
 // MT rows of x per pass (grid.y walks the row groups).
 enum GemvMode { kGemvRows32 = 0, kGemvRows64, kGemvHead };
-template <int MT, int MODE>
+// RU: weight rows multiplied side by side, as many as an item holds, up to three: short rows share the loads of x, and
+// an item of one row (long K) reads nothing twice (one row at the 1.5B widths, behind the wait, with three always:
+// down 5.3 us, 3.9 now; gate/up 4.0, 3.4; q/k/v 2.3, 2.0)
+template <int MT, int MODE, int RU>
 __global__ void __launch_bounds__(kGemvThreads)
 k_gemv(LinearArgs a, GemvPlan p) {
 	extern __shared__ __align__(128) unsigned char smem[];
@@ -193,7 +196,6 @@ k_gemv(LinearArgs a, GemvPlan p) {
 		const int4* wv = (const int4*)(ring + (size_t)sl * slot_bytes);
 		// RU weight rows side by side; one reduction per (row of x, weight row segment). Segments of one
 		// weight row may belong to different warps, so the sums meet in shared memory.
-		constexpr int RU = MT == 1 ? 3 : 1;
 #pragma unroll 1
 		for (int rr = 0; rr < nr; rr += RU) {
 			int acc[RU][MT];
@@ -341,13 +343,13 @@ static size_t gemv_smem_bytes(int mt, int K, int rows_per_block, int slots, int 
 	       (size_t)rows_per_block * 12 + 8 + (size_t)mt * 8 + (size_t)kGemvWarps * kMaxSlots * 8 + 16;
 }
 
-template <int MT, int MODE>
+template <int MT, int MODE, int RU>
 static cudaError_t launch_mode(const LinearArgs& a, int grid_y, cudaStream_t st) {
 	static PerDeviceOnce configured;
 	cudaError_t e = once_per_device(configured, [] {
-		cudaError_t c = cudaFuncSetAttribute(k_gemv<MT, MODE>, cudaFuncAttributeMaxDynamicSharedMemorySize, 220 * 1024);
+		cudaError_t c = cudaFuncSetAttribute(k_gemv<MT, MODE, RU>, cudaFuncAttributeMaxDynamicSharedMemorySize, 220 * 1024);
 		if (c != cudaSuccess) return c;
-		return cudaFuncSetAttribute(k_gemv<MT, MODE>, cudaFuncAttributePreferredSharedMemoryCarveout, cudaSharedmemCarveoutMaxShared);
+		return cudaFuncSetAttribute(k_gemv<MT, MODE, RU>, cudaFuncAttributePreferredSharedMemoryCarveout, cudaSharedmemCarveoutMaxShared);
 	});
 	if (e != cudaSuccess) return e;
 	GemvPlan p;
@@ -388,13 +390,22 @@ static cudaError_t launch_mode(const LinearArgs& a, int grid_y, cudaStream_t st)
 	const size_t smem = gemv_smem_bytes(MT, a.K, rpb, slots, slot_bytes);
 	if (smem > 220 * 1024) return cudaErrorInvalidConfiguration;
 	const int gx = (a.N + rpb - 1) / rpb;
-	return launch_ordered(a.caller_memory == 0, k_gemv<MT, MODE>, dim3(gx, grid_y), dim3(kGemvThreads), smem, st, a, p);
+	return launch_ordered(a.caller_memory == 0, k_gemv<MT, MODE, RU>, dim3(gx, grid_y), dim3(kGemvThreads), smem, st, a, p);
 }
 
+template <int MT, int RU>
+static cudaError_t launch_rows(const LinearArgs& a, int grid_y, cudaStream_t st) {
+	if (a.best != nullptr) return launch_mode<MT, kGemvHead, RU>(a, grid_y, st);
+	return a.out64 ? launch_mode<MT, kGemvRows64, RU>(a, grid_y, st) : launch_mode<MT, kGemvRows32, RU>(a, grid_y, st);
+}
 template <int MT>
 static cudaError_t launch_mt(const LinearArgs& a, int grid_y, cudaStream_t st) {
-	if (a.best != nullptr) return launch_mode<MT, kGemvHead>(a, grid_y, st);
-	return a.out64 ? launch_mode<MT, kGemvRows64>(a, grid_y, st) : launch_mode<MT, kGemvRows32>(a, grid_y, st);
+	if constexpr (MT == 1) {
+		const int rows = a.K * 2 <= kItemBytes ? kItemBytes / a.K : 1;      // per item
+		if (rows >= 3) return launch_rows<1, 3>(a, grid_y, st);
+		if (rows == 2) return launch_rows<1, 2>(a, grid_y, st);
+	}
+	return launch_rows<MT, 1>(a, grid_y, st);
 }
 
 cudaError_t launch_linear_gemv(const LinearArgs& a, cudaStream_t st) {
