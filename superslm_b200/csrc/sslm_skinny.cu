@@ -253,6 +253,11 @@ k_skinny(const __grid_constant__ CUtensorMap map_w, const __grid_constant__ CUte
 	const int ntiles = tile0 < tiles ? (tiles - tile0 + tile_step - 1) / tile_step : 0;
 	const int total = ntiles * nkb;                          // stages this block consumes
 
+	// The channel that a thread of the epilogue finishes, its fold constants asked for ahead of the weights: behind the
+	// exchange the load took half a microsecond, and behind the weights it holds up the dependency wait.
+	Channel c{};
+	if (warp >= 2)
+		c = channel_of(a, tile0 * kWRows + (splits > 1 ? rank * (kWRows / splits) + ((int)threadIdx.x - 64) % (kWRows / splits) : (warp & 3) * 32 + lane));
 	if (threadIdx.x == 0) {
 		for (int s = 0; s < stages; ++s) {
 			bar_init(full_bar(s), 1);
@@ -346,7 +351,6 @@ k_skinny(const __grid_constant__ CUtensorMap map_w, const __grid_constant__ CUte
 				else if (a.rowmax != nullptr) atomicMax(&a.rowmax[(size_t)m * 4], kRowmaxTimeout);
 			}
 		};
-		Channel c = channel_of(a, tile0 * kWRows + q * 32 + lane);      // (fold constants: ahead of the wait)
 		pdl_wait();
 		if (splits > 1) {
 			// ---- one tile: send every peer the accumulator rows it finishes, finish 128 / splits of them
@@ -369,7 +373,6 @@ k_skinny(const __grid_constant__ CUtensorMap map_w, const __grid_constant__ CUte
 			all_in = ok;
 			if (!__all_sync(0xffffffffu, acc_ok && ok)) refuse();      // (what was sent for a tile given up on is garbage: the rows say so)
 			const int my = et % rows;          // (rows divides 128 and the epilogue's thread count: one channel per thread)
-			c = channel_of(a, tile0 * kWRows + rank * rows + my);
 			const int first = tile0 * kWRows + rank * rows;
 			const bool one_seg = a.nseg == 1 || channel_of(a, first).seg == channel_of(a, min(first + rows, a.N) - 1).seg;
 			const int group = rows < 32 ? rows : 32;      // lanes that hold neighbouring channels of the same row
