@@ -222,7 +222,8 @@ SSLM_API sslm_status sslm_b200_set_device(int ordinal);
  * in_scales: M pairs (m, e); out_scales: M pairs; row_status: M reference
  * SslmForwardStatus ordinals (0 = Ok). use_tensor_cores: 0 forces the streaming GEMV
  * kernel, 1 lets M > 8 take the activation-major tcgen05 kernel, 2 lets up to 256 rows take the
- * weights-first one where it is the better of the two. */
+ * weights-first one where it is the better of the two, 3 up to eight rows the one whose weights wait in shared memory,
+ * where they fit. */
 SSLM_API sslm_status sslm_b200_linear(const int8_t* x, const int8_t* w, const int32_t* fold, int32_t M,
                              int32_t N, int32_t K, const int64_t* in_scales, int64_t site_m,
                              int64_t site_e, int32_t use_tensor_cores, int32_t* out_folded,
@@ -243,7 +244,7 @@ SSLM_API sslm_status sslm_b200_last_call_ms(sslm_workspace ws, float* ms, uint64
  * (the streaming kernel ran instead) and the reason code of the last refusal. */
 SSLM_API sslm_status sslm_b200_tc_stats(uint64_t* launches, uint64_t* refusals, int32_t* last_reason);
 /* Launches of the tensor-core linear kernels, first n of: the activation-major one per tile shape (rows x weight
- * columns) 128 x 64, 128 x 128, 256 x 64, 256 x 128; the weights-first one. Lets a test assert which of them
+ * columns) 128 x 64, 128 x 128, 256 x 64, 256 x 128; the weights-first one; the one of up to eight rows. Lets a test assert which of them
  * served a shape. */
 SSLM_API sslm_status sslm_b200_tc_variant_counts(uint64_t* counts, int32_t n);
 

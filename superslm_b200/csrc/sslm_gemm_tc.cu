@@ -758,6 +758,8 @@ void tc_count(bool launched, int reason) {
 	g_tc_variant[4].fetch_add(1);
 }
 
+void tc_count_few() { g_tc_variant[5].fetch_add(1); }
+
 void tc_debug_withhold(int launches) { g_debug_withhold.store(launches < 0 ? 0 : launches); }
 
 bool launch_linear_tc(const LinearArgs& a, cudaStream_t st) {

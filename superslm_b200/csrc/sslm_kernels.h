@@ -171,6 +171,8 @@ struct LinearArgs {
 };
 // HBM-bound small-M path: bulk-copy weight streaming through a shared-memory ring, dp4a.
 cudaError_t launch_linear_gemv(const LinearArgs& a, cudaStream_t st);
+// up to eight rows, the weights waiting in shared memory (sslm_few.cu). Returns false where they do not fit.
+bool launch_linear_few(const LinearArgs& a, cudaStream_t st);
 // tensor-core path for M > 8 rows (tcgen05 kind::i8, TMA-fed). Returns false when the
 // shape is not supported by that kernel (caller then uses the GEMV path).
 bool launch_linear_tc(const LinearArgs& a, cudaStream_t st);
@@ -180,6 +182,7 @@ bool launch_linear_skinny(const LinearArgs& a, cudaStream_t st);
 // shared by the two tensor-core kernels: [rows, k] int8 map, box 128 bytes x box_rows, 128-byte swizzle
 bool tc_tensor_map(const void* ptr, int rows, int k, int box_rows, bool cache, CUtensorMap* out);
 void tc_count(bool launched, int reason);      // of the weights-first kernel
+void tc_count_few();                           // of launch_linear_few, in the counts per variant only
 bool tc_debug_take();      // one launch of those tc_debug_withhold asked for
 // Tests of the bounded waits: the next `launches` tensor-core launches arm their first weight-tile
 // barrier in block 0 without requesting the tile, so that the wait on it runs out (no fault, no
