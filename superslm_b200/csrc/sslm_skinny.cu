@@ -42,7 +42,11 @@ constexpr int kMaxStages = 12;
 
 template <int NB>
 struct SkCfg {
-	static constexpr int kEpiWarps = NB >= 64 ? 8 : 4;
+	// Four epilogue warps per 16 columns (each reads a quarter of the lanes), 16 at most: with eight, gate/up of 256 rows at
+	// the 1.5B widths spent 8.5 of 14.5 us in its epilogue. A step of 120 rows 13.46 -> 13.05 ms / 5, of 21 rows of 0.5B
+	// 18.8 -> 18.25 ms / 15. Not for 64 columns: a clustered block of 16 leaves no registers for a second one beside
+	// it (64 rows: 8 % slower), and without clusters it gains nothing.
+	static constexpr int kEpiWarps = NB == 64 ? 8 : (NB / 4 < 16 ? NB / 4 : 16);
 	static constexpr int kThreads = 64 + 32 * kEpiWarps;
 	static constexpr uint32_t kWBytes = kWRows * kKBlock, kXBytes = NB * kKBlock, kStageBytes = kWBytes + kXBytes;
 	static constexpr uint32_t kTmemCols = 2 * NB < 32 ? 32 : 2 * NB;      // two accumulator stages
