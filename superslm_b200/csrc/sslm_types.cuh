@@ -105,6 +105,7 @@ struct SoftmaxConsts {
 // All per-row working buffers of one call (device pointers into a workspace arena).
 struct RowBatch {
 	int m;                       // rows
+	int ask_ahead;               // k_qkv_post asks for the rows' old K pages
 	const RowDesc* rows;
 	int8_t* x;  Scale* xs;       // residual stream in / out            [m, hidden]
 	int8_t* a;  Scale* as;       // stream after the attention residual [m, hidden]
