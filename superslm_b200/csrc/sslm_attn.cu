@@ -25,6 +25,7 @@
 
 #include <algorithm>
 #include <atomic>
+#include <initializer_list>
 
 #include "sslm_cluster.cuh"
 #include "sslm_kernels.h"
@@ -196,7 +197,7 @@ __device__ __forceinline__ void prefetch_l2(const void* p) { asm volatile("prefe
 // HD = head_dim (32, 64 or 128); threads = 2 * HD.
 template <int HD>
 __global__ void __launch_bounds__(2 * HD, HD == 128 ? 4 : 8)
-k_attention(RowBatch b, Dims d, const LayerDev* layer, int layer_index, KvPoolDev pool, int cp, int reverse_rows) {
+k_attention(RowBatch b, Dims d, const __grid_constant__ LayerDev layer, int layer_index, KvPoolDev pool, int cp, int reverse_rows) {
 	extern __shared__ __align__(16) unsigned char smem[];
 	// blocks start in index order: with reverse_rows the last (widest) rows of a prefill chunk go first
 	const int r = reverse_rows ? (int)gridDim.y - 1 - (int)blockIdx.y : (int)blockIdx.y;
@@ -222,7 +223,7 @@ k_attention(RowBatch b, Dims d, const LayerDev* layer, int layer_index, KvPoolDe
 		for (int j = t; j < (n64 >> 4); j += kAttnThreads)
 			s.pbase[j] = (int64_t)pages[min(j, npages - 1)] * (kPageTokens * HD);
 	}
-	if (t < 3 * G) s.fold[t] = layer->f_ctx[3 * kvh * G + t];      // (weights: ahead of the wait)
+	if (t < 3 * G) s.fold[t] = layer.f_ctx[3 * kvh * G + t];      // (weights: ahead of the wait)
 	__syncthreads();
 	constexpr int kRowsPerLine = 128 / HD;
 	for (int pos = t * kRowsPerLine; pos < n - 1; pos += kAttnThreads * kRowsPerLine)
@@ -489,13 +490,24 @@ __device__ __forceinline__ void shared_row_words(const int8_t* row, int c, uint3
 
 // (Registers: left to itself the compiler takes 56 to 80, and at 64 some forms spill: 24 rows of 500 to
 // 1,500 positions at the 1.5B widths, two slices each, took 1,970 us a token then, 1,810 in 80, 1,730 in 100.)
-template <int HD, bool STAGED>
+//
+// SITE: the q/k/v site of a decode row runs here too (k_qkv_post, which states the reference's lines), so a launch and its
+// boundary go and the staging hides behind the projection. Every block codes and rotates its kv head's q rows; the
+// one whose slice ends with the row lands K and V, straight into its staged rows as well. All blocks of a row come to the
+// same verdict from the same words; rank 0 speaks for it. kSiteBias: a bias joins every element, so the blocks exchange
+// their elements' maximum (and whether one of them left its domain) before anything is coded.
+enum FewSite { kSiteApart = 0, kSitePlain, kSiteBias };
+struct QkvSite {
+	const int32_t *rope_cos, *rope_sin;
+};
+template <int HD, bool STAGED, int SITE, bool W64>
 __global__ void __launch_bounds__(2 * HD, 1)
-k_attention_few(RowBatch b, Dims d, const LayerDev* layer, Scale c_ctx, int layer_index, KvPoolDev pool, int cp, int splits,
-                int whole_row, int chunk) {
+k_attention_few(RowBatch b, Dims d, const __grid_constant__ LayerDev layer, int layer_index, KvPoolDev pool, int cp, int splits,
+                int whole_row, int chunk, QkvSite site) {
+	static_assert(SITE == kSiteApart || STAGED, "K and V land in the staged rows");
 	using S = FewSmem<HD>;
 	extern __shared__ __align__(16) unsigned char smem[];
-	__shared__ __align__(8) unsigned long long s_bars[4];
+	__shared__ __align__(8) unsigned long long s_bars[SITE == kSiteBias ? 5 : 4];
 	constexpr int kThreads = 2 * HD, kWarps = kThreads / 32, NW = HD / 16;
 	const int r = (int)blockIdx.y, kvh = (int)blockIdx.x / splits, split = (int)blockIdx.x % splits;
 	const int G = d.heads / d.kv_heads;
@@ -512,6 +524,7 @@ k_attention_few(RowBatch b, Dims d, const LayerDev* layer, Scale c_ctx, int laye
 		exchange_init(bar(1), (uint32_t)(splits * G * 8) + more(1));
 		exchange_init(bar(2), (uint32_t)(G * HD * 4) + more(2));
 		exchange_init(bar(3), 4u * cluster_blocks + more(3));
+		if (SITE == kSiteBias) exchange_init(bar(4), 8u * cluster_blocks);
 		exchange_fence_init();
 	}
 	// ahead of the kernel that lands this step's K / V rows: the page table, the old rows
@@ -529,13 +542,13 @@ k_attention_few(RowBatch b, Dims d, const LayerDev* layer, Scale c_ctx, int laye
 		const int32_t* pages = b.rows[r].pages + p0 / kPageTokens;
 		for (int j = t; j < (n64 >> 4); j += kThreads) s.pbase[j] = (int64_t)pages[min(j, npages - 1)] * (kPageTokens * HD);
 	}
-	if (t < 3 * G) s.fold[t] = layer->f_ctx[3 * kvh * G + t];
+	if (t < 3 * G) s.fold[t] = layer.f_ctx[3 * kvh * G + t];
 	if (t < 8) {
 		s.mx[t] = INT32_MIN;
 		s.sum[t] = 0ull;
 	}
 	if (t == 8) s.misc[0] = 0u;
-	const FunnelFold fold_ctx = funnel_prefold(nullptr, 0, c_ctx);
+	const FunnelFold fold_ctx = funnel_prefold(nullptr, 0, layer.c_ctx);
 	__syncthreads();
 	auto stage_k = [&](int from, int to) {
 		for (int i = from * (HD / 16) + t; i < to * (HD / 16); i += kThreads) {
@@ -551,7 +564,7 @@ k_attention_few(RowBatch b, Dims d, const LayerDev* layer, Scale c_ctx, int laye
 	};
 	if (STAGED) {
 		stage_k(0, old);
-		stage_v(0, old_pages);
+		stage_v(0, SITE != kSiteApart ? npages : old_pages);      // (a new position's byte of the last page follows)
 		// (pages between the slice's end and the next group of four are read against zero probabilities)
 		for (int i = npages * HD + t; i < (n64 >> 4) * HD; i += kThreads)
 			*(int4*)(s.vs + (size_t)(i / HD) * S::kVStride + (i % HD) * 16) = make_int4(0, 0, 0, 0);
@@ -560,21 +573,198 @@ k_attention_few(RowBatch b, Dims d, const LayerDev* layer, Scale c_ctx, int laye
 		for (int pos = t * kRowsPerLine; pos < old; pos += kThreads * kRowsPerLine)
 			prefetch_l2(kplane + s.pbase[pos >> 4] + (pos & 15) * HD);
 	}
+	// the q/k/v site, ahead of the projection: the normed row's scale, RoPE words, landing constants, biases
+	using T = typename WideOf<W64>::T;
+	using Y = typename WideOf<W64 || SITE == kSiteBias>::T;
+	__shared__ uint32_t s_bank[SITE != kSiteApart ? 64 : 1];
+	__shared__ __align__(16) uint32_t s_q[SITE != kSiteApart ? 2 * HD : 4];
+	__shared__ unsigned long long s_biased[16];      // per block: its q elements' maximum, and bit 32: a K / V element without a sum
+	__shared__ SoftmaxConsts s_consts;
+	__shared__ int32_t s_failed;      // status word of a softmax constant's refusal
+	const int H = d.hidden, KV = d.kv_hidden, pos = width - 1, slot = pos % kPageTokens;
+	const bool has_q = t < G * (HD / 4), lands = pos >= p0 && pos < p0 + n && t < HD / 2;      // (threads take four elements of either)
+	const bool is_k = t < HD / 4;
+	const int dd = (4 * t) & (HD - 1);                // channel of both
+	const int e_q = kvh * G * HD + 4 * t, e_kv = H + (is_k ? 0 : KV) + kvh * HD + dd;
+	Scale ns{0, 0}, kh{0, 0};
+	FunnelFold fold_q{};
+	int2 rc = make_int2(0, 0), rs = make_int2(0, 0);
+	int64_t r_t = 0, e_t = 0, r_a = 0, term_q[4], term_kv[4];
+	int bexp = 0;
+	bool gate = true;
+	uint32_t bad_q = 0, bad_kv = 0;
+	const int64_t *bias_q = nullptr, *bias_k = nullptr, *bias_v = nullptr;
+	if constexpr (SITE != kSiteApart) {
+		ns = b.ns[r];
+		fold_q = funnel_prefold(&ns, 1, layer.c_q);
+		const size_t at = (size_t)pos * (HD / 2) + (dd >> 1);
+		if (has_q || lands) {
+			rc = *(const int2*)(site.rope_cos + at);
+			rs = *(const int2*)(site.rope_sin + at);
+		}
+		if (lands) {
+			const int64_t* rec = (is_k ? layer.k_recip : layer.v_recip) + 3 * kvh;
+			e_t = rec[1];
+			r_t = rec[2];
+		}
+		if (warp == kWarps - 1 && lane < d.kv_heads) kh = Scale{layer.sm_khead[2 * lane], layer.sm_khead[2 * lane + 1]};
+		if (t == 0) s_failed = 0;
+	}
+	if constexpr (SITE == kSiteBias) {
+		bias_q = layer.b_q;
+		bias_k = layer.b_k;
+		bias_v = layer.b_v;
+		r_a = dyn_recip(ns.m);
+		gate = bias_exponent_in_domain(ns.e, &bexp);
+		auto terms = [&](int e, bool in, int64_t (&out)[4], uint32_t& bad) {
+			const int64_t* bp = e < H ? bias_q : (e < H + KV ? bias_k : bias_v);
+			const int off = e < H ? e : (e < H + KV ? e - H : e - H - KV);
+#pragma unroll
+			for (int j = 0; j < 4; ++j) {
+				out[j] = 0;
+				if (in && bp != nullptr && gate && !bias_term(bp[off + j], r_a, bexp, &out[j])) bad = 1;
+			}
+		};
+		terms(e_q, has_q, term_q, bad_q);
+		terms(e_kv, lands, term_kv, bad_kv);
+	}
 	cluster_arrive();
 	cluster_wait();
 	pdl_wait();
 	pdl_release();
+	bool live, ok = true;
+	int32_t verdict = 0;      // (written behind the last exchange, when every block of the row has read the row's word)
+	IExpFast fx;
+	uint32_t qw[NW];
+	if constexpr (SITE != kSiteApart) {
+		const T* row = (const T*)b.wide + (size_t)r * b.wide_ld;
+		T xq[4] = {0, 0, 0, 0}, xkv[4] = {0, 0, 0, 0};
+		if (has_q) load_quad(row + e_q, xq);
+		if (lands) load_quad(row + e_kv, xkv);
+		unsigned long long mx = __ldcg(&b.rowmax[(size_t)r * 4]);
+		const bool refused = __ldcg(&b.status[r]) != 0;
+		Bank bank{s_bank, 0};
+		Y yq[4], ykv[4];
+#pragma unroll
+		for (int j = 0; j < 4; ++j) {
+			yq[j] = xq[j];
+			ykv[j] = xkv[j];
+		}
+		int32_t st = kOk;
+		int at_site = kSiteQ;
+		if constexpr (SITE == kSiteBias) {
+			uint32_t top = 0;
+#pragma unroll
+			for (int j = 0; j < 4; ++j) {
+				int64_t sum;
+				if (!bias_accumulate((int64_t)xq[j], term_q[j], &sum)) bad_q = 1;
+				yq[j] = sum;
+				const unsigned long long a = sum < 0 ? ~(unsigned long long)sum + 1ull : (unsigned long long)sum;
+				top = max(top, a > 0xFFFFFFFFull ? 0xFFFFFFFFu : (uint32_t)a);      // (anything above 2^31 is refused alike)
+				if (!bias_accumulate((int64_t)xkv[j], term_kv[j], &sum)) bad_kv = 1;
+				ykv[j] = sum;
+			}
+			top = block_max_u32(bad_q != 0u ? 0xFFFFFFFFu : min(top, 0xFFFFFFFEu), bank);
+			const bool bad = __syncthreads_or((int)bad_kv) != 0;
+			if (t < (int)cluster_blocks) exchange_send(&s_biased[my_rank], bar(4), (uint32_t)t, (unsigned long long)top | (bad ? 1ull << 32 : 0ull));
+			ok = exchange_wait(bar(4));
+			uint32_t m = 0, any = 0;
+			for (uint32_t j = 0; j < cluster_blocks; ++j) {
+				m = max(m, (uint32_t)s_biased[j]);
+				any |= (uint32_t)(s_biased[j] >> 32);
+			}
+			bad_kv = any;
+			if (bias_q != nullptr) {
+				mx = (unsigned long long)m;
+				if (!gate) st = kRoundingDivideExponentOutOfDomain;
+				else if (m == 0xFFFFFFFFu) st = kBiasReconcileProductOutOfDomain;
+			}
+		}
+		const QuadFunnel fp = quad_funnel(mx, fold_q);
+		if constexpr (SITE == kSiteBias) {
+			if (st == kOk && (bad_kv != 0u || !gate) && (bias_k != nullptr || bias_v != nullptr) && fp.status == kOk) {
+				st = gate ? kBiasReconcileProductOutOfDomain : kRoundingDivideExponentOutOfDomain;
+				at_site = kSiteKv;
+			}
+		}
+		if (st == kOk) st = fp.status;
+		live = !refused && st == kOk;
+		if (!refused) verdict = pack_status(st, at_site, b.layer);
+		asm volatile("cp.async.wait_all;" ::: "memory");
+		__syncthreads();      // the staged rows and pages are there
+		if (live) {
+			if (has_q) {
+				const uint32_t w = rope_quad(code_quad(yq, fp), rc, rs);
+				s_q[t] = w;
+				if (split == 0) *(uint32_t*)(b.qrot + (size_t)r * H + e_q) = w;      // (traces read it)
+			}
+			if (lands) {
+				const Lander l = make_lander(ns.m, r_t, ns.e, e_t);
+				uint32_t sat = 0;
+				int lc[4];
+#pragma unroll
+				for (int j = 0; j < 4; ++j) {
+					const int64_t a = (int64_t)ykv[j];
+					const unsigned long long mag = a < 0 ? ~(unsigned long long)a + 1ull : (unsigned long long)a;
+					bool s1;
+					if (l.fast && mag <= (1ull << 31)) {
+						const uint64_t m = land_magnitude((uint32_t)mag, l);
+						s1 = m > 127;
+						const int c = s1 ? 127 : (int)m;
+						lc[j] = ((a < 0) != l.neg) ? -c : c;
+					} else {
+						lc[j] = (int)clamp127(landing_rescale(a, ns.m, r_t, ns.e, e_t, &s1, nullptr));
+					}
+					sat += s1 ? 1u : 0u;
+				}
+				const int64_t page = s.pbase[(pos - p0) >> 4];      // (byte offset)
+				if (is_k) {
+					const uint32_t w = rope_quad(pack4(lc[0], lc[1], lc[2], lc[3]), rc, rs);
+					*(uint32_t*)(s.ks + (size_t)(pos - p0) * S::kKStride + dd) = w;
+					*(uint32_t*)(const_cast<int8_t*>(kplane) + page + slot * HD + dd) = w;
+				} else {
+#pragma unroll
+					for (int j = 0; j < 4; ++j) {
+						s.vs[(size_t)((pos - p0) >> 4) * S::kVStride + (dd + j) * kPageTokens + slot] = (int8_t)lc[j];
+						const_cast<int8_t*>(vplane)[page + (dd + j) * kPageTokens + slot] = (int8_t)lc[j];
+					}
+				}
+				if (sat != 0u) {
+					atomicAdd(&b.sat[r], (unsigned long long)sat);
+					if (layer_index < b.sat_ld) atomicAdd(&b.sat_layer[(size_t)r * b.sat_ld + layer_index], sat);
+				}
+			}
+			if (warp == kWarps - 1) {
+				// softmax constants per kv head, as in k_qkv_post; any head's refusal is the row's
+				int32_t cst = kOk;
+				if (lane < d.kv_heads) {
+					SoftmaxConsts sc;
+					cst = softmax_consts(fp.out, kh, (uint64_t)pos + 1, &sc);
+					if (lane == kvh) s_consts = sc;
+				}
+				const uint32_t failing = __ballot_sync(0xffffffffu, cst != kOk);
+				if (failing != 0u && lane == __ffs(failing) - 1) s_failed = pack_status(cst, kSiteSoftmaxConsts, b.layer);
+			}
+		}
+		__syncthreads();
+		if (live && s_failed != 0) {
+			verdict = s_failed;
+			live = false;
+		}
+		fx = iexp_fast_prepare(s_consts);
+		shared_row_words<HD>((const int8_t*)s_q + min(g, G - 1) * HD, c, qw);
+	} else {
 	// A row that an earlier site refused is sat out: zero contributions, but every exchange. (Only this
 	// kernel's last step can refuse the row, when every block has long read the word.)
-	const bool live = __ldcg(&b.status[r]) == 0;
-	const IExpFast fx = iexp_fast_prepare(b.smc[(size_t)r * d.kv_heads + kvh]);
-	uint32_t qw[NW];
+	live = __ldcg(&b.status[r]) == 0;
+	fx = iexp_fast_prepare(b.smc[(size_t)r * d.kv_heads + kvh]);
 	load_row_words<HD>(b.qrot + (size_t)r * d.hidden + (size_t)(kvh * G + min(g, G - 1)) * HD, c, qw);
 	if (STAGED) {
 		stage_k(old, n);
 		stage_v(old_pages, npages);
 		asm volatile("cp.async.wait_all;" ::: "memory");
 		__syncthreads();
+	}
 	}
 
 	// ---- stage 1: scores, 8 positions per MMA group, groups dealt round-robin to the warps; lanes beyond
@@ -615,7 +805,7 @@ k_attention_few(RowBatch b, Dims d, const LayerDev* layer, Scale c_ctx, int laye
 	__syncthreads();
 	// ---- exchange 1: every slice's maxima
 	for (int i = t; i < splits * G; i += kThreads) exchange_send(&s.rx_max[split * 8 + i % G], bar(0), kv_rank0 + (uint32_t)(i / G), (uint32_t)s.mx[i % G]);
-	bool ok = exchange_wait(bar(0));
+	ok = exchange_wait(bar(0)) && ok;
 
 	// ---- stage 2: softmax, (head, 128-position chunk) pairs dealt to the warps, a lane takes 4 consecutive
 	// positions: exponentials and their sums, the score's place then holds the element's (shift, remainder)
@@ -757,8 +947,12 @@ k_attention_few(RowBatch b, Dims d, const LayerDev* layer, Scale c_ctx, int laye
 	if (t < (int)cluster_blocks) exchange_send(&s.rx_top[my_rank], bar(3), (uint32_t)t, s.misc[0]);
 	ok = exchange_wait(bar(3)) && ok;
 	if (__builtin_expect(!__all_sync(0xffffffffu, ok), 0)) {
-		give_up(4);
+		give_up(SITE == kSiteBias ? 5 : 4);
 		return;
+	}
+	if (SITE != kSiteApart && my_rank == 0 && t == 0) {      // (every block has read them)
+		b.rowmax[(size_t)r * 4] = 0ull;
+		if (verdict != 0) atomicCAS(&b.status[r], 0, verdict);
 	}
 	if (!live) return;
 	for (uint32_t j = 0; j < cluster_blocks; ++j) top = max(top, s.rx_top[j]);
@@ -825,7 +1019,7 @@ struct TileSmem {
 
 template <int HD>
 __global__ void __launch_bounds__(kTileThreads, 2)
-k_attention_tile(RowBatch b, Dims d, const LayerDev* layer, int layer_index, KvPoolDev pool, int tq) {
+k_attention_tile(RowBatch b, Dims d, const __grid_constant__ LayerDev layer, int layer_index, KvPoolDev pool, int tq) {
 	using L = TileSmem<HD>;
 	constexpr int KS = HD / 32;          // MMA steps along the head dimension
 	constexpr int NGW = HD / 16;         // 8-channel groups a warp owns in P.V
@@ -857,7 +1051,7 @@ k_attention_tile(RowBatch b, Dims d, const LayerDev* layer, int layer_index, KvP
 	const int nblk = (width + kTileKeys - 1) / kTileKeys;
 	const int8_t* kplane = pool.base + kv_plane_offset(d, pool, layer_index, kvh, 0);
 	const int8_t* vplane = pool.base + kv_plane_offset(d, pool, layer_index, kvh, 1);
-	if (t < 3 * G) l_fold[t] = layer->f_ctx[3 * kvh * G + t];
+	if (t < 3 * G) l_fold[t] = layer.f_ctx[3 * kvh * G + t];
 	pdl_wait();
 	pdl_release();
 	if (t < kTileRows) {
@@ -1093,7 +1287,7 @@ k_attention_tile(RowBatch b, Dims d, const LayerDev* layer, int layer_index, KvP
 }
 
 template <int HD>
-static cudaError_t launch_attn_tile(const RowBatch& b, const Dims& d, const LayerDev* layer, int layer_index, KvPoolDev pool,
+static cudaError_t launch_attn_tile(const RowBatch& b, const Dims& d, const LayerDev& layer, int layer_index, KvPoolDev pool,
                                     cudaStream_t st) {
 	const int G = d.heads / d.kv_heads;
 	const int tq = kTileRows / G;
@@ -1192,7 +1386,7 @@ static __device__ __noinline__ uint4 chunk_prob_exact(uint32_t p0, uint32_t p1, 
 
 template <int HD>
 __global__ void __launch_bounds__(kChunkThreads, 2)
-k_attention_chunk(RowBatch b, Dims d, const LayerDev* layer, int layer_index, KvPoolDev pool, ChunkPlan pl) {
+k_attention_chunk(RowBatch b, Dims d, const __grid_constant__ LayerDev layer, int layer_index, KvPoolDev pool, ChunkPlan pl) {
 	using L = ChunkSmem<HD>;
 	constexpr int KS = HD / 32;          // MMA steps along the head dimension
 	constexpr int NT = HD / 32;          // 8-channel tiles a warp owns in P.V (a quarter of the channels)
@@ -1264,7 +1458,7 @@ k_attention_chunk(RowBatch b, Dims d, const LayerDev* layer, int layer_index, Kv
 		const int page = (rank + (i >> 3) * sub) * 8 + (i & 7);
 		pbase[i] = page * kPageTokens < width ? (int64_t)pages[page] * (kPageTokens * HD) : 0;
 	}
-	if (t < 3 * G) l_fold[t] = layer->f_ctx[3 * kvh * G + t];
+	if (t < 3 * G) l_fold[t] = layer.f_ctx[3 * kvh * G + t];
 	if (t < kChunkRows) {
 		rmax[t] = INT32_MIN;
 		rsum[t] = 0ull;
@@ -1605,7 +1799,7 @@ static bool chunk_plan(const Dims& d, int m, int width, ChunkPlan* out) {
 	return found;
 }
 template <int HD>
-static cudaError_t launch_attn_chunk(const RowBatch& b, const Dims& d, const LayerDev* layer, int layer_index, KvPoolDev pool,
+static cudaError_t launch_attn_chunk(const RowBatch& b, const Dims& d, const LayerDev& layer, int layer_index, KvPoolDev pool,
                                      const ChunkPlan& p, cudaStream_t st) {
 	RowBatch rb = b;
 	rb.debug_withhold = p.cluster > 1 ? exchange_debug_take(kExchangeAttnChunk) : 0;
@@ -1640,14 +1834,17 @@ struct AttnPlan {
 static std::atomic<int> g_forced_splits{-1};     // -1: not set yet (the environment decides), 0: automatic
 void attn_force_splits(int splits) { g_forced_splits.store(splits < 0 ? 0 : splits); }
 
-static AttnPlan attn_plan(const Dims& d, int m, int max_width) {
-	AttnPlan p;
+static int forced_splits() {
 	int forced = g_forced_splits.load();
 	if (forced < 0) {      // SSLM_B200_ATTN_SPLITS=n fixes the slices per kv head (tuning, tests)
 		const char* e = getenv("SSLM_B200_ATTN_SPLITS");
 		forced = e ? atoi(e) : 0;
 		g_forced_splits.store(forced < 0 ? 0 : forced);
 	}
+	return forced;
+}
+static AttnPlan attn_plan(const Dims& d, int m, int max_width, int forced) {
+	AttnPlan p;
 	// Clusters of 16 blocks need a GPC to themselves and there are eight: up to six rows get one each.
 	// Otherwise a cluster has at most 8 blocks (the portable size).
 	const int cluster_max = m <= 6 ? 16 : 8;
@@ -1674,11 +1871,28 @@ static AttnPlan attn_plan(const Dims& d, int m, int max_width) {
 	}
 	return p;
 }
-constexpr size_t kFewSmemMax = 225 * 1024;
+constexpr size_t kFewSmemMax = 223 * 1024;
+static size_t few_smem(const Dims& d, int cp) {
+	const int G = d.heads / d.kv_heads;
+	return d.head_dim == 128 ? FewSmem<128>::bytes(G, cp, true) : (d.head_dim == 64 ? FewSmem<64>::bytes(G, cp, true) : FewSmem<32>::bytes(G, cp, true));
+}
+// The q/k/v site of decode rows runs inside their attention clusters from two rows on. Apart / inside, ms for 6 or 16 tokens:
+// 1.5B 2 rows 6.34 / 6.10, 5 rows 20.0 / 19.7, 12 rows 7.69 / 7.44; 0.5B (biases) 21 rows 18.4 / 17.7, 30 rows 6.78 / 6.75.
+// Not for one row (1.5B 18.1 / 18.4, 0.5B 2.69 / 2.91): the streaming projections leave an attention block no registers
+// beside them, and without a row kernel in between nothing hides its prologue.
+AttnChoice attn_choose(const Dims& d, const LayerDev& h, int m, int max_width, int chunk) {
+	AttnChoice c{forced_splits(), kSiteApart};
+	if (chunk || m < 2) return c;
+	const AttnPlan p = attn_plan(d, m, max_width, c.forced);
+	if (p.splits == 0 || p.whole_row == 0 || few_smem(d, p.cp) > kFewSmemMax) return c;
+	const bool bias = h.b_q != nullptr || h.b_k != nullptr || h.b_v != nullptr;
+	c.site = bias ? kSiteBias : kSitePlain;
+	return c;
+}
 
 template <int HD>
-static cudaError_t launch_attn(const RowBatch& b, const Dims& d, const LayerDev* layer, const LayerDev& h, int layer_index, KvPoolDev pool,
-                               const AttnPlan& p, int reverse_rows, cudaStream_t st) {
+static cudaError_t launch_attn(const RowBatch& b, const Dims& d, const LayerDev& layer, int layer_index, KvPoolDev pool,
+                               const AttnPlan& p, int reverse_rows, int site, const QkvSite& qs, cudaStream_t st) {
 	const int G = d.heads / d.kv_heads;
 	if (p.splits == 0)
 		return launch_pdl(k_attention<HD>, dim3(d.kv_heads, b.m), dim3(2 * HD), attn_smem_bytes(G, p.cp), st, b, d, layer, layer_index,
@@ -1700,8 +1914,10 @@ static cudaError_t launch_attn(const RowBatch& b, const Dims& d, const LayerDev*
 	attr[1].val.programmaticStreamSerializationAllowed = 1;
 	cfg.attrs = attr;
 	cfg.numAttrs = pdl_enabled() ? 2 : 1;
-	return cudaLaunchKernelEx(&cfg, staged ? k_attention_few<HD, true> : k_attention_few<HD, false>, rb, d, layer, h.c_ctx, layer_index, pool,
-	                          p.cp, p.splits, p.whole_row, reverse_rows);
+	auto kernel = staged ? k_attention_few<HD, true, kSiteApart, false> : k_attention_few<HD, false, kSiteApart, false>;
+	if (site == kSitePlain) kernel = b.wide64 ? k_attention_few<HD, true, kSitePlain, true> : k_attention_few<HD, true, kSitePlain, false>;
+	if (site == kSiteBias) kernel = b.wide64 ? k_attention_few<HD, true, kSiteBias, true> : k_attention_few<HD, true, kSiteBias, false>;
+	return cudaLaunchKernelEx(&cfg, kernel, rb, d, layer, layer_index, pool, p.cp, p.splits, p.whole_row, reverse_rows, qs);
 }
 
 // (The attributes are the kernel's, not the model's: limits for the largest group, so that mapping one model
@@ -1718,8 +1934,12 @@ static cudaError_t configure_hd() {
 		return e;
 	};
 	cudaError_t e = set((const void*)k_attention<HD>, (int)attn_smem_bytes(group, kAttnMaxSlice), false);
-	if (e == cudaSuccess) e = set((const void*)k_attention_few<HD, true>, (int)kFewSmemMax, true);
-	if (e == cudaSuccess) e = set((const void*)k_attention_few<HD, false>, (int)FewSmem<HD>::bytes(group, kAttnMaxSlice, false), true);
+	for (const void* few : {(const void*)k_attention_few<HD, true, kSiteApart, false>, (const void*)k_attention_few<HD, true, kSitePlain, false>,
+	                        (const void*)k_attention_few<HD, true, kSitePlain, true>, (const void*)k_attention_few<HD, true, kSiteBias, false>,
+	                        (const void*)k_attention_few<HD, true, kSiteBias, true>})
+		if (e == cudaSuccess) e = set(few, (int)kFewSmemMax, true);
+	if (e == cudaSuccess)
+		e = set((const void*)k_attention_few<HD, false, kSiteApart, false>, (int)FewSmem<HD>::bytes(group, kAttnMaxSlice, false), true);
 	if (e == cudaSuccess) e = set((const void*)k_attention_tile<HD>, (int)TileSmem<HD>::kBytes, false);
 	if (e == cudaSuccess) e = set((const void*)k_attention_chunk<HD>, (int)ChunkSmem<HD>::bytes(kChunkSteps), false);
 	return e;
@@ -1737,8 +1957,9 @@ cudaError_t attn_configure(const Dims& d) {
 	return cudaErrorInvalidConfiguration;
 }
 
-bool launch_attention(const RowBatch& b, const Dims& d, const LayerDev* layer, const LayerDev& h, int layer_index,
-                      KvPoolDev pool, int max_width, int reverse_rows, cudaStream_t st, cudaError_t* err) {
+bool launch_attention(const RowBatch& b, const Dims& d, const LayerDev& layer, int layer_index,
+                      KvPoolDev pool, int max_width, int reverse_rows, const AttnChoice& choice, const int32_t* cos, const int32_t* sin,
+                      cudaStream_t st, cudaError_t* err) {
 	// Prefill chunks (rows at consecutive positions of one sequence), by what a whole prompt took with each
 	// kernel. Tiles with the scores kept (k_attention_chunk) from 64 rows and 512 positions on: below, a row's
 	// own blocks are as fast and a tile's fixed part is not paid back (300 rows of the 28-layer model: 3.3 ms
@@ -1774,11 +1995,12 @@ bool launch_attention(const RowBatch& b, const Dims& d, const LayerDev* layer, c
 		if (err) *err = e;
 		return false;
 	}
-	const AttnPlan p = attn_plan(d, b.m, max_width);
+	const AttnPlan p = attn_plan(d, b.m, max_width, choice.forced);
+	const QkvSite qs{cos, sin};
 	cudaError_t e;
-	if (d.head_dim == 128) e = launch_attn<128>(b, d, layer, h, layer_index, pool, p, reverse_rows, st);
-	else if (d.head_dim == 64) e = launch_attn<64>(b, d, layer, h, layer_index, pool, p, reverse_rows, st);
-	else e = launch_attn<32>(b, d, layer, h, layer_index, pool, p, reverse_rows, st);
+	if (d.head_dim == 128) e = launch_attn<128>(b, d, layer, layer_index, pool, p, reverse_rows, choice.site, qs, st);
+	else if (d.head_dim == 64) e = launch_attn<64>(b, d, layer, layer_index, pool, p, reverse_rows, choice.site, qs, st);
+	else e = launch_attn<32>(b, d, layer, layer_index, pool, p, reverse_rows, choice.site, qs, st);
 	if (err) *err = e;
 	return p.whole_row != 0;
 }

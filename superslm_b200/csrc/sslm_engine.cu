@@ -126,7 +126,7 @@ extern "C" sslm_status sslm_model_map(const void* data, size_t size, sslm_model*
 	bytes += L * ((H + 2 * KV) * H + H * H + 2 * I * H + H * I + 2 * H);
 	bytes += L * 12 * ((H + 2 * KV) + H + 2 * I + H + c.heads);
 	bytes += L * (2 * c.kv_heads * 3 * 8 + c.kv_heads * 2 * 8);
-	bytes += 2 * (size_t)c.context_cap * (c.head_dim / 2) * 4 + 1025 * 4 + L * sizeof(LayerDev);
+	bytes += 2 * (size_t)c.context_cap * (c.head_dim / 2) * 4 + 1025 * 4;
 	bytes += L * (H + 2 * KV) * 8;                       // q/k/v bias codes, when the artifact has them
 	bytes += (L * 28 + 64) * 256;
 	if (!cuda_ok(cudaMalloc((void**)&m->arena.base, bytes))) {
@@ -262,7 +262,6 @@ extern "C" sslm_status sslm_model_map(const void* data, size_t size, sslm_model*
 		ld.c_mlp_res = read_scale(v, p + "mlp_residual", &ok);
 		if (!ok) return fail(SSLM_ARTIFACT_REJECTED);
 	}
-	m->d_layers = (LayerDev*)up.put(m->h_layers.data(), L * sizeof(LayerDev));
 	if (!up.ok) return fail(SSLM_ALLOCATION_FAILED);
 	// decode schemas (src/sslm_abi.cpp:1196-1218): a malformed SCM1 section refuses the artifact
 	if (v.has(kSecSchemaMasks)) {

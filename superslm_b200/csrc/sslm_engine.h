@@ -95,7 +95,6 @@ struct sslm_model_s {
 	uint8_t hash[32]{};
 	DeviceArena arena;
 	std::vector<sslm::LayerDev> h_layers;
-	sslm::LayerDev* d_layers = nullptr;
 	const int8_t* d_embed = nullptr;
 	const int8_t* d_head = nullptr;
 	const int8_t* d_final_gain = nullptr;

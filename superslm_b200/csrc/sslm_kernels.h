@@ -100,13 +100,14 @@ inline int exchange_debug_take(ExchangeKernel kernel) {
 
 // ---- per-row sites (sslm_rows.cu)
 cudaError_t rows_configure(const Dims& d);
-// (the host's copy `h` of a layer record carries the site constants into the launch parameters)
+// (A layer's record travels in the launch parameters: read from memory, its pointers cost a kernel's prologue a trip to HBM
+// before the next one could start.)
 // first rows of a call: embed or resume, then an RMSNorm with `gain` (nullptr: none)
 // (It enters the call's new pages into the page tables: when it is refused, nothing behind it may be launched.)
 cudaError_t launch_begin(const RowBatch& b, const Dims& d, const int8_t* embed, Scale c_embed, const RowSource* src, const int8_t* gain,
                          Scale c_norm, int site_norm, cudaStream_t st);
 inline std::atomic<int> g_refuse_begin{0};      // tests: the next launches of it that count as refused by the runtime
-void launch_qkv_post(const RowBatch& b, const Dims& d, const LayerDev* layer, const LayerDev& h, int layer_index, KvPoolDev pool,
+void launch_qkv_post(const RowBatch& b, const Dims& d, const LayerDev& h, int layer_index, KvPoolDev pool,
                      const int32_t* cos, const int32_t* sin, cudaStream_t st);
 void launch_ctx_funnel(const RowBatch& b, const Dims& d, const LayerDev& h, cudaStream_t st);
 // A residual site: funnel of the projection row, reconciliation with the stream, and the RMSNorm of
@@ -202,10 +203,18 @@ void launch_lora_u(const RowBatch& b, const int8_t* x, int k_in, int layer, int 
 cudaError_t attn_configure(const Dims& d);
 // slices per kv head of later attention launches (0: chosen per launch); for tuning and tests
 void attn_force_splits(int splits);
+// How the attention of m rows will run, decided ahead of the q/k/v site: site != 0 says that it takes that site over
+// (launch_qkv_post is then left out).
+struct AttnChoice {
+	int forced;      // slices per kv head asked for (attn_force_splits), 0: none
+	int site;
+};
+AttnChoice attn_choose(const Dims& d, const LayerDev& h, int m, int max_width, int chunk);
 // Returns true when the launch also ran the attention-context funnel (codes in b.ctx, scale in
 // b.cs); otherwise b.ctxw / rowmax slot 3 are filled and launch_ctx_funnel must follow.
-bool launch_attention(const RowBatch& b, const Dims& d, const LayerDev* layer, const LayerDev& h, int layer_index,
-                      KvPoolDev pool, int max_width, int reverse_rows, cudaStream_t st, cudaError_t* err);
+bool launch_attention(const RowBatch& b, const Dims& d, const LayerDev& layer, int layer_index,
+                      KvPoolDev pool, int max_width, int reverse_rows, const AttnChoice& choice, const int32_t* cos, const int32_t* sin,
+                      cudaStream_t st, cudaError_t* err);
 // gather `planes` planes of a sequence's pages, from plane0 on, into the reference's canonical block layout
 // [layer][K|V][kv_head][position][head_dim] with `span` positions per plane; positions beyond
 // `valid(layer)` are zero

@@ -376,6 +376,35 @@ __device__ __forceinline__ uint32_t rope_quad(uint32_t w, int2 c, int2 s) {
 	             rope_round((int64_t)x1 * c.y - (int64_t)y1 * s.y), rope_round((int64_t)x1 * s.y + (int64_t)y1 * c.y));
 }
 
+// ---------------------------------------------------------------------- softmax constants
+// of one kv head of a row: sm = Combine(S[q], softmax_khead) -> C30 constants -> width gate
+__device__ __forceinline__ int32_t softmax_consts(Scale q, Scale kh, uint64_t width, SoftmaxConsts* sc) {
+	sc->c = IExpConsts{0, 0, 0};
+	sc->peak = 0;
+	if (!fits_i32(q.m) || !fits_i32(kh.m)) return kCarriedScaleMantissaOutOfDomain;
+	const Scale sm = combine(q, kh);
+	if (!fits_i32(sm.m)) return kCarriedScaleMantissaOutOfDomain;
+	if (iexp_scale_constants(sm.m, sm.e, &sc->c) != 0) return kIExpScaleDerivationOutOfDomain;
+	if (!softmax_width_in_domain(sc->c.q_b, sc->c.q_c, width, &sc->peak)) return kSoftmaxRowWidthOutOfDomain;
+	// q_ln2 == 0: every element's construction is refused by the reference (IExpConstruct's q_ln2 >= 1 check) ->
+	// SoftmaxKernelRefused. The attention kernels' 32-bit element form also needs q_ln2 <= q_b; that holds for every
+	// constant triple iexp_scale_constants returns and needs no test here: q_ln2 = floor(LN2_Q * r / 2^s) and
+	// q_b = floor(B_Q * r / 2^s) with the same unsigned reciprocal r and the same shift s, and LN2_Q < B_Q, so the
+	// floors are ordered the same way.
+	return sc->c.q_ln2 < 1 ? kSoftmaxKernelRefused : kOk;
+}
+
+// -------------------------------------------------------------------------- q/k/v bias
+// The bias term of one element, false when it leaves int64. A bias code inside 32 bits keeps the
+// product with the row's reciprocal (at most 2^32) inside 64; others take the 128-bit composite.
+__device__ __forceinline__ bool bias_term(int64_t bias, int64_t r_a, int bexp, int64_t* term) {
+	if (bias == (int64_t)(int32_t)bias && r_a > 0 && (uint64_t)r_a <= ((uint64_t)1 << 32)) {
+		*term = rdivpot64(bias * r_a, bexp);
+		return true;
+	}
+	return bias_reconcile(bias, r_a, bexp, term);
+}
+
 // ------------------------------------------------------------- loads of a wide row
 // (past the L1: the projection that wrote the row may have been running when this block started)
 template <bool W64> struct WideOf { using T = int32_t; };

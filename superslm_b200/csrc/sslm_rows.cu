@@ -291,16 +291,6 @@ k_begin(RowBatch b, Dims d, const int8_t* embed, Scale c_embed, const RowSource*
 	set_status(b, r, st, site, b.layer);
 }
 
-// The bias term of one element, false when it leaves int64. A bias code inside 32 bits keeps the
-// product with the row's reciprocal (at most 2^32) inside 64; others take the 128-bit composite.
-__device__ __forceinline__ bool bias_term(int64_t bias, int64_t r_a, int bexp, int64_t* term) {
-	if (bias == (int64_t)(int32_t)bias && r_a > 0 && (uint64_t)r_a <= ((uint64_t)1 << 32)) {
-		*term = rdivpot64(bias * r_a, bexp);
-		return true;
-	}
-	return bias_reconcile(bias, r_a, bexp, term);
-}
-
 // After the fused q/k/v projection: q funnel (ProjectAndFunnel's tail,
 // forward_sites.cpp:1114-1146), K/V landing with the saturation counter (LandTokenKVRow
 // :1397-1415, LandingRescale :513-653), RoPE on q and on the landed K (:1748-1787,
@@ -312,7 +302,7 @@ __device__ __forceinline__ bool bias_term(int64_t bias, int64_t r_a, int bexp, i
 // lanes derive the softmax constants, a serial scalar chain that needs only the q scale, meanwhile.
 template <int NV, bool W64, bool BIAS>
 __global__ void __launch_bounds__(NV == 1 ? 704 : (NV == 4 ? 352 : 832), NV == 4 ? 2 : 1)
-k_qkv_post(RowBatch b, Dims d, const LayerDev* layer, Scale c_q, int layer_index, KvPoolDev pool, const int32_t* rope_cos,
+k_qkv_post(RowBatch b, Dims d, const __grid_constant__ LayerDev lw, int layer_index, KvPoolDev pool, const int32_t* rope_cos,
            const int32_t* rope_sin) {
 	using T = typename WideOf<W64>::T;
 	__shared__ uint32_t s_bank[64];
@@ -324,13 +314,12 @@ k_qkv_post(RowBatch b, Dims d, const LayerDev* layer, Scale c_q, int layer_index
 	const int nq = (H + 2 * KV) >> 2;
 	// ahead of the projection: the normed row's scale (written by the previous residual site),
 	// the position, its RoPE row and page, the site constants
-	const LayerDev& lw = *layer;
 	const Scale ns = b.ns[r];
 	const int pos = b.rows[r].pos;
 	const int page = b.rows[r].pages[pos / kPageTokens];
 	const int slot = pos % kPageTokens;
 	const int64_t *bias_q = BIAS ? lw.b_q : nullptr, *bias_k = BIAS ? lw.b_k : nullptr, *bias_v = BIAS ? lw.b_v : nullptr;
-	const FunnelFold fold_q = funnel_prefold(&ns, 1, c_q);
+	const FunnelFold fold_q = funnel_prefold(&ns, 1, lw.c_q);
 	Scale kh{0, 0};
 	const int kv_lane = (int)threadIdx.x - qt;
 	if (scalar_warp && kv_lane < d.kv_heads) kh = Scale{lw.sm_khead[2 * kv_lane], lw.sm_khead[2 * kv_lane + 1]};
@@ -468,29 +457,7 @@ k_qkv_post(RowBatch b, Dims d, const LayerDev* layer, Scale c_q, int layer_index
 		int32_t st = kOk;
 		if (kv_lane < d.kv_heads) {
 			SoftmaxConsts sc;
-			sc.c = IExpConsts{0, 0, 0};
-			sc.peak = 0;
-			if (!fits_i32(fp.out.m) || !fits_i32(kh.m)) {
-				st = kCarriedScaleMantissaOutOfDomain;
-			} else {
-				const Scale sm = combine(fp.out, kh);
-				if (!fits_i32(sm.m)) {
-					st = kCarriedScaleMantissaOutOfDomain;
-				} else if (iexp_scale_constants(sm.m, sm.e, &sc.c) != 0) {
-					st = kIExpScaleDerivationOutOfDomain;
-				} else if (!softmax_width_in_domain(sc.c.q_b, sc.c.q_c, (uint64_t)pos + 1, &sc.peak)) {
-					st = kSoftmaxRowWidthOutOfDomain;
-				} else if (sc.c.q_ln2 < 1) {
-					// q_ln2 == 0: every element's construction is refused by the reference
-					// (IExpConstruct's q_ln2 >= 1 check) -> SoftmaxKernelRefused.
-					// The attention kernel's 32-bit element form also needs q_ln2 <= q_b; that holds
-					// for every constant triple iexp_scale_constants returns and needs no test here:
-					// q_ln2 = floor(LN2_Q * r / 2^s) and q_b = floor(B_Q * r / 2^s) with the same
-					// unsigned reciprocal r and the same shift s, and LN2_Q < B_Q, so the floors are
-					// ordered the same way.
-					st = kSoftmaxKernelRefused;
-				}
-			}
+			st = softmax_consts(fp.out, kh, (uint64_t)pos + 1, &sc);
 			b.smc[(size_t)r * d.kv_heads + kv_lane] = sc;
 		}
 		// the first failing head speaks for the row
@@ -1034,7 +1001,7 @@ cudaError_t launch_begin(const RowBatch& b, const Dims& d, const int8_t* embed, 
 	if (nv == 1) return go(k_begin<1>);
 	return nv == 4 ? go(k_begin<4>) : go(k_begin<8>);
 }
-void launch_qkv_post(const RowBatch& b, const Dims& d, const LayerDev* layer, const LayerDev& h, int layer_index, KvPoolDev pool,
+void launch_qkv_post(const RowBatch& b, const Dims& d, const LayerDev& h, int layer_index, KvPoolDev pool,
                      const int32_t* cos, const int32_t* sin, cudaStream_t st) {
 	const int nq = d.qkv_rows / 4;
 	// one more warp than the quads need: it derives the softmax constants (a 704-thread block at most)
@@ -1042,7 +1009,7 @@ void launch_qkv_post(const RowBatch& b, const Dims& d, const LayerDev* layer, co
 	if (quad_threads(nq, nv) > (nv == 1 ? 672 : 320)) nv = quad_threads(nq, 4) <= 320 ? 4 : 8;
 	const int t = quad_threads(nq, nv) + 32;
 	const bool bias = h.b_q != nullptr || h.b_k != nullptr || h.b_v != nullptr;
-	auto go = [&](auto kernel) { launch_pdl(kernel, dim3(b.m), dim3(t), 0, st, b, d, layer, h.c_q, layer_index, pool, cos, sin); };
+	auto go = [&](auto kernel) { launch_pdl(kernel, dim3(b.m), dim3(t), 0, st, b, d, h, layer_index, pool, cos, sin); };
 	auto pick = [&](auto nvc) {
 		constexpr int NV = decltype(nvc)::value;
 		if (b.wide64) bias ? go(k_qkv_post<NV, true, true>) : go(k_qkv_post<NV, true, false>);
