@@ -543,6 +543,11 @@ extern "C" sslm_status sslm_workspace_destroy(sslm_workspace ws) {
 
 extern "C" sslm_status sslm_b200_last_call_ms(sslm_workspace ws, float* ms, uint64_t* launches) {
 	if (!ws) return SSLM_INVALID_ARGUMENT;
+	if (ws->timed) {
+		ws->timed = false;
+		cudaSetDevice(ws->device);
+		cudaEventElapsedTime(&ws->last_ms, ws->ev0, ws->ev1);
+	}
 	if (ms) *ms = ws->last_ms;
 	if (launches) *launches = ws->launches;
 	return SSLM_OK;

@@ -61,6 +61,7 @@ struct sslm_workspace_s {
 	int32_t* d_logits = nullptr;
 	cudaEvent_t ev0 = nullptr, ev1 = nullptr;
 	float last_ms = 0.f;
+	bool timed = false;           // ev0 and ev1 hold a finished call whose time last_ms does not have yet
 	uint64_t launches = 0;
 	bool launch_failed = false;   // a kernel launch of the current call was refused by the runtime
 	// optional per-site trace (sslm_b200_trace): host buffer that receives one record per traced
