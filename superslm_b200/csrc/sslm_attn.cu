@@ -2,7 +2,7 @@
 // contractions on the tensor cores (mma.sync m16n8k32, exact int32 accumulation). A row is one token's q heads
 // over positions 0..pos, cut by kv head, so that each K / V byte of a sequence leaves HBM once per kv head:
 //
-//   k_attention        many decode rows: a block of head_dim/16 warps owns one kv head of a row and meets nobody
+//   k_attention        many decode rows: a block owns one kv head of a row and meets nobody
 //   k_attention_few    few rows: the row is cut along its width as well; its blocks form a thread-block cluster
 //                      and exchange maxima, sums and partial contexts through distributed shared memory
 //   k_attention_chunk  prefill chunks: tiles of 32 query rows, wide ones cut over a cluster, scores kept
@@ -60,7 +60,6 @@ __device__ __forceinline__ IExpFast iexp_fast_prepare(const SoftmaxConsts& k) {
 }
 // *parts = (z << 24) | rem with x = z * q_ln2 + rem (rem < q_ln2 < 2^24, z <= 30): the second
 // softmax pass rebuilds the element from it (iexp_from_parts) instead of dividing again.
-constexpr uint32_t kPartsOfZero = 63u << 24;      // parts that rebuild to the value 0 (shift by 63)
 __device__ __forceinline__ int64_t iexp_fast(uint32_t dq, const IExpFast& f, uint32_t* parts) {
 	const uint32_t x = min(dq, f.clip);
 	uint32_t z = (uint32_t)__float_as_int(__fmaf_rz(__uint2float_rn(x), f.inv_ln2, 8388608.0f)) - 0x4B000000u;
@@ -116,6 +115,49 @@ static __device__ __noinline__ uint2 prob_pair_exact(int64_t e0, int64_t e1, uns
 	const float rinv = 32768.0f / (float)tot;
 	return make_uint2(prob_q15(e0, tot, rinv), prob_q15(e1, tot, rinv));
 }
+// A row's constants of the probability pass. pf = (base^2 + q_c) 2^-z 32768 / total in float is within
+// pf 2^-21 (five roundings) + 32768 / total (the element's own floor) of the quotient, so its floor is the
+// probability unless the nearest integer from 1 up is that close; those take prob_q15. Below 1 it is 0.
+struct ChunkProb {
+	float c, qc, eps;
+};
+__device__ __forceinline__ ChunkProb chunk_prob(unsigned long long total, const IExpFast& f) {
+	ChunkProb p;
+	p.c = 32768.0f / (float)(total > 1ull ? total : 1ull);
+	p.qc = (float)f.qc;
+	p.eps = p.c * 1.01f;
+	return p;
+}
+constexpr uint32_t kBaseOfZero = 63u << 24;      // (shift, base) of an element that counts for nothing
+__device__ __forceinline__ int64_t chunk_exp(uint32_t dq, const IExpFast& f, uint32_t* parts) {
+	const uint32_t x = min(dq, f.clip);
+	uint32_t z = (uint32_t)__float_as_int(__fmaf_rz(__uint2float_rn(x), f.inv_ln2, 8388608.0f)) - 0x4B000000u;
+	uint32_t rem = x - z * f.ln2;
+	if (rem >= f.ln2) {
+		rem -= f.ln2;
+		++z;
+	}
+	const uint32_t base = (uint32_t)f.qb - rem;      // 1 .. q_b < 2^24
+	*parts = (z << 24) + base;
+	return (int64_t)(((uint64_t)base * base + (uint64_t)f.qc) >> z);
+}
+__device__ __forceinline__ uint32_t chunk_prob_of(uint32_t parts, const ChunkProb& p, float* near) {
+	const float bf = __uint2float_rn(parts & 0xFFFFFFu);
+	const float pf = fmaf(bf, bf, p.qc) * __int_as_float(__float_as_int(p.c) - (int)((parts >> 24) << 23));
+	const float whole = fmaxf((pf + 8388608.0f) - 8388608.0f, 1.0f);
+	*near = fminf(*near, fmaf(pf, -4.76837158203125e-07f, fabsf(pf - whole)));
+	return (uint32_t)__float_as_int(__fadd_rz(pf, 8388608.0f));      // (low 16 bits)
+}
+static __device__ __noinline__ uint4 chunk_prob_exact(uint32_t p0, uint32_t p1, uint32_t p2, uint32_t p3, int64_t qc, unsigned long long total) {
+	const unsigned long long tot = total > 1ull ? total : 1ull;
+	const float rinv = 32768.0f / (float)tot;
+	auto one = [&](uint32_t p) {
+		const uint64_t base = p & 0xFFFFFFu;
+		return (p >> 24) == 63u ? 0u : prob_q15((int64_t)((base * base + (uint64_t)qc) >> (p >> 24)), tot, rinv);
+	};
+	return make_uint4(one(p0), one(p1), one(p2), one(p3));
+}
+
 // bytes 0 (low plane) or 1 (high plane) of four probabilities, packed into one word
 __device__ __forceinline__ uint32_t pack_plane(uint32_t p0, uint32_t p1, uint32_t p2, uint32_t p3, int byte) {
 	const uint32_t sel = byte ? 0x0051u : 0x0040u;
@@ -194,15 +236,15 @@ __device__ __forceinline__ void prefetch_l2(const void* p) { asm volatile("prefe
 //   1  scores (tensor cores) and the row maximum per head
 //   2  e_k per element and the row total, then p_k = (e_k << 15) / total
 //   3  P.V (tensor cores), per-head context fold, row maximum for the funnel kernel that follows
-// HD = head_dim (32, 64 or 128); threads = 2 * HD.
-template <int HD>
-__global__ void __launch_bounds__(2 * HD, HD == 128 ? 4 : 8)
+// HD = head_dim (32, 64 or 128); a warp owns NDB blocks of eight channels, so threads = 4 * HD / NDB.
+template <int HD, int NDB>
+__global__ void __launch_bounds__(4 * HD / NDB, (HD == 128 ? 2 : 4) * NDB)
 k_attention(RowBatch b, Dims d, const __grid_constant__ LayerDev layer, int layer_index, KvPoolDev pool, int cp, int reverse_rows) {
 	extern __shared__ __align__(16) unsigned char smem[];
 	// blocks start in index order: with reverse_rows the last (widest) rows of a prefill chunk go first
 	const int r = reverse_rows ? (int)gridDim.y - 1 - (int)blockIdx.y : (int)blockIdx.y;
 	const int kvh = (int)blockIdx.x;
-	constexpr int kAttnThreads = 2 * HD, kAttnWarps = kAttnThreads / 32;
+	constexpr int kAttnThreads = 4 * HD / NDB, kAttnWarps = kAttnThreads / 32;
 	const int G = d.heads / d.kv_heads;
 	const int t = threadIdx.x, warp = t >> 5, lane = t & 31;
 	const int g = lane >> 2, c = lane & 3;
@@ -295,14 +337,14 @@ k_attention(RowBatch b, Dims d, const __grid_constant__ LayerDev layer, int laye
 				const uint32_t m = (uint32_t)s.mx[h];
 				const int4 v = *(const int4*)&row[k4];
 				uint32_t q0, q1, q2, q3;
-				const int64_t e0 = iexp_fast(m - (uint32_t)v.x, fx, &q0);
-				int64_t e1 = iexp_fast(m - (uint32_t)v.y, fx, &q1);
-				int64_t e2 = iexp_fast(m - (uint32_t)v.z, fx, &q2);
-				int64_t e3 = iexp_fast(m - (uint32_t)v.w, fx, &q3);
+				const int64_t e0 = chunk_exp(m - (uint32_t)v.x, fx, &q0);
+				int64_t e1 = chunk_exp(m - (uint32_t)v.y, fx, &q1);
+				int64_t e2 = chunk_exp(m - (uint32_t)v.z, fx, &q2);
+				int64_t e3 = chunk_exp(m - (uint32_t)v.w, fx, &q3);
 				if (k4 + 3 >= n) {       // the row's last group: positions beyond its end count for nothing
-					if (k4 + 1 >= n) { e1 = 0; q1 = kPartsOfZero; }
-					if (k4 + 2 >= n) { e2 = 0; q2 = kPartsOfZero; }
-					e3 = 0; q3 = kPartsOfZero;
+					if (k4 + 1 >= n) { e1 = 0; q1 = kBaseOfZero; }
+					if (k4 + 2 >= n) { e2 = 0; q2 = kBaseOfZero; }
+					e3 = 0; q3 = kBaseOfZero;
 				}
 				tot = (unsigned long long)(e0 + e1) + (unsigned long long)(e2 + e3);
 				*(int4*)&row[k4] = make_int4((int)q0, (int)q1, (int)q2, (int)q3);
@@ -324,16 +366,14 @@ k_attention(RowBatch b, Dims d, const __grid_constant__ LayerDev layer, int laye
 		for (int task = warp; task < G * nchunk; task += kAttnWarps) {
 			const int h = task / nchunk, k4 = (task - h * nchunk) * 128 + lane * 4;
 			if (k4 < n4) {
-				const ProbRow pr = prob_row(s.sum[h]);
+				const ChunkProb pr = chunk_prob(s.sum[h], fx);
 				const int4 v = *(const int4*)&s.sc[(size_t)h * cp + k4];
-				const int64_t e0 = iexp_from_parts((uint32_t)v.x, fx), e1 = iexp_from_parts((uint32_t)v.y, fx);
-				const int64_t e2 = iexp_from_parts((uint32_t)v.z, fx), e3 = iexp_from_parts((uint32_t)v.w, fx);
-				bool unsure = false;
-				uint32_t p0 = prob_fast(e0, pr, &unsure), p1 = prob_fast(e1, pr, &unsure);
-				uint32_t p2 = prob_fast(e2, pr, &unsure), p3 = prob_fast(e3, pr, &unsure);
-				if (unsure) {
-					const uint2 a = prob_pair_exact(e0, e1, pr.tot), b2 = prob_pair_exact(e2, e3, pr.tot);
-					p0 = a.x; p1 = a.y; p2 = b2.x; p3 = b2.y;
+				float near = 1.0f;
+				uint32_t p0 = chunk_prob_of((uint32_t)v.x, pr, &near), p1 = chunk_prob_of((uint32_t)v.y, pr, &near);
+				uint32_t p2 = chunk_prob_of((uint32_t)v.z, pr, &near), p3 = chunk_prob_of((uint32_t)v.w, pr, &near);
+				if (near < pr.eps) {
+					const uint4 x = chunk_prob_exact((uint32_t)v.x, (uint32_t)v.y, (uint32_t)v.z, (uint32_t)v.w, fx.qc, s.sum[h]);
+					p0 = x.x; p1 = x.y; p2 = x.z; p3 = x.w;
 				}
 				*(uint32_t*)&s.pl[(size_t)h * cp + k4] = pack_plane(p0, p1, p2, p3, 0);
 				*(uint32_t*)&s.ph[(size_t)h * cp + k4] = pack_plane(p0, p1, p2, p3, 1);
@@ -350,7 +390,6 @@ k_attention(RowBatch b, Dims d, const __grid_constant__ LayerDev layer, int laye
 	// 8..15). Nothing is predicated: the page table and the planes are padded to whole groups, and
 	// lanes of MMA rows beyond the group's heads read head 0's probabilities (their output rows are
 	// never stored).
-	constexpr int NDB = 2;            // 8-channel blocks per warp
 	int accl[NDB][4], acch[NDB][4];
 #pragma unroll
 	for (int i = 0; i < NDB; ++i)
@@ -821,14 +860,14 @@ k_attention_few(RowBatch b, Dims d, const __grid_constant__ LayerDev layer, int 
 				int32_t* row = s.sc + (size_t)h * cp;
 				const int4 v = *(const int4*)&row[k4];
 				uint32_t q0, q1, q2, q3;
-				const int64_t e0 = iexp_fast((uint32_t)m - (uint32_t)v.x, fx, &q0);
-				int64_t e1 = iexp_fast((uint32_t)m - (uint32_t)v.y, fx, &q1);
-				int64_t e2 = iexp_fast((uint32_t)m - (uint32_t)v.z, fx, &q2);
-				int64_t e3 = iexp_fast((uint32_t)m - (uint32_t)v.w, fx, &q3);
+				const int64_t e0 = chunk_exp((uint32_t)m - (uint32_t)v.x, fx, &q0);
+				int64_t e1 = chunk_exp((uint32_t)m - (uint32_t)v.y, fx, &q1);
+				int64_t e2 = chunk_exp((uint32_t)m - (uint32_t)v.z, fx, &q2);
+				int64_t e3 = chunk_exp((uint32_t)m - (uint32_t)v.w, fx, &q3);
 				if (k4 + 3 >= n) {       // the slice's last group: positions beyond its end count for nothing
-					if (k4 + 1 >= n) { e1 = 0; q1 = kPartsOfZero; }
-					if (k4 + 2 >= n) { e2 = 0; q2 = kPartsOfZero; }
-					e3 = 0; q3 = kPartsOfZero;
+					if (k4 + 1 >= n) { e1 = 0; q1 = kBaseOfZero; }
+					if (k4 + 2 >= n) { e2 = 0; q2 = kBaseOfZero; }
+					e3 = 0; q3 = kBaseOfZero;
 				}
 				tot = (unsigned long long)(e0 + e1) + (unsigned long long)(e2 + e3);
 				*(int4*)&row[k4] = make_int4((int)q0, (int)q1, (int)q2, (int)q3);
@@ -853,16 +892,14 @@ k_attention_few(RowBatch b, Dims d, const __grid_constant__ LayerDev layer, int 
 			if (k4 < n4) {
 				unsigned long long total = s.rx_sum[h];
 				for (int j = 1; j < splits; ++j) total += s.rx_sum[j * 8 + h];
-				const ProbRow pr = prob_row(total);
+				const ChunkProb pr = chunk_prob(total, fx);
 				const int4 v = *(const int4*)&s.sc[(size_t)h * cp + k4];
-				const int64_t e0 = iexp_from_parts((uint32_t)v.x, fx), e1 = iexp_from_parts((uint32_t)v.y, fx);
-				const int64_t e2 = iexp_from_parts((uint32_t)v.z, fx), e3 = iexp_from_parts((uint32_t)v.w, fx);
-				bool unsure = false;
-				uint32_t q0 = prob_fast(e0, pr, &unsure), q1 = prob_fast(e1, pr, &unsure);
-				uint32_t q2 = prob_fast(e2, pr, &unsure), q3 = prob_fast(e3, pr, &unsure);
-				if (unsure) {
-					const uint2 a = prob_pair_exact(e0, e1, pr.tot), a2 = prob_pair_exact(e2, e3, pr.tot);
-					q0 = a.x; q1 = a.y; q2 = a2.x; q3 = a2.y;
+				float near = 1.0f;
+				uint32_t q0 = chunk_prob_of((uint32_t)v.x, pr, &near), q1 = chunk_prob_of((uint32_t)v.y, pr, &near);
+				uint32_t q2 = chunk_prob_of((uint32_t)v.z, pr, &near), q3 = chunk_prob_of((uint32_t)v.w, pr, &near);
+				if (near < pr.eps) {
+					const uint4 x = chunk_prob_exact((uint32_t)v.x, (uint32_t)v.y, (uint32_t)v.z, (uint32_t)v.w, fx.qc, total);
+					q0 = x.x; q1 = x.y; q2 = x.z; q3 = x.w;
 				}
 				*(uint32_t*)&s.pl[(size_t)h * cp + k4] = pack_plane(q0, q1, q2, q3, 0);
 				*(uint32_t*)&s.ph[(size_t)h * cp + k4] = pack_plane(q0, q1, q2, q3, 1);
@@ -1339,49 +1376,6 @@ struct ChunkSmem {
 
 __device__ __forceinline__ void ldmatrix4(uint32_t addr, uint32_t& r0, uint32_t& r1, uint32_t& r2, uint32_t& r3) {
 	asm volatile("ldmatrix.sync.aligned.m8n8.x4.shared.b16 {%0, %1, %2, %3}, [%4];" : "=r"(r0), "=r"(r1), "=r"(r2), "=r"(r3) : "r"(addr) : "memory");
-}
-
-// A row's constants of the probability pass. pf = (base^2 + q_c) 2^-z 32768 / total in float is within
-// pf 2^-21 (five roundings) + 32768 / total (the element's own floor) of the quotient, so its floor is the
-// probability unless the nearest integer from 1 up is that close; those take prob_q15. Below 1 it is 0.
-struct ChunkProb {
-	float c, qc, eps;
-};
-__device__ __forceinline__ ChunkProb chunk_prob(unsigned long long total, const IExpFast& f) {
-	ChunkProb p;
-	p.c = 32768.0f / (float)(total > 1ull ? total : 1ull);
-	p.qc = (float)f.qc;
-	p.eps = p.c * 1.01f;
-	return p;
-}
-constexpr uint32_t kBaseOfZero = 63u << 24;      // (shift, base) of an element that counts for nothing
-__device__ __forceinline__ int64_t chunk_exp(uint32_t dq, const IExpFast& f, uint32_t* parts) {
-	const uint32_t x = min(dq, f.clip);
-	uint32_t z = (uint32_t)__float_as_int(__fmaf_rz(__uint2float_rn(x), f.inv_ln2, 8388608.0f)) - 0x4B000000u;
-	uint32_t rem = x - z * f.ln2;
-	if (rem >= f.ln2) {
-		rem -= f.ln2;
-		++z;
-	}
-	const uint32_t base = (uint32_t)f.qb - rem;      // 1 .. q_b < 2^24
-	*parts = (z << 24) + base;
-	return (int64_t)(((uint64_t)base * base + (uint64_t)f.qc) >> z);
-}
-__device__ __forceinline__ uint32_t chunk_prob_of(uint32_t parts, const ChunkProb& p, float* near) {
-	const float bf = __uint2float_rn(parts & 0xFFFFFFu);
-	const float pf = fmaf(bf, bf, p.qc) * __int_as_float(__float_as_int(p.c) - (int)((parts >> 24) << 23));
-	const float whole = fmaxf((pf + 8388608.0f) - 8388608.0f, 1.0f);
-	*near = fminf(*near, fmaf(pf, -4.76837158203125e-07f, fabsf(pf - whole)));
-	return (uint32_t)__float_as_int(__fadd_rz(pf, 8388608.0f));      // (low 16 bits)
-}
-static __device__ __noinline__ uint4 chunk_prob_exact(uint32_t p0, uint32_t p1, uint32_t p2, uint32_t p3, int64_t qc, unsigned long long total) {
-	const unsigned long long tot = total > 1ull ? total : 1ull;
-	const float rinv = 32768.0f / (float)tot;
-	auto one = [&](uint32_t p) {
-		const uint64_t base = p & 0xFFFFFFu;
-		return (p >> 24) == 63u ? 0u : prob_q15((int64_t)((base * base + (uint64_t)qc) >> (p >> 24)), tot, rinv);
-	};
-	return make_uint4(one(p0), one(p1), one(p2), one(p3));
 }
 
 template <int HD>
@@ -1894,9 +1888,16 @@ template <int HD>
 static cudaError_t launch_attn(const RowBatch& b, const Dims& d, const LayerDev& layer, int layer_index, KvPoolDev pool,
                                const AttnPlan& p, int reverse_rows, int site, const QkvSite& qs, cudaStream_t st) {
 	const int G = d.heads / d.kv_heads;
-	if (p.splits == 0)
-		return launch_pdl(k_attention<HD>, dim3(d.kv_heads, b.m), dim3(2 * HD), attn_smem_bytes(G, p.cp), st, b, d, layer, layer_index,
-		                  pool, p.cp, reverse_rows);
+	if (p.splits == 0) {
+		// Twice the warps per block for decode rows: the blocks of the widest rows end last, and theirs is a chain. ms for 4 tokens,
+		// 2 * head_dim threads / 4 * head_dim: 0.5B 45 rows 5.19 / 4.76, 80 5.75 / 5.44, 250 8.31 / 8.03; 1.5B 100 rows 7.89 / 7.71,
+		// 180 9.52 / 9.07. Not with 128 channels and about one block per multiprocessor (64 rows 31.9 / 32.5 for 16
+		// tokens, 80 7.22 / 7.32 for 4), nor for the short rows of a prompt (150 rows: 2.32 / 2.39).
+		const int blocks = d.kv_heads * b.m;
+		const bool wide = reverse_rows == 0 && (HD < 128 || 4 * blocks >= 5 * sm_count());
+		return launch_pdl(wide ? k_attention<HD, 1> : k_attention<HD, 2>, dim3(d.kv_heads, b.m), dim3(wide ? 4 * HD : 2 * HD), attn_smem_bytes(G, p.cp), st,
+		                  b, d, layer, layer_index, pool, p.cp, reverse_rows);
+	}
 	const bool staged = FewSmem<HD>::bytes(G, p.cp, true) <= kFewSmemMax;
 	RowBatch rb = b;
 	rb.debug_withhold = exchange_debug_take(kExchangeAttnFew);
@@ -1933,7 +1934,8 @@ static cudaError_t configure_hd() {
 		if (e == cudaSuccess) e = cudaFuncSetAttribute(f, cudaFuncAttributePreferredSharedMemoryCarveout, cudaSharedmemCarveoutMaxShared);
 		return e;
 	};
-	cudaError_t e = set((const void*)k_attention<HD>, (int)attn_smem_bytes(group, kAttnMaxSlice), false);
+	cudaError_t e = set((const void*)k_attention<HD, 1>, (int)attn_smem_bytes(group, kAttnMaxSlice), false);
+	if (e == cudaSuccess) e = set((const void*)k_attention<HD, 2>, (int)attn_smem_bytes(group, kAttnMaxSlice), false);
 	for (const void* few : {(const void*)k_attention_few<HD, true, kSiteApart, false>, (const void*)k_attention_few<HD, true, kSitePlain, false>,
 	                        (const void*)k_attention_few<HD, true, kSitePlain, true>, (const void*)k_attention_few<HD, true, kSiteBias, false>,
 	                        (const void*)k_attention_few<HD, true, kSiteBias, true>})
