@@ -696,11 +696,23 @@ k_res(RowBatch b, Dims d, ResSite a) {
 	set_status(b, r, st, site, site_layer);
 }
 
+// scalars of an activation row
+struct ActRow {
+	float fg, fg_lo, fu, fu_lo;
+	uint32_t dg, du;
+	int live;
+	FunnelFold fold;
+};
+
 // gate / up funnels -> SwiGLU activation site (MlpActSite, forward_sites.cpp:796-864).
 //
 // The activation row is the longest a row site walks (intermediate width, three codes per element).
 // While rows are few its time is one block's chain, so a row is cut over a cluster of `gridDim.x`
 // blocks, which meet once, for the maximum of the products; on a prefill chunk two blocks share a row.
+// What depends on the row alone (two scale folds, two funnels, the product's fold: a quarter of the instructions) one warp
+// derives for the block, while the others wait for their elements: 64 rows of 8,960 1.6 % a step, a prompt of
+// 37 3 %. Not with five quads a thread, where it costs registers (prompt of 300: 1.7 % longer), nor for the fewest rows,
+// whose chain the extra trip through shared memory only lengthens.
 // DENSE: in 72 registers instead of 80, for one more block per multiprocessor at some widths (launch_act)
 template <int NV, bool W64, bool DENSE = false>
 __global__ void __launch_bounds__(DENSE ? 288 : (NV == 5 ? 352 : 384), NV == 1 ? 1 : (DENSE ? 3 : 2))
@@ -710,6 +722,8 @@ k_act(RowBatch b, Dims d, Scale c_gate, Scale c_up, Scale c_act, const int32_t* 
 	__shared__ int32_t table[1025];     // the sigmoid table
 	__shared__ int32_t gsil[256];       // g * sigmoid(g) for the 255 gate codes, this row's scale
 	__shared__ uint32_t s_peer[8];      // every block's largest product
+	__shared__ ActRow s_row;
+	__shared__ Scale s_gate;
 	__shared__ __align__(8) unsigned long long s_arrived;
 	Bank bank{s_bank, 0};
 	const int r = blockIdx.y, n = d.inter, nq = n >> 2;
@@ -717,9 +731,15 @@ k_act(RowBatch b, Dims d, Scale c_gate, Scale c_up, Scale c_act, const int32_t* 
 	const int per = (nq + (int)blocks - 1) / (int)blocks, q0 = (int)rank * per, q1 = min(nq, q0 + per);
 	// ahead of the gate/up projection: the normed row's scale (written by the residual site
 	// before that projection ran) and the sigmoid table
-	const Scale ns = b.ns[r];
+	const bool shared = NV <= 2 && b.m >= 16;
+	const bool scalar_thread = !shared || threadIdx.x < 32;
 	for (int i = threadIdx.x; i < 1025; i += blockDim.x) table[i] = silu_table[i];
-	const FunnelFold fold_g = funnel_prefold(&ns, 1, c_gate), fold_u = funnel_prefold(&ns, 1, c_up);
+	FunnelFold fold_g{}, fold_u{};
+	if (scalar_thread) {
+		const Scale ns = b.ns[r];
+		fold_g = funnel_prefold(&ns, 1, c_gate);
+		fold_u = funnel_prefold(&ns, 1, c_up);
+	}
 	const uint32_t arrived = cta_addr(&s_arrived);
 	if (blocks > 1) {
 		if (threadIdx.x == 0) {
@@ -744,28 +764,54 @@ k_act(RowBatch b, Dims d, Scale c_gate, Scale c_up, Scale c_act, const int32_t* 
 			xu[v][0] = xu[v][1] = xu[v][2] = xu[v][3] = 0;
 		}
 	}
-	const unsigned long long mxg = __ldcg(&b.rowmax[(size_t)r * 4 + 1]), mxu = __ldcg(&b.rowmax[(size_t)r * 4 + 2]);
-	const bool refused = __ldcg(&b.status[r]) != 0;
-	const QuadFunnel fg = quad_funnel(mxg, fold_g);
-	const QuadFunnel fu = quad_funnel(mxu, fold_u);
-	int32_t st = fg.status != kOk ? fg.status : fu.status;
-	int site = fg.status != kOk ? kSiteGate : kSiteUp;
-	if (st == kOk && !silu_scale_in_domain(fg.out)) {
-		st = kSiluScaleOutOfDomain;
-		site = kSiteSilu;
+	bool refused = false;
+	int32_t st = kOk;
+	int site = kSiteGate;
+	Scale inc[2] = {Scale{0, 0}, Scale{0, 0}};
+	QuadFunnel fg{}, fu{};
+	bool live = false;
+	if (scalar_thread) {
+		const unsigned long long mxg = __ldcg(&b.rowmax[(size_t)r * 4 + 1]), mxu = __ldcg(&b.rowmax[(size_t)r * 4 + 2]);
+		refused = __ldcg(&b.status[r]) != 0;
+		const QuadFunnel qg = quad_funnel(mxg, fold_g), qu = quad_funnel(mxu, fold_u);
+		inc[0] = qg.out;
+		inc[1] = qu.out;
+		st = qg.status != kOk ? qg.status : qu.status;
+		site = qg.status != kOk ? kSiteGate : kSiteUp;
+		if (st == kOk && !silu_scale_in_domain(qg.out)) {
+			st = kSiluScaleOutOfDomain;
+			site = kSiteSilu;
+		}
+		fg = qg;
+		fu = qu;
+		live = !refused && st == kOk;
+		if (shared && threadIdx.x == 0) {
+			s_row.fg = qg.f; s_row.fg_lo = qg.f_lo; s_row.dg = qg.d;
+			s_row.fu = qu.f; s_row.fu_lo = qu.f_lo; s_row.du = qu.d;
+			s_row.live = live;
+			s_gate = qg.out;
+		}
 	}
-	const bool live = !refused && st == kOk;
-	__syncthreads();      // the table is complete
+	__syncthreads();      // the table and the row's scalars are complete
+	if (shared) {
+		live = s_row.live != 0;
+		fg.f = s_row.fg; fg.f_lo = s_row.fg_lo; fg.d = s_row.dg;
+		fu.f = s_row.fu; fu.f_lo = s_row.fu_lo; fu.d = s_row.du;
+	}
 	if (live) {
 		// the sigmoid depends only on the gate code and the row's gate scale: 255 evaluations per
 		// block instead of one per element
-		const int ge = (int)fg.out.e;
-		for (int t = threadIdx.x; t < 255; t += blockDim.x) gsil[t] = (t - 127) * silu_sigmoid_q15(table, t - 127, fg.out.m, ge);
+		const int64_t gm = shared ? s_gate.m : inc[0].m;
+		const int ge = (int)(shared ? s_gate.e : inc[0].e);
+		for (int t = threadIdx.x; t < 255; t += blockDim.x) gsil[t] = (t - 127) * silu_sigmoid_q15(table, t - 127, gm, ge);
 	}
 	__syncthreads();
+	FunnelFold fold_act{};
+	if (scalar_thread) {      // (read behind the barrier of the maximum that it will meet)
+		fold_act = funnel_prefold(inc, 2, c_act);
+		if (shared && threadIdx.x == 0) s_row.fold = fold_act;
+	}
 	// products g * sigmoid(g) * u, |.| <= 127 * 2^15 * 127 < 2^29
-	const Scale inc[2] = {fg.out, fu.out};
-	const FunnelFold fold_act = funnel_prefold(inc, 2, c_act);   // ahead of the maximum it will meet
 	int32_t w[NV][4];
 	uint32_t mx = 0;
 	if (live) {
@@ -801,7 +847,7 @@ k_act(RowBatch b, Dims d, Scale c_gate, Scale c_up, Scale c_act, const int32_t* 
 		if (!refused && rank == 0) set_status(b, r, st, site, b.layer);
 		return;
 	}
-	const QuadFunnel fp = quad_funnel((unsigned long long)mx, fold_act);
+	const QuadFunnel fp = quad_funnel((unsigned long long)mx, shared ? s_row.fold : fold_act);
 	if (fp.status != kOk) {
 		if (rank == 0) set_status(b, r, fp.status, kSiteAct, b.layer);
 		return;
@@ -828,12 +874,6 @@ k_act(RowBatch b, Dims d, Scale c_gate, Scale c_up, Scale c_act, const int32_t* 
 // (210 a quad and warp, half of the slots): 2,047 rows of 8,960 take 47 us in place of 73, of which the
 // 165 MB that move need 26.
 constexpr int kActWorkers = 256, kActThreads = kActWorkers + 64, kActStages = 4;
-struct ActRow {
-	float fg, fg_lo, fu, fu_lo;
-	uint32_t dg, du;
-	int live;
-	FunnelFold fold;
-};
 __global__ void __launch_bounds__(kActThreads, 3)
 k_act_many(RowBatch b, Dims d, Scale c_gate, Scale c_up, Scale c_act, const int32_t* silu_table) {
 	extern __shared__ __align__(128) int4 stage[];      // [kActStages][gate, up][worker], then the products [quads of a row]
