@@ -122,8 +122,9 @@ extern "C" sslm_status sslm_b200_linear_resident(const int8_t* d_x, const int8_t
 	a.seg_lora[0] = a.seg_lora[1] = a.seg_lora[2] = -1;
 	a.caller_memory = 1;
 	// nothing ran yet if the projection's launch is refused: the array still reads zero. From two rows on
-	// the tensor cores (45 rows of 1536 x 8960: 85 us as six passes of the streaming kernel).
-	const bool tc = M >= 2 && (launch_linear_skinny(a, st) || (M > 8 && launch_linear_tc(a, st)));
+	// the tensor cores (45 rows of 1536 x 8960: 85 us as six passes of the streaming kernel); up to eight rows, where the
+	// projection fits, with the weights waiting in shared memory (11,008 x 2,048, 2 rows: 14.4 us back to back, 11.9 so).
+	const bool tc = M >= 2 && (launch_linear_few(a, st) || launch_linear_skinny(a, st) || (M > 8 && launch_linear_tc(a, st)));
 	if (!tc && launch_linear_gemv(a, st) != cudaSuccess) return SSLM_ALLOCATION_FAILED;
 	const int threads = N >= 4096 ? 1024 : (N >= 1024 ? 256 : 128);
 	launch_pdl(k_resident_funnel, dim3(M), dim3(threads), 0, st, (const int32_t*)d_out_folded, (int)N, peak, (const Scale*)d_in_scales,

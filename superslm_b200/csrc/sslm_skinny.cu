@@ -257,11 +257,10 @@ k_skinny(const __grid_constant__ CUtensorMap map_w, const __grid_constant__ CUte
 	const int ntiles = tile0 < tiles ? (tiles - tile0 + tile_step - 1) / tile_step : 0;
 	const int total = ntiles * nkb;                          // stages this block consumes
 
-	// The channel that a thread of the epilogue finishes, its fold constants asked for ahead of the weights: behind the
-	// exchange the load took half a microsecond, and behind the weights it holds up the dependency wait.
+	// The channel that a thread of a clustered block's epilogue finishes, its fold constants asked for ahead of the weights:
+	// behind the exchange the load took half a microsecond, and behind the weights it holds up the dependency wait.
 	Channel c{};
-	if (warp >= 2)
-		c = channel_of(a, tile0 * kWRows + (splits > 1 ? rank * (kWRows / splits) + ((int)threadIdx.x - 64) % (kWRows / splits) : (warp & 3) * 32 + lane));
+	if (warp >= 2 && splits > 1) c = channel_of(a, tile0 * kWRows + rank * (kWRows / splits) + ((int)threadIdx.x - 64) % (kWRows / splits));
 	if (threadIdx.x == 0) {
 		for (int s = 0; s < stages; ++s) {
 			bar_init(full_bar(s), 1);
@@ -355,6 +354,7 @@ k_skinny(const __grid_constant__ CUtensorMap map_w, const __grid_constant__ CUte
 				else if (a.rowmax != nullptr) atomicMax(&a.rowmax[(size_t)m * 4], kRowmaxTimeout);
 			}
 		};
+		if (splits == 1) c = channel_of(a, tile0 * kWRows + q * 32 + lane);      // (not ahead of the block's set-up, which would wait for it)
 		pdl_wait();
 		if (splits > 1) {
 			// ---- one tile: send every peer the accumulator rows it finishes, finish 128 / splits of them
