@@ -117,6 +117,7 @@ k_linear_few(const __grid_constant__ CUtensorMap map_w, LinearArgs a, FewPlan p)
 	int acc[4] = {0, 0, 0, 0};
 	if (nkb > 0 && !__all_sync(0xffffffffu, bounded_wait<false>(bar, 0))) {
 		s_timeout = 1;
+		bounded_wait<false>(bar, 0);      // (boxes that are late must not land in a shared memory given up)
 	} else {
 		const int row = lane & 15;
 		const uint32_t wrow = mine + (uint32_t)row * kBlockBytes, sw = (uint32_t)(row & 7), half = (uint32_t)lane >> 4;
