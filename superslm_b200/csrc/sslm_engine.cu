@@ -466,7 +466,8 @@ sslm_workspace_s* create_workspace(sslm_model_s* model, const sslm_config& cfg, 
 	ok = ok && cuda_ok(cudaMalloc((void**)&w->d_up, rows * kUpBytesPerRow));
 	ok = ok && cuda_ok(cudaMallocHost((void**)&w->h_down, rows * kDownBytesPerRow));
 	ok = ok && cuda_ok(cudaMalloc((void**)&w->d_down, rows * kDownBytesPerRow));
-	ok = ok && cuda_ok(cudaEventCreate(&w->ev0)) && cuda_ok(cudaEventCreate(&w->ev1));
+	for (auto& pair : w->ev)
+		for (cudaEvent_t& e : pair) ok = ok && cuda_ok(cudaEventCreate(&e));
 	if (ok && rows > 8) {
 		// K slices times tiles never exceeds the SM count, and a tile is at most 256 x 64
 		// accumulators, so 16 MiB holds every case the tensor-core path picks
@@ -497,8 +498,9 @@ static void destroy_workspace(sslm_workspace_s* w) {
 	cudaFree(w->d_down);
 	cudaFreeHost(w->h_up);
 	cudaFreeHost(w->h_down);
-	if (w->ev0) cudaEventDestroy(w->ev0);
-	if (w->ev1) cudaEventDestroy(w->ev1);
+	for (auto& pair : w->ev)
+		for (cudaEvent_t e : pair)
+			if (e) cudaEventDestroy(e);
 	for (cudaEvent_t e : w->prof_events) cudaEventDestroy(e);
 	if (w->stream) cudaStreamDestroy(w->stream);
 	delete w;
@@ -544,9 +546,12 @@ extern "C" sslm_status sslm_workspace_destroy(sslm_workspace ws) {
 extern "C" sslm_status sslm_b200_last_call_ms(sslm_workspace ws, float* ms, uint64_t* launches) {
 	if (!ws) return SSLM_INVALID_ARGUMENT;
 	if (ws->timed) {
+		const cudaEvent_t* ev = ws->ev[ws->ev_now ^ 1];
+		if (!cuda_ok(cudaEventElapsedTime(&ws->last_ms, ev[0], ev[1]))) {
+			cudaGetLastError();
+			return SSLM_ALLOCATION_FAILED;
+		}
 		ws->timed = false;
-		cudaSetDevice(ws->device);
-		cudaEventElapsedTime(&ws->last_ms, ws->ev0, ws->ev1);
 	}
 	if (ms) *ms = ws->last_ms;
 	if (launches) *launches = ws->launches;

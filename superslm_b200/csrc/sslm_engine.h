@@ -59,9 +59,10 @@ struct sslm_workspace_s {
 	unsigned int* d_tc_counters = nullptr;
 	int32_t* logit_capture = nullptr;   // host buffer for full logit rows (tests), or nullptr
 	int32_t* d_logits = nullptr;
-	cudaEvent_t ev0 = nullptr, ev1 = nullptr;
+	cudaEvent_t ev[2][2] = {};    // start and end: of the call at hand [ev_now] and of the last completed one [ev_now ^ 1]
+	int ev_now = 0;
 	float last_ms = 0.f;
-	bool timed = false;           // ev0 and ev1 hold a finished call whose time last_ms does not have yet
+	bool timed = false;           // last_ms does not have the last completed call's time yet
 	uint64_t launches = 0;
 	bool launch_failed = false;   // a kernel launch of the current call was refused by the runtime
 	// optional per-site trace (sslm_b200_trace): host buffer that receives one record per traced
