@@ -563,7 +563,7 @@ k_attention_few(RowBatch b, Dims d, const __grid_constant__ LayerDev layer, int 
 		exchange_init(bar(1), (uint32_t)(splits * G * 8) + more(1));
 		exchange_init(bar(2), (uint32_t)(G * HD * 4) + more(2));
 		exchange_init(bar(3), 4u * cluster_blocks + more(3));
-		if (SITE == kSiteBias) exchange_init(bar(4), 8u * cluster_blocks);
+		if (SITE == kSiteBias) exchange_init(bar(4), 8u * cluster_blocks + more(4));
 		exchange_fence_init();
 	}
 	// ahead of the kernel that lands this step's K / V rows: the page table, the old rows

@@ -95,7 +95,7 @@ def test_exchange_that_runs_out(gpu_lib, kernel, exchange, shape, n, call):
     eng = abi.Engine(gpu_lib, art, blocks=1, max_chunk=n)
     arm = gpu_lib.dll.sslm_b200_debug_withhold_exchange
     arm.argtypes = [C.c_int32, C.c_int32]
-    assert arm(kernel, 4) == arm(4, 0) == abi.ST["SSLM_INVALID_ARGUMENT"]
+    assert arm(kernel, 5) == arm(4, 0) == abi.ST["SSLM_INVALID_ARGUMENT"]
     failed = abi.ST["SSLM_ALLOCATION_FAILED"]
     try:
         s = eng.new_seq()
@@ -118,6 +118,62 @@ def test_exchange_that_runs_out(gpu_lib, kernel, exchange, shape, n, call):
         assert 0.2 < took < 5.0      # waits of a quarter of a second: four exchanges and six times that on the way out
         assert s.decode(2, sh.layers) == want_toks[1:]
         assert abi.parse_save_blob(s.save(), sh.hidden)["kv"] == ps.kv.tobytes()
+    finally:
+        arm(-1, 0)
+        eng.close()
+
+
+# batches whose q/k/v site runs inside the attention cluster: (shape, adapted, bias_bits, prompts, exchange). Clusters of 16 blocks
+# (up to six rows), of 8, and of 2; with biases there is a fifth exchange.
+SITE_EXCHANGES = [("mini1.5b", False, 0, (300, 40), x) for x in range(4)] + [("mini0.5b", False, 30, (300, 40, 5), x) for x in range(5)] + \
+                 [("tiny", True, 36, (200, 30), 4), ("tiny", True, 0, (200, 30), 1), ("small", False, 36, (70, 5, 30, 64, 1, 20, 9, 16), 4),
+                  ("small", False, 30, (20, 5), 4), ("small", False, 30, (20, 5), 0)]
+
+
+@pytest.mark.parametrize("shape,adapted,bias_bits,lengths,exchange", SITE_EXCHANGES)
+def test_exchange_of_a_batch_that_runs_out(gpu_lib, shape, adapted, bias_bits, lengths, exchange):
+    """Row 0 of a batch gives up inside its cluster in the first layer: the call fails, no sequence moves, and the next calls give
+    the oracle's tokens, K/V bytes and saturation counts (the failed call's own landings stay counted, as any refused call's)."""
+    sh = A.SHAPES[shape]
+    art = A.build_synthetic_model(shape, 0x7280, 320, bias_bits=bias_bits)
+    adp = A.build_synthetic_adapter(art, 0x7281, 16, A.PEFT_ORDER) if adapted else None
+    eng = abi.Engine(gpu_lib, art, blocks=len(lengths), max_batch=len(lengths), max_chunk=320)
+
+    def holds(s):      # the positions that count, their K/V, where the sequence stands, its saturation count
+        b = abi.parse_save_blob(s.save(), sh.hidden)
+        kv = np.frombuffer(b["kv"], dtype=np.int8).reshape(sh.layers, 2, sh.kv_heads, 320, sh.head_dim)
+        return kv[:, :, :, :b["context_length"]].tobytes(), b["context_length"], b["layer_index"], b["kv_saturation_count"]
+
+    arm = gpu_lib.dll.sslm_b200_debug_withhold_exchange
+    arm.argtypes = [C.c_int32, C.c_int32]
+    try:
+        handle = eng.map_adapter(adp) if adapted else None
+        seqs, want = [], []
+        for i, n in enumerate(lengths):
+            prompt = A.stream_uniform(0x7290 + i, "prompt", n, 0, sh.vocab - 1)
+            want.append(run_port(art, prompt, 4, adp))
+            s = eng.new_seq()
+            if adapted:
+                s.set_adapter(handle)
+            assert s.prefill(prompt, 320) == n
+            seqs.append(s)
+        got = [eng.decode_step(seqs, sh.layers)]
+        before = [holds(s) for s in seqs]
+        assert arm(1, exchange) == 0
+        t = time.perf_counter()
+        assert eng.decode_step(seqs, sh.layers)[0] == abi.ST["SSLM_ALLOCATION_FAILED"]
+        assert 0.2 < time.perf_counter() - t < 5.0
+        after = [holds(s) for s in seqs]
+        assert [a[:3] for a in after] == [b[:3] for b in before] and [a[3] for a in after[1:]] == [b[3] for b in before[1:]]
+        again = after[0][3] - before[0][3]
+        assert 0 <= again <= 2 * sh.kv_hidden
+        got += [eng.decode_step(seqs, sh.layers) for _ in range(3)]
+        assert [status for status, _ in got] == [0] * 4
+        for i, (s, (tokens, ps)) in enumerate(zip(seqs, want)):
+            assert [step[i] for _, step in got] == tokens
+            blob = abi.parse_save_blob(s.save(), sh.hidden)
+            assert blob["kv"] == ps.kv.tobytes()
+            assert blob["kv_saturation_count"] == ps.s.kv_saturation_count + (again if i == 0 else 0)
     finally:
         arm(-1, 0)
         eng.close()
