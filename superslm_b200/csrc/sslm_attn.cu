@@ -58,9 +58,8 @@ __device__ __forceinline__ IExpFast iexp_fast_prepare(const SoftmaxConsts& k) {
 	f.inv_ln2 = (1.0f / (float)f.ln2) * 0.9999995f;
 	return f;
 }
-// *parts = (z << 24) | rem with x = z * q_ln2 + rem (rem < q_ln2 < 2^24, z <= 30): the second
-// softmax pass rebuilds the element from it (iexp_from_parts) instead of dividing again.
-__device__ __forceinline__ int64_t iexp_fast(uint32_t dq, const IExpFast& f, uint32_t* parts) {
+// The element by itself: k_attention_tile, which keeps nothing between its walks. (x = z * q_ln2 + rem, rem < q_ln2 < 2^24, z <= 30)
+__device__ __forceinline__ int64_t iexp_fast(uint32_t dq, const IExpFast& f) {
 	const uint32_t x = min(dq, f.clip);
 	uint32_t z = (uint32_t)__float_as_int(__fmaf_rz(__uint2float_rn(x), f.inv_ln2, 8388608.0f)) - 0x4B000000u;
 	uint32_t rem = x - z * f.ln2;
@@ -69,12 +68,7 @@ __device__ __forceinline__ int64_t iexp_fast(uint32_t dq, const IExpFast& f, uin
 		++z;
 	}
 	const int32_t base = f.qb - (int32_t)rem;
-	*parts = (z << 24) | rem;
 	return (int64_t)((uint64_t)((int64_t)base * (int64_t)base + f.qc) >> z);
-}
-__device__ __forceinline__ int64_t iexp_from_parts(uint32_t parts, const IExpFast& f) {
-	const int32_t base = f.qb - (int32_t)(parts & 0xFFFFFFu);
-	return ((int64_t)base * (int64_t)base + f.qc) >> (parts >> 24);
 }
 // Q15 probability floor((e << 15) / tot), 0 <= e <= tot, 1 <= tot < 2^63.
 //
@@ -129,6 +123,8 @@ __device__ __forceinline__ ChunkProb chunk_prob(unsigned long long total, const 
 	return p;
 }
 constexpr uint32_t kBaseOfZero = 63u << 24;      // (shift, base) of an element that counts for nothing
+// The element of the kernels that keep their scores; *parts, its (shift, base) word, takes the score's place and the
+// probability pass reads it instead of dividing again.
 __device__ __forceinline__ int64_t chunk_exp(uint32_t dq, const IExpFast& f, uint32_t* parts) {
 	const uint32_t x = min(dq, f.clip);
 	uint32_t z = (uint32_t)__float_as_int(__fmaf_rz(__uint2float_rn(x), f.inv_ln2, 8388608.0f)) - 0x4B000000u;
@@ -1210,9 +1206,8 @@ k_attention_tile(RowBatch b, Dims d, const __grid_constant__ LayerDev layer, int
 			const int k0 = blk * kTileKeys + 32 * ph + 8 * j + 2 * c;
 #pragma unroll
 			for (int q = 0; q < 2; ++q) {
-				uint32_t parts;
-				const int64_t ea = iexp_fast((uint32_t)mx_a - (uint32_t)acc[j][q], fa, &parts);
-				const int64_t eb = iexp_fast((uint32_t)mx_b - (uint32_t)acc[j][2 + q], fb, &parts);
+				const int64_t ea = iexp_fast((uint32_t)mx_a - (uint32_t)acc[j][q], fa);
+				const int64_t eb = iexp_fast((uint32_t)mx_b - (uint32_t)acc[j][2 + q], fb);
 				sum_a += k0 + q <= lim_a ? (unsigned long long)ea : 0ull;
 				sum_b += k0 + q <= lim_b ? (unsigned long long)eb : 0ull;
 			}
@@ -1250,9 +1245,8 @@ k_attention_tile(RowBatch b, Dims d, const __grid_constant__ LayerDev layer, int
 			bool unsure = false;
 #pragma unroll
 			for (int q = 0; q < 2; ++q) {
-				uint32_t parts;
-				ea[q] = iexp_fast((uint32_t)mx_a - (uint32_t)acc[j][q], fa, &parts);
-				eb[q] = iexp_fast((uint32_t)mx_b - (uint32_t)acc[j][2 + q], fb, &parts);
+				ea[q] = iexp_fast((uint32_t)mx_a - (uint32_t)acc[j][q], fa);
+				eb[q] = iexp_fast((uint32_t)mx_b - (uint32_t)acc[j][2 + q], fb);
 				// (an element beyond its row's limit may exceed the row's total: it is dropped below, whatever it gives)
 				pa[q] = prob_fast(ea[q], pr_a, &unsure);
 				pb[q] = prob_fast(eb[q], pr_b, &unsure);
@@ -2046,11 +2040,9 @@ __global__ void k_int_sweep(int which, const int64_t* a, const int64_t* b, const
 			k.c = IExpConsts{b[i], c[i], e[i] >> 32};
 			k.peak = (int64_t)(uint32_t)e[i] << 16;
 			const IExpFast f = iexp_fast_prepare(k);
-			uint32_t parts = 0;
-			const int64_t v = iexp_fast((uint32_t)a[i], f, &parts);
+			const int64_t v = iexp_fast((uint32_t)a[i], f);
 			o0 = v;
 			o1 = (v < 0 || v > k.peak) ? 1 : 0;       // the reference's per-element bound
-			o2 = iexp_from_parts(parts, f);
 			break;
 		}
 		case 8: {      // Q15 probability: floor((e << 15) / total), 0 <= e <= total
@@ -2096,7 +2088,7 @@ __global__ void k_int_sweep(int which, const int64_t* a, const int64_t* b, const
 			o2 = nd.root;
 			break;
 		}
-		case 13: {      // the prefill kernels' softmax element; o1 its (shift, base) word
+		case 13: {      // the softmax element of the kernels that keep their scores; o1 its (shift, base) word
 			SoftmaxConsts k;
 			k.c = IExpConsts{b[i], c[i], e[i]};
 			k.peak = 0;
