@@ -201,18 +201,26 @@ k_linear_few(const __grid_constant__ CUtensorMap map_w, LinearArgs a, FewPlan p)
 }
 
 constexpr int kSmemMax = 220 * 1024;
-constexpr int kRegs = 80;
+// what a block takes beside its dynamic shared memory, as compiled: registers of a warp (given out in units of 256), shared memory
+struct FewCost {
+	int warp_regs, fixed_smem;
+};
 
 bool launch(LinearArgs& a, cudaStream_t st) {
 	static PerDeviceOnce configured;
-	if (once_per_device(configured, [] {
-		    cudaError_t e = cudaFuncSetAttribute(k_linear_few, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmemMax);
+	static FewCost costs[kMaxDevices];
+	FewCost& cost = costs[current_device_ordinal()];
+	if (once_per_device(configured, [&cost] {
+		    cudaFuncAttributes f;
+		    cudaError_t e = cudaFuncGetAttributes(&f, k_linear_few);
+		    if (e == cudaSuccess) cost = FewCost{(f.numRegs * 32 + 255) / 256 * 256, (int)f.sharedSizeBytes + 1024};      // (1 KB is the system's)
+		    if (e == cudaSuccess) e = cudaFuncSetAttribute(k_linear_few, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmemMax);
 		    if (e == cudaSuccess) e = cudaFuncSetAttribute(k_linear_few, cudaFuncAttributePreferredSharedMemoryCarveout, cudaSharedmemCarveoutMaxShared);
 		    return e;
 	    }) != cudaSuccess)
 		return false;
-	// The fewest tiles per block with which all blocks run at once and leave room for those of the row kernel in front
-	// (a second wave of 100 KB blocks began 6 us after the first).
+	// The fewest tiles per block with which all blocks run at once (a second wave of 100 KB blocks began 6 us after the first)
+	// beside those of the row kernel in front, which has a block per row and may still hold a multiprocessor each.
 	const int kblocks = (a.K + kBlockBytes - 1) / kBlockBytes, tiles = (a.N + kTileRows - 1) / kTileRows, sms = sm_count();
 	for (int per = 1; per <= kMaxWarps; ++per) {
 		FewPlan p;
@@ -223,8 +231,8 @@ bool launch(LinearArgs& a, cudaStream_t st) {
 		const int warps = per * p.warps_k, blocks = (tiles + per - 1) / per;
 		const int smem = 1024 + warps * p.blocks_k * kBoxBytes + a.M * p.x_stride;
 		if (smem > kSmemMax) return false;
-		const int resident = std::min({2, 226 * 1024 / (smem + 5 * 1024), 65536 / (kRegs * 32 * warps)});
-		if (blocks > resident * sms - 8) continue;
+		const int resident = std::min({2, 228 * 1024 / (smem + cost.fixed_smem), 65536 / (cost.warp_regs * warps)});
+		if (blocks > resident * sms - kFewRows) continue;
 		CUtensorMap map;
 		if (!tc_tensor_map(a.w, a.N, a.K, kTileRows, a.caller_memory == 0, &map)) return false;
 		a.debug_withhold = tc_debug_take() ? 1 : 0;
