@@ -240,8 +240,8 @@ SSLM_API sslm_status sslm_b200_linear_bench(int32_t M, int32_t N, int32_t K, int
  * sslm_decode_step that ran on `ws`, and the number of kernels launched on it so far. */
 SSLM_API sslm_status sslm_b200_last_call_ms(sslm_workspace ws, float* ms, uint64_t* kernel_launches);
 
-/* Process-wide counters of the tensor-core linear kernel: launches, times it declined a shape
- * (the streaming kernel ran instead) and the reason code of the last refusal. */
+/* Process-wide counters of the tensor-core linear kernels: launches of all of them, times one declined a shape
+ * (another kernel ran instead) and the reason code of the last refusal. */
 SSLM_API sslm_status sslm_b200_tc_stats(uint64_t* launches, uint64_t* refusals, int32_t* last_reason);
 /* Launches of the tensor-core linear kernels, first n of: the activation-major one per tile shape (rows x weight
  * columns) 128 x 64, 128 x 128, 256 x 64, 256 x 128; the weights-first one; the one of up to eight rows. Lets a test assert which of them

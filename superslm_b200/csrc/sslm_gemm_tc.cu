@@ -758,7 +758,10 @@ void tc_count(bool launched, int reason) {
 	g_tc_variant[4].fetch_add(1);
 }
 
-void tc_count_few() { g_tc_variant[5].fetch_add(1); }
+void tc_count_few() {
+	g_tc_launches.fetch_add(1);
+	g_tc_variant[5].fetch_add(1);
+}
 
 void tc_debug_withhold(int launches) { g_debug_withhold.store(launches < 0 ? 0 : launches); }
 

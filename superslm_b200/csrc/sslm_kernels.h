@@ -183,7 +183,7 @@ bool launch_linear_skinny(const LinearArgs& a, cudaStream_t st);
 // shared by the two tensor-core kernels: [rows, k] int8 map, box 128 bytes x box_rows, 128-byte swizzle
 bool tc_tensor_map(const void* ptr, int rows, int k, int box_rows, bool cache, CUtensorMap* out);
 void tc_count(bool launched, int reason);      // of the weights-first kernel
-void tc_count_few();                           // of launch_linear_few, in the counts per variant only
+void tc_count_few();                           // of launch_linear_few
 bool tc_debug_take();      // one launch of those tc_debug_withhold asked for
 // Tests of the bounded waits: the next `launches` tensor-core launches arm their first weight-tile
 // barrier in block 0 without requesting the tile, so that the wait on it runs out (no fault, no
