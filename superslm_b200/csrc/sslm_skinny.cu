@@ -224,8 +224,11 @@ __device__ __forceinline__ uint32_t finish_value(const LinearArgs& a, Channel& c
 	return keep ? mag : 0u;
 }
 
+// (Clustered launches of up to 64 columns count on two blocks per multiprocessor: launch_mode cuts their rings for that. 32-bit rows
+// compile to 96 registers and fewer; for 64-bit rows the compiler is told, left to itself it takes 128 to 168: steps of 24 and 48 rows
+// with adapters 2.36 and 2.58 ms at the 1.5B widths, 2.15 and 2.34 so, 24 rows with four epilogue warps of 128 registers 2.16.)
 template <int NB, int MODE>
-__global__ void __launch_bounds__(SkCfg<NB>::kThreads, 1)
+__global__ void __launch_bounds__(SkCfg<NB>::kThreads, MODE == kRows64 && NB <= 64 ? 2 : 1)
 k_skinny(const __grid_constant__ CUtensorMap map_w, const __grid_constant__ CUtensorMap map_x, LinearArgs a, int stages, int splits) {
 	using Cfg = SkCfg<NB>;
 	constexpr int kEpi = 32 * Cfg::kEpiWarps;

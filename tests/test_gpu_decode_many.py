@@ -32,3 +32,30 @@ def test_every_row_matches_the_oracle(gpu_lib, shape, rows, bias_bits):
                 assert abi.parse_save_blob(s.save(), sh.hidden)["kv"] == ps.kv.tobytes(), i
     finally:
         eng.close()
+
+
+@pytest.mark.parametrize("shape,rows", [("mini1.5b", 17), ("mini1.5b", 32), ("mini3b", 24), ("mini0.5b", 33), ("small", 64), ("tiny", 100)])
+def test_adapted_rows_match_the_oracle(gpu_lib, shape, rows):
+    """64-bit rows in every width of the weights-first kernel from 32 columns on; one row in three has no adapter"""
+    sh = A.SHAPES[shape]
+    art = A.build_synthetic_model(shape, 0x7B80, 64)
+    adp = A.build_synthetic_adapter(art, 0x7B81, 16, A.PEFT_ORDER)
+    prompts = [A.stream_uniform(0x7B82 + i, "prompt", n, 0, sh.vocab - 1) for i, n in enumerate((1, 40, 16))]
+    want = [run_port(art, p, 3, adp if i != 2 else None) for i, p in enumerate(prompts)]
+    eng = abi.Engine(gpu_lib, art, blocks=rows, max_batch=rows, max_chunk=64)
+    try:
+        handle, seqs = eng.map_adapter(adp), []
+        for i in range(rows):
+            seqs.append(eng.new_seq())
+            if i % 3 != 2:
+                seqs[i].set_adapter(handle)
+            assert seqs[i].prefill(prompts[i % 3], 64) == len(prompts[i % 3])
+        got = [eng.decode_step(seqs, sh.layers) for _ in range(3)]
+        assert [status for status, _ in got] == [0] * 3
+        for i, s in enumerate(seqs):
+            tokens, ps = want[i % 3]
+            assert [step[i] for _, step in got] == tokens, i
+            if i < 3 or i >= rows - 3:
+                assert abi.parse_save_blob(s.save(), sh.hidden)["kv"] == ps.kv.tobytes(), i
+    finally:
+        eng.close()
