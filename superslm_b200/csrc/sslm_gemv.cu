@@ -103,7 +103,8 @@ struct GemvPlan {
 enum GemvMode { kGemvRows32 = 0, kGemvRows64, kGemvHead };
 // RU: weight rows multiplied side by side, as many as an item holds, up to three: short rows share the loads of x, and
 // an item of one row (long K) reads nothing twice (one row at the 1.5B widths, behind the wait, with three always:
-// down 5.3 us, 3.9 now; gate/up 4.0, 3.4; q/k/v 2.3, 2.0)
+// down 5.3 us, 3.9 now; gate/up 4.0, 3.4; q/k/v 2.3, 2.0). The vocabulary head takes three where an item holds two as well: with
+// two its loop spills, and the 233 MB of 1,536 columns took 59 us in place of 49.
 template <int MT, int MODE, int RU>
 __global__ void __launch_bounds__(kGemvThreads)
 k_gemv(LinearArgs a, GemvPlan p) {
@@ -395,16 +396,17 @@ static cudaError_t launch_mode(const LinearArgs& a, int grid_y, cudaStream_t st)
 
 template <int MT, int RU>
 static cudaError_t launch_rows(const LinearArgs& a, int grid_y, cudaStream_t st) {
-	if (a.best != nullptr) return launch_mode<MT, kGemvHead, RU>(a, grid_y, st);
 	return a.out64 ? launch_mode<MT, kGemvRows64, RU>(a, grid_y, st) : launch_mode<MT, kGemvRows32, RU>(a, grid_y, st);
 }
 template <int MT>
 static cudaError_t launch_mt(const LinearArgs& a, int grid_y, cudaStream_t st) {
 	if constexpr (MT == 1) {
 		const int rows = a.K * 2 <= kItemBytes ? kItemBytes / a.K : 1;      // per item
+		if (a.best != nullptr) return rows >= 2 ? launch_mode<1, kGemvHead, 3>(a, grid_y, st) : launch_mode<1, kGemvHead, 1>(a, grid_y, st);
 		if (rows >= 3) return launch_rows<1, 3>(a, grid_y, st);
 		if (rows == 2) return launch_rows<1, 2>(a, grid_y, st);
 	}
+	if (a.best != nullptr) return launch_mode<MT, kGemvHead, 1>(a, grid_y, st);
 	return launch_rows<MT, 1>(a, grid_y, st);
 }
 
