@@ -21,6 +21,7 @@
 #include <cuda_runtime.h>
 
 #include <algorithm>
+#include <atomic>
 #include <initializer_list>
 
 #include "sslm_cluster.cuh"
@@ -203,7 +204,7 @@ k_linear_few(const __grid_constant__ CUtensorMap map_w, LinearArgs a, FewPlan p)
 constexpr int kSmemMax = 220 * 1024;
 // what a block takes beside its dynamic shared memory, as compiled: registers of a warp (given out in units of 256), shared memory
 struct FewCost {
-	int warp_regs, fixed_smem;
+	std::atomic<int> warp_regs, fixed_smem;
 };
 
 bool launch(LinearArgs& a, cudaStream_t st) {
@@ -213,7 +214,10 @@ bool launch(LinearArgs& a, cudaStream_t st) {
 	if (once_per_device(configured, [&cost] {
 		    cudaFuncAttributes f;
 		    cudaError_t e = cudaFuncGetAttributes(&f, k_linear_few);
-		    if (e == cudaSuccess) cost = FewCost{(f.numRegs * 32 + 255) / 256 * 256, (int)f.sharedSizeBytes + 1024};      // (1 KB is the system's)
+		    if (e == cudaSuccess) {
+			    cost.warp_regs = (f.numRegs * 32 + 255) / 256 * 256;
+			    cost.fixed_smem = (int)f.sharedSizeBytes + 1024;      // (1 KB is the system's)
+		    }
 		    if (e == cudaSuccess) e = cudaFuncSetAttribute(k_linear_few, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmemMax);
 		    if (e == cudaSuccess) e = cudaFuncSetAttribute(k_linear_few, cudaFuncAttributePreferredSharedMemoryCarveout, cudaSharedmemCarveoutMaxShared);
 		    return e;
@@ -233,6 +237,12 @@ bool launch(LinearArgs& a, cudaStream_t st) {
 		if (smem > kSmemMax) return false;
 		const int resident = std::min({2, 228 * 1024 / (smem + cost.fixed_smem), 65536 / (cost.warp_regs * warps)});
 		if (blocks > resident * sms - kFewRows) continue;
+		// A projection by itself, its weights asked for ahead of nothing: two blocks on a multiprocessor pay from 1,280 columns
+		// and 6,144 channels on. 2, 5, 8 rows, us with the weights-first kernel / here, funnel included: 2,048 x 8,192 12.3 / 12.3,
+		// 13.7 / 12.3, 14.4 / 12.4; 1,280 x 6,144 12.3 / 10.3, 12.3 / 10.8, 12.3 / 12.3; below, 896 x 9,728 10.3 / 12.3, 10.8 / 12.3,
+		// 11.9 / 12.3, 1,536 x 4,096 10.3 / 11.1, 10.3 / 12.1, 10.3 / 12.3. A block each: 1,536 x 17,920 14.4 / 13.4 to 14.4, and
+		// 896 to 11,008 columns of 896 to 2,048 channels 8.2 to 14.4 / 8.2 to 11.8.
+		if (a.caller_memory != 0 && blocks > sms && (a.K < 1280 || a.N < 6144)) return false;
 		CUtensorMap map;
 		if (!tc_tensor_map(a.w, a.N, a.K, kTileRows, a.caller_memory == 0, &map)) return false;
 		a.debug_withhold = tc_debug_take() ? 1 : 0;

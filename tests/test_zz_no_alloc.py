@@ -126,3 +126,23 @@ def test_resident_linear_reports_a_wait_that_ran_out(gpu_lib, M, N, K, given_up)
         arm(0)
     assert (status[:given_up] == 100).all() and (status[given_up:] == 0).all()
     check_resident(gpu_lib, torch, 6, M, N, K)      # nothing of it is left in the fixed array
+
+
+@pytest.mark.parametrize("K,N,M,kind", [(896, 9728, 5, 4), (1536, 4096, 2, 4), (1024, 9728, 3, 4), (1280, 6144, 8, 5), (1280, 6128, 3, 4),
+                                        (2048, 9728, 2, 5), (1536, 17920, 8, 5), (11008, 2048, 2, 5), (896, 1152, 8, 5)])
+def test_which_kernel_serves_a_few_rows(gpu_lib, K, N, M, kind):
+    """weights waiting in shared memory (5) where its blocks have a multiprocessor each or the projection is large, else weights
+    first (4): kinds as sslm_b200_tc_variant_counts orders them"""
+    torch = pytest.importorskip("torch")
+    torch.cuda.set_device(0)
+    from tests.test_gpu_parity import oracle_linear
+    f = gpu_lib.dll.sslm_b200_tc_variant_counts
+    f.argtypes = [C.c_void_p, C.c_int32]
+    counts = np.zeros((2, 6), dtype=np.uint64)
+    x, w, fold, in_scales = make_case(K + N + M, M, N, K, 127)
+    assert f(counts[0].ctypes.data, 6) == 0
+    got = resident_entry(gpu_lib, torch, x, w, fold, in_scales)
+    assert f(counts[1].ctypes.data, 6) == 0
+    assert list(counts[1] - counts[0]) == [int(i == kind) for i in range(6)]
+    for a, b, what in zip(got, oracle_linear(x, w, fold, in_scales, SITE), ("folded", "codes", "scales", "status")):
+        assert (np.asarray(a, dtype=np.int64) == np.asarray(b, dtype=np.int64)).all(), what
