@@ -1368,10 +1368,6 @@ struct ChunkSmem {
 	__host__ __device__ static constexpr size_t bytes(int steps) { return kStage + kScores * steps + kMisc; }
 };
 
-__device__ __forceinline__ void ldmatrix4(uint32_t addr, uint32_t& r0, uint32_t& r1, uint32_t& r2, uint32_t& r3) {
-	asm volatile("ldmatrix.sync.aligned.m8n8.x4.shared.b16 {%0, %1, %2, %3}, [%4];" : "=r"(r0), "=r"(r1), "=r"(r2), "=r"(r3) : "r"(addr) : "memory");
-}
-
 template <int HD>
 __global__ void __launch_bounds__(kChunkThreads, 2)
 k_attention_chunk(RowBatch b, Dims d, const __grid_constant__ LayerDev layer, int layer_index, KvPoolDev pool, ChunkPlan pl) {

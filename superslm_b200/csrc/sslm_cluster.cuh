@@ -98,6 +98,15 @@ static __device__ __noinline__ void exchange_leave(uint32_t bar, int n) {
 		while (!bar_try<true>(bar + 8u * (uint32_t)i, 0) && now_ns() < deadline) __nanosleep(64);
 }
 
+// ---- tiles: a box of a tensor map (a CUtensorMap in the launch parameters) into shared memory, counted on `bar`; four 8 x 16-byte matrices out of it
+__device__ __forceinline__ void tma_2d(uint32_t dst, const void* map, uint32_t bar, int c0, int c1) {
+	asm volatile("cp.async.bulk.tensor.2d.shared::cta.global.mbarrier::complete_tx::bytes [%0], [%1, {%3, %4}], [%2];"
+	             ::"r"(dst), "l"(map), "r"(bar), "r"(c0), "r"(c1) : "memory");
+}
+__device__ __forceinline__ void ldmatrix4(uint32_t addr, uint32_t& r0, uint32_t& r1, uint32_t& r2, uint32_t& r3) {
+	asm volatile("ldmatrix.sync.aligned.m8n8.x4.shared.b16 {%0, %1, %2, %3}, [%4];" : "=r"(r0), "=r"(r1), "=r"(r2), "=r"(r3) : "r"(addr) : "memory");
+}
+
 // ---- slots that some threads fill and others empty, turn by turn
 __device__ __forceinline__ void ring_init(uint32_t bar, uint32_t count) { asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(bar), "r"(count)); }
 __device__ __forceinline__ void ring_arrive(uint32_t bar) { asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(bar) : "memory"); }

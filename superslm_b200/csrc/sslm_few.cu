@@ -39,16 +39,8 @@ struct FewPlan {
 	int x_stride;     // bytes between rows of x in shared memory (16 more than a multiple of 128: no bank conflicts)
 };
 
-__device__ __forceinline__ void tma_2d(uint32_t dst, const CUtensorMap* map, uint32_t bar, int c0, int c1) {
-	asm volatile("cp.async.bulk.tensor.2d.shared::cta.global.mbarrier::complete_tx::bytes [%0], [%1, {%3, %4}], [%2];"
-	             ::"r"(dst), "l"(map), "r"(bar), "r"(c0), "r"(c1) : "memory");
-}
 __device__ __forceinline__ void copy4(uint32_t dst, const void* src) {
 	asm volatile("cp.async.ca.shared.global [%0], [%1], 4;" ::"r"(dst), "l"(src) : "memory");
-}
-__device__ __forceinline__ void ldsm4(uint32_t addr, uint32_t (&r)[4]) {
-	asm volatile("ldmatrix.sync.aligned.m8n8.x4.shared.b16 {%0, %1, %2, %3}, [%4];"
-	             : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]) : "r"(addr) : "memory");
 }
 __device__ __forceinline__ void mma_s8(int (&c)[4], const uint32_t (&a)[4], uint32_t b0, uint32_t b1) {
 	asm volatile(
@@ -127,9 +119,9 @@ k_linear_few(const __grid_constant__ CUtensorMap map_w, LinearArgs a, FewPlan p)
 		for (int k = 0; k < nkb; ++k) {
 			uint32_t w[4][4], x0[4], x1[4];
 #pragma unroll
-			for (int s = 0; s < 4; ++s) ldsm4(wrow + (uint32_t)k * kBoxBytes + (((2u * s + half) ^ sw) << 4), w[s]);
-			ldsm4(xr + (uint32_t)k * kBlockBytes, x0);
-			ldsm4(xr + (uint32_t)k * kBlockBytes + 64u, x1);
+			for (int s = 0; s < 4; ++s) ldmatrix4(wrow + (uint32_t)k * kBoxBytes + (((2u * s + half) ^ sw) << 4), w[s][0], w[s][1], w[s][2], w[s][3]);
+			ldmatrix4(xr + (uint32_t)k * kBlockBytes, x0[0], x0[1], x0[2], x0[3]);
+			ldmatrix4(xr + (uint32_t)k * kBlockBytes + 64u, x1[0], x1[1], x1[2], x1[3]);
 			mma_s8(acc, w[0], x0[0], x0[1]);
 			mma_s8(acc, w[1], x0[2], x0[3]);
 			mma_s8(acc, w[2], x1[0], x1[1]);

@@ -65,11 +65,6 @@ __device__ __forceinline__ void bar_arrive(uint32_t bar) {
 	asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(bar) : "memory");
 }
 __device__ __forceinline__ bool bar_wait(uint32_t bar, uint32_t parity) { return bounded_wait<false>(bar, parity); }
-__device__ __forceinline__ void tma_2d(uint32_t dst, const CUtensorMap* map, uint32_t bar, int c0, int c1) {
-	asm volatile(
-	    "cp.async.bulk.tensor.2d.shared::cta.global.mbarrier::complete_tx::bytes [%0], [%1, {%3, %4}], [%2];"
-	    ::"r"(dst), "l"(map), "r"(bar), "r"(c0), "r"(c1) : "memory");
-}
 // K-major, 128-byte-swizzled operand tile: 8-row groups are 1024 bytes apart
 __device__ __forceinline__ uint64_t smem_desc(uint32_t addr) {
 	return (uint64_t)((addr & 0x3FFFFu) >> 4) | ((uint64_t)1 << 16) | ((uint64_t)(1024 >> 4) << 32) | ((uint64_t)1 << 46) | ((uint64_t)2 << 61);
