@@ -1882,7 +1882,7 @@ static cudaError_t launch_attn(const RowBatch& b, const Dims& d, const LayerDev&
 		// Twice the warps per block for decode rows: the blocks of the widest rows end last, and theirs is a chain. ms for 4 tokens,
 		// 2 * head_dim threads / 4 * head_dim: 0.5B 45 rows 5.19 / 4.76, 80 5.75 / 5.44, 250 8.31 / 8.03; 1.5B 100 rows 7.89 / 7.71,
 		// 180 9.52 / 9.07. Not with 128 channels and about one block per multiprocessor (64 rows 31.9 / 32.5 for 16
-		// tokens, 80 7.22 / 7.32 for 4), nor for the short rows of a prompt (150 rows: 2.32 / 2.39).
+		// tokens, 80 7.22 / 7.32 for 4), nor for the short rows of a prompt (150 rows: 2.32 / 2.39). In 64 registers, with four words spilled from 64 channels on.
 		const int blocks = d.kv_heads * b.m;
 		const bool wide = reverse_rows == 0 && (HD < 128 || 4 * blocks >= 5 * sm_count());
 		return launch_pdl(wide ? k_attention<HD, 1> : k_attention<HD, 2>, dim3(d.kv_heads, b.m), dim3(wide ? 4 * HD : 2 * HD), attn_smem_bytes(G, p.cp), st,

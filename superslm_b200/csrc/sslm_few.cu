@@ -7,8 +7,8 @@
 // What is left behind the wait is short: the rows of x into shared memory, four multiplications a block
 // (mma.sync m16n8k32 s8, fragments by ldmatrix: the weights are the A operand, eight rows of x the B operand, so
 // eight rows cost what one does), one exchange of partial sums between the warps that share the 16 rows, the fold.
-// Bound by the weights' way into shared memory (27.5 MB: 6.7 us from HBM, 3.8 from L2, whatever the form of the copies)
-// and by the latencies of that chain.
+// Bound by the weights' way into shared memory (gate/up: 27.7 MB, 13 us cold, 9.6 in the chain, where it begins a kernel
+// earlier) and by the latencies of that chain (issue slots 7 to 12 % used).
 //
 // Five rows at the 1.5B widths, behind the wait, on the weights-first tcgen05 kernel (k_skinny) / here: q/k/v 3.1 / 2.7 us,
 // o 3.5 / 3.1, gate/up 5.5 / 5.9 (but the row kernel in front 5.4 / 2.9, which its weights no longer crowd out),

@@ -711,8 +711,9 @@ struct ActRow {
 // blocks, which meet once, for the maximum of the products; on a prefill chunk two blocks share a row.
 // What depends on the row alone (two scale folds, two funnels, the product's fold: a quarter of the instructions) one warp
 // derives for the block, while the others wait for their elements: 64 rows of 8,960 1.6 % a step, a prompt of
-// 37 3 %. Not with five quads a thread, where it costs registers (prompt of 300: 1.7 % longer), nor for the fewest rows,
-// whose chain the extra trip through shared memory only lengthens.
+// 37 3 %. Not with five quads a thread, where it costs registers (prompt of 300: 1.7 % longer). From 16 rows on: a step of 16, 24, 32, 48
+// rows 1,503 / 1,480, 1,600 / 1,562, 1,632 / 1,584, 1,793 / 1,764 us apart / shared at the 1.5B widths, 0 to 2 % at 0.5B and 3B; 9 and
+// 12 rows take the same time either way.
 // DENSE: in 72 registers instead of 80, for one more block per multiprocessor at some widths (launch_act)
 template <int NV, bool W64, bool DENSE = false>
 __global__ void __launch_bounds__(DENSE ? 288 : (NV == 5 ? 352 : 384), NV == 1 ? 1 : (DENSE ? 3 : 2))

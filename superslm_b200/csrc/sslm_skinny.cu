@@ -44,7 +44,9 @@ template <int NB>
 struct SkCfg {
 	// Four epilogue warps per 16 columns (each reads a quarter of the lanes), 16 at most: with eight, gate/up of 256 rows at
 	// the 1.5B widths spent 8.5 of 14.5 us in its epilogue. A step of 120 rows 13.46 -> 13.05 ms / 5, of 21 rows of 0.5B
-	// 18.8 -> 18.25 ms / 15. Not for 64 columns: a clustered block of 16 leaves no registers for a second one beside
+	// 18.8 -> 18.25 ms / 15. Eight for 32 columns, against four: a step of 20 to 32 rows of 0.5B 1,175 to 1,230 -> 1,130 to 1,165 us, with
+	// adapters 1,821 to 1,865 -> 1,610 to 1,647, at the 1.5B widths the same within 2 % either way; by itself 2,048 x 2,048 10.9 -> 11.6 us, 8,960 x
+	// 1,536 14.4 -> 13.3. Not for 64 columns: a clustered block of 16 leaves no registers for a second one beside
 	// it (64 rows: 8 % slower), and without clusters it gains nothing.
 	static constexpr int kEpiWarps = NB == 64 ? 8 : (NB / 4 < 16 ? NB / 4 : 16);
 	static constexpr int kThreads = 64 + 32 * kEpiWarps;
