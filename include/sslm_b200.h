@@ -291,7 +291,7 @@ SSLM_API sslm_status sslm_b200_debug_refuse_launch(int32_t launches);
  *   5 a / b (unsigned, small quotient)     6 the funnel's scalars for a one-element row of magnitude a,
  *     incoming scale (b, c), site constant (e >> 32, low half of e): out0/out1 the output scale, out2 status
  *   7 one i-exp softmax element: shifted score a, constants (q_ln2 b, q_b c, q_c e >> 32), peak = low
- *     half of e << 16: out0 value, out1 refused
+ *     half of e << 16: out0 value, out1 refused, out2 the value rebuilt from its (shift, base) word
  *   8 Q15 probability floor((a << 15) / b)
  * and the short forms of the row and attention kernels (out1 = 0 where a form does not cover the operands):
  *   9 code of a in a row of maximum b: out0 32-bit, out1 64-bit elements, out2 0 if the signs agree

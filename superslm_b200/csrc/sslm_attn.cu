@@ -2037,8 +2037,12 @@ __global__ void k_int_sweep(int which, const int64_t* a, const int64_t* b, const
 			k.peak = (int64_t)(uint32_t)e[i] << 16;
 			const IExpFast f = iexp_fast_prepare(k);
 			const int64_t v = iexp_fast((uint32_t)a[i], f);
+			uint32_t word;
+			chunk_exp((uint32_t)a[i], f, &word);
+			const uint64_t base = word & 0xFFFFFFu;
 			o0 = v;
 			o1 = (v < 0 || v > k.peak) ? 1 : 0;       // the reference's per-element bound
+			o2 = (int64_t)((base * base + (uint64_t)f.qc) >> (word >> 24));
 			break;
 		}
 		case 8: {      // Q15 probability: floor((e << 15) / total), 0 <= e <= total

@@ -132,7 +132,7 @@ def test_softmax_element_and_probability_on_the_device(gpu_lib):
     e = pack(qc, peak16)
     got, want = device_sweep(gpu_lib, 7, dq, ln2, qb, e), oracle_sweep(7, dq, ln2, qb, e)
     assert (want[1] == 0).all()
-    assert (got[0] == want[0]).all()
+    assert (got[0] == want[0]).all() and (got[2] == want[0]).all()
     bound = peak16 << 16
     assert (got[1] == ((want[0] < 0) | (want[0] > bound)).astype(I64)).all()
     tot = (rng.integers(1, 1 << 62, N, dtype=I64) >> rng.integers(0, 61, N)).astype(I64)
@@ -224,7 +224,7 @@ def test_norm_quotients_of_the_row_kernels_on_the_device(gpu_lib):
     assert (got[0][covered] == ((h << 32) // root)[covered]).all()
 
 
-def test_softmax_of_the_kernels_that_keep_their_scores(gpu_lib):
+def test_prefill_softmax_on_the_device(gpu_lib):
     rng = np.random.default_rng(9)
     port = H.port()
     sets = []
@@ -235,16 +235,6 @@ def test_softmax_of_the_kernels_that_keep_their_scores(gpu_lib):
            qb.value * qb.value + qc.value <= (1 << 47):
             sets.append((ln2.value, qb.value, qc.value))
     assert len(sets) >= 16
-    lo, hi, limit = (1 << 30), (1 << 31) - 1, None      # the smallest scale that the width gate admits: q_b and the peak at their largest
-    while lo <= hi:
-        m = (lo + hi) // 2
-        ok = port.osc_iexp_scale_constants(m, -53, C.byref(ln2), C.byref(qb), C.byref(qc)) == 0 and qb.value ** 2 + qc.value <= 1 << 47
-        if ok:
-            limit, hi = (ln2.value, qb.value, qc.value), m - 1
-        else:
-            lo = m + 1
-    assert limit[1] ** 2 + limit[2] > 0.9999 * (1 << 47)
-    sets += [limit] * (len(sets) // 4)
     pick = rng.integers(0, len(sets), N)
     ln2, qb, qc = (np.array([sets[i][k] for i in pick], dtype=I64) for k in range(3))
     dq = (rng.integers(0, 34, N) * ln2 + rng.integers(-3, 4, N)).clip(0, (1 << 32) - 1).astype(I64)
@@ -265,5 +255,40 @@ def test_softmax_of_the_kernels_that_keep_their_scores(gpu_lib):
     words[::41] = 63 << 24                                                          # elements that count for nothing
     value[::41] = 0
     got = device_sweep(gpu_lib, 14, words, tot, qc, zeros())
+    want = ((value.astype(np.uint64) << np.uint64(15)) // tot.astype(np.uint64)).astype(I64)
+    assert (got[0] == want).all()
+
+
+def test_softmax_at_the_width_gate_on_the_device(gpu_lib):
+    """the smallest scale that the gate admits: q_b and the peak at their largest"""
+    rng = np.random.default_rng(10)
+    port = H.port()
+    ln2, qb, qc = C.c_int64(0), C.c_int64(0), C.c_int64(0)
+    lo, hi, limit = (1 << 30), (1 << 31) - 1, None
+    while lo <= hi:
+        m = (lo + hi) // 2
+        ok = port.osc_iexp_scale_constants(m, -53, C.byref(ln2), C.byref(qb), C.byref(qc)) == 0 and qb.value ** 2 + qc.value <= 1 << 47
+        if ok:
+            limit, hi = (ln2.value, qb.value, qc.value), m - 1
+        else:
+            lo = m + 1
+    ln2, qb, qc = limit
+    peak = qb ** 2 + qc
+    assert peak > 0.9999 * (1 << 47)
+    dq = (rng.integers(0, 34, N) * ln2 + rng.integers(-3, 4, N)).clip(0, (1 << 32) - 1).astype(I64)
+    dq[::17] = rng.integers(0, 1 << 32, dq[::17].size, dtype=I64)
+    x = np.minimum(dq, 30 * ln2)
+    value = ((qb - x % ln2) ** 2 + qc) >> (x // ln2)
+    got = device_sweep(gpu_lib, 13, dq, zeros() + ln2, zeros() + qb, zeros() + qc)
+    assert (got[0] == value).all()
+    words = got[1]
+    z, base = words >> 24, words & 0xFFFFFF
+    assert ((base * base + qc) >> z == value).all()
+    tot = np.maximum(value, 1) + (rng.integers(0, 1 << 62, N, dtype=I64) >> rng.integers(0, 61, N)) % (peak * 32767)
+    k = rng.integers(1, 1 << 15, N, dtype=I64)
+    near = (value << 15) // k + rng.integers(-2, 3, N, dtype=I64)
+    use = (rng.integers(0, 2, N) == 0) & (near >= value) & (near > 0)
+    tot[use] = near[use]
+    got = device_sweep(gpu_lib, 14, words, tot, zeros() + qc, zeros())
     want = ((value.astype(np.uint64) << np.uint64(15)) // tot.astype(np.uint64)).astype(I64)
     assert (got[0] == want).all()
