@@ -274,8 +274,8 @@ SSLM_API sslm_status sslm_b200_debug_withhold_tc_load(int32_t launches);
 /* The same for the words that the blocks of a cluster send each other: block 0 of the next launch of
  * `kernel` waits for more than will come in one of its exchanges. kernel 0: the weights-first linear kernel
  * where K is cut over a cluster (exchange 0); 1: attention of few rows (0 maxima, 1 sums, 2 contexts, 3 the
- * funnel's maximum, 4 the biased elements' maximum where the q/k/v site runs inside; elsewhere 4 changes nothing);
- * 2: attention of prefill chunks in tiles cut over a cluster (0 to 2); 3: the activation site (0). kernel -1 takes
+ * funnel's maximum); 2: attention of prefill chunks in tiles cut over a cluster (0 to 2); 3: the activation
+ * site (0); 5: attention of few biased rows with the q/k/v site inside (0 the biased elements' maximum). kernel -1 takes
  * the request back. */
 SSLM_API sslm_status sslm_b200_debug_withhold_exchange(int32_t kernel, int32_t exchange);
 /* Tests only: the first kernel of each of the next `launches` (0..16) row groups counts as refused by the CUDA

@@ -1890,7 +1890,7 @@ static cudaError_t launch_attn(const RowBatch& b, const Dims& d, const LayerDev&
 	}
 	const bool staged = FewSmem<HD>::bytes(G, p.cp, true) <= kFewSmemMax;
 	RowBatch rb = b;
-	rb.debug_withhold = exchange_debug_take(kExchangeAttnFew);
+	rb.debug_withhold = site == kSiteBias && exchange_debug_take(kExchangeAttnSite) ? 5 : exchange_debug_take(kExchangeAttnFew);
 	cudaLaunchConfig_t cfg = {};
 	cfg.gridDim = dim3(d.kv_heads * p.splits, b.m);
 	cfg.blockDim = dim3(2 * HD);

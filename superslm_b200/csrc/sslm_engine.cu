@@ -599,7 +599,7 @@ extern "C" sslm_status sslm_b200_debug_refuse_launch(int32_t launches) {
 	return SSLM_OK;
 }
 extern "C" sslm_status sslm_b200_debug_withhold_exchange(int32_t kernel, int32_t exchange) {
-	static const int kExchanges[kExchangeKernels] = {1, 5, 3, 1};
+	static const int kExchanges[kExchangeKernels] = {1, 4, 3, 1, 0, 1};
 	if (kernel >= kExchangeKernels || (kernel >= 0 && (exchange < 0 || exchange >= kExchanges[kernel]))) return SSLM_INVALID_ARGUMENT;
 	g_withheld_exchange.store(kernel < 0 ? 0u : (uint32_t)kernel << 8 | (uint32_t)(exchange + 1));
 	return SSLM_OK;

@@ -90,7 +90,8 @@ inline int sm_count() {
 // The next launch of one kernel that exchanges words over a cluster arms one of its exchanges, in block 0,
 // with four bytes more than will come: that block's wait runs out. One word: 0 for none, else
 // kernel << 8 | exchange + 1.
-enum ExchangeKernel { kExchangeLinear = 0, kExchangeAttnFew, kExchangeAttnChunk, kExchangeAct, kExchangeKernels };
+// (4 names no kernel; 5 is the fifth exchange of attention with the q/k/v site of biased rows inside)
+enum ExchangeKernel { kExchangeLinear = 0, kExchangeAttnFew, kExchangeAttnChunk, kExchangeAct, kExchangeAttnSite = 5, kExchangeKernels };
 inline std::atomic<uint32_t> g_withheld_exchange{0};
 inline int exchange_debug_take(ExchangeKernel kernel) {
 	uint32_t w = g_withheld_exchange.load(std::memory_order_relaxed);

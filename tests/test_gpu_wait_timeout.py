@@ -95,7 +95,7 @@ def test_exchange_that_runs_out(gpu_lib, kernel, exchange, shape, n, call):
     eng = abi.Engine(gpu_lib, art, blocks=1, max_chunk=n)
     arm = gpu_lib.dll.sslm_b200_debug_withhold_exchange
     arm.argtypes = [C.c_int32, C.c_int32]
-    assert arm(kernel, 5) == arm(4, 0) == abi.ST["SSLM_INVALID_ARGUMENT"]
+    assert arm(kernel, 4) == arm(4, 0) == abi.ST["SSLM_INVALID_ARGUMENT"]
     failed = abi.ST["SSLM_ALLOCATION_FAILED"]
     try:
         s = eng.new_seq()
@@ -123,11 +123,14 @@ def test_exchange_that_runs_out(gpu_lib, kernel, exchange, shape, n, call):
         eng.close()
 
 
-# batches whose q/k/v site runs inside the attention cluster: (shape, adapted, bias_bits, prompts, exchange). Clusters of 16 blocks
-# (up to six rows), of 8, and of 2; with biases there is a fifth exchange.
-SITE_EXCHANGES = [("mini1.5b", False, 0, (300, 40), x) for x in range(4)] + [("mini0.5b", False, 30, (300, 40, 5), x) for x in range(5)] + \
-                 [("tiny", True, 36, (200, 30), 4), ("tiny", True, 0, (200, 30), 1), ("small", False, 36, (70, 5, 30, 64, 1, 20, 9, 16), 4),
-                  ("small", False, 30, (20, 5), 4), ("small", False, 30, (20, 5), 0)]
+# batches whose q/k/v site runs inside the attention cluster: (shape, adapted, bias_bits, prompts, kernel and exchange). Clusters of 16
+# blocks (up to six rows), of 8, and of 2; with biases there is a fifth exchange.
+SITE = (5, 0)
+SITE_EXCHANGES = [("mini1.5b", False, 0, (300, 40), (1, x)) for x in range(4)] + \
+                 [("mini0.5b", False, 30, (300, 40, 5), x) for x in ((1, 0), (1, 1), (1, 2), (1, 3), SITE)] + \
+                 [("tiny", True, 36, (200, 30), SITE), ("tiny", True, 0, (200, 30), (1, 1)),
+                  ("small", False, 36, (70, 5, 30, 64, 1, 20, 9, 16), SITE), ("small", False, 30, (20, 5), SITE),
+                  ("small", False, 30, (20, 5), (1, 0))]
 
 
 @pytest.mark.parametrize("shape,adapted,bias_bits,lengths,exchange", SITE_EXCHANGES)
@@ -159,7 +162,7 @@ def test_exchange_of_a_batch_that_runs_out(gpu_lib, shape, adapted, bias_bits, l
             seqs.append(s)
         got = [eng.decode_step(seqs, sh.layers)]
         before = [holds(s) for s in seqs]
-        assert arm(1, exchange) == 0
+        assert arm(*exchange) == 0
         t = time.perf_counter()
         assert eng.decode_step(seqs, sh.layers)[0] == abi.ST["SSLM_ALLOCATION_FAILED"]
         assert 0.2 < time.perf_counter() - t < 5.0
