@@ -6,7 +6,7 @@ import ctypes as C
 import numpy as np
 import pytest
 
-from tests.test_gpu_parity import gpu_linear, linear_case_inputs, oracle_linear, tc_launches
+from tests.test_gpu_parity import gpu_linear, linear_case_inputs, oracle_linear
 
 pytestmark = pytest.mark.gpu
 
@@ -26,10 +26,9 @@ def test_layer_with_its_weights_waiting_matches_the_oracle(gpu_lib, K, N, M):
     f.argtypes = [C.c_void_p, C.c_int32]
     counts = np.zeros((2, 6), dtype=np.uint64)
     assert f(counts[0].ctypes.data, 6) == 0
-    before = tc_launches(gpu_lib)
     got = gpu_linear(gpu_lib, x, w, fold, in_scales, site, 3)
     assert f(counts[1].ctypes.data, 6) == 0
-    assert list(counts[1] - counts[0]) == [0, 0, 0, 0, 0, 1] and tc_launches(gpu_lib) - before == 1
+    assert list(counts[1] - counts[0]) == [0, 0, 0, 0, 0, 1]
     for a, b, what in zip(got, want, ("folded", "codes", "scales", "status")):
         assert (np.asarray(a, dtype=np.int64) == np.asarray(b, dtype=np.int64)).all(), what
 
@@ -50,3 +49,11 @@ def test_request_that_never_comes(gpu_lib):
     want, got = oracle_linear(x, w, fold, in_scales, site), gpu_linear(gpu_lib, x, w, fold, in_scales, site, 3)
     for a, b in zip(got, want):
         assert (np.asarray(a, dtype=np.int64) == np.asarray(b, dtype=np.int64)).all()
+
+
+def test_its_launches_are_in_the_process_wide_count(gpu_lib):
+    from tests.test_gpu_parity import tc_launches
+    x, w, fold, in_scales = linear_case_inputs(144, 129, 7)
+    before = tc_launches(gpu_lib)
+    gpu_linear(gpu_lib, x, w, fold, in_scales, (1090717716, -44), 3)
+    assert tc_launches(gpu_lib) - before == 1
